@@ -10,6 +10,7 @@
 #include "../kernels/comm_kernels.cuh"
 #include "../kernels/embbag.cuh"
 #include "../kernels/kv_pack.cuh"
+#include "../kernels/decoder.cuh"
 #include "../kernels/moe_dispatch.cuh"
 #include "../kernels/fp8_gemm.cuh"
 #include "../mem/vmm.h"
@@ -222,6 +223,123 @@ static void kv_pack_send(torch::Tensor src_k, torch::Tensor src_v, int64_t dst_k
   check_rc(fl_kv_pack_send(&a, (int)num_ctas, cur_stream()), "fl_kv_pack_send");
 }
 
+// ------------------------------------------------------------------------------------------------ decoder
+static int dec_dtype(const torch::Tensor& t) {
+  TORCH_CHECK(t.is_cuda() && (t.scalar_type() == torch::kBFloat16 || t.scalar_type() == torch::kHalf), "bf16 or fp16 on the GPU expected");
+  return t.scalar_type() == torch::kBFloat16 ? FL_DEC_BF16 : FL_DEC_FP16;
+}
+static void dec_like(const c10::optional<torch::Tensor>& t, const torch::Tensor& as, int64_t numel, const char* what) {
+  TORCH_CHECK(!t.has_value() || (t->is_cuda() && t->scalar_type() == as.scalar_type() && t->is_contiguous() && t->numel() == numel), what);
+}
+static const long long* dec_i64(const c10::optional<torch::Tensor>& t, int64_t numel, const char* what) {
+  if (!t.has_value()) return nullptr;
+  TORCH_CHECK(t->is_cuda() && t->scalar_type() == torch::kInt64 && t->is_contiguous() && t->numel() == numel, what);
+  return reinterpret_cast<const long long*>(t->data_ptr<int64_t>());
+}
+static FlPagedKv dec_kv(torch::Tensor k_pool, torch::Tensor v_pool, torch::Tensor table, int64_t layout, int64_t layer, int64_t layers,
+                        int64_t num_blocks, int64_t block_size, int64_t kv_heads, int64_t dim) {
+  TORCH_CHECK(k_pool.is_cuda() && v_pool.is_cuda() && k_pool.is_contiguous() && v_pool.is_contiguous(), "pools: contiguous on the GPU");
+  TORCH_CHECK(table.is_cuda() && table.scalar_type() == torch::kInt32 && table.is_contiguous() && table.dim() == 2, "block_table: [batch, blocks] int32");
+  TORCH_CHECK(layer >= 0 && layer < layers && block_size > 0, "layer out of range");
+  const int64_t need = num_blocks * layers * block_size * kv_heads * dim;
+  TORCH_CHECK(k_pool.numel() >= need && v_pool.numel() >= need, "pools smaller than num_blocks pages");
+  FlPagedKv kv;
+  kv.k = k_pool.data_ptr(); kv.v = v_pool.data_ptr();
+  kv.block_table = table.data_ptr<int>(); kv.table_stride = (int)table.size(1);
+  kv.layout = (int)layout; kv.layer = (int)layer; kv.layers = (int)layers; kv.num_blocks = (int)num_blocks;
+  kv.block_size = (int)block_size; kv.heads = (int)kv_heads;
+  return kv;
+}
+static void dec_embed(torch::Tensor tokens, c10::optional<torch::Tensor> pos, torch::Tensor embed, c10::optional<torch::Tensor> pos_embed,
+                      torch::Tensor x, int64_t seq, int64_t offset) {
+  const int dt = dec_dtype(x);
+  const int64_t rows = tokens.numel(), H = embed.size(1);
+  TORCH_CHECK(embed.scalar_type() == x.scalar_type() && embed.is_contiguous() && x.is_contiguous() && x.numel() == rows * H, "x: [rows, hidden] like embed");
+  if (pos_embed.has_value()) dec_like(pos_embed, x, pos_embed->size(0) * H, "pos_embed: [positions, hidden]");
+  c10::cuda::CUDAGuard guard(x.device());
+  check_rc(fl_dec_embed(dt, dec_i64(tokens, rows, "tokens: int64"), dec_i64(pos, rows, "positions: int64"), embed.data_ptr(), opt_ptr(pos_embed),
+                        x.data_ptr(), rows, (int)H, (int)seq, (int)offset, embed.size(0), pos_embed.has_value() ? pos_embed->size(0) : 0,
+                        cur_stream()), "fl_dec_embed");
+}
+static void dec_add_norm(torch::Tensor x, c10::optional<torch::Tensor> y, c10::optional<torch::Tensor> y_bias, torch::Tensor w,
+                         c10::optional<torch::Tensor> b, torch::Tensor h, double eps) {
+  const int dt = dec_dtype(x);
+  const int64_t H = w.numel(), rows = x.numel() / H;
+  TORCH_CHECK(x.is_contiguous() && x.numel() == rows * H && w.scalar_type() == x.scalar_type() && w.is_contiguous(), "x: [rows, hidden]");
+  dec_like(y, x, x.numel(), "y: like x"); dec_like(y_bias, x, H, "y_bias: [hidden]"); dec_like(b, x, H, "b: [hidden]"); dec_like(h, x, x.numel(), "h: like x");
+  c10::cuda::CUDAGuard guard(x.device());
+  check_rc(fl_dec_add_norm(dt, x.data_ptr(), opt_ptr(y), opt_ptr(y_bias), w.data_ptr(), opt_ptr(b), h.data_ptr(), rows, (int)H, (float)eps,
+                           cur_stream()), "fl_dec_add_norm");
+}
+static void dec_qkv(torch::Tensor qkv, c10::optional<torch::Tensor> bias, c10::optional<torch::Tensor> rope, c10::optional<torch::Tensor> pos,
+                    int64_t seq, torch::Tensor k_pool, torch::Tensor v_pool, torch::Tensor table, int64_t layout, int64_t layer,
+                    int64_t layers, int64_t num_blocks, int64_t block_size, int64_t heads, int64_t kv_heads, int64_t dim) {
+  const int dt = dec_dtype(qkv);
+  const int64_t width = (heads + 2 * kv_heads) * dim, rows = qkv.numel() / width;
+  TORCH_CHECK(qkv.is_contiguous() && qkv.numel() == rows * width, "qkv: [rows, (heads + 2 kv_heads) * dim]");
+  TORCH_CHECK(k_pool.scalar_type() == qkv.scalar_type() && v_pool.scalar_type() == qkv.scalar_type(), "pools of the model's type expected");
+  TORCH_CHECK(pos.has_value() ? table.size(0) >= rows : (seq > 0 && table.size(0) * seq >= rows), "block_table: one row per request");
+  TORCH_CHECK(!rope.has_value() || (rope->is_cuda() && rope->scalar_type() == torch::kFloat32 && rope->is_contiguous() && rope->size(-1) == dim),
+              "rope: [positions, dim] fp32");
+  dec_like(bias, qkv, width, "bias: [(heads + 2 kv_heads) * dim]");
+  c10::cuda::CUDAGuard guard(qkv.device());
+  const FlPagedKv kv = dec_kv(k_pool, v_pool, table, layout, layer, layers, num_blocks, block_size, kv_heads, dim);
+  check_rc(fl_dec_qkv(dt, qkv.data_ptr(), opt_ptr(bias), rope.has_value() ? rope->data_ptr<float>() : nullptr, rope.has_value() ? rope->size(0) : 0,
+                      dec_i64(pos, rows, "positions: int64"), rows, (int)seq, (int)heads, (int)dim, &kv, cur_stream()), "fl_dec_qkv");
+}
+static void dec_act(torch::Tensor h, c10::optional<torch::Tensor> bias, torch::Tensor out, int64_t kind) {
+  const int dt = dec_dtype(h);
+  const int64_t F = out.size(-1), rows = out.numel() / F;
+  TORCH_CHECK(h.is_contiguous() && out.is_contiguous() && out.scalar_type() == h.scalar_type() &&
+              h.numel() == rows * F * (kind == FL_ACT_SILU_GATED ? 2 : 1), "h: [rows, ffn] (gate and up: [rows, 2 ffn])");
+  dec_like(bias, h, F, "bias: [ffn]");
+  c10::cuda::CUDAGuard guard(h.device());
+  check_rc(fl_dec_act(dt, (int)kind, h.data_ptr(), opt_ptr(bias), out.data_ptr(), rows, (int)F, cur_stream()), "fl_dec_act");
+}
+static std::tuple<int64_t, int64_t, int64_t> dec_attention_plan(int64_t batch, int64_t heads, int64_t kv_heads, int64_t dim, int64_t capacity) {
+  long long ws = 0;
+  int tickets = 0, splits = 1;
+  check_rc(fl_dec_attention_plan((int)batch, (int)heads, (int)kv_heads, (int)dim, (int)capacity, &ws, &tickets, &splits), "fl_dec_attention_plan");
+  return {(int64_t)ws, (int64_t)tickets, (int64_t)splits};
+}
+static void dec_attention(torch::Tensor qkv, torch::Tensor pos, torch::Tensor k_pool, torch::Tensor v_pool, torch::Tensor table, int64_t layer,
+                          int64_t layers, int64_t num_blocks, int64_t block_size, int64_t heads, int64_t kv_heads, int64_t dim, torch::Tensor out,
+                          int64_t splits, c10::optional<torch::Tensor> ws, c10::optional<torch::Tensor> tickets) {
+  const int dt = dec_dtype(qkv);
+  const int64_t width = (heads + 2 * kv_heads) * dim, batch = qkv.numel() / width;
+  TORCH_CHECK(qkv.is_contiguous() && qkv.numel() == batch * width && table.size(0) >= batch, "qkv: [batch, (heads + 2 kv_heads) * dim]");
+  TORCH_CHECK(k_pool.scalar_type() == qkv.scalar_type() && v_pool.scalar_type() == qkv.scalar_type(), "pools of the model's type expected");
+  dec_like(out, qkv, batch * heads * dim, "out: [batch, heads * dim]");
+  if (splits > 1) {
+    const auto need = dec_attention_plan(batch, heads, kv_heads, dim, table.size(1) * block_size);
+    TORCH_CHECK(splits <= std::get<2>(need) && ws.has_value() && ws->is_cuda() && ws->scalar_type() == torch::kFloat32 && ws->numel() >= std::get<0>(need) &&
+                tickets.has_value() && tickets->is_cuda() && tickets->scalar_type() == torch::kInt32 && tickets->numel() >= std::get<1>(need),
+                "workspace smaller than dec_attention_plan asks for");
+  }
+  c10::cuda::CUDAGuard guard(qkv.device());
+  const FlPagedKv kv = dec_kv(k_pool, v_pool, table, FL_KV_LBSHD, layer, layers, num_blocks, block_size, kv_heads, dim);
+  check_rc(fl_dec_attention(dt, qkv.data_ptr(), width, dec_i64(pos, batch, "positions: int64"), &kv, out.data_ptr(), (int)batch, (int)heads, (int)dim,
+                            (int)splits, ws.has_value() ? ws->data_ptr<float>() : nullptr, tickets.has_value() ? tickets->data_ptr<int>() : nullptr,
+                            cur_stream()), "fl_dec_attention");
+}
+static torch::Tensor dec_argmax(torch::Tensor logits) {
+  const int dt = dec_dtype(logits);
+  TORCH_CHECK(logits.dim() == 2 && logits.is_contiguous(), "logits: [rows, vocab]");
+  c10::cuda::CUDAGuard guard(logits.device());
+  auto out = torch::empty({logits.size(0)}, logits.options().dtype(torch::kInt64));
+  check_rc(fl_dec_argmax(dt, logits.data_ptr(), reinterpret_cast<long long*>(out.data_ptr<int64_t>()), (int)logits.size(0), logits.size(1),
+                         cur_stream()), "fl_dec_argmax");
+  return out;
+}
+static void dec_advance(torch::Tensor next, torch::Tensor tokens, torch::Tensor pos, torch::Tensor history, int64_t pos0) {
+  const int64_t B = next.numel();
+  TORCH_CHECK(history.dim() == 2 && history.size(1) == B, "history: [steps, batch]");
+  c10::cuda::CUDAGuard guard(next.device());
+  check_rc(fl_dec_advance(dec_i64(next, B, "next: int64"), const_cast<long long*>(dec_i64(tokens, B, "tokens: int64")),
+                          const_cast<long long*>(dec_i64(pos, B, "pos: int64")), const_cast<long long*>(dec_i64(history, history.numel(), "history: int64")),
+                          pos0, (int)B, (int)history.size(0), cur_stream()), "fl_dec_advance");
+}
+
 // ------------------------------------------------------------------------------------------------ MoE
 static void moe_dispatch(torch::Tensor x, torch::Tensor topk_idx, c10::optional<torch::Tensor> row_scale,
                          int64_t num_experts, int64_t experts_per_rank, int64_t cap, int64_t rank, int64_t world,
@@ -356,6 +474,14 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("barrier", &barrier);
   m.def("embbag", &embbag);
   m.def("kv_pack_send", &kv_pack_send);
+  m.def("dec_embed", &dec_embed);
+  m.def("dec_add_norm", &dec_add_norm);
+  m.def("dec_qkv", &dec_qkv);
+  m.def("dec_act", &dec_act);
+  m.def("dec_attention_plan", &dec_attention_plan);
+  m.def("dec_attention", &dec_attention);
+  m.def("dec_argmax", &dec_argmax);
+  m.def("dec_advance", &dec_advance);
   m.def("moe_dispatch", &moe_dispatch);
   m.def("moe_zero_tail", &moe_zero_tail);
   m.def("moe_combine", &moe_combine);

@@ -14,6 +14,7 @@
 #include "../csrc/kernels/fp8_gemm.cuh"
 #include "../csrc/kernels/grouped_gemm.cuh"
 #include "../csrc/kernels/kv_pack.cuh"
+#include "../csrc/kernels/decoder.cuh"
 #include "../csrc/kernels/moe_dispatch.cuh"
 #include "../csrc/kernels/moe_dispatch_noalloc.cuh"
 #include "../csrc/kernels/shadow_reduce.cuh"

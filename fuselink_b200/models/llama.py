@@ -6,9 +6,11 @@ CMakeLists.txt:116-149: model_llama2, model_opt, model_gpt2).
 
 The reference's serving experiment builds `st::model::Gpt<T>` from an external library with dummy weights
 (experiments/serving/model.hh:165-177) and a table of model shapes (common_gpt_hyper_params.h:10-131).
-Here the model is plain PyTorch (library attention / GEMMs: not a named hot path), tensor-parallel over a
-process group, with random-init bf16 weights; what is hand-written is the KV hand-off between the stages
-(csrc/kernels/kv_pack.cu), which this model feeds layer by layer through ``on_layer_done``.
+Here the matrix products and the attention over a prompt are library calls, tensor-parallel over a process group, with
+random-init bf16 weights; hand-written are the KV hand-off between the stages (csrc/kernels/kv_pack.cu), which this model
+feeds layer by layer through ``on_layer_done``, and, for bf16 and fp16 on the GPU, every pass between the products and the
+attention of a decoding step (csrc/kernels/decoder.cu).  The operation-by-operation formulation below is the same
+computation, rounded at the same places; it serves the CPU, fp32 and head sizes the kernels do not take.
 
 Paged KV layouts (block = `block_size` tokens):
   prefill pool  [block][layer][head][slot][dim]   (FL_KV_BLHSD)
@@ -22,7 +24,10 @@ from typing import Callable, Optional
 import torch
 import torch.nn.functional as F
 
+from .._ext import require_native
+
 KV_BLHSD, KV_LBSHD = 0, 1
+_ACT = {"llama": 0, "opt": 1, "gpt2": 2}          # FlDecAct
 
 
 @dataclass
@@ -178,6 +183,95 @@ class LlamaShard(torch.nn.Module):
     def _logits(self, x):
         return (self._norm(x, self.final_norm, self.final_norm_b) @ self.lm_head.t()).float()
 
+    # ------------------------------------------------------------------------------------------- fused passes
+    def _fused(self, pool: torch.Tensor) -> bool:
+        """Whether csrc/kernels/decoder.cu takes this shard: 16-bit weights and pools on the GPU, rows and heads in whole
+        16-byte vectors (a rotated head in two halves of them), heads of at most 128."""
+        cfg, w = self.cfg, self.embed
+        return (w.is_cuda and pool.is_cuda and w.dtype == pool.dtype and w.dtype in (torch.bfloat16, torch.float16)
+                and cfg.hidden % 8 == 0 and cfg.hidden <= 32768 and self.f_local % 8 == 0 and cfg.head_dim % 16 == 0 and cfg.head_dim <= 128)
+
+    def _rope_table(self, positions: int):
+        """fp32 [positions, D]: the cosines, then the sines, of every position's angles; made once for at least 4096
+        positions.  Tables that were outgrown are kept, since a captured graph may hold their addresses."""
+        if self.cfg.arch != "llama":
+            return None
+        tables = self.__dict__.setdefault("_rope_tables", [])
+        if tables and tables[-1].shape[0] >= positions:
+            return tables[-1]
+        n = max(4096, 1 << (positions - 1).bit_length())
+        D, dev = self.cfg.head_dim, self.embed.device
+        inv = 1.0 / (self.cfg.rope_theta ** (torch.arange(0, D, 2, device=dev, dtype=torch.float32) / D))
+        ang = torch.arange(n, device=dev).float().unsqueeze(-1) * inv
+        table = torch.cat([ang.cos(), ang.sin()], -1).contiguous()
+        if not torch.cuda.is_current_stream_capturing():       # another stream may be the next to use it
+            torch.cuda.current_stream(dev).synchronize()
+            tables.append(table)
+        return table
+
+    def _layers_fused(self, x, pos, seq, k_pool, v_pool, table, layout, num_blocks, attend, on_layer_done=None):
+        """Every layer on x [rows, hidden]; ``attend(l, qkv)`` returns the attention output [rows, h_local * D].  Returns
+        (x, y, bias): the residual stream without the last branch, the branch and its bias (final_norm adds them up)."""
+        C, cfg = require_native(), self.cfg
+        rows, kind = x.shape[0], _ACT[cfg.arch]
+        rope = self._rope_table(table.shape[1] * cfg.block_size)
+        h = torch.empty_like(x)
+        act = torch.empty(rows, self.f_local, dtype=x.dtype, device=x.device)
+        y = bias = None
+        for l in range(cfg.layers):
+            C.dec_add_norm(x, y, bias, self.n1[l], self.n1b[l], h, cfg.eps)
+            qkv = h @ self.wqkv[l].t()
+            C.dec_qkv(qkv, self.bqkv[l], rope, pos, seq, k_pool, v_pool, table, layout, l, cfg.layers, num_blocks, cfg.block_size,
+                      self.h_local, self.kvh_local, cfg.head_dim)
+            if on_layer_done is not None:
+                on_layer_done(l)                                                # KV of this layer may leave now
+            y = self._allreduce(attend(l, qkv) @ self.wo[l].t())
+            C.dec_add_norm(x, y, self.bo[l], self.n2[l], self.n2b[l], h, cfg.eps)
+            C.dec_act(h @ self.w13[l].t(), self.b13[l], act, kind)
+            y, bias = self._allreduce(act @ self.w2[l].t()), self.b2[l]
+        return x, y, bias
+
+    def _choose_fused(self, x, y, bias):
+        C = require_native()
+        h = torch.empty_like(x)
+        C.dec_add_norm(x, y, bias, self.final_norm, self.final_norm_b, h, self.cfg.eps)
+        return C.dec_argmax(h @ self.lm_head.t())
+
+    def _prefill_fused(self, tokens, k_pool, v_pool, block_table, on_layer_done, last_pos):
+        C, cfg = require_native(), self.cfg
+        B, S = tokens.shape
+        D, hl, kl = cfg.head_dim, self.h_local, self.kvh_local
+        x = torch.empty(B * S, cfg.hidden, dtype=self.embed.dtype, device=tokens.device)
+        C.dec_embed(tokens.contiguous(), None, self.embed, self.pos_embed, x, S, cfg.pos_offset)
+        table = block_table[:B, : S // cfg.block_size].int().contiguous()
+        num_blocks = k_pool.numel() // (cfg.layers * kl * cfg.block_size * D)
+
+        def attend(l, qkv):
+            q, k, v = qkv.view(B, S, hl + 2 * kl, D).split([hl, kl, kl], 2)
+            o = F.scaled_dot_product_attention(q.transpose(1, 2), k.transpose(1, 2), v.transpose(1, 2), is_causal=True, enable_gqa=hl != kl)
+            return o.transpose(1, 2).reshape(B * S, hl * D)
+
+        x, y, bias = self._layers_fused(x, None, S, k_pool, v_pool, table, KV_BLHSD, num_blocks, attend, on_layer_done)
+        at = torch.arange(B, device=x.device) * S + (S - 1 if last_pos is None else last_pos)
+        return self._choose_fused(x[at], y[at], bias)
+
+    def _decode_fused(self, tokens, positions, k_pool, v_pool, block_table, num_blocks):
+        C, cfg = require_native(), self.cfg
+        B, D, hl, kl, dev = tokens.shape[0], cfg.head_dim, self.h_local, self.kvh_local, tokens.device
+        positions, table = positions.contiguous(), block_table.int().contiguous()
+        x = torch.empty(B, cfg.hidden, dtype=self.embed.dtype, device=dev)
+        C.dec_embed(tokens.contiguous(), positions, self.embed, self.pos_embed, x, 1, cfg.pos_offset)
+        floats, tickets, splits = C.dec_attention_plan(B, hl, kl, D, table.shape[1] * cfg.block_size)
+        ws = torch.empty(floats, device=dev) if splits > 1 else None              # one step's layers take turns in it
+        tk = torch.zeros(tickets, dtype=torch.int32, device=dev) if splits > 1 else None
+        out = torch.empty(B, hl * D, dtype=x.dtype, device=dev)
+
+        def attend(l, qkv):
+            C.dec_attention(qkv, positions, k_pool, v_pool, table, l, cfg.layers, num_blocks, cfg.block_size, hl, kl, D, out, splits, ws, tk)
+            return out
+
+        return self._choose_fused(*self._layers_fused(x, positions, 1, k_pool, v_pool, table, KV_LBSHD, num_blocks, attend))
+
     # ------------------------------------------------------------------------------------------- prefill
     @torch.no_grad()
     def prefill(self, tokens: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, block_table: torch.Tensor,
@@ -188,6 +282,8 @@ class LlamaShard(torch.nn.Module):
         B, S = tokens.shape
         bs, D, L = cfg.block_size, cfg.head_dim, cfg.layers
         assert S % bs == 0
+        if self._fused(k_pool):
+            return self._prefill_fused(tokens, k_pool, v_pool, block_table, on_layer_done, last_pos)
         nblk = S // bs
         kp = k_pool.view(-1, L, self.kvh_local, bs, D)
         vp = v_pool.view(-1, L, self.kvh_local, bs, D)
@@ -217,6 +313,8 @@ class LlamaShard(torch.nn.Module):
         cfg = self.cfg
         B = tokens.shape[0]
         bs, D, L = cfg.block_size, cfg.head_dim, cfg.layers
+        if self._fused(k_pool):
+            return self._decode_fused(tokens, positions, k_pool, v_pool, block_table, num_pool_blocks)
         kp = k_pool.view(L, num_pool_blocks, bs, self.kvh_local, D)
         vp = v_pool.view(L, num_pool_blocks, bs, self.kvh_local, D)
         bt = block_table.long()

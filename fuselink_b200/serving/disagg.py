@@ -202,7 +202,9 @@ class DecodeStage:
         self.graph = None
         self.g_tokens = torch.zeros(B, dtype=torch.long, device=dev)
         self.g_pos = torch.zeros(B, dtype=torch.long, device=dev)
-        self.g_out = None
+        # tokens of every step; the captured step feeds itself: it takes g_tokens at g_pos, notes the result here, puts it
+        # into g_tokens and advances g_pos, so decoding is nothing but replays
+        self.g_hist = torch.zeros(p.num_decoding_step, B, dtype=torch.long, device=dev)
 
     def _step(self, tokens, pos):
         link = self.link
@@ -220,7 +222,8 @@ class DecodeStage:
             torch.cuda.current_stream().wait_stream(side)
             g = torch.cuda.CUDAGraph()
             with torch.cuda.graph(g):
-                self.g_out = self._step(self.g_tokens, self.g_pos)
+                out = self._step(self.g_tokens, self.g_pos)
+                self.link.C.dec_advance(out, self.g_tokens, self.g_pos, self.g_hist, self.p.input_len)
             self.graph = g
         except Exception as e:  # noqa: BLE001 - capture is an optimisation; the eager loop is always valid
             self.graph = None
@@ -239,19 +242,21 @@ class DecodeStage:
             self.g_pos.copy_(pos)
             self._capture()                     # one-off set-up, outside the timed loop
         d0.record()
-        for _ in range(p.num_decoding_step):
-            if self.graph is not None:
-                self.g_tokens.copy_(tokens)
-                self.g_pos.copy_(pos)
+        if self.graph is not None:
+            self.g_tokens.copy_(tokens)
+            self.g_pos.copy_(pos)
+            for _ in range(p.num_decoding_step):
                 self.graph.replay()
-                tokens = self.g_out.clone()
-            else:
+            gen = torch.cat([tokens.unsqueeze(1), self.g_hist.t()], 1)
+        else:
+            for _ in range(p.num_decoding_step):
                 tokens = self._step(tokens, pos)
-            out.append(tokens)
-            pos = pos + 1
+                out.append(tokens)
+                pos = pos + 1
+            gen = torch.stack(out, 1)
         d1.record()
         device_sync(self.dev)
-        return torch.stack(out, 1), d0.elapsed_time(d1)
+        return gen, d0.elapsed_time(d1)
 
     def run(self) -> StageReport:
         p, link = self.p, self.link

@@ -1,0 +1,116 @@
+"""The fused decoder passes (csrc/kernels/decoder.cu) against the same operations in fp32 / PyTorch."""
+import math
+
+import pytest
+import torch
+import torch.nn.functional as F
+
+pytestmark = pytest.mark.gpu
+DT = [torch.bfloat16, torch.float16]
+
+
+def _eps(dt):
+    return 2.0 ** -8 if dt == torch.bfloat16 else 2.0 ** -11          # half a unit in the last place, relative
+
+
+def _rand(*shape, dt, seed):
+    return torch.randn(*shape, generator=torch.Generator(device="cuda").manual_seed(seed), device="cuda").to(dt)
+
+
+@pytest.mark.parametrize("dt", DT)
+@pytest.mark.parametrize("batch,heads,kv_heads,dim,bs,lens", [
+    (1, 1, 1, 64, 16, [1]), (3, 4, 2, 64, 16, [15, 16, 17]), (2, 32, 8, 128, 16, [2049, 700]), (2, 12, 12, 80, 8, [129, 1]),
+    (2, 24, 2, 128, 5, [333, 1000]), (17, 8, 8, 96, 16, [7 * i + 1 for i in range(17)]),
+])
+def test_paged_attention_of_one_token(dt, batch, heads, kv_heads, dim, bs, lens):
+    from fuselink_b200 import C
+    L, layer, maxblk = 2, 1, max(lens) // bs + 3
+    nb = batch * maxblk
+    kp, vp = (_rand(L, nb, bs, kv_heads, dim, dt=dt, seed=s) for s in (1, 2))
+    bt = torch.randperm(nb, generator=torch.Generator().manual_seed(3)).view(batch, maxblk).int().cuda()
+    qkv = _rand(batch, (heads + 2 * kv_heads) * dim, dt=dt, seed=4)
+    pos = torch.tensor(lens, device="cuda") - 1
+    out = torch.full((batch, heads * dim), float("nan"), dtype=dt, device="cuda")
+    ws, tk, splits = C.dec_attention_plan(batch, heads, kv_heads, dim, maxblk * bs)
+    w, t = torch.empty(max(ws, 1), device="cuda"), torch.zeros(tk, dtype=torch.int32, device="cuda")
+    for _ in range(2):                                                # the second run finds the tickets as the first left them
+        C.dec_attention(qkv, pos, kp, vp, bt, layer, L, nb, bs, heads, kv_heads, dim, out, splits, w, t)
+    assert not t.any()
+    for b, n in enumerate(lens):
+        k, v = (p[layer][bt[b].long()].reshape(-1, kv_heads, dim)[:n].float().repeat_interleave(heads // kv_heads, 1) for p in (kp, vp))
+        q = qkv[b, : heads * dim].view(heads, dim).float()
+        want = torch.einsum("hn,nhd->hd", (torch.einsum("hd,nhd->hn", q, k) / math.sqrt(dim)).softmax(-1), v).reshape(-1)
+        # the probabilities are rounded to the type before the second product (a sum of at most max|v| x eps), and the result
+        assert (out[b].float() - want).abs().max() <= 2 * _eps(dt) * v.abs().max() + 1e-5
+
+
+@pytest.mark.parametrize("dt", DT)
+@pytest.mark.parametrize("rows,hidden", [(1, 64), (5, 768), (200, 2048), (3, 8192), (2, 20480), (150, 1032)])
+@pytest.mark.parametrize("ln", [False, True])
+def test_add_norm(dt, rows, hidden, ln):
+    from fuselink_b200 import C
+    from fuselink_b200.models.llama import _ln, _rms
+    x, y = _rand(rows, hidden, dt=dt, seed=1), _rand(rows, hidden, dt=dt, seed=2)
+    yb, w, b = (_rand(hidden, dt=dt, seed=s) for s in (3, 4, 5))
+    for yy, bias in ((None, None), (y, None), (y, yb)):
+        xs, h = x.clone(), torch.empty_like(x)
+        C.dec_add_norm(xs, yy, bias, w, b if ln else None, h, 1e-5)
+        want_x = x if yy is None else x + (yy if bias is None else yy + bias)
+        assert torch.equal(xs, want_x)
+        want = _ln(want_x, w, b, 1e-5) if ln else _rms(want_x, w, 1e-5)
+        # The sums are taken in another order, so a value next to the middle between two neighbours may be rounded to the other
+        # one, 2 eps away relatively: the result, and with the RMS norm also the normalised value before it meets its weight.
+        # The layer norm adds its bias to a product that may cancel it: the absolute term.
+        assert ((h - want).float().abs() <= (2.02 if ln else 4.05) * _eps(dt) * want.float().abs() + (2e-6 if ln else 0)).all()
+
+
+@pytest.mark.parametrize("model,dt", [("tiny", torch.bfloat16), ("tiny_opt", torch.float16), ("tiny_gpt2", torch.bfloat16)])
+@pytest.mark.parametrize("batch,length", [(1, 16), (3, 48)])
+def test_fused_layers_match_the_operations(model, dt, batch, length, monkeypatch):
+    """Prefill and two decoding steps with the kernels and without them: pages and tokens."""
+    from fuselink_b200.models.llama import MODEL_ZOO, LlamaShard
+    cfg = MODEL_ZOO[model]
+    net = LlamaShard(cfg, device="cuda", seed=2, dtype=dt)
+    net.lm_head = net.embed.roll(1, 0).clone()         # next tokens that win by a margin
+    net.embed.mul_(50)
+    bs, D, kl, L = cfg.block_size, cfg.head_dim, cfg.kv_heads, cfg.layers
+    per = length // bs + 1
+    nb = batch * per
+    bt = torch.randperm(nb, generator=torch.Generator().manual_seed(1)).view(batch, per).int().cuda()
+    toks = torch.randint(0, cfg.vocab, (batch, length), generator=torch.Generator().manual_seed(2)).cuda()
+    res = []
+    for fused in (True, False):
+        if not fused:
+            monkeypatch.setattr(LlamaShard, "_fused", lambda self, pool: False)
+        kp, vp = (torch.zeros(nb * L * kl * bs * D, dtype=dt, device="cuda") for _ in range(2))
+        first = net.prefill(toks, kp, vp, bt)
+        kd, vd = (p.view(nb, L, kl, bs, D).permute(1, 0, 3, 2, 4).contiguous().view(-1) for p in (kp, vp))
+        t, out = first, [first]
+        for s in range(2):
+            t = net.decode_step(t, torch.full((batch,), length + s, device="cuda"), kd, vd, bt, nb)
+            out.append(t)
+        res.append((torch.stack(out), kp, vp, kd, vd))
+    assert torch.equal(res[0][0], res[1][0])
+    for a, b in zip(res[0][1:], res[1][1:]):
+        # two layers of a handful of roundings each
+        assert (a.float() - b.float()).norm() <= 4 * _eps(dt) * b.float().norm()
+
+
+@pytest.mark.parametrize("rows,vocab", [(1, 1), (3, 1000), (16, 50257), (2, 128256)])
+def test_argmax(rows, vocab):
+    from fuselink_b200 import C
+    x = _rand(rows, vocab, dt=torch.bfloat16, seed=3)
+    got = C.dec_argmax(x)
+    best = x.float().max(1, keepdim=True).values
+    first = (x.float() == best).int().argmax(1)
+    assert torch.equal(got, first)
+
+
+@pytest.mark.parametrize("kind,ffn", [(0, 512), (1, 24), (2, 3072)])
+def test_activation(kind, ffn):
+    from fuselink_b200 import C
+    h, b = _rand(7, ffn * (2 if kind == 0 else 1), dt=torch.bfloat16, seed=1), _rand(ffn, dt=torch.bfloat16, seed=2)
+    out = torch.empty(7, ffn, dtype=torch.bfloat16, device="cuda")
+    C.dec_act(h, None if kind == 0 else b, out, kind)
+    want = F.silu(h[:, :ffn]) * h[:, ffn:] if kind == 0 else F.relu(h + b) if kind == 1 else F.gelu(h + b, approximate="tanh")
+    assert ((out - want).float().abs() <= 2.02 * 2.0 ** -8 * want.float().abs() + 1e-6).all()
