@@ -277,24 +277,29 @@ __global__ void __launch_bounds__(256) dec_act_kernel(const T* h, const T* bias,
 
 // ---- attention of one new token over its pages --------------------------------------------------------------------------
 // Bound by reading every cached key and value once.  A warp takes 16 tokens of one KV head at a time and reads them straight
-// from the pool into the fragments of m16n8k16 products, 16 bytes per lane and load, all of a step's loads issued before its
-// first product; nothing is staged in shared memory and no page is gathered first.  Two orders that the products do not fix
-// make that possible: the contraction index of q.k may run over the head dimension in any order, so lane t of a quad takes
-// columns 8 t .. 8 t + 7 of each 32; the output columns of p.v may be dealt out in any order, so lane group g takes columns
-// 8 g .. 8 g + 7 of each 64.  The rows of a product are the query heads that share the KV head (8 at most per CTA; the other
-// eight rows are zero).  The eight warps of a CTA walk different tokens and merge their (max, sum, output) in shared memory;
-// where batch x KV heads leaves SMs idle the context is cut into `splits` more parts, merged by the last CTA to finish.
-constexpr int ATT_WARPS = 8;
+// from the pool into the fragments of m16n8k16 products, 16 bytes per lane and load; nothing is staged in shared memory and
+// no page is gathered first.  Two orders that the products do not fix make that possible: the contraction index of q.k may
+// run over the head dimension in any order, so lane t of a quad takes columns 8 t .. 8 t + 7 of each 32; the output columns
+// of p.v may be dealt out in any order, so lane group g takes columns 8 g .. 8 g + 7 of each 64.  The rows of a product are
+// the query heads that share the KV head (8 at most per CTA; the other eight rows are zero).  The values of a step are
+// requested before its scores are computed and the next step's keys right after them, so a warp always has 4 to 8 KB on the
+// way.  The warps of a CTA walk different tokens; the context is cut further over the CTAs of a cluster, which merge their
+// (max, sum, output) through distributed shared memory.  16 x 2048 tokens, 8 KV heads of 128: 64 us per layer with one CTA of
+// eight warps per (request, head) and all of a step's loads waited for at once.
 constexpr int ATT_G = 8;          // query heads per CTA
 
-template <typename T, int DP>     // DP: head dimension rounded up to a multiple of 64
-__global__ void __launch_bounds__(ATT_WARPS * 32) dec_attention_kernel(const T* q, long long q_stride, const long long* pos,
-                                                                        const FlPagedKv kv, T* out, int heads, int dim, int group,
-                                                                        int gparts, float scale_log2, float* ws, int* tickets) {
+__device__ __forceinline__ float ld_cluster_f32(uint32_t addr) {
+  float v;
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr));
+  return v;
+}
+
+template <typename T, int DP, int W, bool PAGE16>   // DP: head dimension rounded up to a multiple of 64; PAGE16: pages of whole 16s
+__global__ void __launch_bounds__(W * 32, 16 / W) dec_attention_kernel(const T* q, long long q_stride, const long long* pos, const FlPagedKv kv,
+                                                                        T* out, int heads, int dim, int group, int gparts, float scale_log2) {
   constexpr int KJ = DP / 32, VC = DP / 64;
-  __shared__ float s_m[ATT_WARPS][ATT_G], s_l[ATT_WARPS][ATT_G];
-  __shared__ float s_o[ATT_WARPS][ATT_G][DP];
-  __shared__ int s_last;
+  __shared__ float s_m[W][ATT_G], s_l[W][ATT_G], c_m[ATT_G], c_l[ATT_G];
+  __shared__ float s_o[W][ATT_G][DP + 4];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
   const int kh = blockIdx.x / gparts, gp = blockIdx.x - kh * gparts, b = blockIdx.y, split = blockIdx.z, splits = gridDim.z;
   const int h0 = kh * group + gp * ATT_G, nh = min(ATT_G, group - gp * ATT_G);
@@ -302,12 +307,42 @@ __global__ void __launch_bounds__(ATT_WARPS * 32) dec_attention_kernel(const T* 
   const long long cap = (long long)kv.table_stride * bs;
   const int len = (int)min(max(pos[b] + 1, 0ll), cap);
   const int* table = kv.block_table + (long long)b * kv.table_stride;
+  const long long tok_stride = (long long)kv.heads * dim;
 
   // this warp's tokens: whole groups of 16, dealt out evenly over the warps of all splits
-  const int units = (len + 15) / 16, nw = splits * ATT_WARPS, w = split * ATT_WARPS + warp;
+  const int units = (len + 15) / 16, nw = splits * W, w = split * W + warp;
   const int per = units / nw, extra = units % nw;
   const int first = (w * per + min(w, extra)) * 16;
   const int last = min(len, first + (per + (w < extra ? 1 : 0)) * 16);
+
+  // page ids: with PAGE16 one per step, fetched a step ahead; otherwise looked up token by token
+  auto page_of = [&](int base) -> int { return PAGE16 && base < last ? table[base / bs] : -1; };
+  auto row_of = [&](const void* pool, int blk, int base, int tok) -> const T* {
+    int slot;
+    if (PAGE16) {
+      slot = base % bs + (tok - base);
+    } else {
+      blk = tok < last ? table[tok / bs] : -1;
+      slot = tok % bs;
+    }
+    if (tok >= last || blk < 0 || blk >= kv.num_blocks) return nullptr;
+    return reinterpret_cast<const T*>(pool) + (((long long)kv.layer * kv.num_blocks + blk) * bs + slot) * tok_stride + kh * dim;
+  };
+  uint4 kr[2][KJ];
+  auto load_keys = [&](int base, int blk) {
+#pragma unroll
+    for (int p = 0; p < 2; ++p) {
+      const T* r = row_of(kv.k, blk, base, base + 8 * p + g);
+#pragma unroll
+      for (int j = 0; j < KJ; ++j) {
+        const int d = 32 * j + 8 * t;
+        kr[p][j] = make_uint4(0, 0, 0, 0);
+        if (r != nullptr && d < dim) kr[p][j] = ld_nc_v4(r + d);
+      }
+    }
+  };
+  int blk = page_of(first), blk_next = page_of(first + 16);
+  load_keys(first, blk);
 
   uint32_t qa[KJ][4];
 #pragma unroll
@@ -324,32 +359,11 @@ __global__ void __launch_bounds__(ATT_WARPS * 32) dec_attention_kernel(const T* 
     for (int j = 0; j < 8; ++j) o[c][j][0] = o[c][j][1] = 0.f;
   float m = -INFINITY, l = 0.f;
 
-  // address of token `tok`'s row of this head in the key (or value) pool, 0 if its page id is bad
-  auto row_of = [&](const void* pool, int tok) -> const T* {
-    const int pg = tok / bs;
-    const int blk = table[pg];
-    if (blk < 0 || blk >= kv.num_blocks) return nullptr;
-    return reinterpret_cast<const T*>(pool) +
-           ((((long long)kv.layer * kv.num_blocks + blk) * bs + (tok - pg * bs)) * kv.heads + kh) * dim;
-  };
-
   for (int base = first; base < last; base += 16) {
-    uint4 kr[2][KJ], vr[4][VC];
-#pragma unroll
-    for (int p = 0; p < 2; ++p) {
-      const int tok = base + 8 * p + g;
-      const T* r = tok < last ? row_of(kv.k, tok) : nullptr;
-#pragma unroll
-      for (int j = 0; j < KJ; ++j) {
-        const int d = 32 * j + 8 * t;
-        kr[p][j] = make_uint4(0, 0, 0, 0);
-        if (r != nullptr && d < dim) kr[p][j] = ld_nc_v4(r + d);
-      }
-    }
+    uint4 vr[4][VC];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      const int tok = base + 2 * t + (i & 1) + 8 * (i >> 1);
-      const T* r = tok < last ? row_of(kv.v, tok) : nullptr;
+      const T* r = row_of(kv.v, blk, base, base + 2 * t + (i & 1) + 8 * (i >> 1));
 #pragma unroll
       for (int c = 0; c < VC; ++c) {
         const int d = 64 * c + 8 * g;
@@ -369,6 +383,9 @@ __global__ void __launch_bounds__(ATT_WARPS * 32) dec_attention_kernel(const T* 
 #pragma unroll
       for (int e = 0; e < 2; ++e) s[p][e] = base + 8 * p + 2 * t + e < last ? s[p][e] * scale_log2 : -INFINITY;
     }
+    blk = blk_next;
+    blk_next = page_of(base + 32);
+    load_keys(base + 16, blk);
     float mx = fmaxf(fmaxf(s[0][0], s[0][1]), fmaxf(s[1][0], s[1][1]));
     mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
     mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
@@ -406,56 +423,49 @@ __global__ void __launch_bounds__(ATT_WARPS * 32) dec_attention_kernel(const T* 
 #pragma unroll
   for (int c = 0; c < VC; ++c)
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      s_o[warp][g][64 * c + 16 * t + j] = o[c][j][0];
-      s_o[warp][g][64 * c + 16 * t + 8 + j] = o[c][j][1];
+    for (int j = 0; j < 8; j += 4) {
+      *reinterpret_cast<float4*>(&s_o[warp][g][64 * c + 16 * t + j]) = make_float4(o[c][j][0], o[c][j + 1][0], o[c][j + 2][0], o[c][j + 3][0]);
+      *reinterpret_cast<float4*>(&s_o[warp][g][64 * c + 16 * t + 8 + j]) = make_float4(o[c][j][1], o[c][j + 1][1], o[c][j + 2][1], o[c][j + 3][1]);
     }
   __syncthreads();
-  // merge the warps; with one split this is the result
+  // merge the warps: with one split this is the result, otherwise it replaces the first warp's part
   const int cells = nh * dim;
-  const long long unit = ((long long)b * gridDim.x + blockIdx.x);
-  float* part = ws + (unit * splits + split) * (ATT_G * (DP + 2));
-  for (int i = threadIdx.x; i < cells; i += blockDim.x) {
+  T* res = out + (long long)b * heads * dim + (long long)h0 * dim;
+  for (int i = threadIdx.x; i < cells; i += W * 32) {
     const int hg = i / dim, d = i - hg * dim;
     float mm = -INFINITY;
 #pragma unroll
-    for (int x = 0; x < ATT_WARPS; ++x) mm = fmaxf(mm, s_m[x][hg]);
+    for (int x = 0; x < W; ++x) mm = fmaxf(mm, s_m[x][hg]);
     float acc = 0.f, ll = 0.f;
 #pragma unroll
-    for (int x = 0; x < ATT_WARPS; ++x) {
+    for (int x = 0; x < W; ++x) {
       const float e = s_m[x][hg] == -INFINITY ? 0.f : exp2f(s_m[x][hg] - mm);
       acc += e * s_o[x][hg][d];
       ll += e * s_l[x][hg];
     }
     if (splits == 1) {
-      out[(long long)b * heads * dim + (long long)(h0 + hg) * dim + d] = T(ll > 0.f ? acc / ll : 0.f);
+      res[i] = T(ll > 0.f ? acc / ll : 0.f);
     } else {
-      part[hg * (DP + 2) + d] = acc;
-      if (d == 0) { part[hg * (DP + 2) + DP] = mm; part[hg * (DP + 2) + DP + 1] = ll; }
+      s_o[0][hg][d] = acc;
+      if (d == 0) { c_m[hg] = mm; c_l[hg] = ll; }
     }
   }
   if (splits == 1) return;
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0) s_last = atomicAdd(tickets + unit, 1) == splits - 1;
-  __syncthreads();
-  if (!s_last) return;
-  __threadfence();
-  const float* all = ws + unit * splits * (ATT_G * (DP + 2));
-  for (int i = threadIdx.x; i < cells; i += blockDim.x) {
+  cluster_sync_all();
+  for (int i = split * W * 32 + threadIdx.x; i < cells; i += splits * W * 32) {
     const int hg = i / dim, d = i - hg * dim;
+    const uint32_t am = smem_u32(&c_m[hg]), al = smem_u32(&c_l[hg]), ao = smem_u32(&s_o[0][hg][d]);
     float mm = -INFINITY;
-    for (int x = 0; x < splits; ++x) mm = fmaxf(mm, __ldcg(all + (x * ATT_G + hg) * (DP + 2) + DP));
+    for (int x = 0; x < splits; ++x) mm = fmaxf(mm, ld_cluster_f32(map_to_cta(am, x)));
     float acc = 0.f, ll = 0.f;
     for (int x = 0; x < splits; ++x) {
-      const float* r = all + (x * ATT_G + hg) * (DP + 2);
-      const float pm = __ldcg(r + DP), e = pm == -INFINITY ? 0.f : exp2f(pm - mm);
-      acc += e * __ldcg(r + d);
-      ll += e * __ldcg(r + DP + 1);
+      const float pm = ld_cluster_f32(map_to_cta(am, x)), e = pm == -INFINITY ? 0.f : exp2f(pm - mm);
+      acc += e * ld_cluster_f32(map_to_cta(ao, x));
+      ll += e * ld_cluster_f32(map_to_cta(al, x));
     }
-    out[(long long)b * heads * dim + (long long)(h0 + hg) * dim + d] = T(ll > 0.f ? acc / ll : 0.f);
+    res[i] = T(ll > 0.f ? acc / ll : 0.f);
   }
-  if (threadIdx.x == 0) tickets[unit] = 0;
+  cluster_sync_all();                            // nobody leaves while its part is being read
 }
 
 // ---- greedy choice ----------------------------------------------------------------------------------------------------------
@@ -575,37 +585,44 @@ extern "C" int fl_dec_act(int dtype, int kind, const void* h, const void* bias, 
   return (int)cudaGetLastError();
 }
 
-// Two CTAs' worth of work per SM, as long as every warp still gets about 64 tokens of a full context.
-extern "C" int fl_dec_attention_plan(int batch, int heads, int kv_heads, int dim, int capacity, long long* ws_floats, int* tickets,
-                                     int* splits) {
-  if (batch < 1 || kv_heads < 1 || heads < kv_heads || heads % kv_heads || dim < 8 || dim % 8 || dim > 128) return -2;
-  const int group = heads / kv_heads, gparts = (group + fl::ATT_G - 1) / fl::ATT_G, units = batch * kv_heads * gparts;
-  int s = (2 * 148 + units - 1) / units;
-  const int most = (capacity + 64 * fl::ATT_WARPS - 1) / (64 * fl::ATT_WARPS);
-  if (s > most) s = most;
-  if (s < 1) s = 1;
-  const int dp = dim <= 64 ? 64 : 128;
-  *splits = s;
-  *tickets = units;
-  *ws_floats = s > 1 ? (long long)units * s * fl::ATT_G * (dp + 2) : 0;
-  return 0;
+template <typename T, int DP, int W>
+static int launch_attention(const void* q, long long q_stride, const long long* pos, const FlPagedKv* kv, void* out, int batch, int heads,
+                            int dim, int group, int gparts, int splits, cudaStream_t stream) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(kv->heads * gparts, batch, splits);
+  cfg.blockDim = dim3(W * 32, 1, 1);
+  cfg.stream = stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = 1; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = splits;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  const float scale = 1.4426950408889634f / sqrtf((float)dim);
+  auto kernel = kv->block_size % 16 == 0 ? fl::dec_attention_kernel<T, DP, W, true> : fl::dec_attention_kernel<T, DP, W, false>;
+  return (int)cudaLaunchKernelEx(&cfg, kernel, (const T*)q, q_stride, pos, *kv, (T*)out, heads, dim, group, gparts, scale);
 }
 
+// How the context is cut: enough CTAs for sixteen warps per SM (a warp keeps 4 to 8 KB on the way, and that many saturate
+// the memory), but no warp below 32 tokens of a full context and at most 8 CTAs per cluster.  Where even that leaves SMs
+// idle (a few requests with long contexts) the CTAs get eight warps instead of four.
 extern "C" int fl_dec_attention(int dtype, const void* q, long long q_stride, const long long* pos, const FlPagedKv* kv, void* out,
-                                int batch, int heads, int dim, int splits, float* ws, int* tickets, cudaStream_t stream) {
+                                int batch, int heads, int dim, cudaStream_t stream) {
   if (batch < 1 || batch > 65535 || kv->heads < 1 || heads % kv->heads || dim < 8 || dim % 8 || dim > 128 || kv->layout != FL_KV_LBSHD)
     return -2;
-  if (splits < 1 || splits > 65535 || (splits > 1 && (ws == nullptr || tickets == nullptr))) return -3;
   const int group = heads / kv->heads, gparts = (group + fl::ATT_G - 1) / fl::ATT_G;
-  const dim3 grid(kv->heads * gparts, batch, splits);
-  const float scale = 1.4426950408889634f / sqrtf((float)dim);
+  const long long units = (long long)batch * kv->heads * gparts, cap = (long long)kv->table_stride * kv->block_size;
+  long long splits = 4 * 148 / units;
+  if (splits > (cap + 127) / 128) splits = (cap + 127) / 128;
+  if (splits > 8) splits = 8;
+  if (splits < 1) splits = 1;
+  const bool wide = units * splits <= 2 * 148 && cap >= splits * 8 * 32;
+#define FL_ATT(D, W) return launch_attention<T, D, W>(q, q_stride, pos, kv, out, batch, heads, dim, group, gparts, (int)splits, stream)
   FL_DEC_TYPES(dtype, {
-    if (dim <= 64)
-      fl::dec_attention_kernel<T, 64><<<grid, fl::ATT_WARPS * 32, 0, stream>>>((const T*)q, q_stride, pos, *kv, (T*)out, heads, dim, group, gparts, scale, ws, tickets);
-    else
-      fl::dec_attention_kernel<T, 128><<<grid, fl::ATT_WARPS * 32, 0, stream>>>((const T*)q, q_stride, pos, *kv, (T*)out, heads, dim, group, gparts, scale, ws, tickets);
+    if (dim <= 64) { if (wide) FL_ATT(64, 8); else FL_ATT(64, 4); }
+    else { if (wide) FL_ATT(128, 8); else FL_ATT(128, 4); }
   });
-  return (int)cudaGetLastError();
+#undef FL_ATT
+  return 0;
 }
 
 extern "C" int fl_dec_argmax(int dtype, const void* logits, long long* out, int rows, long long vocab, cudaStream_t stream) {

@@ -28,11 +28,9 @@ int fl_dec_add_norm(int dtype, void* x, const void* y, const void* y_bias, const
 int fl_dec_qkv(int dtype, void* qkv, const void* bias, const float* rope, long long rope_rows, const long long* pos, long long rows,
                int seq, int heads, int dim, const FlPagedKv* kv, cudaStream_t stream);
 int fl_dec_act(int dtype, int kind, const void* h, const void* bias, void* out, long long rows, int ffn, cudaStream_t stream);
-// floats of workspace and number of zeroed words fl_dec_attention needs
-int fl_dec_attention_plan(int batch, int heads, int kv_heads, int dim, int capacity, long long* ws_floats, int* tickets, int* splits);
 // out [batch, heads * dim] = attention of q [batch] (row stride q_stride) over positions 0 .. pos of the request's pages
 int fl_dec_attention(int dtype, const void* q, long long q_stride, const long long* pos, const FlPagedKv* kv, void* out, int batch,
-                     int heads, int dim, int splits, float* ws, int* tickets, cudaStream_t stream);
+                     int heads, int dim, cudaStream_t stream);
 // out[row] = index of the largest value of logits[row] (the first of equals; NaN counts as largest)
 int fl_dec_argmax(int dtype, const void* logits, long long* out, int rows, long long vocab, cudaStream_t stream);
 // one decoding step's bookkeeping: history[pos - pos0][b] = next[b]; tokens = next; pos += 1

@@ -296,30 +296,16 @@ static void dec_act(torch::Tensor h, c10::optional<torch::Tensor> bias, torch::T
   c10::cuda::CUDAGuard guard(h.device());
   check_rc(fl_dec_act(dt, (int)kind, h.data_ptr(), opt_ptr(bias), out.data_ptr(), rows, (int)F, cur_stream()), "fl_dec_act");
 }
-static std::tuple<int64_t, int64_t, int64_t> dec_attention_plan(int64_t batch, int64_t heads, int64_t kv_heads, int64_t dim, int64_t capacity) {
-  long long ws = 0;
-  int tickets = 0, splits = 1;
-  check_rc(fl_dec_attention_plan((int)batch, (int)heads, (int)kv_heads, (int)dim, (int)capacity, &ws, &tickets, &splits), "fl_dec_attention_plan");
-  return {(int64_t)ws, (int64_t)tickets, (int64_t)splits};
-}
 static void dec_attention(torch::Tensor qkv, torch::Tensor pos, torch::Tensor k_pool, torch::Tensor v_pool, torch::Tensor table, int64_t layer,
-                          int64_t layers, int64_t num_blocks, int64_t block_size, int64_t heads, int64_t kv_heads, int64_t dim, torch::Tensor out,
-                          int64_t splits, c10::optional<torch::Tensor> ws, c10::optional<torch::Tensor> tickets) {
+                          int64_t layers, int64_t num_blocks, int64_t block_size, int64_t heads, int64_t kv_heads, int64_t dim, torch::Tensor out) {
   const int dt = dec_dtype(qkv);
   const int64_t width = (heads + 2 * kv_heads) * dim, batch = qkv.numel() / width;
   TORCH_CHECK(qkv.is_contiguous() && qkv.numel() == batch * width && table.size(0) >= batch, "qkv: [batch, (heads + 2 kv_heads) * dim]");
   TORCH_CHECK(k_pool.scalar_type() == qkv.scalar_type() && v_pool.scalar_type() == qkv.scalar_type(), "pools of the model's type expected");
   dec_like(out, qkv, batch * heads * dim, "out: [batch, heads * dim]");
-  if (splits > 1) {
-    const auto need = dec_attention_plan(batch, heads, kv_heads, dim, table.size(1) * block_size);
-    TORCH_CHECK(splits <= std::get<2>(need) && ws.has_value() && ws->is_cuda() && ws->scalar_type() == torch::kFloat32 && ws->numel() >= std::get<0>(need) &&
-                tickets.has_value() && tickets->is_cuda() && tickets->scalar_type() == torch::kInt32 && tickets->numel() >= std::get<1>(need),
-                "workspace smaller than dec_attention_plan asks for");
-  }
   c10::cuda::CUDAGuard guard(qkv.device());
   const FlPagedKv kv = dec_kv(k_pool, v_pool, table, FL_KV_LBSHD, layer, layers, num_blocks, block_size, kv_heads, dim);
   check_rc(fl_dec_attention(dt, qkv.data_ptr(), width, dec_i64(pos, batch, "positions: int64"), &kv, out.data_ptr(), (int)batch, (int)heads, (int)dim,
-                            (int)splits, ws.has_value() ? ws->data_ptr<float>() : nullptr, tickets.has_value() ? tickets->data_ptr<int>() : nullptr,
                             cur_stream()), "fl_dec_attention");
 }
 static torch::Tensor dec_argmax(torch::Tensor logits) {
@@ -478,7 +464,6 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("dec_add_norm", &dec_add_norm);
   m.def("dec_qkv", &dec_qkv);
   m.def("dec_act", &dec_act);
-  m.def("dec_attention_plan", &dec_attention_plan);
   m.def("dec_attention", &dec_attention);
   m.def("dec_argmax", &dec_argmax);
   m.def("dec_advance", &dec_advance);

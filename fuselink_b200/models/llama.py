@@ -261,13 +261,10 @@ class LlamaShard(torch.nn.Module):
         positions, table = positions.contiguous(), block_table.int().contiguous()
         x = torch.empty(B, cfg.hidden, dtype=self.embed.dtype, device=dev)
         C.dec_embed(tokens.contiguous(), positions, self.embed, self.pos_embed, x, 1, cfg.pos_offset)
-        floats, tickets, splits = C.dec_attention_plan(B, hl, kl, D, table.shape[1] * cfg.block_size)
-        ws = torch.empty(floats, device=dev) if splits > 1 else None              # one step's layers take turns in it
-        tk = torch.zeros(tickets, dtype=torch.int32, device=dev) if splits > 1 else None
         out = torch.empty(B, hl * D, dtype=x.dtype, device=dev)
 
         def attend(l, qkv):
-            C.dec_attention(qkv, positions, k_pool, v_pool, table, l, cfg.layers, num_blocks, cfg.block_size, hl, kl, D, out, splits, ws, tk)
+            C.dec_attention(qkv, positions, k_pool, v_pool, table, l, cfg.layers, num_blocks, cfg.block_size, hl, kl, D, out)
             return out
 
         return self._choose_fused(*self._layers_fused(x, positions, 1, k_pool, v_pool, table, KV_LBSHD, num_blocks, attend))
