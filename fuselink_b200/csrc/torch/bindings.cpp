@@ -9,6 +9,7 @@
 #include "../kernels/shadow_reduce.cuh"
 #include "../kernels/comm_kernels.cuh"
 #include "../kernels/embbag.cuh"
+#include "../kernels/interact.cuh"
 #include "../kernels/kv_pack.cuh"
 #include "../kernels/decoder.cuh"
 #include "../kernels/moe_dispatch.cuh"
@@ -189,6 +190,34 @@ static void embbag(bool backward, torch::Tensor weights, torch::Tensor indices, 
   a.out_peers = to_peers(peers); a.lr = (float)lr; a.status = reinterpret_cast<int*>(status_addr);
   if (backward) check_rc(fl_embbag_a2a_bwd_sgd(&a, (int)num_ctas, cur_stream()), "fl_embbag_a2a_bwd_sgd");
   else check_rc(fl_embbag_a2a_fwd(&a, (int)num_ctas, cur_stream()), "fl_embbag_a2a_fwd");
+}
+
+// Pairwise-dot interaction: out [B, ld] = x | upper triangle of z z^T | zeros, z = x and the pooled vectors of the sample.
+static FlInteractArgs interact_args(const torch::Tensor& x, const torch::Tensor& pooled, const torch::Tensor& wide) {
+  for (const auto& t : {x, pooled, wide})
+    TORCH_CHECK(t.is_cuda() && t.scalar_type() == torch::kFloat32 && t.is_contiguous(), "interact: contiguous fp32 CUDA tensors expected");
+  TORCH_CHECK(x.dim() == 2 && pooled.dim() == 3 && wide.dim() == 2 && pooled.size(0) == x.size(0) && wide.size(0) == x.size(0) &&
+              pooled.size(2) == x.size(1), "x: [B, dim], pooled: [B, vectors - 1, dim], out: [B, ld]");
+  FlInteractArgs a;
+  memset(&a, 0, sizeof a);
+  a.x = x.data_ptr<float>(); a.pooled = pooled.data_ptr<float>();
+  a.batch = x.size(0); a.vectors = (int)pooled.size(1) + 1; a.dim = (int)x.size(1); a.ld = wide.size(1);
+  return a;
+}
+static void interact_fwd(torch::Tensor x, torch::Tensor pooled, torch::Tensor out) {
+  FlInteractArgs a = interact_args(x, pooled, out);
+  c10::cuda::CUDAGuard guard(x.device());
+  a.out = out.data_ptr<float>();
+  check_rc(fl_interact_fwd(&a, cur_stream()), "fl_interact_fwd");
+}
+static void interact_bwd(torch::Tensor x, torch::Tensor pooled, torch::Tensor dout, torch::Tensor dx, torch::Tensor dpooled, double scale) {
+  FlInteractArgs a = interact_args(x, pooled, dout);
+  for (const auto& t : {dx, dpooled})
+    TORCH_CHECK(t.is_cuda() && t.scalar_type() == torch::kFloat32 && t.is_contiguous(), "interact: contiguous fp32 CUDA tensors expected");
+  TORCH_CHECK(dx.numel() == x.numel() && dpooled.numel() == pooled.numel(), "gradients: as large as the vectors");
+  c10::cuda::CUDAGuard guard(x.device());
+  a.dout = dout.data_ptr<float>(); a.dx = dx.data_ptr<float>(); a.dpooled = dpooled.data_ptr<float>(); a.scale = (float)scale;
+  check_rc(fl_interact_bwd(&a, cur_stream()), "fl_interact_bwd");
 }
 
 // ------------------------------------------------------------------------------------------------ KV
@@ -463,6 +492,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("dec_embed", &dec_embed);
   m.def("dec_add_norm", &dec_add_norm);
   m.def("dec_qkv", &dec_qkv);
+  m.def("interact_fwd", &interact_fwd);
+  m.def("interact_bwd", &interact_bwd);
   m.def("dec_act", &dec_act);
   m.def("dec_attention", &dec_attention);
   m.def("dec_argmax", &dec_argmax);

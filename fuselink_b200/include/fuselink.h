@@ -13,6 +13,7 @@
 #include "../csrc/kernels/embbag.cuh"
 #include "../csrc/kernels/fp8_gemm.cuh"
 #include "../csrc/kernels/grouped_gemm.cuh"
+#include "../csrc/kernels/interact.cuh"
 #include "../csrc/kernels/kv_pack.cuh"
 #include "../csrc/kernels/decoder.cuh"
 #include "../csrc/kernels/moe_dispatch.cuh"

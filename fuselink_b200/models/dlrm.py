@@ -69,6 +69,55 @@ def _mlp(sizes, last_act: bool) -> nn.Sequential:
     return nn.Sequential(*layers)
 
 
+class _Interaction(torch.autograd.Function):
+    """[B, width] from the bottom MLP's vectors x and the pooled vectors: x, the dot products of all pairs, zeros up to
+    ``width``.  The pooled vectors' gradient, times ``scale``, goes straight into ``gpooled``; ``anchor`` (a leaf that wants a
+    gradient and gets none) has the backward run whether or not x wants one."""
+
+    @staticmethod
+    def forward(ctx, x, pooled, gpooled, scale, width, iu, anchor):
+        # The kernel's products are tf32, so it needs the caller's leave.  Below 16 vectors, unless they come in fours, the
+        # library answers in fp32 at some batch sizes although it has it; those products stay the library's.
+        n = pooled.shape[1] + 1
+        if torch.backends.cuda.matmul.allow_tf32 and (n >= 16 or n % 4 == 0):
+            out = torch.empty(x.shape[0], width, dtype=x.dtype, device=x.device)
+            require_native().interact_fwd(x, pooled, out)
+        else:
+            z = torch.cat([x.unsqueeze(1), pooled], dim=1)
+            inter = torch.bmm(z, z.transpose(1, 2))[:, iu[0], iu[1]]
+            out = F.pad(torch.cat([x, inter], dim=1), (0, width - x.shape[1] - inter.shape[1]))
+        ctx.save_for_backward(x)
+        ctx.pooled, ctx.gpooled, ctx.scale = pooled, gpooled, scale
+        return out
+
+    @staticmethod
+    @torch.autograd.function.once_differentiable
+    def backward(ctx, dout):
+        x, = ctx.saved_tensors
+        dx = torch.empty_like(x)
+        require_native().interact_bwd(x, ctx.pooled, dout.contiguous(), dx, ctx.gpooled, ctx.scale)
+        return dx, None, None, None, None, None, None
+
+
+class _PaddedLinear(torch.autograd.Function):
+    """F.linear(r[:, :in], weight, bias) for rows r that are padded with zeros to an aligned width: the gradients' products
+    run over the padded width.  At an odd number of columns (479 for 26 tables) they miss the library's aligned kernels."""
+
+    @staticmethod
+    def forward(ctx, r, weight, bias):
+        ctx.save_for_backward(r, weight)
+        return F.linear(r[:, : weight.shape[1]], weight, bias)
+
+    @staticmethod
+    @torch.autograd.function.once_differentiable
+    def backward(ctx, dy):
+        r, weight = ctx.saved_tensors
+        n = weight.shape[1]
+        dr = dy @ F.pad(weight, (0, r.shape[1] - n)) if ctx.needs_input_grad[0] else None
+        dw = (dy.t() @ r)[:, :n].contiguous() if ctx.needs_input_grad[1] else None
+        return dr, dw, dy.sum(0) if ctx.needs_input_grad[2] else None
+
+
 class DLRM(nn.Module):
     def __init__(self, cfg: DLRMConfig, heap: Optional[SymmetricHeap] = None, rank: int = 0, world: int = 1,
                  device="cuda", seed: int = 0, name: str = "dlrm"):
@@ -119,6 +168,9 @@ class DLRM(nn.Module):
 
     def sparse_backward_launch(self, grad_pooled: torch.Tensor):
         self.gpooled.local.copy_(grad_pooled)
+        self._grad_ready()
+
+    def _grad_ready(self):
         barrier(self.heap, self.name + ":b", signal=True, wait=False)
         self.launches += 1
 
@@ -141,6 +193,29 @@ class DLRM(nn.Module):
         inter = zz[:, self.iu0, self.iu1]
         return self.top(torch.cat([x, inter], dim=1)).squeeze(-1)
 
+    def _fused_dense(self, dense: torch.Tensor) -> bool:
+        """Whether csrc/kernels/interact.cu takes the interaction: fp32 on the GPU, at most 28 vectors of whole 128 columns, and
+        a dense side that is what __init__ made (no hooks, no replaced or converted layers, no override, no autocast), since the
+        first layer of the top MLP is then called through its weight."""
+        if not (dense.is_cuda and dense.dtype == torch.float32 and self.cfg.dim % 128 == 0 and self.cfg.num_tables <= 27
+                and type(self).dense_forward is DLRM.dense_forward and not torch.is_autocast_enabled("cuda")):
+            return False
+        first = self.top[0]
+        return (type(first) is nn.Linear and type(self.top) is nn.Sequential and "dense_forward" not in self.__dict__
+                and not any(m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks for m in (self.top, first))
+                and all(p.dtype == torch.float32 and p.is_cuda for p in self.dense_parameters()))
+
+    def _dense_forward_fused(self, dense: torch.Tensor, pooled: torch.Tensor) -> torch.Tensor:
+        """dense_forward with the gradient of ``pooled`` (over the ranks' mean) written to the buffer the tables' owners read."""
+        x = self.bottom(dense).contiguous()
+        n = self.n_inter + self.cfg.dim
+        width = (n + 7) // 8 * 8
+        anchor = torch.empty(0, device=x.device, requires_grad=True)
+        r = _Interaction.apply(x, pooled, self.gpooled.local, 1.0 / self.world, width, (self.iu0, self.iu1), anchor)
+        first = self.top[0]
+        y = _PaddedLinear.apply(r, first.weight, first.bias)
+        return self.top[1:](y).squeeze(-1)
+
     def dense_parameters(self):
         return list(self.bottom.parameters()) + list(self.top.parameters())
 
@@ -148,12 +223,13 @@ class DLRM(nn.Module):
     def train_step(self, dense: torch.Tensor, indices: torch.Tensor, labels: torch.Tensor, opt: torch.optim.Optimizer):
         """Forward + backward + SGD on dense and sparse parameters.  Returns the (detached) loss."""
         fused = self.heap is not None          # a heap was given: the fused kernels (on host memory only in tests that model them)
+        direct = fused and self._fused_dense(dense)      # the pooled vectors' gradient is written where the owners read it
         if fused:
             self.sparse_forward_launch(indices)
-            pooled = self.sparse_forward_wait().detach().requires_grad_(True)
+            pooled = self.sparse_forward_wait().detach().requires_grad_(not direct)
         else:
             pooled = self._pooled_reference(indices).requires_grad_(True)
-        logits = self.dense_forward(dense, pooled)
+        logits = (self._dense_forward_fused if direct else self.dense_forward)(dense, pooled)
         loss = F.binary_cross_entropy_with_logits(logits, labels)
         loss.backward()
         work = flat = grads = None
@@ -165,12 +241,16 @@ class DLRM(nn.Module):
             flat = _flatten_dense_tensors(grads)
             work = dist.all_reduce(flat, async_op=True)
         # the loss is a mean over the local batch; the global objective is the mean over ranks
-        gp = pooled.grad / self.world if self.world > 1 else pooled.grad
-        if fused:
-            self.sparse_backward_launch(gp)
-            self.sparse_backward_apply(indices)
+        if direct:
+            self._grad_ready()
         else:
-            self._sparse_backward_reference(indices, gp)
+            gp = pooled.grad / self.world if self.world > 1 else pooled.grad
+            if fused:
+                self.sparse_backward_launch(gp)
+            else:
+                self._sparse_backward_reference(indices, gp)
+        if fused:
+            self.sparse_backward_apply(indices)
         if work is not None:
             work.wait()
             flat /= self.world
