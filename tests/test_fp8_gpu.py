@@ -141,3 +141,34 @@ def test_fp8_throughput_smoke():
     torch.cuda.synchronize()
     ms = e0.elapsed_time(e1) / 10
     print(f"\n[fp8 gemm smoke] 8192x4096x4096 e4m3 1x128: {ms:.3f} ms  {2.0 * cap * N * K / ms / 1e9:.0f} TFLOP/s")
+
+
+@pytest.mark.parametrize("K", [128, 384, 1024, 1152, 3072])            # one block, an odd number, whole and partial groups of eight
+@pytest.mark.parametrize("cap,counts", [(0, None), (256, [0, 130, 256, 1]), (200, [7, 0, 200, 129]), (128, [0, 0, 0])])
+@pytest.mark.parametrize("offset", [0, 4])                              # 4: addresses that are multiples of 8 bytes only
+def test_row_quantizer_over_groups(K, cap, counts, offset):
+    """Rows that hold tokens, up to a whole tile, and no others."""
+    from fuselink_b200 import C
+    from fuselink_b200.ops import fp8
+    rows = cap * len(counts) if counts else 77
+    x = _mk([rows * K + offset], 3.0, seed=K)[offset:].view(rows, K)
+    x[0] = 0
+    cnt = torch.tensor(counts, dtype=torch.int32, device="cuda") if counts else None
+    q = torch.full((rows * K + offset,), 5, dtype=torch.uint8, device="cuda")[offset:].view(rows, K).view(fp8.FP8)
+    s = torch.full((rows, K // 128), -1.0, device="cuda")
+    C.fp8_quantize_rows(x, q, s, cnt, cap)
+    used = torch.ones(rows, dtype=torch.bool, device="cuda")
+    for g, n in enumerate(counts or []):
+        used[g * cap + min((n + 127) // 128 * 128, cap):(g + 1) * cap] = False
+    rq, rs = fp8.ref_quantize_rows(x)
+    torch.testing.assert_close(s[used], rs[used], rtol=1e-6, atol=0)
+    assert (q[used].float() - rq[used].float()).abs().max() <= 32 if used.any() else True
+    assert (s[~used] == -1).all() and (q[~used].view(torch.uint8) == 5).all()
+
+
+def test_block_quantizer_at_8_byte_addresses():
+    from fuselink_b200.ops import fp8
+    w = _mk([2 * 256 * 384 + 4], 0.05, seed=2)[4:].view(2, 256, 384)
+    q, s = fp8.quantize_blocks(w)
+    q0, s0 = fp8.quantize_blocks(w.clone())
+    assert torch.equal(q.view(torch.uint8), q0.view(torch.uint8)) and torch.equal(s, s0)
