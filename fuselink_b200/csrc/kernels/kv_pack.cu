@@ -17,36 +17,68 @@ __device__ __forceinline__ long long page_base(int layout, int nblocks, int laye
                                : ((long long)layer * nblocks + blk) * page_elems;
 }
 
-__global__ void __launch_bounds__(256) kv_pack_send_kernel(const FlKvSendArgs a) {
+// v / d for v, d < 2^16, with m = ceil(2^32 / d): the error m d - 2^32 is below d, so v times it stays below 2^32
+__device__ __forceinline__ unsigned div16(unsigned v, unsigned m, unsigned d) { return d == 1 ? v : __umulhi(v, m); }
+
+// Bound by memory: a page at a time per CTA, four 16-byte copies per thread requested before the first is stored, six CTAs per
+// SM.  The page's request comes from a table of running totals in shared memory, and the next page's ids are fetched while this
+// one is copied; with a walk over the requests' counts and two divisions per 16 bytes 16 x 2048 tokens of 32 layers took
+// 1968 us, now 1540 (8.6 GB of bytes: 1310 us).  ORDER: the order inside a page differs.
+constexpr int KV_BATCH = 1024;      // requests whose running totals are kept; larger batches walk the counts
+
+template <bool ORDER, bool SMALL>   // SMALL: a page of fewer than 2^16 vectors
+__global__ void __launch_bounds__(256, 6) kv_pack_send_kernel(const FlKvSendArgs a) {
   const int H = a.heads, S = a.block_size, D = a.head_dim;
-  const int vec_per_row = D / 8;                       // 16-byte vectors per (head, slot) row
-  const int vec_per_page = H * S * vec_per_row;
+  const unsigned vec_per_row = D / 8;                  // 16-byte vectors per (head, slot) row
+  const unsigned vec_per_page = (unsigned)H * S * vec_per_row;
   const long long page_elems = (long long)H * S * D;
   const int nl = a.layer_end - a.layer_begin;
+  const bool dst_shd = a.dst_layout == FL_KV_LBSHD;
+  const unsigned inner = dst_shd ? H : S;              // rows run over (outer, inner) in the destination, the other way in the source
+  const unsigned outer = dst_shd ? S : H;
+  const unsigned mrow = SMALL ? 0xffffffffu / vec_per_row + 1 : 0, minner = SMALL ? 0xffffffffu / inner + 1 : 0;
 
-  // total pages over the batch (batch is small: scan)
+  __shared__ int s_end[KV_BATCH];
   __shared__ int s_total;
+  if (a.batch <= KV_BATCH)
+    for (int b = threadIdx.x; b < a.batch; b += blockDim.x) s_end[b] = max(0, min(a.num_blocks[b], a.max_blocks));
+  __syncthreads();
   if (threadIdx.x == 0) {
     int tot = 0;
-    for (int b = 0; b < a.batch; ++b) tot += min(a.num_blocks[b], a.max_blocks);
+    for (int b = 0; b < a.batch; ++b) {
+      tot += a.batch <= KV_BATCH ? s_end[b] : max(0, min(a.num_blocks[b], a.max_blocks));
+      if (a.batch <= KV_BATCH) s_end[b] = tot;
+    }
     s_total = tot;
   }
   __syncthreads();
   const long long units = (long long)s_total * nl * 2;
 
-  for (long long u = blockIdx.x; u < units; u += gridDim.x) {
-    const int kv = (int)(u & 1);
-    long long r = u >> 1;
-    const int layer = a.layer_begin + (int)(r % nl);
-    int pg = (int)(r / nl);
-    int b = 0;
-    for (; b < a.batch; ++b) {
-      const int nb = min(a.num_blocks[b], a.max_blocks);
-      if (pg < nb) break;
-      pg -= nb;
+  auto page_ids = [&](long long u) -> int2 {
+    if (u >= units) return make_int2(-1, -1);
+    int pg = (int)((u >> 1) / nl), b = 0;
+    if (a.batch <= KV_BATCH) {
+      for (int hi = a.batch - 1; b < hi;) {              // the first request that ends behind pg
+        const int mid = (b + hi) / 2;
+        if (s_end[mid] <= pg) b = mid + 1; else hi = mid;
+      }
+      if (b > 0) pg -= s_end[b - 1];
+    } else {
+      for (; b < a.batch; ++b) {
+        const int nb = max(0, min(a.num_blocks[b], a.max_blocks));
+        if (pg < nb) break;
+        pg -= nb;
+      }
     }
-    const int sblk = a.src_block_table[(long long)b * a.max_blocks + pg];
-    const int dblk = a.dst_block_table[(long long)b * a.max_blocks + pg];
+    const long long at = (long long)b * a.max_blocks + pg;
+    return make_int2(a.src_block_table[at], a.dst_block_table[at]);
+  };
+  int2 next = page_ids(blockIdx.x);
+  for (long long u = blockIdx.x; u < units; u += gridDim.x) {
+    const int sblk = next.x, dblk = next.y;
+    next = page_ids(u + gridDim.x);
+    const int kv = (int)(u & 1);
+    const int layer = a.layer_begin + (int)((u >> 1) % nl);
     if (sblk < 0 || sblk >= a.src_num_blocks || dblk < 0 || dblk >= a.dst_num_blocks) {
       if (threadIdx.x == 0) report(a.status, kBadIndex, 1000);
       continue;  // skip the access, keep going
@@ -55,20 +87,20 @@ __global__ void __launch_bounds__(256) kv_pack_send_kernel(const FlKvSendArgs a)
                                page_base(a.src_layout, a.src_num_blocks, a.layers, page_elems, sblk, layer);
     __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(kv ? a.dst_v : a.dst_k) +
                          page_base(a.dst_layout, a.dst_num_blocks, a.layers, page_elems, dblk, layer);
-    if (a.src_layout == a.dst_layout) {
-      for (int v = threadIdx.x; v < vec_per_page; v += blockDim.x)
-        st_v4(reinterpret_cast<uint4*>(dst) + v, ld_nc_v4(reinterpret_cast<const uint4*>(src) + v));
-    } else {
-      // page-internal order differs: [head][slot][dim] <-> [slot][head][dim]; iterate in destination order
-      const bool dst_shd = a.dst_layout == FL_KV_LBSHD;
-      for (int v = threadIdx.x; v < vec_per_page; v += blockDim.x) {
-        const int d8 = v % vec_per_row;
-        const int rw = v / vec_per_row;
-        int h, s;
-        if (dst_shd) { s = rw / H; h = rw % H; } else { h = rw / S; s = rw % S; }
-        const int src_v = dst_shd ? ((h * S + s) * vec_per_row + d8) : ((s * H + h) * vec_per_row + d8);
-        st_v4(reinterpret_cast<uint4*>(dst) + v, ld_nc_v4(reinterpret_cast<const uint4*>(src) + src_v));
-      }
+    auto source_of = [&](unsigned v) -> unsigned {       // iterates in destination order
+      if (!ORDER) return v;
+      const unsigned rw = SMALL ? div16(v, mrow, vec_per_row) : v / vec_per_row;
+      const unsigned o = SMALL ? div16(rw, minner, inner) : rw / inner;
+      return ((rw - o * inner) * outer + o) * vec_per_row + (v - rw * vec_per_row);
+    };
+    for (unsigned v = threadIdx.x; v < vec_per_page; v += 4 * 256) {
+      uint4 r[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (v + i * 256 < vec_per_page) r[i] = ld_nc_v4(reinterpret_cast<const uint4*>(src) + source_of(v + i * 256));
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (v + i * 256 < vec_per_page) st_v4(reinterpret_cast<uint4*>(dst) + v + i * 256, r[i]);
     }
   }
 
@@ -102,7 +134,10 @@ extern "C" int fl_kv_pack_send(const FlKvSendArgs* a, int num_ctas, cudaStream_t
   if (a->layer_begin < 0 || a->layer_end > a->layers || a->layer_begin >= a->layer_end) return -2;
   if (a->batch < 1 || a->max_blocks < 1) return -3;
   if (!a->cta_counter) return -4;
-  if (num_ctas <= 0) num_ctas = 148 * 4;
-  fl::kv_pack_send_kernel<<<num_ctas, 256, 0, stream>>>(*a);
+  if (num_ctas <= 0) num_ctas = 148 * 6;
+  const bool order = a->src_layout != a->dst_layout, small = (long long)a->heads * a->block_size * (a->head_dim / 8) < 65536;
+  auto kernel = order ? (small ? fl::kv_pack_send_kernel<true, true> : fl::kv_pack_send_kernel<true, false>)
+                      : fl::kv_pack_send_kernel<false, true>;
+  kernel<<<num_ctas, 256, 0, stream>>>(*a);
   return (int)cudaGetLastError();
 }

@@ -140,3 +140,34 @@ def test_online_trace_batches_with_pool_credits():
     finally:
         for h in heaps:
             h.close()
+
+
+@pytest.mark.parametrize("H,S,D,layout", [(1, 1, 8, 1), (3, 5, 24, 1), (12, 16, 64, 1), (64, 64, 128, 1), (7, 16, 128, 0)])
+@pytest.mark.parametrize("batch", [1, 37, 1500])                       # the last: more requests than the table of totals holds
+def test_kv_pack_send_over_page_shapes(H, S, D, layout, batch):
+    """Odd head counts and page sizes, pages of 2^16 vectors and more, empty requests; every page lands, nothing else moves."""
+    from fuselink_b200 import C
+    L, maxb = 2, 3
+    if H * S * D * batch > 1 << 24:
+        batch = 5
+    g = torch.Generator().manual_seed(batch)
+    nb = torch.randint(0, maxb + 1, (batch,), generator=g).int()
+    nb[0] = maxb
+    n = batch * maxb
+    src = [torch.randn(n, L, H, S, D, generator=g).to(torch.bfloat16).cuda() for _ in range(2)]
+    shape = (n, L, H, S, D) if layout == 0 else (L, n, S, H, D)
+    dst = [torch.full(shape, -7.0, dtype=torch.bfloat16, device="cuda") for _ in range(2)]
+    sbt, dbt = (torch.randperm(n, generator=g).view(batch, maxb).int().cuda() for _ in range(2))
+    status, counter = torch.zeros(8, dtype=torch.int32, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+    C.kv_pack_send(src[0], src[1], dst[0].data_ptr(), dst[1].data_ptr(), 0, layout, n, n, L, H, S, D, 1, 2, sbt, dbt, nb.cuda(),
+                   None, 0, 0, 1, counter, 0, status.data_ptr())
+    mask = torch.arange(maxb).unsqueeze(0) < nb.unsqueeze(1)
+    si, di = sbt.cpu()[mask].long().cuda(), dbt.cpu()[mask].long().cuda()
+    for s, d in zip(src, dst):
+        want = torch.full_like(d, -7.0)
+        if layout == 0:
+            want[di, 1] = s[si, 1]
+        else:
+            want[1, di] = s[si, 1].transpose(1, 2)
+        assert torch.equal(d, want)
+    assert not status.any()
