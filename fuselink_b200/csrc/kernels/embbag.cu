@@ -35,44 +35,48 @@ __device__ __forceinline__ void red_add_f4(float* p, float4 v) {
 }
 
 // grid: persistent; each warp walks bags  w, w + nwarps, ...   bag id = t_local * B_global + b
-template <int MAXL>
-__global__ void __launch_bounds__(256) embbag_fwd_kernel(const FlEmbBagArgs a) {
+// Bound by the latency of rows that are anywhere in memory: what counts is how many are on the way.  Rows are requested EB_ROWS
+// at a time (32 warps of 64 registers per SM, 160 KB on the way) and the next bag's indices before this bag's rows.  With a
+// bag's 20 rows at once, 16 warps per SM and the indices waited for first, 26 tables x 65536 bags of 20 took 2276 us (DRAM at
+// 28 % of its peak, L2 at 21 %); now 1950 us.
+constexpr int EB_ROWS = 10;
+
+__global__ void __launch_bounds__(256, 4) embbag_fwd_kernel(const FlEmbBagArgs a) {
   const int lane = threadIdx.x & 31;
   const long long nwarps = (long long)gridDim.x * (blockDim.x >> 5);
   const long long nbags = (long long)a.t_local * a.b_global;
-  const int vec_per_lane = a.dim / 128;  // float4 per lane
-  for (long long bag = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); bag < nbags; bag += nwarps) {
+  long long bag = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  long long next_idx = bag < nbags && lane < a.pooling ? a.indices[bag * a.pooling + lane] : 0;
+  for (; bag < nbags; bag += nwarps) {
     const int t = (int)(bag / a.b_global);
     const int b = (int)(bag - (long long)t * a.b_global);
-    const long long* idx = a.indices + bag * a.pooling;
     // lanes load the bag's indices once, then broadcast
-    long long my_idx = 0;
-    if (lane < a.pooling) {
-      my_idx = idx[lane];
-      if (my_idx < 0 || my_idx >= a.rows) {  // bounds check: skip the access, record it
-        report(a.status, kBadIndex, 900);
-        my_idx = -1;
-      }
+    long long my_idx = next_idx;
+    if (my_idx < 0 || my_idx >= a.rows) {  // bounds check: skip the access, record it
+      report(a.status, kBadIndex, 900);
+      my_idx = -1;
     }
+    next_idx = bag + nwarps < nbags && lane < a.pooling ? a.indices[(bag + nwarps) * a.pooling + lane] : 0;
     const float* table = a.weights + (long long)t * a.rows * a.dim;
     const int owner = b / a.b_local;
     const int bl = b - owner * a.b_local;
     float* out = reinterpret_cast<float*>(a.out_peers.p[owner]) +
                  ((long long)bl * a.t_total + (a.t_first + t)) * a.dim;
-    for (int v = 0; v < vec_per_lane; ++v) {
+    for (int c = lane * 4; c < a.dim; c += 128) {
       float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-      float4 r[MAXL];
+      for (int j0 = 0; j0 < a.pooling; j0 += EB_ROWS) {
+        float4 r[EB_ROWS];
 #pragma unroll
-      for (int j = 0; j < MAXL; ++j) {
-        const long long ij = __shfl_sync(0xffffffffu, my_idx, j);
-        r[j] = (j < a.pooling && ij >= 0) ? ld_f4(table + ij * a.dim + v * 128 + lane * 4)
-                                          : make_float4(0.f, 0.f, 0.f, 0.f);
-      }
+        for (int j = 0; j < EB_ROWS; ++j) {
+          const long long ij = __shfl_sync(0xffffffffu, my_idx, (j0 + j) & 31);
+          r[j] = (j0 + j < a.pooling && ij >= 0) ? ld_f4(table + ij * a.dim + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
 #pragma unroll
-      for (int j = 0; j < MAXL; ++j) {
-        acc.x += r[j].x; acc.y += r[j].y; acc.z += r[j].z; acc.w += r[j].w;
+        for (int j = 0; j < EB_ROWS; ++j) {
+          acc.x += r[j].x; acc.y += r[j].y; acc.z += r[j].z; acc.w += r[j].w;
+        }
       }
-      st_f4(out + v * 128 + lane * 4, acc);
+      st_f4(out + c, acc);
     }
   }
 }
@@ -112,58 +116,64 @@ __global__ void __launch_bounds__(256) embbag_bwd_kernel(const FlEmbBagArgs a) {
   }
 }
 
-// Backward with a per-CTA accumulator for the first `hot` rows of the table.  With ids ordered by frequency a handful of rows
-// take a large share of all updates (Zipf(1.05) over 1M rows: the first 64 rows get about 40 %, row 0 alone 9 %), and every
-// one of them is a vector reduction on the same few L2 lines, one after the other.  Here a CTA works on ONE table
-// (blockIdx.y), sums the updates of those rows in shared memory and sends each row to global memory once, when it is done.
-template <int MAXL>
-__global__ void __launch_bounds__(256) embbag_bwd_hot_kernel(const FlEmbBagArgs a, const int hot) {
-  extern __shared__ __align__(16) float hot_acc[];            // [hot][dim]
+// Backward with accumulators for the first `hot` rows of the table.  With ids ordered by frequency a handful of rows take a
+// large share of all updates (Zipf(1.05) over 1M rows: the first 24 rows get 30 %, row 0 alone 7 %), and every one of them is a
+// vector reduction on the same few L2 lines, one after the other.  Here a CTA works on ONE table (blockIdx.y), and each warp
+// sums the updates of those rows in shared memory of its own, which takes no atomics; a row is sent to global memory once per
+// warp, at the end.  The next bag's indices and gradient are fetched a bag ahead, and a bag's updates of other rows leave one
+// after the other before its hot ones.  26 tables x 65536 bags of 20: 5177 us without accumulators, 3785 us with 64 rows shared
+// by eight warps (atomics on shared memory are compare-and-swap loops, and the warps retry against each other on the hottest
+// rows); here 3370 us with 8 rows, 3122 with 16, 3021 with 24 (48 KB, 16 warps per SM).
+constexpr int EB_WARPS = 4;
+
+__global__ void __launch_bounds__(EB_WARPS * 32) embbag_bwd_hot_kernel(const FlEmbBagArgs a, const int hot) {
+  extern __shared__ __align__(16) float hot_acc[];            // [warp][hot][dim]
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int t = blockIdx.y;
-  const int vec_per_lane = a.dim / 128;
-  for (int i = threadIdx.x; i < hot * a.dim; i += blockDim.x) hot_acc[i] = 0.f;
-  __syncthreads();
+  float* acc = hot_acc + warp * hot * a.dim;
+  for (int i = lane * 4; i < hot * a.dim; i += 128) *reinterpret_cast<float4*>(acc + i) = make_float4(0.f, 0.f, 0.f, 0.f);
   float* table = a.weights_rw + (long long)t * a.rows * a.dim;
-  const int nwarps = gridDim.x * (blockDim.x >> 5);
-  for (int b = blockIdx.x * (blockDim.x >> 5) + warp; b < a.b_global; b += nwarps) {
-    const long long* idx = a.indices + ((long long)t * a.b_global + b) * a.pooling;
-    long long my_idx = -1;
-    if (lane < a.pooling) {
-      my_idx = idx[lane];
-      if (my_idx < 0 || my_idx >= a.rows) {
-        report(a.status, kBadIndex, 902);
-        my_idx = -1;
-      }
+  const long long* indices = a.indices + (long long)t * a.b_global * a.pooling;
+  auto grad_at = [&](int b) -> const float* {
+    const int owner = b / a.b_local, bl = b - owner * a.b_local;
+    return reinterpret_cast<const float*>(a.out_peers.p[owner]) + ((long long)bl * a.t_total + (a.t_first + t)) * a.dim + lane * 4;
+  };
+  const int nwarps = gridDim.x * EB_WARPS;
+  int b = blockIdx.x * EB_WARPS + warp;
+  long long next_idx = b < a.b_global && lane < a.pooling ? indices[(long long)b * a.pooling + lane] : 0;
+  float4 next_g = b < a.b_global ? ld_f4_coherent(grad_at(b)) : make_float4(0.f, 0.f, 0.f, 0.f);   // peers wrote it this step: no .nc
+  while (b < a.b_global) {
+    const long long my_idx = next_idx;
+    float4 gv = next_g;
+    const int nb = a.b_global - b > nwarps ? b + nwarps : a.b_global;
+    if (nb < a.b_global) {
+      next_idx = lane < a.pooling ? indices[(long long)nb * a.pooling + lane] : 0;
+      next_g = ld_f4_coherent(grad_at(nb));
     }
-    const int owner = b / a.b_local;
-    const int bl = b - owner * a.b_local;
-    const float* g = reinterpret_cast<const float*>(a.out_peers.p[owner]) +
-                     ((long long)bl * a.t_total + (a.t_first + t)) * a.dim;
-    for (int v = 0; v < vec_per_lane; ++v) {
-      float4 gv = ld_f4_coherent(g + v * 128 + lane * 4);
+    const bool bad = my_idx < 0 || my_idx >= a.rows;
+    if (bad) report(a.status, kBadIndex, 902);
+    const bool mine = lane < a.pooling && !bad;
+    const unsigned cold = __ballot_sync(0xffffffffu, mine && my_idx >= hot), warm = __ballot_sync(0xffffffffu, mine && my_idx < hot);
+    for (int c = 0; c < a.dim; c += 128) {
+      if (c) gv = ld_f4_coherent(grad_at(b) + c);
       gv.x *= -a.lr; gv.y *= -a.lr; gv.z *= -a.lr; gv.w *= -a.lr;
-#pragma unroll
-      for (int j = 0; j < MAXL; ++j) {
-        const long long ij = __shfl_sync(0xffffffffu, my_idx, j);
-        if (j >= a.pooling || ij < 0) continue;
-        if (ij < hot) {
-          float* s = hot_acc + ij * a.dim + v * 128 + lane * 4;
-          atomicAdd(s + 0, gv.x); atomicAdd(s + 1, gv.y); atomicAdd(s + 2, gv.z); atomicAdd(s + 3, gv.w);
-        } else {
-          red_add_f4(table + ij * a.dim + v * 128 + lane * 4, gv);
-        }
+      for (unsigned m = cold; m; m &= m - 1)
+        red_add_f4(table + __shfl_sync(0xffffffffu, my_idx, __ffs(m) - 1) * a.dim + c + lane * 4, gv);
+      for (unsigned m = warm; m; m &= m - 1) {
+        float4* s = reinterpret_cast<float4*>(acc + __shfl_sync(0xffffffffu, (int)my_idx, __ffs(m) - 1) * a.dim + c + lane * 4);
+        float4 x = *s;
+        x.x += gv.x; x.y += gv.y; x.z += gv.z; x.w += gv.w;
+        *s = x;
       }
     }
+    b = nb;
   }
-  __syncthreads();
-  for (int r = warp; r < hot; r += (blockDim.x >> 5)) {
-    for (int v = 0; v < vec_per_lane; ++v) {
-      const float4 x = *reinterpret_cast<const float4*>(hot_acc + r * a.dim + v * 128 + lane * 4);
+  for (int r = 0; r < hot; ++r)
+    for (int c = lane * 4; c < a.dim; c += 128) {
+      const float4 x = *reinterpret_cast<const float4*>(acc + r * a.dim + c);
       const bool nz = x.x != 0.f || x.y != 0.f || x.z != 0.f || x.w != 0.f;
-      if (__any_sync(0xffffffffu, nz)) red_add_f4(table + (long long)r * a.dim + v * 128 + lane * 4, x);
+      if (__any_sync(0xffffffffu, nz)) red_add_f4(table + (long long)r * a.dim + c, x);
     }
-  }
 }
 
 }  // namespace fl
@@ -180,8 +190,7 @@ extern "C" int fl_embbag_a2a_fwd(const FlEmbBagArgs* a, int num_ctas, cudaStream
   int rc = check(a);
   if (rc) return rc;
   if (num_ctas <= 0) num_ctas = 148 * 8;
-  if (a->pooling <= 20) fl::embbag_fwd_kernel<20><<<num_ctas, 256, 0, stream>>>(*a);
-  else fl::embbag_fwd_kernel<32><<<num_ctas, 256, 0, stream>>>(*a);
+  fl::embbag_fwd_kernel<<<num_ctas, 256, 0, stream>>>(*a);
   return (int)cudaGetLastError();
 }
 
@@ -192,16 +201,16 @@ extern "C" int fl_embbag_a2a_bwd_sgd(const FlEmbBagArgs* a, int num_ctas, cudaSt
   int hot = a->hot_rows;
   if (hot == 0) {
     static int dflt = -2;
-    if (dflt == -2) { const char* e = getenv("FUSELINK_EMBBAG_HOT_ROWS"); dflt = e ? atoi(e) : 64; }
+    if (dflt == -2) { const char* e = getenv("FUSELINK_EMBBAG_HOT_ROWS"); dflt = e ? atoi(e) : 24; }
     hot = dflt;
   }
   if ((long long)hot > a->rows) hot = (int)a->rows;
-  while (hot > 0 && (size_t)hot * a->dim * sizeof(float) > 48 * 1024) hot /= 2;    // stays within the default shared-memory limit
+  while (hot > 0 && (size_t)hot * a->dim * sizeof(float) * fl::EB_WARPS > 48 * 1024) hot /= 2;    // stays within the default shared-memory limit
   if (hot > 0 && a->t_local > 0) {
-    dim3 grid(num_ctas / a->t_local > 0 ? num_ctas / a->t_local : 1, a->t_local);
-    const size_t smem = (size_t)hot * a->dim * sizeof(float);
-    if (a->pooling <= 20) fl::embbag_bwd_hot_kernel<20><<<grid, 256, smem, stream>>>(*a, hot);
-    else fl::embbag_bwd_hot_kernel<32><<<grid, 256, smem, stream>>>(*a, hot);
+    // at least about 8 bags per warp: below that its accumulator is cleared and flushed for a handful of updates
+    const int most = (a->b_global + 8 * fl::EB_WARPS - 1) / (8 * fl::EB_WARPS), want = 2 * num_ctas / a->t_local;
+    dim3 grid(want < 1 ? 1 : want < most ? want : most, a->t_local);
+    fl::embbag_bwd_hot_kernel<<<grid, fl::EB_WARPS * 32, (size_t)hot * a->dim * sizeof(float) * fl::EB_WARPS, stream>>>(*a, hot);
     return (int)cudaGetLastError();
   }
   if (a->pooling <= 20) fl::embbag_bwd_kernel<20><<<num_ctas, 256, 0, stream>>>(*a);
