@@ -13,6 +13,7 @@
 #include "../kernels/kv_pack.cuh"
 #include "../kernels/decoder.cuh"
 #include "../kernels/moe_dispatch.cuh"
+#include "../kernels/moe_route.cuh"
 #include "../kernels/fp8_gemm.cuh"
 #include "../mem/vmm.h"
 #include "../monitor/monitor.h"
@@ -380,6 +381,44 @@ static void moe_dispatch(torch::Tensor x, torch::Tensor topk_idx, c10::optional<
   a.reuse_slots = reuse_slots; a.status = reinterpret_cast<int*>(status_addr);
   check_rc(fl_moe_dispatch(&a, cur_stream()), "fl_moe_dispatch");
 }
+// logits [T, E] bf16, bias [E] -> probs [T, E], weights [T, k], experts [T, k] as int32 and int64, first-choice shares [E], aux []
+static std::vector<torch::Tensor> moe_route(torch::Tensor logits, torch::Tensor bias, int64_t topk) {
+  TORCH_CHECK(logits.is_cuda() && logits.scalar_type() == torch::kBFloat16 && logits.is_contiguous() && logits.dim() == 2, "logits: [tokens, experts] bf16");
+  TORCH_CHECK(bias.device() == logits.device() && bias.scalar_type() == torch::kFloat32 && bias.is_contiguous() && bias.numel() == logits.size(1), "bias: [experts] fp32");
+  c10::cuda::CUDAGuard guard(logits.device());
+  const int64_t T = logits.size(0), E = logits.size(1);
+  const auto f = logits.options().dtype(torch::kFloat32);
+  FlMoeRouteArgs a;
+  memset(&a, 0, sizeof a);
+  a.tokens = (int)T; a.experts = (int)E; a.topk = (int)topk;
+  auto probs = torch::empty({T, E}, f), w = torch::empty({T, topk}, f), share = torch::empty({E}, f), aux = torch::empty({}, f);
+  auto part = torch::empty({fl_moe_route_blocks(a.tokens), 2, E}, f);
+  auto idx = torch::empty({T, topk}, f.dtype(torch::kInt32)), idx64 = torch::empty({T, topk}, f.dtype(torch::kInt64));
+  a.logits = logits.data_ptr(); a.bias = bias.data_ptr<float>(); a.probs = probs.data_ptr<float>(); a.w = w.data_ptr<float>();
+  a.idx = idx.data_ptr<int>(); a.idx64 = reinterpret_cast<long long*>(idx64.data_ptr<int64_t>());
+  a.part = part.data_ptr<float>(); a.share = share.data_ptr<float>(); a.aux = aux.data_ptr<float>();
+  check_rc(fl_moe_route(&a, cur_stream()), "fl_moe_route");
+  return {probs, w, idx, idx64, share, aux};
+}
+static torch::Tensor moe_route_bwd(torch::Tensor probs, torch::Tensor w, torch::Tensor idx, torch::Tensor share,
+                                   c10::optional<torch::Tensor> dw, c10::optional<torch::Tensor> daux) {
+  TORCH_CHECK(probs.is_cuda() && w.size(0) == probs.size(0) && share.numel() == probs.size(1), "what moe_route returned");
+  for (const auto& t : {probs, w, share})
+    TORCH_CHECK(t.scalar_type() == torch::kFloat32 && t.is_contiguous(), "contiguous fp32 expected");
+  TORCH_CHECK(idx.scalar_type() == torch::kInt32 && idx.is_contiguous() && idx.sizes() == w.sizes(), "idx: [tokens, topk] int32");
+  for (const auto& t : {dw, daux})
+    TORCH_CHECK(!t.has_value() || (t->is_cuda() && t->scalar_type() == torch::kFloat32 && t->is_contiguous()), "gradients: contiguous fp32");
+  TORCH_CHECK((!dw.has_value() || dw->numel() == w.numel()) && (!daux.has_value() || daux->numel() == 1), "gradients: as large as the outputs");
+  c10::cuda::CUDAGuard guard(probs.device());
+  FlMoeRouteArgs a;
+  memset(&a, 0, sizeof a);
+  a.tokens = (int)probs.size(0); a.experts = (int)probs.size(1); a.topk = (int)w.size(1);
+  auto out = torch::empty(probs.sizes(), probs.options().dtype(torch::kBFloat16));
+  a.probs = probs.data_ptr<float>(); a.w = w.data_ptr<float>(); a.idx = idx.data_ptr<int>(); a.share = share.data_ptr<float>();
+  a.dw = (const float*)opt_ptr(dw); a.daux = (const float*)opt_ptr(daux); a.dlogits = out.data_ptr();
+  check_rc(fl_moe_route_bwd(&a, cur_stream()), "fl_moe_route_bwd");
+  return out;
+}
 static void moe_zero_tail(int64_t buf, int64_t counts, int64_t experts_local, int64_t cap, int64_t width) {
   check_rc(fl_moe_zero_tail(reinterpret_cast<void*>(buf), reinterpret_cast<const int*>(counts), (int)experts_local,
                             (int)cap, (int)width, cur_stream()), "fl_moe_zero_tail");
@@ -492,6 +531,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("dec_embed", &dec_embed);
   m.def("dec_add_norm", &dec_add_norm);
   m.def("dec_qkv", &dec_qkv);
+  m.def("moe_route", &moe_route);
+  m.def("moe_route_bwd", &moe_route_bwd);
   m.def("interact_fwd", &interact_fwd);
   m.def("interact_bwd", &interact_bwd);
   m.def("dec_act", &dec_act);

@@ -18,6 +18,7 @@
 #include "../csrc/kernels/decoder.cuh"
 #include "../csrc/kernels/moe_dispatch.cuh"
 #include "../csrc/kernels/moe_dispatch_noalloc.cuh"
+#include "../csrc/kernels/moe_route.cuh"
 #include "../csrc/kernels/shadow_reduce.cuh"
 #include "../csrc/mem/vmm.h"
 #include "../csrc/monitor/monitor.h"

@@ -13,6 +13,7 @@ from typing import Optional
 import torch
 import torch.nn as nn
 
+from .._ext import require_native
 from ..ops import gemm, ref
 from ..ops.moe import MoEConfig, MoEFunction, MoEWorkspace, balanced_placement, expert_home
 from ..parallel.symm import SymmetricHeap
@@ -49,6 +50,33 @@ def load_balancing_loss(probs: torch.Tensor, idx: torch.Tensor, num_experts: int
     me = probs.mean(0)
     ce = torch.nn.functional.one_hot(idx[:, 0].long(), num_experts).float().mean(0)
     return (me * ce).sum() * num_experts
+
+
+class _Route(torch.autograd.Function):
+    """(weights, experts as int32 and int64, load-balancing loss) from the router's logits (csrc/kernels/moe_route.cu).  A gradient that is itself to be
+    differentiated is taken through the framework's operations."""
+
+    @staticmethod
+    def forward(ctx, logits, bias, topk):
+        probs, w, idx, idx64, share, aux = require_native().moe_route(logits, bias, topk)
+        ctx.save_for_backward(logits, bias, probs, w, idx, share)
+        ctx.mark_non_differentiable(idx, idx64)
+        ctx.set_materialize_grads(False)
+        return w, idx, idx64, aux
+
+    @staticmethod
+    def backward(ctx, dw, _, __, daux):
+        logits, bias, probs, w, idx, share = ctx.saved_tensors
+        if dw is None and daux is None:
+            return None, None, None
+        if torch.is_grad_enabled():
+            chosen = torch.softmax(logits.float() + bias, dim=-1)
+            cw = chosen.gather(1, idx.long())
+            outs = ((cw / cw.sum(dim=-1, keepdim=True), dw), (load_balancing_loss(chosen, idx, logits.shape[1]), daux))
+            used = [(o, g) for o, g in outs if g is not None]
+            return torch.autograd.grad([o for o, _ in used], logits, [g for _, g in used], create_graph=True)[0], None, None
+        f = lambda g: None if g is None else g.contiguous()
+        return require_native().moe_route_bwd(probs, w.detach(), idx, share, f(dw), f(daux)), None, None
 
 
 class MoELayer(nn.Module):
@@ -144,7 +172,11 @@ class MoELayer(nn.Module):
         xr = x
         if self.training and self.noisy_gate == "jitter":
             xr = x * torch.empty_like(x).uniform_(1.0 - self.jitter_eps, 1.0 + self.jitter_eps)
-        logits = (xr @ self.router.t()).float() + self.router_bias
+        y = xr @ self.router.t()
+        if self._fused_route(y):
+            w, idx, self.last_topk_idx, self.l_aux = _Route.apply(y, self.router_bias, self.cfg.topk)
+            return self._drop(w, idx), idx
+        logits = y.float() + self.router_bias
         probs = torch.softmax(logits, dim=-1)
         if self.training and self.noisy_gate == "rsample":
             noisy = logits - torch.log(-torch.log(torch.rand_like(logits).clamp_min(1e-20)))   # Gumbel-max sampling
@@ -155,12 +187,25 @@ class MoELayer(nn.Module):
         w = w / w.sum(dim=-1, keepdim=True)
         self.last_topk_idx = idx.detach()       # what reshadow() looks at
         self.l_aux = load_balancing_loss(probs, idx, self.cfg.num_experts)
+        return self._drop(w, idx), idx.int()
+
+    def _fused_route(self, y: torch.Tensor) -> bool:
+        """Whether csrc/kernels/moe_route.cu takes these logits: bf16 on the GPU, at most 64 experts and 8 choices, a bias that
+        wants no gradient and no noise."""
+        E, b = self.cfg.num_experts, self.router_bias
+        return (y.is_cuda and y.dtype == torch.bfloat16 and y.dim() == 2 and y.shape[0] > 0 and y.is_contiguous() and E <= 64
+                and self.cfg.topk <= min(8, E) and not (self.training and self.noisy_gate == "rsample")
+                and b.dtype == torch.float32 and b.device == y.device and b.numel() == y.shape[1] == E and b.is_contiguous()
+                and not b.requires_grad)
+
+    def _drop(self, w: torch.Tensor, idx: torch.Tensor) -> torch.Tensor:
+        """The weights without the choices over an expert's capacity, where the layer drops them."""
         if self.drop_tokens and self.capacity_factor > 0:
-            cap = expert_capacity(x.shape[0], self.cfg.num_experts, self.cfg.topk, self.capacity_factor, self.min_capacity)
+            cap = expert_capacity(w.shape[0], self.cfg.num_experts, self.cfg.topk, self.capacity_factor, self.min_capacity)
             keep = capacity_keep_mask(idx, self.cfg.num_experts, cap)
             self.dropped_fraction = 1.0 - keep.float().mean()
             w = w * keep.to(w.dtype)
-        return w, idx.int()
+        return w
 
     def home(self, e: int):
         """(owner rank, local index) of expert e."""
