@@ -99,6 +99,22 @@ class _Interaction(torch.autograd.Function):
         return dx, None, None, None, None, None, None
 
 
+_GRAM_ROWS = 1024
+
+
+def _gram(dy: torch.Tensor, r: torch.Tensor) -> torch.Tensor:
+    """dy^T r over slices of _GRAM_ROWS rows, the slices' results added up in fp32.  The library's aligned tf32 kernels keep one
+    running sum over all rows, and its rounding shows: against fp64 the relative error is 2.94e-4 below 8192 rows, 3.31e-4 at
+    65536.  In slices it is 2.94e-4 at any number of rows, which is also what the kernels for odd widths give."""
+    B = dy.shape[0]
+    n = B // _GRAM_ROWS
+    if n < 2:
+        return dy.t() @ r
+    m = n * _GRAM_ROWS
+    out = torch.bmm(dy[:m].view(n, _GRAM_ROWS, -1).transpose(1, 2), r[:m].view(n, _GRAM_ROWS, -1)).sum(0)
+    return out if m == B else out.addmm_(dy[m:].t(), r[m:])
+
+
 class _PaddedLinear(torch.autograd.Function):
     """F.linear(r[:, :in], weight, bias) for rows r that are padded with zeros to an aligned width: the gradients' products
     run over the padded width.  At an odd number of columns (479 for 26 tables) they miss the library's aligned kernels."""
@@ -114,7 +130,7 @@ class _PaddedLinear(torch.autograd.Function):
         r, weight = ctx.saved_tensors
         n = weight.shape[1]
         dr = dy @ F.pad(weight, (0, r.shape[1] - n)) if ctx.needs_input_grad[0] else None
-        dw = (dy.t() @ r)[:, :n].contiguous() if ctx.needs_input_grad[1] else None
+        dw = _gram(dy.contiguous(), r)[:, :n].contiguous() if ctx.needs_input_grad[1] else None
         return dr, dw, dy.sum(0) if ctx.needs_input_grad[2] else None
 
 

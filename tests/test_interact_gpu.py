@@ -62,3 +62,21 @@ def test_train_step_takes_the_general_path_where_the_kernel_does_not_apply(table
         torch.testing.assert_close(a.gpooled.local, c.gpooled.local)
     finally:
         heap.close()
+
+
+@pytest.mark.parametrize("columns", [131, 183, 479])
+@pytest.mark.parametrize("batch", [300, 2053, 8192, 20011, 65536])           # one slice, slices and a remainder, slices only
+def test_weight_gradient_over_the_padded_width_is_as_exact_as_over_its_own(columns, batch, monkeypatch):
+    from fuselink_b200.models.dlrm import _PaddedLinear
+    monkeypatch.setattr(torch.backends.cuda.matmul, "allow_tf32", True)
+    g = torch.Generator(device="cuda").manual_seed(columns)
+    r = torch.zeros(batch, (columns + 7) // 8 * 8, device="cuda")
+    r[:, :columns] = torch.randn(batch, columns, generator=g, device="cuda")
+    dy = torch.randn(batch, 1024, generator=g, device="cuda").relu_()
+    w, b = (torch.randn(*s, generator=g, device="cuda").requires_grad_(True) for s in ((1024, columns), (1024,)))
+    _PaddedLinear.apply(r, w, b).backward(dy)
+    x = r[:, :columns].contiguous()
+    want = dy.double().t() @ x.double()
+    err, lib = ((t.double() - want).norm() / want.norm() for t in (w.grad, dy.t() @ x))
+    # both are mostly the rounding of the factors to tf32, equal in the two; 1 % covers the order of the sums
+    assert err <= 1.01 * lib
