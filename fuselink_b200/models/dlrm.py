@@ -69,6 +69,16 @@ def _mlp(sizes, last_act: bool) -> nn.Sequential:
     return nn.Sequential(*layers)
 
 
+def _tf32_allowed() -> bool:
+    """Whether the program lets fp32 products run in tf32.  `fp32_precision` answers for both of the framework's settings; the
+    older flag raises once the newer setting has been used."""
+    matmul = torch.backends.cuda.matmul
+    try:
+        return matmul.fp32_precision == "tf32"
+    except AttributeError:                     # versions that have the flag alone
+        return matmul.allow_tf32
+
+
 class _Interaction(torch.autograd.Function):
     """[B, width] from the bottom MLP's vectors x and the pooled vectors: x, the dot products of all pairs, zeros up to
     ``width``.  The pooled vectors' gradient, times ``scale``, goes straight into ``gpooled``; ``anchor`` (a leaf that wants a
@@ -79,7 +89,7 @@ class _Interaction(torch.autograd.Function):
         # The kernel's products are tf32, so it needs the caller's leave.  Below 16 vectors, unless they come in fours, the
         # library answers in fp32 at some batch sizes although it has it; those products stay the library's.
         n = pooled.shape[1] + 1
-        if torch.backends.cuda.matmul.allow_tf32 and (n >= 16 or n % 4 == 0):
+        if _tf32_allowed() and (n >= 16 or n % 4 == 0):
             out = torch.empty(x.shape[0], width, dtype=x.dtype, device=x.device)
             require_native().interact_fwd(x, pooled, out)
         else:

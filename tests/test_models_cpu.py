@@ -287,3 +287,18 @@ def test_baseline_layer_gives_the_same_result_under_any_expert_placement():
     x = torch.randn(64, 128).to(torch.bfloat16)
     assert torch.equal(a(x), b(x)) and torch.equal(a.w2[0], b.w2[7]) and a.homes is None
     assert BaselineMoELayer(cfg, 0, 1, device="cpu", seed=3, placement="balanced").homes is None      # one rank: nothing to even out
+
+
+@pytest.mark.parametrize("setting,allowed", [
+    ("", False), ("matmul.allow_tf32 = True", True), ("matmul.allow_tf32 = False", False), ("matmul.fp32_precision = 'tf32'", True),
+    ("matmul.fp32_precision = 'ieee'", False), ("torch.backends.fp32_precision = 'tf32'", True),
+    ("torch.backends.fp32_precision = 'tf32'; matmul.fp32_precision = 'ieee'", False), ("torch.set_float32_matmul_precision('high')", True),
+])
+def test_tf32_permission_under_both_interfaces(setting, allowed):
+    """In a process each, since the settings are the process's and using both raises."""
+    import subprocess
+    import sys
+    code = f"import torch; matmul = torch.backends.cuda.matmul; {setting}\nfrom fuselink_b200.models.dlrm import _tf32_allowed; print(_tf32_allowed())"
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
+    assert r.returncode == 0, r.stderr
+    assert r.stdout.strip() == str(allowed)
