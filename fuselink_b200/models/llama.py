@@ -232,10 +232,12 @@ class LlamaShard(torch.nn.Module):
         return x, y, bias
 
     def _choose_fused(self, x, y, bias):
+        """The tokens chosen at [..., hidden] positions of the residual stream; ``x`` is overwritten."""
         C = require_native()
         h = torch.empty_like(x)
         C.dec_add_norm(x, y, bias, self.final_norm, self.final_norm_b, h, self.cfg.eps)
-        return C.dec_argmax(h @ self.lm_head.t())
+        logits = h @ self.lm_head.t()
+        return C.dec_argmax(logits.view(-1, logits.shape[-1])).view(logits.shape[:-1])
 
     def _prefill_fused(self, tokens, k_pool, v_pool, block_table, on_layer_done, last_pos):
         C, cfg = require_native(), self.cfg
@@ -252,8 +254,10 @@ class LlamaShard(torch.nn.Module):
             return o.transpose(1, 2).reshape(B * S, hl * D)
 
         x, y, bias = self._layers_fused(x, None, S, k_pool, v_pool, table, KV_BLHSD, num_blocks, attend, on_layer_done)
-        at = torch.arange(B, device=x.device) * S + (S - 1 if last_pos is None else last_pos)
-        return self._choose_fused(x[at], y[at], bias)
+        # indexed per request, so that a position counts from the request's own end or is out of its range
+        at = (slice(None), -1) if last_pos is None else (torch.arange(B, device=x.device), last_pos)
+        x, y = (t.view(B, S, -1)[at] for t in (x, y))
+        return self._choose_fused(x.contiguous(), y.contiguous(), bias)
 
     def _decode_fused(self, tokens, positions, k_pool, v_pool, block_table, num_blocks):
         C, cfg = require_native(), self.cfg

@@ -1,0 +1,122 @@
+"""The fused route of the decoder (models/llama.py over csrc/kernels/decoder.cu) takes the calls that the operation-by-operation
+route takes and answers alike: both on host memory, the kernels as plain PyTorch with the same arguments."""
+import math
+
+import pytest
+import torch
+import torch.nn.functional as F
+
+from fuselink_b200.models import llama
+from fuselink_b200.models.llama import KV_BLHSD, MODEL_ZOO, LlamaShard
+
+
+class Kernels:
+    """What the kernels are specified to do (decoder.cuh), values rounded at the same places."""
+
+    def dec_embed(self, tokens, pos, embed, pos_embed, x, seq, offset):
+        tokens = tokens.reshape(-1)
+        x.copy_(embed[tokens])
+        if pos_embed is not None:
+            x += pos_embed[(torch.arange(tokens.numel()) % seq if pos is None else pos) + offset]
+
+    def dec_add_norm(self, x, y, y_bias, w, b, h, eps):
+        if y is not None:
+            x += y if y_bias is None else y + y_bias
+        h.copy_(llama._rms(x, w, eps) if b is None else llama._ln(x, w, b, eps))
+
+    def dec_qkv(self, qkv, bias, rope, pos, seq, k_pool, v_pool, table, layout, layer, layers, num_blocks, bs, heads, kv_heads, dim):
+        rows = torch.arange(qkv.shape[0])
+        at, req = (rows % seq, rows // seq) if pos is None else (pos, rows)
+        if bias is not None:
+            qkv += bias
+        y = qkv.view(len(rows), heads + 2 * kv_heads, dim)
+        if rope is not None:
+            cos, sin = (rope[at].unsqueeze(1)[..., s] for s in (slice(0, dim // 2), slice(dim // 2, None)))
+            z = y[:, :heads + kv_heads].float()
+            a, b = z[..., :dim // 2], z[..., dim // 2:]
+            y[:, :heads + kv_heads] = torch.cat([a * cos - b * sin, b * cos + a * sin], -1).to(qkv.dtype)
+        page, slot = table.long()[req, at // bs], at % bs
+        for pool, v in ((k_pool, y[:, heads:heads + kv_heads]), (v_pool, y[:, heads + kv_heads:])):
+            if layout == KV_BLHSD:
+                pool.view(num_blocks, layers, kv_heads, bs, dim)[page, layer, :, slot] = v
+            else:
+                pool.view(layers, num_blocks, bs, kv_heads, dim)[layer, page, slot] = v
+
+    def dec_act(self, h, bias, out, kind):
+        if kind == 0:
+            out.copy_(F.silu(h[:, :out.shape[1]]) * h[:, out.shape[1]:])
+        else:
+            out.copy_(F.relu(h + bias) if kind == 1 else F.gelu(h + bias, approximate="tanh"))
+
+    def dec_attention(self, qkv, pos, k_pool, v_pool, table, layer, layers, num_blocks, bs, heads, kv_heads, dim, out):
+        for b in range(qkv.shape[0]):
+            n = int(pos[b]) + 1
+            k, v = (p.view(layers, num_blocks, bs, kv_heads, dim)[layer][table[b].long()].reshape(-1, kv_heads, dim)[:n].float()
+                    .repeat_interleave(heads // kv_heads, 1) for p in (k_pool, v_pool))
+            q = qkv[b, :heads * dim].view(heads, dim).float()
+            p = (torch.einsum("hd,nhd->hn", q, k) / math.sqrt(dim)).softmax(-1)
+            out[b] = torch.einsum("hn,nhd->hd", p, v).reshape(-1).to(out.dtype)
+
+    def dec_argmax(self, logits):
+        assert logits.dim() == 2
+        return logits.float().argmax(-1)
+
+
+FUSED, PLAIN = True, False
+
+
+@pytest.fixture
+def route(monkeypatch):
+    """route(FUSED) and route(PLAIN) choose the route of the calls that follow."""
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: True)      # nothing to wait for on host memory
+    monkeypatch.setattr(llama, "require_native", Kernels)
+    return lambda fused: monkeypatch.setattr(LlamaShard, "_fused", lambda self, pool: fused)
+
+
+def _net(model, dtype=torch.bfloat16):
+    net = LlamaShard(MODEL_ZOO[model], device="cpu", seed=2, dtype=dtype)
+    net.lm_head = net.embed.roll(1, 0).clone()         # next tokens that win by a margin
+    net.embed.mul_(50)
+    return net
+
+
+def _prefill(net, tokens, table=None, blocks=None, **kw):
+    cfg, (B, S) = net.cfg, tokens.shape
+    per = S // cfg.block_size
+    if table is None:
+        table = torch.randperm(B * per, generator=torch.Generator().manual_seed(1)).view(B, per).int()
+    pools = [torch.zeros((blocks or B * per) * cfg.layers * cfg.kv_heads * cfg.block_size * cfg.head_dim, dtype=net.embed.dtype) for _ in range(2)]
+    return net.prefill(tokens, *pools, table, **kw), *pools
+
+
+def _tokens(net, B, S):
+    return torch.randint(0, net.cfg.vocab, (B, S), generator=torch.Generator().manual_seed(5))
+
+
+def _alike(a, b, dtype=torch.bfloat16):
+    assert torch.equal(a[0], b[0])
+    for x, y in zip(a[1:], b[1:]):
+        assert (x.float() - y.float()).norm() <= 4 * (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11) * y.float().norm()
+
+
+@pytest.mark.parametrize("model", ["tiny", "tiny_opt", "tiny_gpt2"])
+@pytest.mark.parametrize("last_pos", [None, 3, -1, -20, torch.tensor([0, 31, 7]), torch.tensor([-1, 5, -32]), torch.tensor([4, -2, 9], dtype=torch.int32),
+                                      torch.tensor([[1, 2, 3], [4, 5, -6]])])
+def test_the_position_that_gives_the_first_token(model, last_pos, route):
+    """Positions count from the request's own end where they are negative, in either route."""
+    net = _net(model)
+    toks = _tokens(net, 3, 32)
+    res = []
+    for r in (FUSED, PLAIN):
+        route(r)
+        res.append(_prefill(net, toks, last_pos=last_pos))
+    _alike(*res)
+
+
+@pytest.mark.parametrize("last_pos", [32, -33, torch.tensor([0, 40, 1])])
+def test_a_position_outside_the_prompt_is_an_error(last_pos, route):
+    net = _net("tiny")
+    for r in (FUSED, PLAIN):
+        route(r)
+        with pytest.raises(IndexError):
+            _prefill(net, _tokens(net, 3, 32), last_pos=last_pos)
