@@ -386,12 +386,15 @@ __global__ void __launch_bounds__(W * 32, 16 / W) dec_attention_kernel(const T* 
     blk = blk_next;
     blk_next = page_of(base + 32);
     load_keys(base + 16, blk);
+    const float m_old = m;
     float mx = fmaxf(fmaxf(s[0][0], s[0][1]), fmaxf(s[1][0], s[1][1]));
     mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
     mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
-    const float mn = fmaxf(m, mx);               // finite: at least one token of the step is in range
-    const float f = exp2f(m - mn);
-    m = mn;
+    // A score may be -inf (an infinite key): 0 stands in for a maximum of -inf, so that a step of nothing else adds nothing.
+    // One that is NaN or +inf makes the sums NaN, and NaN they stay.
+    m = fmaxf(m, mx);
+    const float mn = m == -INFINITY ? 0.f : m;
+    const float f = exp2f(m_old - mn);
     float add = 0.f;
 #pragma unroll
     for (int p = 0; p < 2; ++p)
@@ -439,12 +442,12 @@ __global__ void __launch_bounds__(W * 32, 16 / W) dec_attention_kernel(const T* 
     float acc = 0.f, ll = 0.f;
 #pragma unroll
     for (int x = 0; x < W; ++x) {
-      const float e = s_m[x][hg] == -INFINITY ? 0.f : exp2f(s_m[x][hg] - mm);
+      const float e = s_l[x][hg] == 0.f ? 0.f : exp2f(s_m[x][hg] - mm);       // a part without weight; not one whose sum is NaN
       acc += e * s_o[x][hg][d];
       ll += e * s_l[x][hg];
     }
     if (splits == 1) {
-      res[i] = T(ll > 0.f ? acc / ll : 0.f);
+      res[i] = T(len > 0 ? acc / ll : 0.f);
     } else {
       s_o[0][hg][d] = acc;
       if (d == 0) { c_m[hg] = mm; c_l[hg] = ll; }
@@ -459,11 +462,11 @@ __global__ void __launch_bounds__(W * 32, 16 / W) dec_attention_kernel(const T* 
     for (int x = 0; x < splits; ++x) mm = fmaxf(mm, ld_cluster_f32(map_to_cta(am, x)));
     float acc = 0.f, ll = 0.f;
     for (int x = 0; x < splits; ++x) {
-      const float pm = ld_cluster_f32(map_to_cta(am, x)), e = pm == -INFINITY ? 0.f : exp2f(pm - mm);
+      const float pl = ld_cluster_f32(map_to_cta(al, x)), e = pl == 0.f ? 0.f : exp2f(ld_cluster_f32(map_to_cta(am, x)) - mm);
       acc += e * ld_cluster_f32(map_to_cta(ao, x));
-      ll += e * ld_cluster_f32(map_to_cta(al, x));
+      ll += e * pl;
     }
-    res[i] = T(ll > 0.f ? acc / ll : 0.f);
+    res[i] = T(len > 0 ? acc / ll : 0.f);
   }
   cluster_sync_all();                            // nobody leaves while its part is being read
 }

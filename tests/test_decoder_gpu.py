@@ -42,6 +42,38 @@ def test_paged_attention_of_one_token(dt, batch, heads, kv_heads, dim, bs, lens)
 
 
 @pytest.mark.parametrize("dt", DT)
+@pytest.mark.parametrize("kv_heads,dim,bs,lens", [(2, 64, 16, [40, 5]), (8, 128, 16, [2049, 1500]), (2, 80, 8, [300, 90]), (4, 64, 32, [1000] * 160)])
+@pytest.mark.parametrize("value,where", [(float("nan"), "first"), (float("nan"), "last"), (float("nan"), "all"), (float("inf"), "first"), (float("-inf"), "first"),
+                                         (float("-inf"), "last"), (float("-inf"), "all")])
+def test_paged_attention_passes_on_what_is_not_finite(dt, kv_heads, dim, bs, lens, value, where):
+    """A NaN or infinite score makes the head NaN, as a softmax does; one of -inf (here a whole step of 16 tokens, before or behind
+    finite ones) weighs nothing, and nothing but such scores is NaN.  Other heads and requests are as without."""
+    from fuselink_b200 import C
+    heads, batch, maxblk = 2 * kv_heads, len(lens), max(lens) // bs + 1
+    nb = batch * maxblk
+    kp, vp = (_rand(1, nb, bs, kv_heads, dim, dt=dt, seed=s) for s in (1, 2))
+    bt = torch.randperm(nb, generator=torch.Generator().manual_seed(3)).view(batch, maxblk).int().cuda()
+    qkv = _rand(batch, (heads + 2 * kv_heads) * dim, dt=dt, seed=4)
+    qkv[:, 0:heads * dim:dim] = 1                                   # every query's first column: the score gets the key's infinity
+    n = lens[0]
+    for tok in dict(first=range(min(16, n - 1)), last=range((n - 1) // 16 * 16, n), all=range(n))[where]:
+        kp[0, bt[0, tok // bs].long(), tok % bs, 1, 0] = value
+    pos = torch.tensor(lens, device="cuda") - 1
+    out = torch.empty(batch, heads * dim, dtype=dt, device="cuda")
+    C.dec_attention(qkv, pos, kp, vp, bt, 0, 1, nb, bs, heads, kv_heads, dim, out)
+    for b in (0, batch - 1):
+        k, v = (p[0][bt[b].long()].reshape(-1, kv_heads, dim)[:lens[b]].float().repeat_interleave(2, 1) for p in (kp, vp))
+        q = qkv[b, : heads * dim].view(heads, dim).float()
+        want = torch.einsum("hn,nhd->hd", ((q.unsqueeze(0) * k).sum(-1).t() / math.sqrt(dim)).softmax(-1), v).reshape(-1)
+        got = out[b].float()
+        if b == 0:
+            assert want.view(heads, dim)[2:4].isnan().all() == (value != float("-inf") or where == "all")
+        assert torch.equal(got.isnan(), want.isnan())
+        # as above: the probabilities' rounding to the type and the result's
+        assert ((got - want).abs()[~want.isnan()] <= 2 * _eps(dt) * v.abs().max() + 1e-5).all()
+
+
+@pytest.mark.parametrize("dt", DT)
 @pytest.mark.parametrize("rows,hidden", [(1, 64), (5, 768), (200, 2048), (3, 8192), (2, 20480), (150, 1032)])
 @pytest.mark.parametrize("ln", [False, True])
 def test_add_norm(dt, rows, hidden, ln):
