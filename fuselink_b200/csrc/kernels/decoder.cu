@@ -14,6 +14,7 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <math.h>
+#include <initializer_list>
 #include "../common/fl_ptx.cuh"
 
 namespace fl {
@@ -534,6 +535,13 @@ static unsigned grid_for(long long items) {
   return (unsigned)(ctas < 1 ? 1 : ctas > 148ll * 64 ? 148 * 64 : ctas);
 }
 
+// every access is 16 bytes wide; a null pointer is an argument that is not given
+static bool aligned(std::initializer_list<const void*> pointers) {
+  uintptr_t all = 0;
+  for (const void* p : pointers) all |= reinterpret_cast<uintptr_t>(p);
+  return (all & 15) == 0;
+}
+
 #define FL_DEC_TYPES(dtype, ...)                                             \
   do {                                                                       \
     if ((dtype) == FL_DEC_BF16) { using T = __nv_bfloat16; __VA_ARGS__; }    \
@@ -544,6 +552,7 @@ static unsigned grid_for(long long items) {
 extern "C" int fl_dec_embed(int dtype, const long long* tokens, const long long* pos, const void* embed, const void* pos_embed, void* x,
                             long long rows, int hidden, int seq, int offset, long long vocab, long long pos_rows, cudaStream_t stream) {
   if (hidden % 8 || hidden < 8 || rows < 0 || (pos == nullptr && pos_embed != nullptr && seq < 1)) return -2;
+  if (!aligned({embed, pos_embed, x})) return -4;
   if (rows == 0) return 0;
   FL_DEC_TYPES(dtype, (fl::dec_embed_kernel<T><<<grid_for(rows * (hidden / 8)), 256, 0, stream>>>(
                           tokens, pos, (const T*)embed, (const T*)pos_embed, (T*)x, rows, hidden / 8, seq < 1 ? 1 : seq, offset, vocab, pos_rows)));
@@ -553,6 +562,7 @@ extern "C" int fl_dec_embed(int dtype, const long long* tokens, const long long*
 extern "C" int fl_dec_add_norm(int dtype, void* x, const void* y, const void* y_bias, const void* w, const void* b, void* h, long long rows,
                                int hidden, float eps, cudaStream_t stream) {
   if (hidden % 8 || hidden < 8 || hidden > 8 * 4 * 1024 || rows < 0 || rows > 0x7fffffffll) return -2;
+  if (!aligned({x, y, y_bias, w, b, h})) return -4;
   if (rows == 0) return 0;
   const int vecs = hidden / 8;
   // few rows: one vector per thread, as many threads as that takes; many rows: two per thread keeps more CTAs resident
@@ -567,6 +577,7 @@ extern "C" int fl_dec_add_norm(int dtype, void* x, const void* y, const void* y_
 extern "C" int fl_dec_qkv(int dtype, void* qkv, const void* bias, const float* rope, long long rope_rows, const long long* pos,
                           long long rows, int seq, int heads, int dim, const FlPagedKv* kv, cudaStream_t stream) {
   if (dim % 16 || dim < 16 || heads < 1 || kv->heads < 1 || kv->block_size < 1 || rows < 0 || (pos == nullptr && seq < 1)) return -2;
+  if (!aligned({qkv, bias, kv->k, kv->v})) return -4;
   if (rows == 0) return 0;
   FL_DEC_TYPES(dtype, (fl::dec_qkv_kernel<T><<<grid_for(rows * (heads + 2 * kv->heads) * (dim / 16)), 256, 0, stream>>>(
                           (T*)qkv, (const T*)bias, rope, rope_rows, pos, rows, seq, heads, dim, *kv)));
@@ -575,6 +586,7 @@ extern "C" int fl_dec_qkv(int dtype, void* qkv, const void* bias, const float* r
 
 extern "C" int fl_dec_act(int dtype, int kind, const void* h, const void* bias, void* out, long long rows, int ffn, cudaStream_t stream) {
   if (ffn % 8 || ffn < 8 || rows < 0) return -2;
+  if (!aligned({h, bias, out})) return -4;
   if (rows == 0) return 0;
   const unsigned grid = grid_for(rows * (ffn / 8));
 #define FL_ACT(K) fl::dec_act_kernel<T, K><<<grid, 256, 0, stream>>>((const T*)h, (const T*)bias, (T*)out, rows, ffn)
@@ -610,8 +622,10 @@ static int launch_attention(const void* q, long long q_stride, const long long* 
 // idle (a few requests with long contexts) the CTAs get eight warps instead of four.
 extern "C" int fl_dec_attention(int dtype, const void* q, long long q_stride, const long long* pos, const FlPagedKv* kv, void* out,
                                 int batch, int heads, int dim, cudaStream_t stream) {
-  if (batch < 1 || batch > 65535 || kv->heads < 1 || heads % kv->heads || dim < 8 || dim % 8 || dim > 128 || kv->layout != FL_KV_LBSHD)
+  if (batch < 1 || batch > 65535 || kv->heads < 1 || heads % kv->heads || dim < 8 || dim % 8 || dim > 128 || kv->layout != FL_KV_LBSHD ||
+      q_stride % 8)
     return -2;
+  if (!aligned({q, kv->k, kv->v})) return -4;
   const int group = heads / kv->heads, gparts = (group + fl::ATT_G - 1) / fl::ATT_G;
   const long long units = (long long)batch * kv->heads * gparts, cap = (long long)kv->table_stride * kv->block_size;
   long long splits = 4 * 148 / units;

@@ -14,6 +14,8 @@ struct FlPagedKv {
   int layout, layer, layers, num_blocks, block_size, heads;
 };
 
+// Tensors of the model's type start at a multiple of 16 bytes (the logits of the greedy choice may start anywhere); otherwise the
+// call returns -4 and launches nothing.
 #ifdef __cplusplus
 extern "C" {
 #endif

@@ -18,6 +18,7 @@ Paged KV layouts (block = `block_size` tokens):
 """
 from __future__ import annotations
 
+import itertools
 from dataclasses import dataclass
 from typing import Callable, Optional
 
@@ -185,11 +186,28 @@ class LlamaShard(torch.nn.Module):
 
     # ------------------------------------------------------------------------------------------- fused passes
     def _fused(self, pool: torch.Tensor) -> bool:
-        """Whether csrc/kernels/decoder.cu takes this shard: 16-bit weights and pools on the GPU, rows and heads in whole
-        16-byte vectors (a rotated head in two halves of them), heads of at most 128."""
+        """Whether csrc/kernels/decoder.cu takes this shard."""
+        return self.embed.is_cuda and self._fits(pool)
+
+    def _fits(self, pool: torch.Tensor) -> bool:
+        """16-bit weights and pools, rows and heads in whole 16-byte vectors (a rotated head in two halves of them), heads of at
+        most 128; and what the kernels read themselves (everything but the matrices) of one type on one device, contiguous, from
+        a multiple of 16 bytes on.  Asked on every call, since the weights are plain attributes: 30 to 60 us, beside 2 ms for the
+        launches of an eager decoding step."""
         cfg, w = self.cfg, self.embed
-        return (w.is_cuda and pool.is_cuda and w.dtype == pool.dtype and w.dtype in (torch.bfloat16, torch.float16)
-                and cfg.hidden % 8 == 0 and cfg.hidden <= 32768 and self.f_local % 8 == 0 and cfg.head_dim % 16 == 0 and cfg.head_dim <= 128)
+        dtype, device = w.dtype, w.device
+        if not (dtype in (torch.bfloat16, torch.float16) and cfg.hidden % 8 == 0 and cfg.hidden <= 32768 and self.f_local % 8 == 0
+                and cfg.head_dim % 16 == 0 and cfg.head_dim <= 128):
+            return False
+        for t in itertools.chain((w, pool, self.pos_embed, self.final_norm, self.final_norm_b), self.n1, self.n1b, self.n2, self.n2b,
+                                 self.bqkv, self.bo, self.b13, self.b2):
+            if t is not None and (t.data_ptr() & 15 or t.dtype != dtype or t.device != device or not t.is_contiguous()):
+                return False
+        return True
+
+    @staticmethod
+    def _same_kind(t: torch.Tensor, as_: torch.Tensor) -> bool:
+        return t.dtype == as_.dtype and t.device == as_.device and t.is_contiguous() and t.data_ptr() % 16 == 0
 
     def _rope_table(self, positions: int):
         """fp32 [positions, D]: the cosines, then the sines, of every position's angles; made once for at least 4096
@@ -283,7 +301,7 @@ class LlamaShard(torch.nn.Module):
         B, S = tokens.shape
         bs, D, L = cfg.block_size, cfg.head_dim, cfg.layers
         assert S % bs == 0
-        if self._fused(k_pool):
+        if self._fused(k_pool) and self._same_kind(v_pool, k_pool):
             return self._prefill_fused(tokens, k_pool, v_pool, block_table, on_layer_done, last_pos)
         nblk = S // bs
         kp = k_pool.view(-1, L, self.kvh_local, bs, D)
@@ -314,7 +332,7 @@ class LlamaShard(torch.nn.Module):
         cfg = self.cfg
         B = tokens.shape[0]
         bs, D, L = cfg.block_size, cfg.head_dim, cfg.layers
-        if self._fused(k_pool):
+        if self._fused(k_pool) and self._same_kind(v_pool, k_pool):
             return self._decode_fused(tokens, positions, k_pool, v_pool, block_table, num_pool_blocks)
         kp = k_pool.view(L, num_pool_blocks, bs, self.kvh_local, D)
         vp = v_pool.view(L, num_pool_blocks, bs, self.kvh_local, D)

@@ -1,6 +1,8 @@
 """The fused route of the decoder (models/llama.py over csrc/kernels/decoder.cu) takes the calls that the operation-by-operation
 route takes and answers alike: both on host memory, the kernels as plain PyTorch with the same arguments."""
+import ctypes
 import math
+import os
 
 import pytest
 import torch
@@ -120,3 +122,55 @@ def test_a_position_outside_the_prompt_is_an_error(last_pos, route):
         route(r)
         with pytest.raises(IndexError):
             _prefill(net, _tokens(net, 3, 32), last_pos=last_pos)
+
+
+def _shifted(t):
+    """The same values from an address that is a multiple of 2 bytes only."""
+    flat = torch.empty(t.numel() + 9, dtype=t.dtype)
+    first = next(i for i in range(1, 9) if flat[i:].data_ptr() % 16 == 2)
+    flat[first:first + t.numel()] = t.reshape(-1)
+    return flat[first:first + t.numel()].view(t.shape)
+
+
+@pytest.mark.parametrize("name", ["embed", "pos_embed", "final_norm", "final_norm_b", "n1", "n1b", "n2", "n2b", "bqkv", "bo", "b13", "b2", "pool"])
+def test_tensors_the_kernels_do_not_take_go_the_general_route(name):
+    pool = torch.zeros(64, dtype=torch.bfloat16)
+    for change in (_shifted, lambda t: t.float(), lambda t: torch.stack([t, t], -1)[..., 0]):
+        net = _net("tiny_opt")
+        assert net._fits(pool)
+        if name == "pool":
+            assert not net._fits(change(pool)) and not net._same_kind(change(pool), pool)
+        elif isinstance(getattr(net, name), list):
+            getattr(net, name)[1] = change(getattr(net, name)[1])
+            assert not net._fits(pool)
+        else:
+            setattr(net, name, change(getattr(net, name)))
+            assert not net._fits(pool)
+
+
+def test_c_entries_refuse_addresses_they_cannot_read():
+    """Every pointer in turn off its 16 bytes; nothing is launched for zero rows, so the addresses are never used."""
+    from fuselink_b200 import build
+    lib = ctypes.CDLL(os.path.join(build.LIB, "libfuselink.so"))
+    P, I, LL, F32 = ctypes.c_void_p, ctypes.c_int, ctypes.c_longlong, ctypes.c_float
+
+    class Kv(ctypes.Structure):
+        _fields_ = [("k", P), ("v", P), ("block_table", P)] + [(n, I) for n in ("table_stride", "layout", "layer", "layers", "num_blocks", "block_size", "heads")]
+
+    def kv(k, v):
+        return ctypes.byref(Kv(k, v, 0x1000, 4, 1, 0, 1, 8, 16, 2))
+
+    calls = [
+        (3, lambda p: lib.fl_dec_embed(I(0), P(8), P(8), P(p[0]), P(p[1]), P(p[2]), LL(0), I(64), I(1), I(0), LL(10), LL(10), P())),
+        (6, lambda p: lib.fl_dec_add_norm(I(0), *map(P, p), LL(0), I(64), F32(1e-5), P())),
+        (4, lambda p: lib.fl_dec_qkv(I(0), P(p[0]), P(p[1]), P(), LL(0), P(8), LL(0), I(1), I(2), I(64), kv(p[2], p[3]), P())),
+        (3, lambda p: lib.fl_dec_act(I(0), I(1), *map(P, p), LL(0), I(64), P())),
+    ]
+    for n, call in calls:
+        assert call([0x100000] * n) == 0
+        for i in range(n):
+            for off in (2, 4, 8):
+                assert call([0x100000 + (off if k == i else 0) for k in range(n)]) == -4
+    attention = lambda q, k, v: lib.fl_dec_attention(I(0), P(q), LL(384), P(8), kv(k, v), P(0x100000), I(1), I(2), I(64), P())
+    for bad in ((2, 0, 0), (0, 4, 0), (0, 0, 8)):
+        assert attention(*(0x100000 + b for b in bad)) == -4
