@@ -70,11 +70,17 @@ __device__ __forceinline__ uint4 pack8(const float* v) {
 template <typename T>
 __device__ __forceinline__ void load8(const T* p, float* v) { unpack8<T>(ld_v4(p), v); }
 
+// An index that framework indexing would refuse: the access is skipped and the status word says which it was.  A plain store, since
+// the word may be in host memory and any one of the values will do.
+__device__ __forceinline__ void note(int* status, int what) {
+  if (status != nullptr) *reinterpret_cast<volatile int*>(status) = what;
+}
+
 // ---- embedding --------------------------------------------------------------------------------------------------------
 template <typename T>
 __global__ void __launch_bounds__(256) dec_embed_kernel(const long long* tokens, const long long* pos, const T* embed, const T* pos_embed,
                                                         T* x, long long rows, int vecs, int seq, int offset, long long vocab,
-                                                        long long pos_rows) {
+                                                        long long pos_rows, int* status) {
   const long long total = rows * vecs;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
     const long long n = i / vecs;
@@ -83,9 +89,13 @@ __global__ void __launch_bounds__(256) dec_embed_kernel(const long long* tokens,
     if (tok < 0) tok += vocab;                      // as indexing does
     uint4 u = make_uint4(0, 0, 0, 0);
     if (tok >= 0 && tok < vocab) u = ld_v4(embed + (tok * vecs + c) * 8);
+    else note(status, FL_DEC_BAD_TOKEN);
     if (pos_embed != nullptr) {
-      const long long p = (pos ? pos[n] : n % seq) + offset;
-      if (p >= 0 && p < pos_rows) {
+      long long p = (pos ? pos[n] : n % seq) + offset;
+      if (p < 0) p += pos_rows;
+      if (p < 0 || p >= pos_rows) {
+        note(status, FL_DEC_BAD_POSITION);
+      } else {
         float a[8], b[8];
         unpack8<T>(u, a);
         load8<T>(pos_embed + (p * vecs + c) * 8, b);
@@ -211,11 +221,12 @@ __global__ void __launch_bounds__(256) dec_qkv_kernel(T* qkv, const T* bias, con
 #pragma unroll
       for (int j = 0; j < 8; ++j) b[j] = Num<T>::round(b[j] + e[j]);
     }
-    if (rotate && at >= 0 && at < rope_rows) {
-      const float* cs = rope + at * dim + c;          // row: half cosines, half sines
+    const long long turn = at < 0 ? -at : at;
+    if (rotate && turn < rope_rows) {
+      const float* cs = rope + turn * dim + c;        // row: half cosines, half sines
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
-        const float co = cs[j], si = cs[half + j], x1 = a[j], x2 = b[j];
+        const float co = cs[j], si = at < 0 ? -cs[half + j] : cs[half + j], x1 = a[j], x2 = b[j];
         a[j] = x1 * co - x2 * si;
         b[j] = x2 * co + x1 * si;
       }
@@ -228,11 +239,14 @@ __global__ void __launch_bounds__(256) dec_qkv_kernel(T* qkv, const T* bias, con
     if (is_q) continue;
     const long long req = pos ? n : n / seq;
     const int kh = hd - heads - (is_v ? kv.heads : 0);
-    const long long page = at / kv.block_size;
-    if (at < 0 || page >= kv.table_stride) continue;
-    const int slot = (int)(at - page * kv.block_size);
-    const int blk = kv.block_table[req * kv.table_stride + page];
-    if (blk < 0 || blk >= kv.num_blocks) continue;
+    long long page = at / kv.block_size;
+    int slot = (int)(at - page * kv.block_size);
+    if (slot < 0) { slot += kv.block_size; page -= 1; }
+    if (page < 0) page += kv.table_stride;            // negative positions and page ids count from the end, as indexing does
+    if (page < 0 || page >= kv.table_stride) { note(kv.status, FL_DEC_BAD_POSITION); continue; }
+    int blk = kv.block_table[req * kv.table_stride + page];
+    if (blk < 0) blk += kv.num_blocks;
+    if (blk < 0 || blk >= kv.num_blocks) { note(kv.status, FL_DEC_BAD_PAGE); continue; }
     const long long row = kv.layout == FL_KV_BLHSD
                               ? (((long long)blk * kv.layers + kv.layer) * kv.heads + kh) * kv.block_size + slot
                               : (((long long)kv.layer * kv.num_blocks + blk) * kv.block_size + slot) * kv.heads + kh;
@@ -326,6 +340,7 @@ __global__ void __launch_bounds__(W * 32, 16 / W) dec_attention_kernel(const T* 
       blk = tok < last ? table[tok / bs] : -1;
       slot = tok % bs;
     }
+    if (blk < 0) blk += kv.num_blocks;
     if (tok >= last || blk < 0 || blk >= kv.num_blocks) return nullptr;
     return reinterpret_cast<const T*>(pool) + (((long long)kv.layer * kv.num_blocks + blk) * bs + slot) * tok_stride + kh * dim;
   };
@@ -362,9 +377,13 @@ __global__ void __launch_bounds__(W * 32, 16 / W) dec_attention_kernel(const T* 
 
   for (int base = first; base < last; base += 16) {
     uint4 vr[4][VC];
+    unsigned there = 0;                            // bit 2 p + e: the token of s[p][e] is in the context and its page in the pool
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      const T* r = row_of(kv.v, blk, base, base + 2 * t + (i & 1) + 8 * (i >> 1));
+      const int tok = base + 2 * t + (i & 1) + 8 * (i >> 1);
+      const T* r = row_of(kv.v, blk, base, tok);
+      if (r != nullptr) there |= 1u << i;
+      else if (tok < last) note(kv.status, FL_DEC_BAD_PAGE);
 #pragma unroll
       for (int c = 0; c < VC; ++c) {
         const int d = 64 * c + 8 * g;
@@ -382,7 +401,7 @@ __global__ void __launch_bounds__(W * 32, 16 / W) dec_attention_kernel(const T* 
         Num<T>::mma(s[p], qa[j][2], qa[j][3], kr[p][j].z, kr[p][j].w);
       }
 #pragma unroll
-      for (int e = 0; e < 2; ++e) s[p][e] = base + 8 * p + 2 * t + e < last ? s[p][e] * scale_log2 : -INFINITY;
+      for (int e = 0; e < 2; ++e) s[p][e] = there >> (2 * p + e) & 1 ? s[p][e] * scale_log2 : -INFINITY;
     }
     blk = blk_next;
     blk_next = page_of(base + 32);
@@ -550,12 +569,14 @@ static bool aligned(std::initializer_list<const void*> pointers) {
   } while (0)
 
 extern "C" int fl_dec_embed(int dtype, const long long* tokens, const long long* pos, const void* embed, const void* pos_embed, void* x,
-                            long long rows, int hidden, int seq, int offset, long long vocab, long long pos_rows, cudaStream_t stream) {
+                            long long rows, int hidden, int seq, int offset, long long vocab, long long pos_rows, int* status,
+                            cudaStream_t stream) {
   if (hidden % 8 || hidden < 8 || rows < 0 || (pos == nullptr && pos_embed != nullptr && seq < 1)) return -2;
   if (!aligned({embed, pos_embed, x})) return -4;
   if (rows == 0) return 0;
   FL_DEC_TYPES(dtype, (fl::dec_embed_kernel<T><<<grid_for(rows * (hidden / 8)), 256, 0, stream>>>(
-                          tokens, pos, (const T*)embed, (const T*)pos_embed, (T*)x, rows, hidden / 8, seq < 1 ? 1 : seq, offset, vocab, pos_rows)));
+                          tokens, pos, (const T*)embed, (const T*)pos_embed, (T*)x, rows, hidden / 8, seq < 1 ? 1 : seq, offset, vocab, pos_rows,
+                          status)));
   return (int)cudaGetLastError();
 }
 

@@ -7,11 +7,17 @@
 enum FlDecDtype : int { FL_DEC_BF16 = 0, FL_DEC_FP16 = 1 };
 enum FlDecAct : int { FL_ACT_SILU_GATED = 0, FL_ACT_RELU = 1, FL_ACT_GELU_TANH = 2 };
 
-// Where the keys and values of a token go.  Layouts are those of kv_pack.cuh; a page id outside the pool is skipped.
+// What a kernel writes to the status word (device memory or mapped host memory, or null) when an index is outside its table; the
+// access is skipped: a row of zeros for the token, no position added, no page written, the page left out of the attention.
+// Negative indices count from the end.
+enum FlDecStatus : int { FL_DEC_BAD_TOKEN = 1, FL_DEC_BAD_POSITION = 2, FL_DEC_BAD_PAGE = 3 };
+
+// Where the keys and values of a token go.  Layouts are those of kv_pack.cuh.
 struct FlPagedKv {
   void* k; void* v;
   const int* block_table; int table_stride;   // [batch][table_stride] page ids
   int layout, layer, layers, num_blocks, block_size, heads;
+  int* status;
 };
 
 // Tensors of the model's type start at a multiple of 16 bytes (the logits of the greedy choice may start anywhere); otherwise the
@@ -21,7 +27,7 @@ extern "C" {
 #endif
 // x[n] = embed[tokens[n]] (+ pos_embed[pos + offset]); pos: positions, or null for n % seq
 int fl_dec_embed(int dtype, const long long* tokens, const long long* pos, const void* embed, const void* pos_embed, void* x,
-                 long long rows, int hidden, int seq, int offset, long long vocab, long long pos_rows, cudaStream_t stream);
+                 long long rows, int hidden, int seq, int offset, long long vocab, long long pos_rows, int* status, cudaStream_t stream);
 // x += y (+ y_bias) where y is given; h = norm(x) * w (+ b): RMS norm without b, layer norm with it
 int fl_dec_add_norm(int dtype, void* x, const void* y, const void* y_bias, const void* w, const void* b, void* h, long long rows,
                     int hidden, float eps, cudaStream_t stream);

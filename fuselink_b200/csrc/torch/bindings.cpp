@@ -267,7 +267,7 @@ static const long long* dec_i64(const c10::optional<torch::Tensor>& t, int64_t n
   return reinterpret_cast<const long long*>(t->data_ptr<int64_t>());
 }
 static FlPagedKv dec_kv(torch::Tensor k_pool, torch::Tensor v_pool, torch::Tensor table, int64_t layout, int64_t layer, int64_t layers,
-                        int64_t num_blocks, int64_t block_size, int64_t kv_heads, int64_t dim) {
+                        int64_t num_blocks, int64_t block_size, int64_t kv_heads, int64_t dim, int64_t status_addr) {
   TORCH_CHECK(k_pool.is_cuda() && v_pool.is_cuda() && k_pool.is_contiguous() && v_pool.is_contiguous(), "pools: contiguous on the GPU");
   TORCH_CHECK(table.is_cuda() && table.scalar_type() == torch::kInt32 && table.is_contiguous() && table.dim() == 2, "block_table: [batch, blocks] int32");
   TORCH_CHECK(layer >= 0 && layer < layers && block_size > 0, "layer out of range");
@@ -278,10 +278,11 @@ static FlPagedKv dec_kv(torch::Tensor k_pool, torch::Tensor v_pool, torch::Tenso
   kv.block_table = table.data_ptr<int>(); kv.table_stride = (int)table.size(1);
   kv.layout = (int)layout; kv.layer = (int)layer; kv.layers = (int)layers; kv.num_blocks = (int)num_blocks;
   kv.block_size = (int)block_size; kv.heads = (int)kv_heads;
+  kv.status = reinterpret_cast<int*>(status_addr);
   return kv;
 }
 static void dec_embed(torch::Tensor tokens, c10::optional<torch::Tensor> pos, torch::Tensor embed, c10::optional<torch::Tensor> pos_embed,
-                      torch::Tensor x, int64_t seq, int64_t offset) {
+                      torch::Tensor x, int64_t seq, int64_t offset, int64_t status_addr) {
   const int dt = dec_dtype(x);
   const int64_t rows = tokens.numel(), H = embed.size(1);
   TORCH_CHECK(embed.scalar_type() == x.scalar_type() && embed.is_contiguous() && x.is_contiguous() && x.numel() == rows * H, "x: [rows, hidden] like embed");
@@ -289,7 +290,7 @@ static void dec_embed(torch::Tensor tokens, c10::optional<torch::Tensor> pos, to
   c10::cuda::CUDAGuard guard(x.device());
   check_rc(fl_dec_embed(dt, dec_i64(tokens, rows, "tokens: int64"), dec_i64(pos, rows, "positions: int64"), embed.data_ptr(), opt_ptr(pos_embed),
                         x.data_ptr(), rows, (int)H, (int)seq, (int)offset, embed.size(0), pos_embed.has_value() ? pos_embed->size(0) : 0,
-                        cur_stream()), "fl_dec_embed");
+                        reinterpret_cast<int*>(status_addr), cur_stream()), "fl_dec_embed");
 }
 static void dec_add_norm(torch::Tensor x, c10::optional<torch::Tensor> y, c10::optional<torch::Tensor> y_bias, torch::Tensor w,
                          c10::optional<torch::Tensor> b, torch::Tensor h, double eps) {
@@ -303,7 +304,8 @@ static void dec_add_norm(torch::Tensor x, c10::optional<torch::Tensor> y, c10::o
 }
 static void dec_qkv(torch::Tensor qkv, c10::optional<torch::Tensor> bias, c10::optional<torch::Tensor> rope, c10::optional<torch::Tensor> pos,
                     int64_t seq, torch::Tensor k_pool, torch::Tensor v_pool, torch::Tensor table, int64_t layout, int64_t layer,
-                    int64_t layers, int64_t num_blocks, int64_t block_size, int64_t heads, int64_t kv_heads, int64_t dim) {
+                    int64_t layers, int64_t num_blocks, int64_t block_size, int64_t heads, int64_t kv_heads, int64_t dim,
+                    int64_t status_addr) {
   const int dt = dec_dtype(qkv);
   const int64_t width = (heads + 2 * kv_heads) * dim, rows = qkv.numel() / width;
   TORCH_CHECK(qkv.is_contiguous() && qkv.numel() == rows * width, "qkv: [rows, (heads + 2 kv_heads) * dim]");
@@ -313,7 +315,7 @@ static void dec_qkv(torch::Tensor qkv, c10::optional<torch::Tensor> bias, c10::o
               "rope: [positions, dim] fp32");
   dec_like(bias, qkv, width, "bias: [(heads + 2 kv_heads) * dim]");
   c10::cuda::CUDAGuard guard(qkv.device());
-  const FlPagedKv kv = dec_kv(k_pool, v_pool, table, layout, layer, layers, num_blocks, block_size, kv_heads, dim);
+  const FlPagedKv kv = dec_kv(k_pool, v_pool, table, layout, layer, layers, num_blocks, block_size, kv_heads, dim, status_addr);
   check_rc(fl_dec_qkv(dt, qkv.data_ptr(), opt_ptr(bias), rope.has_value() ? rope->data_ptr<float>() : nullptr, rope.has_value() ? rope->size(0) : 0,
                       dec_i64(pos, rows, "positions: int64"), rows, (int)seq, (int)heads, (int)dim, &kv, cur_stream()), "fl_dec_qkv");
 }
@@ -327,14 +329,15 @@ static void dec_act(torch::Tensor h, c10::optional<torch::Tensor> bias, torch::T
   check_rc(fl_dec_act(dt, (int)kind, h.data_ptr(), opt_ptr(bias), out.data_ptr(), rows, (int)F, cur_stream()), "fl_dec_act");
 }
 static void dec_attention(torch::Tensor qkv, torch::Tensor pos, torch::Tensor k_pool, torch::Tensor v_pool, torch::Tensor table, int64_t layer,
-                          int64_t layers, int64_t num_blocks, int64_t block_size, int64_t heads, int64_t kv_heads, int64_t dim, torch::Tensor out) {
+                          int64_t layers, int64_t num_blocks, int64_t block_size, int64_t heads, int64_t kv_heads, int64_t dim, torch::Tensor out,
+                          int64_t status_addr) {
   const int dt = dec_dtype(qkv);
   const int64_t width = (heads + 2 * kv_heads) * dim, batch = qkv.numel() / width;
   TORCH_CHECK(qkv.is_contiguous() && qkv.numel() == batch * width && table.size(0) >= batch, "qkv: [batch, (heads + 2 kv_heads) * dim]");
   TORCH_CHECK(k_pool.scalar_type() == qkv.scalar_type() && v_pool.scalar_type() == qkv.scalar_type(), "pools of the model's type expected");
   dec_like(out, qkv, batch * heads * dim, "out: [batch, heads * dim]");
   c10::cuda::CUDAGuard guard(qkv.device());
-  const FlPagedKv kv = dec_kv(k_pool, v_pool, table, FL_KV_LBSHD, layer, layers, num_blocks, block_size, kv_heads, dim);
+  const FlPagedKv kv = dec_kv(k_pool, v_pool, table, FL_KV_LBSHD, layer, layers, num_blocks, block_size, kv_heads, dim, status_addr);
   check_rc(fl_dec_attention(dt, qkv.data_ptr(), width, dec_i64(pos, batch, "positions: int64"), &kv, out.data_ptr(), (int)batch, (int)heads, (int)dim,
                             cur_stream()), "fl_dec_attention");
 }
@@ -528,15 +531,20 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("barrier", &barrier);
   m.def("embbag", &embbag);
   m.def("kv_pack_send", &kv_pack_send);
-  m.def("dec_embed", &dec_embed);
+  m.def("dec_embed", &dec_embed, py::arg("tokens"), py::arg("pos"), py::arg("embed"), py::arg("pos_embed"), py::arg("x"), py::arg("seq"),
+        py::arg("offset"), py::arg("status_addr") = 0);
   m.def("dec_add_norm", &dec_add_norm);
-  m.def("dec_qkv", &dec_qkv);
+  m.def("dec_qkv", &dec_qkv, py::arg("qkv"), py::arg("bias"), py::arg("rope"), py::arg("pos"), py::arg("seq"), py::arg("k_pool"),
+        py::arg("v_pool"), py::arg("table"), py::arg("layout"), py::arg("layer"), py::arg("layers"), py::arg("num_blocks"),
+        py::arg("block_size"), py::arg("heads"), py::arg("kv_heads"), py::arg("dim"), py::arg("status_addr") = 0);
   m.def("moe_route", &moe_route);
   m.def("moe_route_bwd", &moe_route_bwd);
   m.def("interact_fwd", &interact_fwd);
   m.def("interact_bwd", &interact_bwd);
   m.def("dec_act", &dec_act);
-  m.def("dec_attention", &dec_attention);
+  m.def("dec_attention", &dec_attention, py::arg("qkv"), py::arg("pos"), py::arg("k_pool"), py::arg("v_pool"), py::arg("table"),
+        py::arg("layer"), py::arg("layers"), py::arg("num_blocks"), py::arg("block_size"), py::arg("heads"), py::arg("kv_heads"),
+        py::arg("dim"), py::arg("out"), py::arg("status_addr") = 0);
   m.def("dec_argmax", &dec_argmax);
   m.def("dec_advance", &dec_advance);
   m.def("moe_dispatch", &moe_dispatch);

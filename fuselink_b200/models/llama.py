@@ -90,6 +90,22 @@ def _rope(x, pos, theta):
     return torch.cat([x1 * cos - x2 * sin, x2 * cos + x1 * sin], -1).to(x.dtype)
 
 
+class _Status:
+    """A word in pinned host memory in which the decoder kernels note an index outside its table, so that the host can look at it
+    without waiting for them.  A copied or unpickled shard has a word of its own."""
+    WHAT = {1: "a token outside the vocabulary", 2: "a position outside the position embedding or the block table",
+            3: "a page id outside the pool"}
+
+    def __init__(self):
+        self.word = torch.zeros(1, dtype=torch.int32, pin_memory=torch.cuda.is_available())
+
+    def __deepcopy__(self, memo):
+        return _Status()
+
+    def __reduce__(self):
+        return _Status, ()
+
+
 class LlamaShard(torch.nn.Module):
     """One tensor-parallel shard of the model.  ``tp_group`` is None for TP=1.  Column-parallel tensors (QKV, the first
     MLP matrix and their biases) are split over the shards, row-parallel ones (attention output, second MLP matrix) are
@@ -227,11 +243,29 @@ class LlamaShard(torch.nn.Module):
             tables.append(table)
         return table
 
+    def _status_addr(self) -> int:
+        """Where the kernels note a bad index; 0 (nowhere) if the first call of all is one that is being captured."""
+        st = self.__dict__.get("_status")
+        if st is None:
+            if torch.cuda.is_current_stream_capturing():
+                return 0
+            st = self.__dict__.setdefault("_status", _Status())
+        return st.word.data_ptr()
+
+    def check_status(self) -> None:
+        """Raise IndexError if a kernel met a token, position or page id outside its table since the last call.  Does not wait:
+        behind a synchronisation it covers everything before it.  Every fused call begins with it."""
+        st = self.__dict__.get("_status")
+        what = 0 if st is None else int(st.word)
+        if what:
+            st.word.zero_()
+            raise IndexError(f"decoder: {_Status.WHAT.get(what, what)}")
+
     def _layers_fused(self, x, pos, seq, k_pool, v_pool, table, layout, num_blocks, attend, on_layer_done=None):
         """Every layer on x [rows, hidden]; ``attend(l, qkv)`` returns the attention output [rows, h_local * D].  Returns
         (x, y, bias): the residual stream without the last branch, the branch and its bias (final_norm adds them up)."""
         C, cfg = require_native(), self.cfg
-        rows, kind = x.shape[0], _ACT[cfg.arch]
+        rows, kind, status = x.shape[0], _ACT[cfg.arch], self._status_addr()
         rope = self._rope_table(table.shape[1] * cfg.block_size)
         h = torch.empty_like(x)
         act = torch.empty(rows, self.f_local, dtype=x.dtype, device=x.device)
@@ -240,7 +274,7 @@ class LlamaShard(torch.nn.Module):
             C.dec_add_norm(x, y, bias, self.n1[l], self.n1b[l], h, cfg.eps)
             qkv = h @ self.wqkv[l].t()
             C.dec_qkv(qkv, self.bqkv[l], rope, pos, seq, k_pool, v_pool, table, layout, l, cfg.layers, num_blocks, cfg.block_size,
-                      self.h_local, self.kvh_local, cfg.head_dim)
+                      self.h_local, self.kvh_local, cfg.head_dim, status)
             if on_layer_done is not None:
                 on_layer_done(l)                                                # KV of this layer may leave now
             y = self._allreduce(attend(l, qkv) @ self.wo[l].t())
@@ -258,13 +292,19 @@ class LlamaShard(torch.nn.Module):
         return C.dec_argmax(logits.view(-1, logits.shape[-1])).view(logits.shape[:-1])
 
     def _prefill_fused(self, tokens, k_pool, v_pool, block_table, on_layer_done, last_pos):
+        self.check_status()
         C, cfg = require_native(), self.cfg
         B, S = tokens.shape
         D, hl, kl = cfg.head_dim, self.h_local, self.kvh_local
+        table = block_table[:, : S // cfg.block_size].int().contiguous()
+        if table.shape != (B, S // cfg.block_size):
+            raise RuntimeError(f"block table of {tuple(block_table.shape)} for {B} prompts of {S // cfg.block_size} pages")
+        if self.pos_embed is not None and S + cfg.pos_offset > self.pos_embed.shape[0]:
+            raise IndexError(f"prompts of {S} tokens, {self.pos_embed.shape[0] - cfg.pos_offset} positions")
+        num_blocks = k_pool.view(-1, cfg.layers, kl, cfg.block_size, D).shape[0]
+        v_pool.view(num_blocks, -1)
         x = torch.empty(B * S, cfg.hidden, dtype=self.embed.dtype, device=tokens.device)
-        C.dec_embed(tokens.contiguous(), None, self.embed, self.pos_embed, x, S, cfg.pos_offset)
-        table = block_table[:B, : S // cfg.block_size].int().contiguous()
-        num_blocks = k_pool.numel() // (cfg.layers * kl * cfg.block_size * D)
+        C.dec_embed(tokens.contiguous(), None, self.embed, self.pos_embed, x, S, cfg.pos_offset, self._status_addr())
 
         def attend(l, qkv):
             q, k, v = qkv.view(B, S, hl + 2 * kl, D).split([hl, kl, kl], 2)
@@ -278,15 +318,20 @@ class LlamaShard(torch.nn.Module):
         return self._choose_fused(x.contiguous(), y.contiguous(), bias)
 
     def _decode_fused(self, tokens, positions, k_pool, v_pool, block_table, num_blocks):
-        C, cfg = require_native(), self.cfg
+        self.check_status()
+        C, cfg, status = require_native(), self.cfg, self._status_addr()
         B, D, hl, kl, dev = tokens.shape[0], cfg.head_dim, self.h_local, self.kvh_local, tokens.device
+        if block_table.shape[0] != B:
+            raise RuntimeError(f"block table of {tuple(block_table.shape)} for {B} sequences")
+        for pool in (k_pool, v_pool):
+            pool.view(cfg.layers, num_blocks, cfg.block_size, kl, D)
         positions, table = positions.contiguous(), block_table.int().contiguous()
         x = torch.empty(B, cfg.hidden, dtype=self.embed.dtype, device=dev)
-        C.dec_embed(tokens.contiguous(), positions, self.embed, self.pos_embed, x, 1, cfg.pos_offset)
+        C.dec_embed(tokens.contiguous(), positions, self.embed, self.pos_embed, x, 1, cfg.pos_offset, status)
         out = torch.empty(B, hl * D, dtype=x.dtype, device=dev)
 
         def attend(l, qkv):
-            C.dec_attention(qkv, positions, k_pool, v_pool, table, l, cfg.layers, num_blocks, cfg.block_size, hl, kl, D, out)
+            C.dec_attention(qkv, positions, k_pool, v_pool, table, l, cfg.layers, num_blocks, cfg.block_size, hl, kl, D, out, status)
             return out
 
         return self._choose_fused(*self._layers_fused(x, positions, 1, k_pool, v_pool, table, KV_LBSHD, num_blocks, attend))

@@ -32,6 +32,13 @@ HDR_TOKENS, HDR_LENS, HDR_OUTS = 4, 4 + HDR_MAX_BATCH, 4 + 2 * HDR_MAX_BATCH
 HDR_INTS = 4 + 3 * HDR_MAX_BATCH   # [batch, prompt_len, max_blocks, batch_index] + first tokens + prompt lengths + output lengths
 
 
+def check_model(model) -> None:
+    """Behind a synchronisation: raise what the model's kernels noted (models that note nothing have no ``check_status``)."""
+    check = getattr(model, "check_status", None)
+    if check is not None:
+        check()
+
+
 @dataclass
 class ServeParams:
     """The experiment's knobs (TestParams of the reference, experiments/serving/model.hh:31-49)."""
@@ -182,6 +189,7 @@ class PrefillStage:
         if cuda:
             main.wait_stream(self.side)
         device_sync(self.dev)
+        check_model(self.model)
         kv_bytes = 2 * self.ctx_blocks * p.model.layers * link.page_elems * p.elem_bytes
         return StageReport("prefill", elapsed_ms=e0.elapsed_time(k1), compute_ms=e0.elapsed_time(e1), kv_ms=k0.elapsed_time(k1),
                            kv_bytes=kv_bytes, tokens=p.batch_size * p.input_len)
@@ -256,6 +264,7 @@ class DecodeStage:
             gen = torch.stack(out, 1)
         d1.record()
         device_sync(self.dev)
+        check_model(self.model)
         return gen, d0.elapsed_time(d1)
 
     def run(self) -> StageReport:

@@ -24,7 +24,7 @@ from typing import Callable, Iterable, List, Optional
 
 import torch
 
-from .disagg import HDR_INTS, HDR_LENS, HDR_OUTS, KVLink, ServeParams
+from .disagg import HDR_INTS, HDR_LENS, HDR_OUTS, KVLink, ServeParams, check_model
 from ..models.llama import LlamaShard
 from ..utils.timing import device_sync, timing_event
 
@@ -158,6 +158,7 @@ class OnlinePrefill:
                          final=True, num_ctas=1)
         e2.record()
         device_sync(self.dev)
+        check_model(self.model)
         kv_bytes = int(nblocks.sum().item()) * m.layers * link.page_elems * 2 * p.elem_bytes
         st = BatchStats(B, sum(lens), kv_bytes, HDR_INTS * 8, e1.elapsed_time(e2), e0.elapsed_time(e1))
         self.stats.append(st)
@@ -231,6 +232,7 @@ class OnlineDecode:
                 pos = pos + 1
                 gen.append(tokens)
         device_sync(dev)
+        check_model(self.model)
         # give the pool back: credit word on the SENDER's pad counts batches finished on this pool
         self.done_on[i] += 1
         link.C.put_chunks([(self.credit_pad.addr(), self.credit_pad.addr(self.src), 16,

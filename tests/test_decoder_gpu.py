@@ -143,3 +143,86 @@ def test_activation(kind, ffn):
     C.dec_act(h, None if kind == 0 else b, out, kind)
     want = F.silu(h[:, :ffn]) * h[:, ffn:] if kind == 0 else F.relu(h + b) if kind == 1 else F.gelu(h + b, approximate="tanh")
     assert ((out - want).float().abs() <= 2.02 * 2.0 ** -8 * want.float().abs() + 1e-6).all()
+
+
+def _shard(model):
+    from fuselink_b200.models.llama import MODEL_ZOO, LlamaShard
+    net = LlamaShard(MODEL_ZOO[model], device="cuda", seed=2)
+    cfg = net.cfg
+    pools = lambda blocks: [torch.zeros(blocks * cfg.layers * cfg.kv_heads * cfg.block_size * cfg.head_dim, dtype=torch.bfloat16, device="cuda") for _ in range(2)]
+    return net, pools
+
+
+@pytest.mark.parametrize("model", ["tiny", "tiny_gpt2"])
+@pytest.mark.parametrize("token,table,pos,message", [
+    (1000, [0, 1], 20, "token"), (-1001, [0, 1], 20, "token"), (3, [0, 1], 32, "position"), (3, [0, 1], 1 << 40, "position"), (3, [0, 1], -33, "position"),
+    (3, [0, 2], 20, "page"), (3, [-3, 1], 20, "page"), (3, [1 << 30, 1], 20, "page"),
+])
+def test_an_index_outside_its_table_is_an_error(model, token, table, pos, message):
+    """Skipped and noted by the kernels; raised by the next call or by check_status behind a synchronisation."""
+    net, pools = _shard(model)
+    k, v = pools(2)
+    bt = torch.tensor([table], dtype=torch.int32, device="cuda")
+    tok, at = torch.tensor([token], device="cuda"), torch.tensor([pos], device="cuda")
+    ok = torch.tensor([[0, 1]], dtype=torch.int32, device="cuda"), torch.tensor([5], device="cuda")
+    assert net._fused(k)
+    for look in (net.check_status, lambda: net.decode_step(ok[1], ok[1], k, v, ok[0], 2)):
+        net.decode_step(tok, at, k, v, bt, 2)
+        torch.cuda.synchronize()
+        with pytest.raises(IndexError, match=message):
+            look()
+        net.decode_step(ok[1], ok[1], k, v, ok[0], 2)
+        torch.cuda.synchronize()
+        net.check_status()
+    if message != "position":
+        toks = torch.full((1, 32), 7, device="cuda")
+        toks[0, 9] = token
+        net.prefill(toks, k, v, bt)
+        torch.cuda.synchronize()
+        with pytest.raises(IndexError, match=message):
+            net.check_status()
+
+
+@pytest.mark.parametrize("model", ["tiny", "tiny_gpt2"])
+def test_negative_indices_count_from_the_end(model, monkeypatch):
+    """As in the general route: tokens, pages and positions; the pages written are the same."""
+    from fuselink_b200.models.llama import LlamaShard
+    net, pools = _shard(model)
+    res = []
+    for fused in (True, False):
+        if not fused:
+            monkeypatch.setattr(LlamaShard, "_fused", lambda self, pool: False)
+        k, v = pools(6)
+        toks = torch.arange(-48, 48, device="cuda").view(2, 48)
+        net.prefill(toks, k, v, torch.tensor([[0, -1, 2], [-3, 1, 4]], device="cuda"))
+        kd, vd = pools(6)
+        net.decode_step(torch.tensor([-1, 2, 3], device="cuda"), torch.tensor([-1, -20, 7], device="cuda"), kd, vd,
+                        torch.tensor([[0, 1], [2, 3], [-2, -1]], dtype=torch.int32, device="cuda"), 6)
+        torch.cuda.synchronize()
+        net.check_status()
+        n = kd.numel() // net.cfg.layers                                      # the first layer: not yet behind an attention over nothing
+        res.append((k, v, kd[:n], vd[:n]))
+    for a, b in zip(*res):
+        assert torch.equal(a != 0, b != 0)
+        assert (a.float() - b.float()).norm() <= 4 * _eps(torch.bfloat16) * b.float().norm()
+
+
+@pytest.mark.parametrize("bs", [16, 8])
+def test_attention_leaves_out_a_page_outside_the_pool(bs):
+    from fuselink_b200 import C
+    heads, kv_heads, dim, n, maxblk = 4, 2, 64, 300, 300 // bs + 1
+    kp, vp = (_rand(1, maxblk, bs, kv_heads, dim, dt=torch.bfloat16, seed=s) for s in (1, 2))
+    bt = torch.randperm(maxblk, generator=torch.Generator().manual_seed(3)).view(1, maxblk).int().cuda()
+    bad = bt.clone()
+    bad[0, 3], bad[0, 7] = maxblk, -maxblk - 1
+    qkv = _rand(1, (heads + 2 * kv_heads) * dim, dt=torch.bfloat16, seed=4)
+    out, status = torch.empty(1, heads * dim, dtype=torch.bfloat16, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+    C.dec_attention(qkv, torch.tensor([n - 1], device="cuda"), kp, vp, bad, 0, 1, maxblk, bs, heads, kv_heads, dim, out, status.data_ptr())
+    assert status.item() == 3
+    keep = torch.arange(n, device="cuda")
+    keep = keep[(keep // bs != 3) & (keep // bs != 7)]
+    k, v = (p[0][bt[0].long()].reshape(-1, kv_heads, dim)[keep].float().repeat_interleave(2, 1) for p in (kp, vp))
+    q = qkv[0, : heads * dim].view(heads, dim).float()
+    want = torch.einsum("hn,nhd->hd", (torch.einsum("hd,nhd->hn", q, k) / math.sqrt(dim)).softmax(-1), v).reshape(-1)
+    # the probabilities' rounding to the type and the result's
+    assert (out[0].float() - want).abs().max() <= 2 * _eps(torch.bfloat16) * v.abs().max() + 1e-5

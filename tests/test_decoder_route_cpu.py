@@ -15,7 +15,7 @@ from fuselink_b200.models.llama import KV_BLHSD, MODEL_ZOO, LlamaShard
 class Kernels:
     """What the kernels are specified to do (decoder.cuh), values rounded at the same places."""
 
-    def dec_embed(self, tokens, pos, embed, pos_embed, x, seq, offset):
+    def dec_embed(self, tokens, pos, embed, pos_embed, x, seq, offset, status=0):
         tokens = tokens.reshape(-1)
         x.copy_(embed[tokens])
         if pos_embed is not None:
@@ -26,7 +26,7 @@ class Kernels:
             x += y if y_bias is None else y + y_bias
         h.copy_(llama._rms(x, w, eps) if b is None else llama._ln(x, w, b, eps))
 
-    def dec_qkv(self, qkv, bias, rope, pos, seq, k_pool, v_pool, table, layout, layer, layers, num_blocks, bs, heads, kv_heads, dim):
+    def dec_qkv(self, qkv, bias, rope, pos, seq, k_pool, v_pool, table, layout, layer, layers, num_blocks, bs, heads, kv_heads, dim, status=0):
         rows = torch.arange(qkv.shape[0])
         at, req = (rows % seq, rows // seq) if pos is None else (pos, rows)
         if bias is not None:
@@ -50,7 +50,7 @@ class Kernels:
         else:
             out.copy_(F.relu(h + bias) if kind == 1 else F.gelu(h + bias, approximate="tanh"))
 
-    def dec_attention(self, qkv, pos, k_pool, v_pool, table, layer, layers, num_blocks, bs, heads, kv_heads, dim, out):
+    def dec_attention(self, qkv, pos, k_pool, v_pool, table, layer, layers, num_blocks, bs, heads, kv_heads, dim, out, status=0):
         for b in range(qkv.shape[0]):
             n = int(pos[b]) + 1
             k, v = (p.view(layers, num_blocks, bs, kv_heads, dim)[layer][table[b].long()].reshape(-1, kv_heads, dim)[:n].float()
@@ -124,6 +124,59 @@ def test_a_position_outside_the_prompt_is_an_error(last_pos, route):
             _prefill(net, _tokens(net, 3, 32), last_pos=last_pos)
 
 
+@pytest.mark.parametrize("table", [torch.zeros(3, 1, dtype=torch.int32), torch.zeros(2, 2, dtype=torch.int32)])
+def test_a_block_table_that_does_not_cover_the_prompts_is_an_error(table, route):
+    net = _net("tiny")
+    for r in (FUSED, PLAIN):
+        route(r)
+        with pytest.raises((IndexError, RuntimeError)):
+            _prefill(net, _tokens(net, 3, 32), table, blocks=6)
+
+
+def test_prompts_longer_than_the_position_embedding_are_an_error(route):
+    net = _net("tiny_gpt2")
+    net.pos_embed = net.pos_embed[:31].clone()
+    for r in (FUSED, PLAIN):
+        route(r)
+        with pytest.raises(IndexError):
+            _prefill(net, _tokens(net, 1, 32))
+
+
+def test_pools_of_another_size_are_an_error(route):
+    net = _net("tiny")
+    cfg = net.cfg
+    page = cfg.layers * cfg.kv_heads * cfg.block_size * cfg.head_dim
+    for r in (FUSED, PLAIN):
+        route(r)
+        for k, v in ((2 * page, 2 * page + 8), (2 * page + 8, 2 * page)):
+            pools = torch.zeros(k, dtype=torch.bfloat16), torch.zeros(v, dtype=torch.bfloat16)
+            with pytest.raises(RuntimeError):
+                net.prefill(_tokens(net, 1, 32), *pools, torch.tensor([[0, 1]]))
+            with pytest.raises(RuntimeError):
+                net.decode_step(torch.tensor([1]), torch.tensor([3]), *pools, torch.tensor([[0, 1]]), 2)
+        with pytest.raises((IndexError, RuntimeError)):
+            pools = [torch.zeros(2 * page, dtype=torch.bfloat16) for _ in range(2)]
+            net.decode_step(torch.tensor([1, 2]), torch.tensor([3, 3]), *pools, torch.tensor([[0, 1]]), 2)
+
+
+def test_a_noted_index_is_raised_once(route):
+    import copy
+    import pickle
+    net = _net("tiny")
+    net.check_status()
+    route(FUSED)
+    net._status = llama._Status()
+    for call in (net.check_status, lambda: _prefill(net, _tokens(net, 1, 32))):
+        net._status.word[0] = 2
+        with pytest.raises(IndexError, match="position"):
+            call()
+        net.check_status()
+    net._status.word[0] = 1
+    for other in (copy.deepcopy(net), pickle.loads(pickle.dumps(net))):
+        other.check_status()                        # a word of its own
+        assert other._status.word.data_ptr() != net._status.word.data_ptr()
+
+
 def _shifted(t):
     """The same values from an address that is a multiple of 2 bytes only."""
     flat = torch.empty(t.numel() + 9, dtype=t.dtype)
@@ -155,13 +208,13 @@ def test_c_entries_refuse_addresses_they_cannot_read():
     P, I, LL, F32 = ctypes.c_void_p, ctypes.c_int, ctypes.c_longlong, ctypes.c_float
 
     class Kv(ctypes.Structure):
-        _fields_ = [("k", P), ("v", P), ("block_table", P)] + [(n, I) for n in ("table_stride", "layout", "layer", "layers", "num_blocks", "block_size", "heads")]
+        _fields_ = [("k", P), ("v", P), ("block_table", P)] + [(n, I) for n in ("table_stride", "layout", "layer", "layers", "num_blocks", "block_size", "heads")] + [("status", P)]
 
     def kv(k, v):
         return ctypes.byref(Kv(k, v, 0x1000, 4, 1, 0, 1, 8, 16, 2))
 
     calls = [
-        (3, lambda p: lib.fl_dec_embed(I(0), P(8), P(8), P(p[0]), P(p[1]), P(p[2]), LL(0), I(64), I(1), I(0), LL(10), LL(10), P())),
+        (3, lambda p: lib.fl_dec_embed(I(0), P(8), P(8), P(p[0]), P(p[1]), P(p[2]), LL(0), I(64), I(1), I(0), LL(10), LL(10), P(), P())),
         (6, lambda p: lib.fl_dec_add_norm(I(0), *map(P, p), LL(0), I(64), F32(1e-5), P())),
         (4, lambda p: lib.fl_dec_qkv(I(0), P(p[0]), P(p[1]), P(), LL(0), P(8), LL(0), I(1), I(2), I(64), kv(p[2], p[3]), P())),
         (3, lambda p: lib.fl_dec_act(I(0), I(1), *map(P, p), LL(0), I(64), P())),
