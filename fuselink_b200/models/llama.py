@@ -221,6 +221,24 @@ class LlamaShard(torch.nn.Module):
                 return False
         return True
 
+    def _indices(self, t: torch.Tensor) -> torch.Tensor:
+        """Tokens or positions as the kernels read them: int64, contiguous, on the shard's device."""
+        if t.dtype not in (torch.int64, torch.int32):
+            raise IndexError(f"tokens and positions are int64 or int32, not {t.dtype}")
+        return self._here(t.long())
+
+    def _pages(self, table: torch.Tensor) -> torch.Tensor:
+        if table.dtype != torch.int32:              # an id that int32 does not hold must not become one inside the pool
+            table = table.long().clamp(-2 ** 31, 2 ** 31 - 1).int()
+        return self._here(table)
+
+    def _here(self, t: torch.Tensor) -> torch.Tensor:
+        if t.device != self.embed.device:
+            if t.is_cuda:
+                raise RuntimeError(f"tokens, positions and block table on {self.embed.device} expected, not on {t.device}")
+            t = t.to(self.embed.device)
+        return t.contiguous()
+
     @staticmethod
     def _same_kind(t: torch.Tensor, as_: torch.Tensor) -> bool:
         return t.dtype == as_.dtype and t.device == as_.device and t.is_contiguous() and t.data_ptr() % 16 == 0
@@ -296,7 +314,7 @@ class LlamaShard(torch.nn.Module):
         C, cfg = require_native(), self.cfg
         B, S = tokens.shape
         D, hl, kl = cfg.head_dim, self.h_local, self.kvh_local
-        table = block_table[:, : S // cfg.block_size].int().contiguous()
+        tokens, table = self._indices(tokens), self._pages(block_table[:, : S // cfg.block_size])
         if table.shape != (B, S // cfg.block_size):
             raise RuntimeError(f"block table of {tuple(block_table.shape)} for {B} prompts of {S // cfg.block_size} pages")
         if self.pos_embed is not None and S + cfg.pos_offset > self.pos_embed.shape[0]:
@@ -304,7 +322,7 @@ class LlamaShard(torch.nn.Module):
         num_blocks = k_pool.view(-1, cfg.layers, kl, cfg.block_size, D).shape[0]
         v_pool.view(num_blocks, -1)
         x = torch.empty(B * S, cfg.hidden, dtype=self.embed.dtype, device=tokens.device)
-        C.dec_embed(tokens.contiguous(), None, self.embed, self.pos_embed, x, S, cfg.pos_offset, self._status_addr())
+        C.dec_embed(tokens, None, self.embed, self.pos_embed, x, S, cfg.pos_offset, self._status_addr())
 
         def attend(l, qkv):
             q, k, v = qkv.view(B, S, hl + 2 * kl, D).split([hl, kl, kl], 2)
@@ -320,14 +338,14 @@ class LlamaShard(torch.nn.Module):
     def _decode_fused(self, tokens, positions, k_pool, v_pool, block_table, num_blocks):
         self.check_status()
         C, cfg, status = require_native(), self.cfg, self._status_addr()
-        B, D, hl, kl, dev = tokens.shape[0], cfg.head_dim, self.h_local, self.kvh_local, tokens.device
+        B, D, hl, kl, dev = tokens.shape[0], cfg.head_dim, self.h_local, self.kvh_local, self.embed.device
         if block_table.shape[0] != B:
             raise RuntimeError(f"block table of {tuple(block_table.shape)} for {B} sequences")
         for pool in (k_pool, v_pool):
             pool.view(cfg.layers, num_blocks, cfg.block_size, kl, D)
-        positions, table = positions.contiguous(), block_table.int().contiguous()
+        tokens, positions, table = self._indices(tokens), self._indices(positions), self._pages(block_table)
         x = torch.empty(B, cfg.hidden, dtype=self.embed.dtype, device=dev)
-        C.dec_embed(tokens.contiguous(), positions, self.embed, self.pos_embed, x, 1, cfg.pos_offset, status)
+        C.dec_embed(tokens, positions, self.embed, self.pos_embed, x, 1, cfg.pos_offset, status)
         out = torch.empty(B, hl * D, dtype=x.dtype, device=dev)
 
         def attend(l, qkv):

@@ -15,7 +15,14 @@ from fuselink_b200.models.llama import KV_BLHSD, MODEL_ZOO, LlamaShard
 class Kernels:
     """What the kernels are specified to do (decoder.cuh), values rounded at the same places."""
 
+    @staticmethod
+    def _bound(indices, table=None):
+        """The types that the bindings take."""
+        assert all(t is None or (t.dtype == torch.int64 and t.is_contiguous()) for t in indices)
+        assert table is None or (table.dtype == torch.int32 and table.is_contiguous())
+
     def dec_embed(self, tokens, pos, embed, pos_embed, x, seq, offset, status=0):
+        self._bound([tokens, pos])
         tokens = tokens.reshape(-1)
         x.copy_(embed[tokens])
         if pos_embed is not None:
@@ -27,6 +34,7 @@ class Kernels:
         h.copy_(llama._rms(x, w, eps) if b is None else llama._ln(x, w, b, eps))
 
     def dec_qkv(self, qkv, bias, rope, pos, seq, k_pool, v_pool, table, layout, layer, layers, num_blocks, bs, heads, kv_heads, dim, status=0):
+        self._bound([pos], table)
         rows = torch.arange(qkv.shape[0])
         at, req = (rows % seq, rows // seq) if pos is None else (pos, rows)
         if bias is not None:
@@ -51,6 +59,7 @@ class Kernels:
             out.copy_(F.relu(h + bias) if kind == 1 else F.gelu(h + bias, approximate="tanh"))
 
     def dec_attention(self, qkv, pos, k_pool, v_pool, table, layer, layers, num_blocks, bs, heads, kv_heads, dim, out, status=0):
+        self._bound([pos], table)
         for b in range(qkv.shape[0]):
             n = int(pos[b]) + 1
             k, v = (p.view(layers, num_blocks, bs, kv_heads, dim)[layer][table[b].long()].reshape(-1, kv_heads, dim)[:n].float()
@@ -122,6 +131,43 @@ def test_a_position_outside_the_prompt_is_an_error(last_pos, route):
         route(r)
         with pytest.raises(IndexError):
             _prefill(net, _tokens(net, 3, 32), last_pos=last_pos)
+
+
+def _decode(net, tokens, positions, table, nb):
+    cfg = net.cfg
+    g = torch.Generator().manual_seed(6)
+    pools = [torch.randn(cfg.layers * nb * cfg.block_size * cfg.kv_heads * cfg.head_dim, generator=g).to(net.embed.dtype) for _ in range(2)]
+    return net.decode_step(tokens, positions, *pools, table, nb), *pools
+
+
+@pytest.mark.parametrize("model", ["tiny", "tiny_opt", "tiny_gpt2"])
+@pytest.mark.parametrize("form", [lambda t: t.int(), lambda t: t.long(), lambda t: torch.stack([t, t], -1)[..., 0], lambda t: t.t().contiguous().t()])
+def test_forms_of_tokens_positions_and_tables(model, form, route):
+    """int32 and int64, contiguous or not."""
+    net = _net(model)
+    table = torch.tensor([[3, 0], [1, 5], [4, 2]])
+    res = []
+    for r in (FUSED, PLAIN):
+        route(r)
+        first = _prefill(net, form(_tokens(net, 3, 32)), form(table))
+        step = _decode(net, form(_tokens(net, 3, 1)[:, 0]), form(torch.tensor([30, 0, 17])), form(table), 6)
+        res.append((first[0], *first[1:], *step[1:], step[0].float()))
+    _alike(*res)
+
+
+def test_indices_of_other_types_are_an_error(route):
+    net = _net("tiny")
+    table = torch.tensor([[0, 1]])
+    for r in (FUSED, PLAIN):
+        route(r)
+        for dtype in (torch.float32, torch.int16):
+            with pytest.raises((IndexError, RuntimeError)):
+                _prefill(net, _tokens(net, 1, 32).to(dtype), table)
+            with pytest.raises((IndexError, RuntimeError)):
+                _decode(net, torch.tensor([1]).to(dtype), torch.tensor([5]), table, 2)
+        for bad in (1 << 32, -(1 << 32) + 1):
+            with pytest.raises(IndexError):
+                _prefill(net, _tokens(net, 1, 32), torch.tensor([[0, bad]]))
 
 
 @pytest.mark.parametrize("table", [torch.zeros(3, 1, dtype=torch.int32), torch.zeros(2, 2, dtype=torch.int32)])
