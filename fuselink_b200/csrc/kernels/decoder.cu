@@ -534,14 +534,16 @@ __global__ void __launch_bounds__(1024) dec_argmax_kernel(const T* logits, long 
   }
 }
 
-__global__ void dec_advance_kernel(const long long* next, long long* tokens, long long* pos, long long* history, long long pos0, int batch,
-                                   int steps) {
+__global__ void __launch_bounds__(256) dec_advance_kernel(const long long* next, long long* tokens, long long* pos, long long* history,
+                                                          long long* step, int batch, int rows) {
+  const long long k = *step;
   for (int b = threadIdx.x; b < batch; b += blockDim.x) {
-    const long long k = pos[b] - pos0;
-    if (k >= 0 && k < steps) history[k * batch + b] = next[b];
+    if (k >= 0 && k < rows) history[k * batch + b] = next[b];
     tokens[b] = next[b];
     pos[b] += 1;
   }
+  __syncthreads();                          // every thread has read the step
+  if (threadIdx.x == 0) *step = k + 1;
 }
 
 }  // namespace fl
@@ -670,9 +672,9 @@ extern "C" int fl_dec_argmax(int dtype, const void* logits, long long* out, int 
   return (int)cudaGetLastError();
 }
 
-extern "C" int fl_dec_advance(const long long* next, long long* tokens, long long* pos, long long* history, long long pos0, int batch,
-                              int steps, cudaStream_t stream) {
+extern "C" int fl_dec_advance(const long long* next, long long* tokens, long long* pos, long long* history, long long* step, int batch,
+                              int rows, cudaStream_t stream) {
   if (batch < 1) return -2;
-  fl::dec_advance_kernel<<<1, 256, 0, stream>>>(next, tokens, pos, history, pos0, batch, steps);
+  fl::dec_advance_kernel<<<1, 256, 0, stream>>>(next, tokens, pos, history, step, batch, rows);
   return (int)cudaGetLastError();
 }

@@ -41,8 +41,8 @@ int fl_dec_attention(int dtype, const void* q, long long q_stride, const long lo
                      int heads, int dim, cudaStream_t stream);
 // out[row] = index of the largest value of logits[row] (the first of equals; NaN counts as largest)
 int fl_dec_argmax(int dtype, const void* logits, long long* out, int rows, long long vocab, cudaStream_t stream);
-// one decoding step's bookkeeping: history[pos - pos0][b] = next[b]; tokens = next; pos += 1
-int fl_dec_advance(const long long* next, long long* tokens, long long* pos, long long* history, long long pos0, int batch, int steps,
+// one decoding step's bookkeeping: history[step][b] = next[b] where the history has such a row; tokens = next; pos += 1; step += 1
+int fl_dec_advance(const long long* next, long long* tokens, long long* pos, long long* history, long long* step, int batch, int rows,
                    cudaStream_t stream);
 #ifdef __cplusplus
 }

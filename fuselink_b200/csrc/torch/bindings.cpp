@@ -350,13 +350,13 @@ static torch::Tensor dec_argmax(torch::Tensor logits) {
                          cur_stream()), "fl_dec_argmax");
   return out;
 }
-static void dec_advance(torch::Tensor next, torch::Tensor tokens, torch::Tensor pos, torch::Tensor history, int64_t pos0) {
+static void dec_advance(torch::Tensor next, torch::Tensor tokens, torch::Tensor pos, torch::Tensor history, torch::Tensor step) {
   const int64_t B = next.numel();
-  TORCH_CHECK(history.dim() == 2 && history.size(1) == B, "history: [steps, batch]");
+  TORCH_CHECK(history.dim() == 2 && history.size(1) == B, "history: [rows, batch]");
   c10::cuda::CUDAGuard guard(next.device());
   check_rc(fl_dec_advance(dec_i64(next, B, "next: int64"), const_cast<long long*>(dec_i64(tokens, B, "tokens: int64")),
                           const_cast<long long*>(dec_i64(pos, B, "pos: int64")), const_cast<long long*>(dec_i64(history, history.numel(), "history: int64")),
-                          pos0, (int)B, (int)history.size(0), cur_stream()), "fl_dec_advance");
+                          const_cast<long long*>(dec_i64(step, 1, "step: int64")), (int)B, (int)history.size(0), cur_stream()), "fl_dec_advance");
 }
 
 // ------------------------------------------------------------------------------------------------ MoE

@@ -210,9 +210,11 @@ class DecodeStage:
         self.graph = None
         self.g_tokens = torch.zeros(B, dtype=torch.long, device=dev)
         self.g_pos = torch.zeros(B, dtype=torch.long, device=dev)
-        # tokens of every step; the captured step feeds itself: it takes g_tokens at g_pos, notes the result here, puts it
-        # into g_tokens and advances g_pos, so decoding is nothing but replays
-        self.g_hist = torch.zeros(p.num_decoding_step, B, dtype=torch.long, device=dev)
+        # The captured step feeds itself: it takes g_tokens at g_pos, notes the result in row g_step of g_hist, puts it into
+        # g_tokens and advances g_pos and g_step, so decoding is nothing but replays.  Nothing of `p` is in the graph, whose
+        # lengths a caller may change; longer runs than the history has rows for are read out in between.
+        self.g_hist = torch.zeros(max(1, p.num_decoding_step), B, dtype=torch.long, device=dev)
+        self.g_step = torch.zeros(1, dtype=torch.long, device=dev)
 
     def _step(self, tokens, pos):
         link = self.link
@@ -231,7 +233,7 @@ class DecodeStage:
             g = torch.cuda.CUDAGraph()
             with torch.cuda.graph(g):
                 out = self._step(self.g_tokens, self.g_pos)
-                self.link.C.dec_advance(out, self.g_tokens, self.g_pos, self.g_hist, self.p.input_len)
+                self.link.C.dec_advance(out, self.g_tokens, self.g_pos, self.g_hist, self.g_step)
             self.graph = g
         except Exception as e:  # noqa: BLE001 - capture is an optimisation; the eager loop is always valid
             self.graph = None
@@ -253,9 +255,14 @@ class DecodeStage:
         if self.graph is not None:
             self.g_tokens.copy_(tokens)
             self.g_pos.copy_(pos)
-            for _ in range(p.num_decoding_step):
-                self.graph.replay()
-            gen = torch.cat([tokens.unsqueeze(1), self.g_hist.t()], 1)
+            rows = self.g_hist.shape[0]
+            for first in range(0, p.num_decoding_step, rows):
+                n = min(rows, p.num_decoding_step - first)
+                self.g_step.zero_()
+                for _ in range(n):
+                    self.graph.replay()
+                out.append(self.g_hist[:n].clone() if first + n < p.num_decoding_step else self.g_hist[:n])
+            gen = torch.cat([tokens.unsqueeze(1), *(h.t() for h in out[1:])], 1)
         else:
             for _ in range(p.num_decoding_step):
                 tokens = self._step(tokens, pos)

@@ -171,3 +171,29 @@ def test_kv_pack_send_over_page_shapes(H, S, D, layout, batch):
             want[1, di] = s[si, 1].transpose(1, 2)
         assert torch.equal(d, want)
     assert not status.any()
+
+
+@pytest.mark.parametrize("input_len,steps", [(64, 8), (64, 3), (64, 0), (32, 8), (32, 20), (71, 9)])
+def test_decode_stage_follows_its_parameters_after_the_capture(input_len, steps):
+    """Shorter, longer and empty runs from other positions on a stage whose step has been captured: tokens as of an eager stage."""
+    from fuselink_b200.models.llama import MODEL_ZOO, LlamaShard
+    from fuselink_b200.parallel.symm import SymmetricHeap
+    from fuselink_b200.serving.disagg import DecodeStage, KVLink, ServeParams
+    p = ServeParams(model=MODEL_ZOO["tiny"], batch_size=3, input_len=64, num_decoding_step=8)
+    heap, = SymmetricHeap.emulated(1, 32 << 20)
+    try:
+        net = LlamaShard(p.model, device="cuda", seed=1)
+        net.lm_head = net.embed.roll(1, 0).clone()                      # next tokens that win by a margin
+        net.embed.mul_(50)
+        link = KVLink(heap, p, net.kvh_local)
+        for pool in (link.k_pool.local, link.v_pool.local):
+            pool.normal_(generator=torch.Generator(device="cuda").manual_seed(1))
+        stages = [DecodeStage(p, net, link, use_graph=g) for g in (True, False)]
+        first = torch.tensor([5, 900, 31], device="cuda")
+        stages[0].decode(first)
+        assert stages[0].graph is not None
+        p.input_len, p.num_decoding_step = input_len, steps
+        got, want = (s.decode(first + 1)[0] for s in stages)
+        assert got.shape == (3, 1 + steps) and torch.equal(got, want)
+    finally:
+        heap.close()
