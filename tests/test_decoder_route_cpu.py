@@ -247,6 +247,33 @@ def test_tensors_the_kernels_do_not_take_go_the_general_route(name):
             assert not net._fits(pool)
 
 
+@pytest.mark.parametrize("op", ["_embed", "_norm", "_qkv", "_attn_out", "_mlp", "_logits"])
+def test_replaced_operations_go_the_general_route(op):
+    pool = torch.zeros(64, dtype=torch.bfloat16)
+    own = getattr(LlamaShard, op)
+    net = type("Other", (LlamaShard,), {op: lambda self, *a: own(self, *a)})(MODEL_ZOO["tiny"], device="cpu")
+    assert not net._fits(pool)
+    net = type("Same", (LlamaShard,), {"more": 1})(MODEL_ZOO["tiny"], device="cpu")
+    assert net._fits(pool)
+    setattr(net, op, lambda *a: own(net, *a))
+    assert not net._fits(pool)
+
+
+def test_tensor_subclasses_and_autocast_go_the_general_route(monkeypatch):
+    from unittest import mock
+    pool = torch.zeros(64, dtype=torch.bfloat16)
+    net = _net("tiny")
+    monkeypatch.setattr(net, "embed", mock.Mock(is_cuda=True))
+    monkeypatch.setattr(LlamaShard, "_fits", lambda self, pool: True)
+    assert net._fused(pool)
+    monkeypatch.setattr(torch, "is_autocast_enabled", lambda device: device == "cuda")
+    assert not net._fused(pool)
+    monkeypatch.undo()
+    net = _net("tiny")
+    net.n1[0] = net.n1[0].as_subclass(type("Wrapped", (torch.Tensor,), {}))
+    assert not net._fits(pool)
+
+
 def test_c_entries_refuse_addresses_they_cannot_read():
     """Every pointer in turn off its 16 bytes; nothing is launched for zero rows, so the addresses are never used."""
     from fuselink_b200 import build
