@@ -220,20 +220,30 @@ class DLRM(nn.Module):
         return self.top(torch.cat([x, inter], dim=1)).squeeze(-1)
 
     def _fused_dense(self, dense: torch.Tensor) -> bool:
-        """Whether csrc/kernels/interact.cu takes the interaction: fp32 on the GPU, at most 28 vectors of whole 128 columns, and
-        a dense side that is what __init__ made (no hooks, no replaced or converted layers, no override, no autocast), since the
-        first layer of the top MLP is then called through its weight."""
-        if not (dense.is_cuda and dense.dtype == torch.float32 and self.cfg.dim % 128 == 0 and self.cfg.num_tables <= 27
-                and type(self).dense_forward is DLRM.dense_forward and not torch.is_autocast_enabled("cuda")):
+        """Whether csrc/kernels/interact.cu takes the interaction: fp32 on the GPU, at most 28 vectors of whole 128 columns, no
+        autocast, and a dense side that is what __init__ made, since the first layer of the top MLP is then called through its
+        weight and the pooled vectors' gradient does not pass through sparse_backward_launch: no hooks, no replaced or converted
+        layers or methods."""
+        return (dense.is_cuda and dense.dtype == torch.float32 and self.cfg.dim % 128 == 0 and self.cfg.num_tables <= 27
+                and not torch.is_autocast_enabled("cuda") and self._plain_dense() and all(p.is_cuda for p in self.dense_parameters()))
+
+    def _plain_dense(self) -> bool:
+        if any(getattr(type(self), f) is not getattr(DLRM, f) or f in self.__dict__ for f in ("dense_forward", "sparse_backward_launch")):
+            return False
+        if torch.nn.modules.module._has_any_global_hook() or not all(type(m) is nn.Sequential for m in (self.bottom, self.top)):
             return False
         first = self.top[0]
-        return (type(first) is nn.Linear and type(self.top) is nn.Sequential and "dense_forward" not in self.__dict__
-                and not any(m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks for m in (self.top, first))
-                and all(p.dtype == torch.float32 and p.is_cuda for p in self.dense_parameters()))
+        skipped = (self.top, first)                # modules whose __call__ the fused route does not go through
+        return (all(type(m) in (nn.Linear, nn.ReLU) for m in self.bottom) and type(first) is nn.Linear
+                and not any("forward" in m.__dict__ or m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks
+                            for m in skipped)
+                and all(type(p) is nn.Parameter and p.dtype == torch.float32 for p in self.dense_parameters()))
 
     def _dense_forward_fused(self, dense: torch.Tensor, pooled: torch.Tensor) -> torch.Tensor:
         """dense_forward with the gradient of ``pooled`` (over the ranks' mean) written to the buffer the tables' owners read."""
         x = self.bottom(dense).contiguous()
+        if x.data_ptr() % 16:                              # a hook may have put a view of something larger in its place
+            x = x.clone()
         n = self.n_inter + self.cfg.dim
         width = (n + 7) // 8 * 8
         anchor = torch.empty(0, device=x.device, requires_grad=True)

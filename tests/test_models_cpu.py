@@ -302,3 +302,37 @@ def test_tf32_permission_under_both_interfaces(setting, allowed):
     r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
     assert r.returncode == 0, r.stderr
     assert r.stdout.strip() == str(allowed)
+
+
+def test_fused_dense_side_stands_aside_for_what_it_would_skip():
+    """Everything that the fused interaction does not call keeps the general route: replaced layers, methods and forwards, hooks."""
+    from fuselink_b200.models.dlrm import DLRM, DLRMConfig
+    cfg = DLRMConfig(num_tables=3, rows=10, global_batch=4)
+
+    def model(cls=DLRM):
+        return cls(cfg, device="cpu")
+
+    def check(change, plain=False):
+        m = model()
+        undo = change(m)
+        assert m._plain_dense() is plain
+        if undo is not None:
+            undo.remove()
+
+    check(lambda m: None, plain=True)
+    check(lambda m: m.bottom[0].register_forward_hook(lambda *a: None), plain=True)          # called as before
+    for part in (lambda m: m.top, lambda m: m.top[0]):
+        check(lambda m: setattr(part(m), "forward", lambda x: x))
+        check(lambda m: part(m).register_forward_hook(lambda *a: None))
+        check(lambda m: part(m).register_forward_pre_hook(lambda *a: None))
+        check(lambda m: part(m).register_full_backward_hook(lambda *a: None))
+    check(lambda m: torch.nn.modules.module.register_module_forward_hook(lambda *a: None))
+    check(lambda m: setattr(m, "dense_forward", lambda *a: None))
+    check(lambda m: setattr(m, "sparse_backward_launch", lambda *a: None))
+    check(lambda m: m.top.__setitem__(0, torch.nn.Identity()))
+    check(lambda m: setattr(m, "bottom", torch.nn.Identity()))
+    check(lambda m: torch.nn.utils.parametrizations.weight_norm(m.top[0]) and None)
+    check(lambda m: m.top.to(torch.float64) and None)
+    for f in ("dense_forward", "sparse_backward_launch"):
+        assert not model(type("Other", (DLRM,), {f: lambda self, *a: None}))._plain_dense()
+    assert model(type("Same", (DLRM,), {}))._plain_dense()
