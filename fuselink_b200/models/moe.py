@@ -52,9 +52,18 @@ def load_balancing_loss(probs: torch.Tensor, idx: torch.Tensor, num_experts: int
     return (me * ce).sum() * num_experts
 
 
+def _ordinary(t: torch.Tensor) -> bool:
+    """Whether a kernel may read this tensor in place of the framework's operations: no subclass, and neither a function transform
+    (vmap, grad, jvp), forward-mode differentiation, a dispatch mode nor tracing that has to see the operations."""
+    # a batched gradient reaches the backward on a thread without the transform, and shows itself by having no memory
+    return (type(t) in (torch.Tensor, nn.Parameter) and torch._C._has_storage(t) and not torch._C._are_functorch_transforms_active()
+            and torch.autograd.forward_ad._current_level < 0 and torch._C._len_torch_dispatch_stack() == 0
+            and not torch.jit.is_tracing() and not torch.compiler.is_compiling())
+
+
 class _Route(torch.autograd.Function):
-    """(weights, experts as int32 and int64, load-balancing loss) from the router's logits (csrc/kernels/moe_route.cu).  A gradient that is itself to be
-    differentiated is taken through the framework's operations."""
+    """(weights, experts as int32 and int64, load-balancing loss) from the router's logits (csrc/kernels/moe_route.cu).  A gradient
+    that is itself to be differentiated, or a batch of them, is taken through the framework's operations."""
 
     @staticmethod
     def forward(ctx, logits, bias, topk):
@@ -75,6 +84,13 @@ class _Route(torch.autograd.Function):
             outs = ((cw / cw.sum(dim=-1, keepdim=True), dw), (load_balancing_loss(chosen, idx, logits.shape[1]), daux))
             used = [(o, g) for o, g in outs if g is not None]
             return torch.autograd.grad([o for o, _ in used], logits, [g for _, g in used], create_graph=True)[0], None, None
+        if not all(g is None or _ordinary(g) for g in (dw, daux)):            # a batch of gradients (vmap over the backward)
+            T, E = probs.shape
+            d = torch.zeros_like(probs) if daux is None else daux * (E / T) * share.expand(T, E)
+            if dw is not None:
+                total = probs.gather(1, idx.long()).sum(-1, keepdim=True)
+                d = d.scatter_add(1, idx.long(), (dw - (dw * w).sum(-1, keepdim=True)) / total)
+            return (probs * (d - (probs * d).sum(-1, keepdim=True))).to(logits.dtype), None, None
         f = lambda g: None if g is None else g.contiguous()
         return require_native().moe_route_bwd(probs, w.detach(), idx, share, f(dw), f(daux)), None, None
 
@@ -191,12 +207,12 @@ class MoELayer(nn.Module):
 
     def _fused_route(self, y: torch.Tensor) -> bool:
         """Whether csrc/kernels/moe_route.cu takes these logits: bf16 on the GPU, at most 64 experts and 8 choices, a bias that
-        wants no gradient and no noise."""
+        wants no gradient and no noise, and nothing that follows the operations one by one."""
         E, b = self.cfg.num_experts, self.router_bias
         return (y.is_cuda and y.dtype == torch.bfloat16 and y.dim() == 2 and y.shape[0] > 0 and y.is_contiguous() and E <= 64
                 and self.cfg.topk <= min(8, E) and not (self.training and self.noisy_gate == "rsample")
                 and b.dtype == torch.float32 and b.device == y.device and b.numel() == y.shape[1] == E and b.is_contiguous()
-                and not b.requires_grad)
+                and not b.requires_grad and _ordinary(y))
 
     def _drop(self, w: torch.Tensor, idx: torch.Tensor) -> torch.Tensor:
         """The weights without the choices over an expert's capacity, where the layer drops them."""

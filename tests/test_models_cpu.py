@@ -336,3 +336,28 @@ def test_fused_dense_side_stands_aside_for_what_it_would_skip():
     for f in ("dense_forward", "sparse_backward_launch"):
         assert not model(type("Other", (DLRM,), {f: lambda self, *a: None}))._plain_dense()
     assert model(type("Same", (DLRM,), {}))._plain_dense()
+
+
+def test_routing_kernels_stand_aside_for_transforms_and_tracing():
+    from torch.autograd import forward_ad
+    from torch.fx.experimental.proxy_tensor import make_fx
+
+    from fuselink_b200.models.moe import _ordinary
+    x, seen = torch.randn(3, 4), []
+
+    def f(t):
+        seen.append(_ordinary(t))
+        return t * 2
+
+    f(x)
+    assert seen == [True]
+    del seen[:]
+    torch.vmap(f)(x)
+    torch.func.jvp(f, (x,), (x,))
+    torch.func.grad(lambda t: f(t).sum())(x)
+    with forward_ad.dual_level():
+        f(forward_ad.make_dual(x, x))
+    make_fx(f)(x)
+    torch.jit.trace(f, x, check_trace=False)
+    f(x.as_subclass(type("Wrapped", (torch.Tensor,), {})))
+    assert seen and not any(seen)

@@ -49,3 +49,40 @@ def test_gradients_of_one_output_and_of_the_gradient():
     second, = torch.autograd.grad(twice.float().square().sum(), logits)
     assert torch.isfinite(second.float()).all() and second.abs().max() > 0
     assert torch.autograd.grad(w[:, 0].sum(), logits)[0].abs().max() > 0
+
+
+def test_route_under_transforms(monkeypatch):
+    """vmap, jvp and forward mode through MoELayer.route give what the general route gives; so does an ordinary call, through the kernel."""
+    from torch.autograd import forward_ad
+
+    from fuselink_b200.models.moe import MoELayer
+    from fuselink_b200.ops.moe import MoEConfig
+    layer = MoELayer(MoEConfig(hidden=64, ffn=128, num_experts=8, topk=2, tokens=70), None, 0, 1, device="cuda")
+    layer.requires_grad_(False)
+    g = torch.Generator(device="cuda").manual_seed(1)
+    x, d = ((torch.randn(2, 70, 64, generator=g, device="cuda")).to(torch.bfloat16) for _ in range(2))
+    weights = lambda t: layer.route(t)[0]
+
+    def forward_mode():
+        with forward_ad.dual_level():
+            return forward_ad.unpack_dual(weights(forward_ad.make_dual(x[0], d[0])))
+
+    res = []
+    for general in (False, True):
+        if general:
+            monkeypatch.setattr(MoELayer, "_fused_route", lambda self, y: False)
+        res.append((torch.vmap(weights)(x), *torch.func.jvp(weights, (x[0],), (d[0],)), *forward_mode(), weights(x[0])))
+    for a, b in zip(*res):
+        torch.testing.assert_close(a, b, rtol=1e-5, atol=1e-6)
+
+
+def test_a_batch_of_gradients():
+    from fuselink_b200.models.moe import _Route
+    logits = torch.randn(70, 8, device="cuda").to(torch.bfloat16).requires_grad_(True)
+    w, _, _, aux = _Route.apply(logits, torch.zeros(8, device="cuda"), 2)
+    dw, daux = torch.randn(5, 70, 2, device="cuda"), torch.randn(5, device="cuda")
+    for outs, grads in (((w,), (dw,)), ((aux,), (daux,)), ((w, aux), (dw, daux))):
+        got, = torch.autograd.grad(outs, logits, grads, retain_graph=True, is_grads_batched=True)
+        want = torch.stack([torch.autograd.grad(outs, logits, [g[i] for g in grads], retain_graph=True)[0] for i in range(5)])
+        # one rounding to bf16 in either, of sums in another order
+        torch.testing.assert_close(got, want, rtol=2.0 ** -7, atol=1e-6)
