@@ -194,6 +194,12 @@ extern "C" int fl_embbag_a2a_fwd(const FlEmbBagArgs* a, int num_ctas, cudaStream
   return (int)cudaGetLastError();
 }
 
+extern "C" int fl_embbag_hot_rows(int asked, long long rows, int dim) {
+  const long long fit = 48 * 1024 / ((long long)dim * sizeof(float) * fl::EB_WARPS);     // the default shared-memory limit
+  const long long hot = asked < rows ? asked : rows;
+  return (int)(hot < fit ? hot : fit);
+}
+
 extern "C" int fl_embbag_a2a_bwd_sgd(const FlEmbBagArgs* a, int num_ctas, cudaStream_t stream) {
   int rc = check(a);
   if (rc) return rc;
@@ -204,8 +210,7 @@ extern "C" int fl_embbag_a2a_bwd_sgd(const FlEmbBagArgs* a, int num_ctas, cudaSt
     if (dflt == -2) { const char* e = getenv("FUSELINK_EMBBAG_HOT_ROWS"); dflt = e ? atoi(e) : 24; }
     hot = dflt;
   }
-  if ((long long)hot > a->rows) hot = (int)a->rows;
-  while (hot > 0 && (size_t)hot * a->dim * sizeof(float) * fl::EB_WARPS > 48 * 1024) hot /= 2;    // stays within the default shared-memory limit
+  hot = fl_embbag_hot_rows(hot, a->rows, a->dim);
   if (hot > 0 && a->t_local > 0) {
     // at least about 8 bags per warp: below that its accumulator is cleared and flushed for a handful of updates
     const int most = (a->b_global + 8 * fl::EB_WARPS - 1) / (8 * fl::EB_WARPS), want = 2 * num_ctas / a->t_local;

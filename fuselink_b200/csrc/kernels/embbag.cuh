@@ -28,6 +28,8 @@ struct FlEmbBagArgs {
 #ifdef __cplusplus
 extern "C" {
 #endif
+// how many of the `asked` rows the backward sums per warp: as many as a table has and as fit 48 KB for a CTA's four warps
+int fl_embbag_hot_rows(int asked, long long rows, int dim);
 int fl_embbag_a2a_fwd(const FlEmbBagArgs* a, int num_ctas, cudaStream_t stream);
 int fl_embbag_a2a_bwd_sgd(const FlEmbBagArgs* a, int num_ctas, cudaStream_t stream);
 #ifdef __cplusplus

@@ -361,3 +361,14 @@ def test_routing_kernels_stand_aside_for_transforms_and_tracing():
     torch.jit.trace(f, x, check_trace=False)
     f(x.as_subclass(type("Wrapped", (torch.Tensor,), {})))
     assert seen and not any(seen)
+
+
+def test_embedding_rows_summed_per_warp():
+    """Asking for more rows than fit gives as many as fit, not fewer."""
+    import ctypes
+    from fuselink_b200 import build
+    f = ctypes.CDLL(os.path.join(build.LIB, "libfuselink.so")).fl_embbag_hot_rows
+    f.argtypes = [ctypes.c_int, ctypes.c_longlong, ctypes.c_int]
+    for asked, rows, dim, want in [(24, 10 ** 6, 128, 24), (64, 10 ** 6, 128, 24), (10 ** 6, 10 ** 9, 128, 24), (25, 10 ** 6, 128, 24), (23, 10 ** 6, 128, 23), (24, 5, 128, 5),
+                                   (24, 10 ** 6, 256, 12), (24, 10 ** 6, 384, 8), (24, 10 ** 6, 512, 6), (24, 10 ** 6, 3072, 1), (24, 10 ** 6, 4096, 0), (-1, 10 ** 6, 128, -1)]:
+        assert f(asked, rows, dim) == want
