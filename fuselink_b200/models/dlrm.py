@@ -86,8 +86,9 @@ class _Interaction(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, x, pooled, gpooled, scale, width, iu, anchor):
-        # The kernel's products are tf32, so it needs the caller's leave.  Below 16 vectors, unless they come in fours, the
-        # library answers in fp32 at some batch sizes although it has it; those products stay the library's.
+        # The kernel's products are tf32, so it needs the caller's leave.  Where it is taken its results are the library's bits.
+        # Below 16 vectors, unless they come in fours, the library answers in fp32 at some batch sizes although it has that leave
+        # (5 vectors: at 1000 and from 4096 on, not at 2053); those products stay the library's.
         n = pooled.shape[1] + 1
         if _tf32_allowed() and (n >= 16 or n % 4 == 0):
             out = torch.empty(x.shape[0], width, dtype=x.dtype, device=x.device)

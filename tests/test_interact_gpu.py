@@ -36,6 +36,21 @@ def test_interaction(vectors, batch, dim, pad):
     assert ((dp - 0.5 * dz[:, 1:]).abs() <= 0.5 * bound[:, 1:]).all()
 
 
+@pytest.mark.parametrize("vectors", [4, 8, 12, *range(16, 29)])                     # the counts that a step gives to the kernel
+def test_forward_products_are_the_librarys_bits(vectors, monkeypatch):
+    """What the choice between kernel and library in models/dlrm.py rests on, with the library of CUDA 12.8."""
+    from fuselink_b200 import C
+    monkeypatch.setattr(torch.backends.cuda.matmul, "allow_tf32", True)
+    i, j = torch.triu_indices(vectors, vectors, 1, device="cuda")
+    for batch in (1, 2, 7, 64, 128, 300, 1000, 2053, 4096, 20011, 65536):
+        g = torch.Generator(device="cuda").manual_seed(batch)
+        x, pooled = torch.randn(batch, 128, generator=g, device="cuda"), torch.randn(batch, vectors - 1, 128, generator=g, device="cuda")
+        out = torch.empty(batch, (128 + len(i) + 7) // 8 * 8, device="cuda")
+        C.interact_fwd(x, pooled, out)
+        z = torch.cat([x.unsqueeze(1), pooled], 1)
+        assert torch.equal(out[:, 128:128 + len(i)], torch.bmm(z, z.transpose(1, 2))[:, i, j]), batch
+
+
 @pytest.mark.parametrize("tables,tf32", [(6, True), (7, True), (26, True), (26, False)])       # 7 and 27 vectors, and the two kinds of 8
 def test_train_step_takes_the_general_path_where_the_kernel_does_not_apply(tables, tf32, monkeypatch):
     """Same step through the kernel, with a hook on the top MLP (general path) and with frozen bottom layers."""
