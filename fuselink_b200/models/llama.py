@@ -249,21 +249,24 @@ class LlamaShard(torch.nn.Module):
         return t.dtype == as_.dtype and t.device == as_.device and t.is_contiguous() and t.data_ptr() % 16 == 0
 
     def _rope_table(self, positions: int):
-        """fp32 [positions, D]: the cosines, then the sines, of every position's angles; made once for at least 4096
-        positions.  Tables that were outgrown are kept, since a captured graph may hold their addresses."""
+        """fp32 [positions, D]: the cosines, then the sines, of every position's angles; made once per base, head size and device
+        for at least 4096 positions, for eight of those; a ninth is made on every call.  Tables that were outgrown are kept, since
+        a captured graph may hold their addresses."""
         if self.cfg.arch != "llama":
             return None
-        tables = self.__dict__.setdefault("_rope_tables", [])
+        D, theta, dev = self.cfg.head_dim, self.cfg.rope_theta, self.embed.device
+        made = self.__dict__.setdefault("_rope_tables", {})
+        tables = made.get((theta, D, dev), [])
         if tables and tables[-1].shape[0] >= positions:
             return tables[-1]
         n = max(4096, 1 << (positions - 1).bit_length())
-        D, dev = self.cfg.head_dim, self.embed.device
-        inv = 1.0 / (self.cfg.rope_theta ** (torch.arange(0, D, 2, device=dev, dtype=torch.float32) / D))
+        inv = 1.0 / (theta ** (torch.arange(0, D, 2, device=dev, dtype=torch.float32) / D))
         ang = torch.arange(n, device=dev).float().unsqueeze(-1) * inv
         table = torch.cat([ang.cos(), ang.sin()], -1).contiguous()
-        if not torch.cuda.is_current_stream_capturing():       # another stream may be the next to use it
-            torch.cuda.current_stream(dev).synchronize()
+        if not torch.cuda.is_current_stream_capturing() and (tables or len(made) < 8):
+            torch.cuda.current_stream(dev).synchronize()       # another stream may be the next to use it
             tables.append(table)
+            made[theta, D, dev] = tables
         return table
 
     def _status_addr(self) -> int:

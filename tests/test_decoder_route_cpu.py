@@ -155,6 +155,27 @@ def test_forms_of_tokens_positions_and_tables(model, form, route):
     _alike(*res)
 
 
+def test_another_rotation_base_is_followed(route, monkeypatch):
+    import dataclasses
+    from unittest import mock
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)           # tables are kept
+    monkeypatch.setattr(torch.cuda, "current_stream", mock.Mock())
+    net = _net("tiny")
+    net.cfg = dataclasses.replace(net.cfg)
+    for theta in (10000.0, 500000.0, 10000.0):
+        net.cfg.rope_theta = theta
+        res = []
+        for r in (FUSED, PLAIN):
+            route(r)
+            res.append(_prefill(net, _tokens(net, 2, 48)))
+        _alike(*res)
+    assert len(net._rope_tables) == 2
+    for theta in range(20000, 20010):
+        net.cfg.rope_theta = float(theta)
+        assert torch.equal(net._rope_table(100), net._rope_table(4096))
+    assert len(net._rope_tables) == 8 and all(len(t) == 1 for t in net._rope_tables.values())
+
+
 def test_indices_of_other_types_are_an_error(route):
     net = _net("tiny")
     table = torch.tensor([[0, 1]])
