@@ -246,7 +246,7 @@ class LlamaShard(torch.nn.Module):
 
     @staticmethod
     def _same_kind(t: torch.Tensor, as_: torch.Tensor) -> bool:
-        return t.dtype == as_.dtype and t.device == as_.device and t.is_contiguous() and t.data_ptr() % 16 == 0
+        return t.dtype == as_.dtype and t.device == as_.device and t.numel() == as_.numel() and t.is_contiguous() and t.data_ptr() % 16 == 0
 
     def _rope_table(self, positions: int):
         """fp32 [positions, D]: the cosines, then the sines, of every position's angles; made once per base, head size and device
@@ -315,7 +315,7 @@ class LlamaShard(torch.nn.Module):
         h = torch.empty_like(x)
         C.dec_add_norm(x, y, bias, self.final_norm, self.final_norm_b, h, self.cfg.eps)
         logits = h @ self.lm_head.t()
-        return C.dec_argmax(logits.view(-1, logits.shape[-1])).view(logits.shape[:-1])
+        return C.dec_argmax(logits.flatten(0, -2)).view(logits.shape[:-1])
 
     def _prefill_fused(self, tokens, k_pool, v_pool, block_table, on_layer_done, last_pos):
         self.check_status()
@@ -328,7 +328,6 @@ class LlamaShard(torch.nn.Module):
         if self.pos_embed is not None and S + cfg.pos_offset > self.pos_embed.shape[0]:
             raise IndexError(f"prompts of {S} tokens, {self.pos_embed.shape[0] - cfg.pos_offset} positions")
         num_blocks = k_pool.view(-1, cfg.layers, kl, cfg.block_size, D).shape[0]
-        v_pool.view(num_blocks, -1)
         x = torch.empty(B * S, cfg.hidden, dtype=self.embed.dtype, device=tokens.device)
         C.dec_embed(tokens, None, self.embed, self.pos_embed, x, S, cfg.pos_offset, self._status_addr())
 
@@ -340,7 +339,7 @@ class LlamaShard(torch.nn.Module):
         x, y, bias = self._layers_fused(x, None, S, k_pool, v_pool, table, KV_BLHSD, num_blocks, attend, on_layer_done)
         # indexed per request, so that a position counts from the request's own end or is out of its range
         at = (slice(None), -1) if last_pos is None else (torch.arange(B, device=x.device), last_pos)
-        x, y = (t.view(B, S, -1)[at] for t in (x, y))
+        x, y = (t.view(B, S, cfg.hidden)[at] for t in (x, y))
         return self._choose_fused(x.contiguous(), y.contiguous(), bias)
 
     def _decode_fused(self, tokens, positions, k_pool, v_pool, block_table, num_blocks):
@@ -403,7 +402,7 @@ class LlamaShard(torch.nn.Module):
         cfg = self.cfg
         B = tokens.shape[0]
         bs, D, L = cfg.block_size, cfg.head_dim, cfg.layers
-        if self._fused(k_pool) and self._same_kind(v_pool, k_pool):
+        if 0 < B <= 65535 and self._fused(k_pool) and self._same_kind(v_pool, k_pool):
             return self._decode_fused(tokens, positions, k_pool, v_pool, block_table, num_pool_blocks)
         kp = k_pool.view(L, num_pool_blocks, bs, self.kvh_local, D)
         vp = v_pool.view(L, num_pool_blocks, bs, self.kvh_local, D)

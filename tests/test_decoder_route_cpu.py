@@ -60,6 +60,7 @@ class Kernels:
 
     def dec_attention(self, qkv, pos, k_pool, v_pool, table, layer, layers, num_blocks, bs, heads, kv_heads, dim, out, status=0):
         self._bound([pos], table)
+        assert 1 <= qkv.shape[0] <= 65535
         for b in range(qkv.shape[0]):
             n = int(pos[b]) + 1
             k, v = (p.view(layers, num_blocks, bs, kv_heads, dim)[layer][table[b].long()].reshape(-1, kv_heads, dim)[:n].float()
@@ -153,6 +154,16 @@ def test_forms_of_tokens_positions_and_tables(model, form, route):
         step = _decode(net, form(_tokens(net, 3, 1)[:, 0]), form(torch.tensor([30, 0, 17])), form(table), 6)
         res.append((first[0], *first[1:], *step[1:], step[0].float()))
     _alike(*res)
+
+
+@pytest.mark.parametrize("batch", [0, 65536])
+def test_batches_the_attention_kernel_does_not_take(batch, route):
+    """It takes 1 to 65535 requests; other steps keep the general route."""
+    import dataclasses
+    route(FUSED)
+    net = LlamaShard(dataclasses.replace(MODEL_ZOO["tiny"], layers=1, hidden=64, heads=1, kv_heads=1, ffn=64, vocab=16), device="cpu")
+    toks = torch.zeros(batch, dtype=torch.long)
+    assert _decode(net, toks, toks, torch.zeros(batch, 1, dtype=torch.int32), 1)[0].shape == (batch,)
 
 
 def test_another_rotation_base_is_followed(route, monkeypatch):
