@@ -266,6 +266,21 @@ static const long long* dec_i64(const c10::optional<torch::Tensor>& t, int64_t n
   TORCH_CHECK(t->is_cuda() && t->scalar_type() == torch::kInt64 && t->is_contiguous() && t->numel() == numel, what);
   return reinterpret_cast<const long long*>(t->data_ptr<int64_t>());
 }
+// Whether the kernels may read these tensors (None: not given): plain tensors with memory, of `like`'s type and device, contiguous,
+// from a multiple of 16 bytes on.  Native because a shard asks it about some 200 tensors on every call.
+static bool dec_takes(py::list tensors, torch::Tensor like) {
+  const auto dtype = like.scalar_type();
+  const auto device = like.device();
+  for (py::handle h : tensors) {
+    if (h.is_none()) continue;
+    if (!THPVariable_CheckTypeExact(Py_TYPE(h.ptr()))) return false;
+    const at::Tensor& t = THPVariable_Unpack(h.ptr());
+    if (!t.has_storage() || t.scalar_type() != dtype || t.device() != device || !t.is_contiguous() ||
+        (reinterpret_cast<uintptr_t>(t.const_data_ptr()) & 15))
+      return false;
+  }
+  return true;
+}
 static FlPagedKv dec_kv(torch::Tensor k_pool, torch::Tensor v_pool, torch::Tensor table, int64_t layout, int64_t layer, int64_t layers,
                         int64_t num_blocks, int64_t block_size, int64_t kv_heads, int64_t dim, int64_t status_addr) {
   TORCH_CHECK(k_pool.is_cuda() && v_pool.is_cuda() && k_pool.is_contiguous() && v_pool.is_contiguous(), "pools: contiguous on the GPU");
@@ -531,6 +546,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("barrier", &barrier);
   m.def("embbag", &embbag);
   m.def("kv_pack_send", &kv_pack_send);
+  m.def("dec_takes", &dec_takes);
   m.def("dec_embed", &dec_embed, py::arg("tokens"), py::arg("pos"), py::arg("embed"), py::arg("pos_embed"), py::arg("x"), py::arg("seq"),
         py::arg("offset"), py::arg("status_addr") = 0);
   m.def("dec_add_norm", &dec_add_norm);

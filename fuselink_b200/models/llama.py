@@ -18,7 +18,6 @@ Paged KV layouts (block = `block_size` tokens):
 """
 from __future__ import annotations
 
-import itertools
 from dataclasses import dataclass
 from typing import Callable, Optional
 
@@ -29,7 +28,6 @@ from .._ext import require_native
 
 KV_BLHSD, KV_LBSHD = 0, 1
 _OPERATIONS = ("_embed", "_norm", "_qkv", "_attn_out", "_mlp", "_logits")      # what the fused route does by itself
-_PLAIN = (torch.Tensor, torch.nn.Parameter)
 _ACT = {"llama": 0, "opt": 1, "gpt2": 2}          # FlDecAct
 
 
@@ -211,20 +209,15 @@ class LlamaShard(torch.nn.Module):
         """16-bit weights and pools, rows and heads in whole 16-byte vectors (a rotated head in two halves of them), heads of at
         most 128; what the kernels read themselves (everything but the matrices) plain tensors of one type on one device,
         contiguous, from a multiple of 16 bytes on; and the operations of this class, not of a subclass or replaced on the object.
-        Asked on every call, since all of that is plain attributes: 30 us for 32 layers without biases, 100 us with, on a host
-        that takes 2 ms for the launches of an eager decoding step."""
+        Asked on every call, since all of that is plain attributes."""
         cfg, w = self.cfg, self.embed
-        dtype, device = w.dtype, w.device
-        if not (dtype in (torch.bfloat16, torch.float16) and cfg.hidden % 8 == 0 and cfg.hidden <= 32768 and self.f_local % 8 == 0
+        if not (w.dtype in (torch.bfloat16, torch.float16) and cfg.hidden % 8 == 0 and cfg.hidden <= 32768 and self.f_local % 8 == 0
                 and cfg.head_dim % 16 == 0 and cfg.head_dim <= 128):
             return False
         if any(getattr(type(self), op) is not getattr(LlamaShard, op) or op in self.__dict__ for op in _OPERATIONS):
             return False
-        for t in itertools.chain((w, pool, self.pos_embed, self.final_norm, self.final_norm_b), self.n1, self.n1b, self.n2, self.n2b,
-                                 self.bqkv, self.bo, self.b13, self.b2):
-            if t is not None and (type(t) not in _PLAIN or t.data_ptr() & 15 or t.dtype != dtype or t.device != device or not t.is_contiguous()):
-                return False
-        return True
+        return require_native().dec_takes([w, pool, self.pos_embed, self.final_norm, self.final_norm_b, *self.n1, *self.n1b, *self.n2, *self.n2b,
+                                           *self.bqkv, *self.bo, *self.b13, *self.b2], w)
 
     def _indices(self, t: torch.Tensor) -> torch.Tensor:
         """Tokens or positions as the kernels read them: int64, contiguous, on the shard's device."""
