@@ -239,11 +239,11 @@ __global__ void __launch_bounds__(256) dec_qkv_kernel(T* qkv, const T* bias, con
     if (is_q) continue;
     const long long req = pos ? n : n / seq;
     const int kh = hd - heads - (is_v ? kv.heads : 0);
-    long long page = at / kv.block_size;
-    int slot = (int)(at - page * kv.block_size);
+    const int at32 = (int)at;                         // 64-bit divisions are slow; a position beyond 32 bits is in no table
+    int page = at32 / kv.block_size, slot = at32 - page * kv.block_size;
     if (slot < 0) { slot += kv.block_size; page -= 1; }
     if (page < 0) page += kv.table_stride;            // negative positions and page ids count from the end, as indexing does
-    if (page < 0 || page >= kv.table_stride) { note(kv.status, FL_DEC_BAD_POSITION); continue; }
+    if (at32 != at || page < 0 || page >= kv.table_stride) { note(kv.status, FL_DEC_BAD_POSITION); continue; }
     int blk = kv.block_table[req * kv.table_stride + page];
     if (blk < 0) blk += kv.num_blocks;
     if (blk < 0 || blk >= kv.num_blocks) { note(kv.status, FL_DEC_BAD_PAGE); continue; }
@@ -300,7 +300,8 @@ __global__ void __launch_bounds__(256) dec_act_kernel(const T* h, const T* bias,
 // requested before its scores are computed and the next step's keys right after them, so a warp always has 4 to 8 KB on the
 // way.  The warps of a CTA walk different tokens; the context is cut further over the CTAs of a cluster, which merge their
 // (max, sum, output) through distributed shared memory.  16 x 2048 tokens, 8 KV heads of 128: 64 us per layer with one CTA of
-// eight warps per (request, head) and all of a step's loads waited for at once.
+// eight warps per (request, head) and all of a step's loads waited for at once; now 38 us (20 us of bytes).  3 x 400 tokens, 32
+// heads of 64: 7.5 us, of which 0.3 us are the looks at page ids and at sums that are not finite.
 constexpr int ATT_G = 8;          // query heads per CTA
 
 __device__ __forceinline__ float ld_cluster_f32(uint32_t addr) {
@@ -482,8 +483,9 @@ __global__ void __launch_bounds__(W * 32, 16 / W) dec_attention_kernel(const T* 
     for (int x = 0; x < splits; ++x) mm = fmaxf(mm, ld_cluster_f32(map_to_cta(am, x)));
     float acc = 0.f, ll = 0.f;
     for (int x = 0; x < splits; ++x) {
-      const float pl = ld_cluster_f32(map_to_cta(al, x)), e = pl == 0.f ? 0.f : exp2f(ld_cluster_f32(map_to_cta(am, x)) - mm);
-      acc += e * ld_cluster_f32(map_to_cta(ao, x));
+      const float pm = ld_cluster_f32(map_to_cta(am, x)), pl = ld_cluster_f32(map_to_cta(al, x)), po = ld_cluster_f32(map_to_cta(ao, x));
+      const float e = pl == 0.f ? 0.f : exp2f(pm - mm);      // all three on the way before the first is needed
+      acc += e * po;
       ll += e * pl;
     }
     res[i] = T(len > 0 ? acc / ll : 0.f);
