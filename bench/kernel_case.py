@@ -2,9 +2,13 @@
 """Single-GPU cases of the data-movement kernels, for timing and for ncu captures (each ends in seconds).
 
     python bench/kernel_case.py --case copy-ldst|copy-bulk|embbag-fwd|embbag-bwd|kvpack|dispatch|combine [--iters 3]
+    python bench/kernel_case.py --case dec-attention|dec-norm|dec-qkv|dec-act|interact-fwd|interact-bwd|route|quant-rows|quant-blocks
 
 All "peer" buffers are regions of the same GPU (emulated symmetric heap), so the numbers are HBM-bound versions
-of the kernels: bytes moved / time is compared with the measured device-copy bandwidth."""
+of the kernels: bytes moved / time is compared with the measured device-copy bandwidth.  The second line's cases have no peers:
+the decoder's passes at the sizes of llama3_8b (16 requests of 2048 tokens; prefill passes over 16384 rows), the interaction of
+65536 samples of 27 vectors, the routing of 8192 tokens to 8 experts, the fp8 quantisers on 8 experts (1024 of 4096 rows in use;
+weights of 4096 x 14336)."""
 import argparse
 import json
 import os
@@ -82,6 +86,59 @@ def main():
             out = torch.empty_like(x)
             fn = lambda: C.moe_combine(ws.comb.local, w, out, 2)
             nbytes = cfg.tokens * cfg.hidden * 2 * 3
+    elif case.startswith("dec-"):
+        H, heads, kvh, D, F, bs, B, S = 4096, 32, 8, 128, 14336, 16, 16, 2048
+        heaps, rows, eps = [], 16384, 1e-5
+
+        def rnd(*shape):
+            return torch.randn(*shape, device=dev).to(torch.bfloat16)
+
+        if case == "dec-attention":
+            nb = B * (S // bs)
+            kp, vp = (rnd(2, nb, bs, kvh, D) for _ in range(2))
+            bt = torch.randperm(nb, device=dev).view(B, -1).int()
+            qkv, pos, out = rnd(B, (heads + 2 * kvh) * D), torch.full((B,), S - 1, device=dev), torch.empty(B, heads * D, dtype=torch.bfloat16, device=dev)
+            fn = lambda: C.dec_attention(qkv, pos, kp, vp, bt, 1, 2, nb, bs, heads, kvh, D, out)
+            nbytes = 2 * B * S * kvh * D * 2
+        elif case == "dec-norm":
+            x, y, h, w = rnd(rows, H), rnd(rows, H), rnd(rows, H), rnd(H)
+            fn = lambda: C.dec_add_norm(x, y, None, w, None, h, eps)
+            nbytes = 4 * x.numel() * 2
+        elif case == "dec-qkv":
+            qkv, nb = rnd(rows, (heads + 2 * kvh) * D), rows // bs
+            kp, vp = (torch.empty(nb * kvh * bs * D, dtype=torch.bfloat16, device=dev) for _ in range(2))
+            bt = torch.randperm(nb, device=dev).view(rows // S, -1).int()
+            rope = torch.rand(S, D, device=dev)
+            fn = lambda: C.dec_qkv(qkv, None, rope, None, S, kp, vp, bt, 0, 0, 1, nb, bs, heads, kvh, D)
+            nbytes = rows * ((heads + kvh) * 2 + kvh + 2 * kvh) * D * 2         # q and k read and written, v read, k and v to their pages
+        else:
+            h, out = rnd(rows, 2 * F), rnd(rows, F)
+            fn = lambda: C.dec_act(h, None, out, 0)
+            nbytes = (h.numel() + out.numel()) * 2
+    elif case.startswith("interact"):
+        B, n, D, ld = 65536, 27, 128, 480
+        heaps = []
+        x, pooled, out, dx, dp = (torch.randn(*s, device=dev) for s in ((B, D), (B, n - 1, D), (B, ld), (B, D), (B, n - 1, D)))
+        fn = (lambda: C.interact_fwd(x, pooled, out)) if case == "interact-fwd" else (lambda: C.interact_bwd(x, pooled, out, dx, dp, 1.0))
+        nbytes = (B * n * D * (1 if case == "interact-fwd" else 2) + B * ld) * 4
+    elif case == "route":
+        heaps = []
+        logits, bias = torch.randn(8192, 8, device=dev).to(torch.bfloat16), torch.zeros(8, device=dev)
+        fn = lambda: C.moe_route(logits, bias, 2)
+        nbytes = 8192 * (8 * 2 + 8 * 4 + 2 * (4 + 4 + 8))
+    elif case.startswith("quant-"):
+        from fuselink_b200.ops import fp8
+        heaps = []
+        if case == "quant-rows":
+            x, counts = torch.randn(8 * 4096, 4096, device=dev).to(torch.bfloat16), torch.full((8,), 1024, dtype=torch.int32, device=dev)
+            q, s = torch.empty(x.shape, dtype=fp8.FP8, device=dev), torch.empty(8 * 4096, 32, device=dev)
+            fn = lambda: C.fp8_quantize_rows(x, q, s, counts, 4096)
+            nbytes = 8 * 1024 * 4096 * 3
+        else:
+            w = torch.randn(8, 4096, 14336, device=dev).to(torch.bfloat16)
+            q, s = torch.empty(w.shape, dtype=fp8.FP8, device=dev), torch.empty(8, 32, 112, device=dev)
+            fn = lambda: C.fp8_quantize_blocks(w, q, s)
+            nbytes = w.numel() * 3
     else:
         raise SystemExit("unknown case")
     ms = time_kernel(fn, warmup=args.warmup, iters=args.iters)

@@ -2,13 +2,14 @@
 //
 // As framework operations this is a concatenation of the vectors, a batched product, a gather of its upper triangle and a
 // second concatenation; the gradient of the gather sorts one index per output element, and the products have 27 rows.  At
-// 65536 samples of 27 x 128 that took 1.7 ms forward and 8 ms backward (now 0.18 and 0.5 ms).  The vectors are 0.9 GB, so one read of them is 0.14 ms
-// and a read and a write 0.28 ms: here both directions are one kernel that touches every vector once.
+// 65536 samples of 27 x 128 that took 1.7 ms forward and 8 ms backward (now 0.18 and 0.53 ms).  The vectors are 0.9 GB, so one
+// read of them is 0.14 ms and a read and a write 0.28 ms: here both directions are one kernel that touches every vector once.
 //
 // The gradient's products run on the fp32 pipes, as they did as library products: 27 x 28 x 128 multiply-adds per sample are
 // about 760 cycles per SM, and the memory takes about 1250 to deliver the sample.  The forward products have tf32 inputs, and
 // the kernel is for callers that allow those.  The ReLUs behind it pass a gradient or not depending on the sign of values
-// next to zero, so it keeps the order of the sums of the library's m16n8k8 products: the results are the same bits.
+// next to zero, so it keeps the order of the sums of the library's m16n8k8 products: the results are the library's bits (CUDA
+// 12.8; tests/test_interact_gpu.py) at 4, 8, 12 and 16 to 28 vectors, which are the counts that models/dlrm.py sends here.
 //
 // Reference parity: the reference runs this workload through an external DLRM checkout (.gitmodules:5-7).
 #include "interact.cuh"
