@@ -38,38 +38,45 @@ __device__ __forceinline__ void red_add_f4(float* p, float4 v) {
 // Bound by the latency of rows that are anywhere in memory: what counts is how many are on the way.  Rows are requested EB_ROWS
 // at a time (32 warps of 64 registers per SM, 160 KB on the way) and the next bag's indices before this bag's rows.  With a
 // bag's 20 rows at once, 16 warps per SM and the indices waited for first, 26 tables x 65536 bags of 20 took 2276 us (DRAM at
-// 28 % of its peak, L2 at 21 %); now 1950 us.
+// 28 % of its peak, L2 at 21 %); with 32 warps 1950 us, its issue slots 65 % busy: indices broadcast as 64 bits, addresses from 64-bit
+// products, every row behind a select.  Now 1169 us: 32-bit places, and no selects for batches of good indices.
 constexpr int EB_ROWS = 10;
 
+template <typename Place>     // of a row in its table, in units of 16 bytes: 32 bits, or 64 for tables beyond 64 GB
 __global__ void __launch_bounds__(256, 4) embbag_fwd_kernel(const FlEmbBagArgs a) {
   const int lane = threadIdx.x & 31;
   const long long nwarps = (long long)gridDim.x * (blockDim.x >> 5);
   const long long nbags = (long long)a.t_local * a.b_global;
   long long bag = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   long long next_idx = bag < nbags && lane < a.pooling ? a.indices[bag * a.pooling + lane] : 0;
+  const Place vecs = (Place)(a.dim / 4), none = ~(Place)0;
   for (; bag < nbags; bag += nwarps) {
     const int t = (int)(bag / a.b_global);
     const int b = (int)(bag - (long long)t * a.b_global);
-    // lanes load the bag's indices once, then broadcast
-    long long my_idx = next_idx;
-    if (my_idx < 0 || my_idx >= a.rows) {  // bounds check: skip the access, record it
-      report(a.status, kBadIndex, 900);
-      my_idx = -1;
-    }
+    // lanes load the bag's indices once, then broadcast the rows' places
+    const long long my_idx = next_idx;
+    const bool bad = my_idx < 0 || my_idx >= a.rows;       // bounds check: skip the access, record it
+    if (bad) report(a.status, kBadIndex, 900);
+    const Place my_at = bad ? none : (Place)my_idx * vecs;
+    const bool all_good = __all_sync(0xffffffffu, !bad);
     next_idx = bag + nwarps < nbags && lane < a.pooling ? a.indices[(bag + nwarps) * a.pooling + lane] : 0;
-    const float* table = a.weights + (long long)t * a.rows * a.dim;
+    const float* table = a.weights + (long long)t * a.rows * a.dim + lane * 4;
     const int owner = b / a.b_local;
     const int bl = b - owner * a.b_local;
-    float* out = reinterpret_cast<float*>(a.out_peers.p[owner]) +
-                 ((long long)bl * a.t_total + (a.t_first + t)) * a.dim;
-    for (int c = lane * 4; c < a.dim; c += 128) {
+    float* out = reinterpret_cast<float*>(a.out_peers.p[owner]) + ((long long)bl * a.t_total + (a.t_first + t)) * a.dim + lane * 4;
+    for (int c = 0; c < a.dim; c += 128) {
       float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
       for (int j0 = 0; j0 < a.pooling; j0 += EB_ROWS) {
         float4 r[EB_ROWS];
+        if (all_good && j0 + EB_ROWS <= a.pooling) {
 #pragma unroll
-        for (int j = 0; j < EB_ROWS; ++j) {
-          const long long ij = __shfl_sync(0xffffffffu, my_idx, (j0 + j) & 31);
-          r[j] = (j0 + j < a.pooling && ij >= 0) ? ld_f4(table + ij * a.dim + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+          for (int j = 0; j < EB_ROWS; ++j) r[j] = ld_f4(table + c + 4ull * (unsigned long long)__shfl_sync(0xffffffffu, my_at, j0 + j));
+        } else {
+#pragma unroll
+          for (int j = 0; j < EB_ROWS; ++j) {
+            const Place at = __shfl_sync(0xffffffffu, my_at, (j0 + j) & 31);
+            r[j] = (j0 + j < a.pooling && at != none) ? ld_f4(table + c + 4ull * (unsigned long long)at) : make_float4(0.f, 0.f, 0.f, 0.f);
+          }
         }
 #pragma unroll
         for (int j = 0; j < EB_ROWS; ++j) {
@@ -190,7 +197,8 @@ extern "C" int fl_embbag_a2a_fwd(const FlEmbBagArgs* a, int num_ctas, cudaStream
   int rc = check(a);
   if (rc) return rc;
   if (num_ctas <= 0) num_ctas = 148 * 8;
-  fl::embbag_fwd_kernel<<<num_ctas, 256, 0, stream>>>(*a);
+  if ((unsigned long long)a->rows * (a->dim / 4) < 0xffffffffull) fl::embbag_fwd_kernel<unsigned><<<num_ctas, 256, 0, stream>>>(*a);
+  else fl::embbag_fwd_kernel<unsigned long long><<<num_ctas, 256, 0, stream>>>(*a);
   return (int)cudaGetLastError();
 }
 
