@@ -22,6 +22,7 @@
 #include "grouped_gemm.cuh"
 #include "../common/fl_ptx.cuh"
 #include <cuda.h>
+#include <math.h>
 #include <stdio.h>
 #include <stdlib.h>
 #include <string.h>
@@ -1043,6 +1044,38 @@ extern "C" int fl_gemm_get_variant(void) {
   return g_variant;
 }
 
+// Tiles of TM rows that a group of about `rows` rows takes on average, where rows are routed independently of one another (a
+// standard deviation of sqrt(rows)).
+static double expected_tiles(double rows, int TM) {
+  double t = 0.;
+  for (int j = 0; j < 4096; ++j) {
+    const double p = 0.5 * erfc((j * (double)TM - rows) / sqrt(2. * rows));      // more than j * TM rows
+    if (j > 0 && p < 1e-3) break;
+    t += p;
+  }
+  return t;
+}
+
+// The variant for groups of `expect_rows` rows, `dflt` being the one for thousands.  Few rows per group change what pays, all
+// measured in us on 8 groups of 28672 x 4096 and 4096 x 14336 or 16 of 11264 x 2048 and 2048 x 5632 (0 | 1 | 2):
+//   weight gradients: the contraction is those rows, and a tile is all epilogue: 0 below 448 (250 rows: 704 | 758, 191: 264 | 307;
+//     448: 554 | 541);
+//   SWIGLU and DSWIGLU: the wide tiles' single accumulator does not hide such short tiles (448 rows: 321 | 296 | 331; 1000: 1506 |
+//     1491 | 1515); 0 where tiles of 128 rows pad a tenth less than those of 256 (250: 520 | 538 | 553, 125: 358 | 380 | 395);
+//   the others: wide tiles are a tenth cheaper per column, unless their number leaves more pairs idle in the last round (250 rows of
+//     4096 x 14336, 86 tiles on 74 pairs: 289 (1) | 326 (2); 500: 395 | 354; 191 of 2048 x 5632: 90 | 88).
+static int variant_for_rows(const FlGemmDesc* d, int dflt) {
+  const double rows = d->expect_rows;
+  if (d->group_mode == 1) return rows < 448 ? 0 : dflt;
+  if (d->N < 512 || rows >= 1024) return dflt;
+  const double t256 = expected_tiles(rows, 256);
+  if (d->epilogue == FL_EPI_SWIGLU || d->epilogue == FL_EPI_DSWIGLU)
+    return 1.1 * 128 * expected_tiles(rows, 128) < 256 * t256 ? 0 : 1;
+  constexpr double kPairs = 74.;
+  const double wide = d->num_groups * t256 * ((d->N + 511) / 512), pair = d->num_groups * t256 * ((d->N + 255) / 256);
+  return 1.8 * ceil(wide / kPairs) < ceil(pair / kPairs) ? 2 : 1;
+}
+
 extern "C" int fl_grouped_gemm(const FlGemmDesc* d, cudaStream_t stream) {
   using namespace fl;
   g_err[0] = 0;
@@ -1094,6 +1127,7 @@ extern "C" int fl_grouped_gemm(const FlGemmDesc* d, cudaStream_t stream) {
   if (variant == 3) {
     const bool short_k_long_epilogue = d->group_mode == 0 && d->epilogue == FL_EPI_DSWIGLU && d->K < 8192;
     variant = (d->N < 512 || short_k_long_epilogue || d->group_mode == 1) ? 1 : 2;
+    if (d->expect_rows > 0) variant = variant_for_rows(d, variant);
   }
   const bool pair = variant >= 1;
   CUtensorMap tmA, tmB;

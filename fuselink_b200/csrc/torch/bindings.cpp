@@ -47,7 +47,7 @@ static void grouped_gemm(int64_t group_mode, int64_t num_groups, int64_t cap, in
                          c10::optional<torch::Tensor> C, int64_t ldc, int64_t gsc, c10::optional<torch::Tensor> gu,
                          int64_t ldgu, c10::optional<torch::Tensor> dgu, c10::optional<torch::Tensor> row_info,
                          std::vector<int64_t> peers, double sgd_lr, bool zero_tail, int64_t group_m, int64_t max_ctas,
-                         c10::optional<torch::Tensor> status, int64_t peer_rows) {
+                         c10::optional<torch::Tensor> status, int64_t peer_rows, int64_t expect_rows) {
   TORCH_CHECK(A.is_cuda() && B.is_cuda(), "grouped_gemm needs CUDA tensors");
   TORCH_CHECK(A.scalar_type() == torch::kBFloat16 && B.scalar_type() == torch::kBFloat16, "bf16 operands expected");
   c10::cuda::CUDAGuard guard(A.device());
@@ -66,6 +66,7 @@ static void grouped_gemm(int64_t group_mode, int64_t num_groups, int64_t cap, in
   d.peers = to_peers(peers); d.num_peers = (int)peers.size(); d.peer_rows = peer_rows;
   d.sgd_lr = (float)sgd_lr; d.zero_tail = zero_tail; d.group_m = (int)group_m; d.max_ctas = (int)max_ctas;
   d.status = status.has_value() ? status->data_ptr<int>() : nullptr;
+  d.expect_rows = (int)std::min<int64_t>(std::max<int64_t>(expect_rows, 0), INT32_MAX);
   check_rc(fl_grouped_gemm(&d, cur_stream()), "fl_grouped_gemm", fl_gemm_last_error());
 }
 
@@ -531,7 +532,11 @@ static int64_t vmm_remap_slab(int64_t region, int64_t slab, int64_t target, bool
 }
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
-  m.def("grouped_gemm", &grouped_gemm);
+  m.def("grouped_gemm", &grouped_gemm, py::arg("group_mode"), py::arg("num_groups"), py::arg("cap"), py::arg("M"), py::arg("N"), py::arg("K"),
+        py::arg("counts"), py::arg("A"), py::arg("a_mn"), py::arg("lda"), py::arg("gsa"), py::arg("B"), py::arg("b_mn"), py::arg("ldb"), py::arg("gsb"),
+        py::arg("epilogue"), py::arg("C"), py::arg("ldc"), py::arg("gsc"), py::arg("gu"), py::arg("ldgu"), py::arg("dgu"), py::arg("row_info"),
+        py::arg("peers"), py::arg("sgd_lr"), py::arg("zero_tail"), py::arg("group_m"), py::arg("max_ctas"), py::arg("status"), py::arg("peer_rows"),
+        py::arg("expect_rows") = 0);
   m.def("grouped_gemm_wgrad_push", &grouped_gemm_wgrad_push);
   m.def("shadow_update", &shadow_update);
   m.def("gemm_set_variant", [](int64_t v) { fl_gemm_set_variant((int)v); });

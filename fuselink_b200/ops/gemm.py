@@ -10,15 +10,21 @@ from .._ext import require_native
 EPI_STORE, EPI_SWIGLU, EPI_SCATTER, EPI_DSWIGLU, EPI_WGRAD = 0, 1, 2, 3, 4
 
 
+def _expected(a: torch.Tensor, rows: int) -> tuple:
+    """The argument that only launches on a GPU take."""
+    return (int(rows),) if rows > 0 and a.is_cuda else ()
+
+
 def grouped_gemm_rows(a: torch.Tensor, b: torch.Tensor, counts: Optional[torch.Tensor], cap: int, *,
                       b_mn_major: bool = False, epilogue: int = EPI_STORE, out: Optional[torch.Tensor] = None,
                       gu: Optional[torch.Tensor] = None, dgu: Optional[torch.Tensor] = None,
                       row_info: Optional[torch.Tensor] = None, peers: Optional[List[int]] = None, ldc: Optional[int] = None,
                       zero_tail: bool = False, group_m: int = 16, max_ctas: int = 0,
-                      status: Optional[torch.Tensor] = None, peer_rows: int = 0) -> Optional[torch.Tensor]:
+                      status: Optional[torch.Tensor] = None, peer_rows: int = 0, expect_rows: int = 0) -> Optional[torch.Tensor]:
     """M-grouped GEMM: for each group g, ``C_g = A_g @ B_g^T`` over the first counts[g] rows of A_g.
     With the SCATTER epilogue ``peer_rows`` is the number of rows of every receive buffer: a row whose return address
-    lies outside is not stored and the status word reports a bad index.
+    lies outside is not stored and the status word reports a bad index.  ``expect_rows``: rows that a group is expected to have (0:
+    not known); it chooses the tiles and changes no result.
 
     a: [G*cap, K] bf16 token buffer (group g owns rows [g*cap, (g+1)*cap)).
     b: [G, N, K] (K-major, the nn.Linear layout) or, with ``b_mn_major``, [G, K, N].
@@ -39,13 +45,13 @@ def grouped_gemm_rows(a: torch.Tensor, b: torch.Tensor, counts: Optional[torch.T
     ldb = N if b_mn_major else K
     C.grouped_gemm(0, G, cap, 0, N, K, counts, a, False, K, cap * K, b, b_mn_major, ldb, b.shape[1] * b.shape[2],
                    epilogue, out, ldc, gsc, gu if gu is not None else None, gu.shape[1] if gu is not None else 0, dgu,
-                   row_info, peers or [], 0.0, zero_tail, group_m, max_ctas, status, peer_rows)
+                   row_info, peers or [], 0.0, zero_tail, group_m, max_ctas, status, peer_rows, *_expected(a, expect_rows))
     return out
 
 
 def grouped_gemm_wgrad(a: torch.Tensor, b: torch.Tensor, counts: Optional[torch.Tensor], cap: int, G: int, *,
                        out: Optional[torch.Tensor] = None, sgd_lr: float = 0.0, group_m: int = 16, max_ctas: int = 0,
-                       status: Optional[torch.Tensor] = None) -> torch.Tensor:
+                       status: Optional[torch.Tensor] = None, expect_rows: int = 0) -> torch.Tensor:
     """K-grouped GEMM: ``C_g[M, N] = A_g^T @ B_g`` with A_g, B_g the first counts[g] rows of group g in the
     token-major buffers a: [G*cap, M], b: [G*cap, N].  With ``sgd_lr`` the result is applied to ``out`` in place
     (``out -= lr * C``) instead of being stored."""
@@ -56,7 +62,7 @@ def grouped_gemm_wgrad(a: torch.Tensor, b: torch.Tensor, counts: Optional[torch.
         assert sgd_lr == 0.0
         out = torch.empty(G, M, N, dtype=torch.bfloat16, device=a.device)
     C.grouped_gemm(1, G, cap, M, N, 0, counts, a, True, M, cap * M, b, True, N, cap * N, EPI_WGRAD, out, N, M * N,
-                   None, 0, None, None, [], sgd_lr, False, group_m, max_ctas, status, 0)
+                   None, 0, None, None, [], sgd_lr, False, group_m, max_ctas, status, 0, *_expected(a, expect_rows))
     return out
 
 

@@ -115,6 +115,7 @@ class MoEWorkspace:
         self.cap = (cfg.tokens * W + 127) // 128 * 128
         rows = self.epr * self.cap
         H, F, T, k = cfg.hidden, cfg.ffn, cfg.tokens, cfg.topk
+        self.rows_per_slot = max(1, T * W * k // cfg.num_experts)      # that an evenly spread router gives an expert
         bf = torch.bfloat16
         # symmetric (peers write into these)
         self.xd = heap.alloc_tensor([rows, H], bf)        # dispatched tokens
@@ -376,9 +377,9 @@ def moe_forward_experts(ws: MoEWorkspace, w13: torch.Tensor, w2: torch.Tensor) -
         ws.launches += 4
     else:
         gemm.grouped_gemm_rows(ws.xd.local, w13, counts, ws.cap, epilogue=gemm.EPI_SWIGLU, out=ws.act, gu=ws.gu,
-                               zero_tail=True, status=st)
+                               zero_tail=True, status=st, expect_rows=ws.rows_per_slot)
         gemm.grouped_gemm_rows(ws.act, w2, counts, ws.cap, epilogue=gemm.EPI_SCATTER, row_info=ws.info.local,
-                               peers=ws.comb.peers(), ldc=ws.cfg.hidden, status=st, peer_rows=ws.comb.local.shape[0])
+                               peers=ws.comb.peers(), ldc=ws.cfg.hidden, status=st, peer_rows=ws.comb.local.shape[0], expect_rows=ws.rows_per_slot)
     barrier(h, ws.name + ":c", signal=True, wait=False)
     ws.launches += 5
 
@@ -433,19 +434,19 @@ def moe_backward_experts(ws: MoEWorkspace, w13: torch.Tensor, w2: torch.Tensor, 
         ws.launches += 2
     else:
         gemm.grouped_gemm_rows(ws.dyd.local, w2, counts, ws.cap, b_mn_major=True, epilogue=gemm.EPI_DSWIGLU, gu=ws.gu,
-                               dgu=ws.dgu, zero_tail=True, status=st)
+                               dgu=ws.dgu, zero_tail=True, status=st, expect_rows=ws.rows_per_slot)
         if overlap:
             # the copies' weight gradients first: their sum over the ranks starts now and runs beside what follows
             R, S, cut = ws.epr_real, ws.shadows_in_use, ws.epr_real * ws.cap
             end = cut + S * ws.cap
-            early = (gemm.grouped_gemm_wgrad(ws.dgu[cut:end], ws.xd.local[cut:end], counts[R:R + S], ws.cap, S, status=st),
-                     gemm.grouped_gemm_wgrad(ws.dyd.local[cut:end], ws.act[cut:end], counts[R:R + S], ws.cap, S, status=st))
+            early = (gemm.grouped_gemm_wgrad(ws.dgu[cut:end], ws.xd.local[cut:end], counts[R:R + S], ws.cap, S, status=st, expect_rows=ws.rows_per_slot),
+                     gemm.grouped_gemm_wgrad(ws.dyd.local[cut:end], ws.act[cut:end], counts[R:R + S], ws.cap, S, status=st, expect_rows=ws.rows_per_slot))
             ws.launches += 2
             works = ws.reduce_shadow_grads(ws, early) or []
         if need_dx:
             gemm.grouped_gemm_rows(ws.dgu, w13, counts, ws.cap, b_mn_major=True, epilogue=gemm.EPI_SCATTER,
                                    row_info=ws.info.local, peers=ws.dxs.peers(), ldc=cfg.hidden, status=st,
-                                   peer_rows=ws.dxs.local.shape[0], max_ctas=beside)
+                                   peer_rows=ws.dxs.local.shape[0], max_ctas=beside, expect_rows=ws.rows_per_slot)
     shadow_grads = None
     if ws.nshadow:
         # Owned experts as below, on the leading slots.  The copies of the shadowed experts have seen this rank's rows
@@ -454,14 +455,14 @@ def moe_backward_experts(ws: MoEWorkspace, w13: torch.Tensor, w2: torch.Tensor, 
         R, S, cut = ws.epr_real, ws.shadows_in_use, ws.epr_real * ws.cap
         dyd, dgu, act, xd = ws.dyd.local, ws.dgu, ws.act, ws.xd.local
         if sgd_lr:
-            gemm.grouped_gemm_wgrad(dyd[:cut], act[:cut], counts[:R], ws.cap, R, out=w2[:R], sgd_lr=sgd_lr, status=st, max_ctas=beside)
-            gemm.grouped_gemm_wgrad(dgu[:cut], xd[:cut], counts[:R], ws.cap, R, out=w13[:R], sgd_lr=sgd_lr, status=st, max_ctas=beside)
+            gemm.grouped_gemm_wgrad(dyd[:cut], act[:cut], counts[:R], ws.cap, R, out=w2[:R], sgd_lr=sgd_lr, status=st, max_ctas=beside, expect_rows=ws.rows_per_slot)
+            gemm.grouped_gemm_wgrad(dgu[:cut], xd[:cut], counts[:R], ws.cap, R, out=w13[:R], sgd_lr=sgd_lr, status=st, max_ctas=beside, expect_rows=ws.rows_per_slot)
             dw2 = dw13 = None
         else:
             dw2 = torch.empty_like(w2)
             dw13 = torch.empty_like(w13)
-            gemm.grouped_gemm_wgrad(dyd[:cut], act[:cut], counts[:R], ws.cap, R, out=dw2[:R], status=st, max_ctas=beside)
-            gemm.grouped_gemm_wgrad(dgu[:cut], xd[:cut], counts[:R], ws.cap, R, out=dw13[:R], status=st, max_ctas=beside)
+            gemm.grouped_gemm_wgrad(dyd[:cut], act[:cut], counts[:R], ws.cap, R, out=dw2[:R], status=st, max_ctas=beside, expect_rows=ws.rows_per_slot)
+            gemm.grouped_gemm_wgrad(dgu[:cut], xd[:cut], counts[:R], ws.cap, R, out=dw13[:R], status=st, max_ctas=beside, expect_rows=ws.rows_per_slot)
             dw2[R:].zero_()                                          # copy slots: filled in once the sums are complete, empty
             dw13[R:].zero_()                                         # ones stay zero
         pk = ws.push
@@ -478,16 +479,16 @@ def moe_backward_experts(ws: MoEWorkspace, w13: torch.Tensor, w2: torch.Tensor, 
             shadow_grads = S
         elif S:
             end = cut + S * ws.cap                                   # empty copy slots at the end take no part
-            shadow_grads = (gemm.grouped_gemm_wgrad(dgu[cut:end], xd[cut:end], counts[R:R + S], ws.cap, S, status=st),
-                            gemm.grouped_gemm_wgrad(dyd[cut:end], act[cut:end], counts[R:R + S], ws.cap, S, status=st))
+            shadow_grads = (gemm.grouped_gemm_wgrad(dgu[cut:end], xd[cut:end], counts[R:R + S], ws.cap, S, status=st, expect_rows=ws.rows_per_slot),
+                            gemm.grouped_gemm_wgrad(dyd[cut:end], act[cut:end], counts[R:R + S], ws.cap, S, status=st, expect_rows=ws.rows_per_slot))
             ws.launches += 2
     elif sgd_lr:
-        gemm.grouped_gemm_wgrad(ws.dyd.local, ws.act, counts, ws.cap, ws.epr, out=w2, sgd_lr=sgd_lr, status=st)
-        gemm.grouped_gemm_wgrad(ws.dgu, ws.xd.local, counts, ws.cap, ws.epr, out=w13, sgd_lr=sgd_lr, status=st)
+        gemm.grouped_gemm_wgrad(ws.dyd.local, ws.act, counts, ws.cap, ws.epr, out=w2, sgd_lr=sgd_lr, status=st, expect_rows=ws.rows_per_slot)
+        gemm.grouped_gemm_wgrad(ws.dgu, ws.xd.local, counts, ws.cap, ws.epr, out=w13, sgd_lr=sgd_lr, status=st, expect_rows=ws.rows_per_slot)
         dw2 = dw13 = None
     else:
-        dw2 = gemm.grouped_gemm_wgrad(ws.dyd.local, ws.act, counts, ws.cap, ws.epr, status=st)
-        dw13 = gemm.grouped_gemm_wgrad(ws.dgu, ws.xd.local, counts, ws.cap, ws.epr, status=st)
+        dw2 = gemm.grouped_gemm_wgrad(ws.dyd.local, ws.act, counts, ws.cap, ws.epr, status=st, expect_rows=ws.rows_per_slot)
+        dw13 = gemm.grouped_gemm_wgrad(ws.dgu, ws.xd.local, counts, ws.cap, ws.epr, status=st, expect_rows=ws.rows_per_slot)
     # every read of the buffers peers will overwrite next step is enqueued before this signal
     barrier(h, ws.name + ":bx", signal=True, wait=False)
     ws.launches += 6 + (1 if need_dx else 0)
