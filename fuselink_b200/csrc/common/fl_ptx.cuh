@@ -187,6 +187,12 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
   return true;
 }
 
+// ---- programmatic dependent launch --------------------------------------------------------------------
+// wait: everything that the kernels before this one in the stream have written is there (they have ended).  launch: the next kernel,
+// if it was launched to start early, may be started once every CTA of this grid has come here or left.
+__device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ---- proxy fences -----------------------------------------------------------------------------------
 // generic-proxy writes (st.shared / st.global) -> async proxy (TMA, tcgen05) visibility
 __device__ __forceinline__ void fence_proxy_async_smem() {

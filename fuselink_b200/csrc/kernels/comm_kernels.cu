@@ -87,6 +87,7 @@ __global__ void __launch_bounds__(1024) put_chunks_kernel(const FlPutArgs a) {
     }
   }
   __syncthreads();
+  grid_dep_launch();
 
   unsigned long long chunks_before = 0;
   bool live = true;
@@ -153,12 +154,16 @@ __global__ void __launch_bounds__(1024) put_chunks_kernel(const FlPutArgs a) {
 }
 
 __global__ void wait_flags_kernel(const FlWaitArgs a) {
+  grid_dep_launch();
+  grid_dep_wait();
   const int i = threadIdx.x;
   if (i < a.n) wait_flag_ge(a.flag[i], a.want[i], a.status, 700 + i, a.limit_ns ? a.limit_ns : (uint64_t)FL_FLAG_WAIT_NS);
 }
 
 __global__ void barrier_kernel(FlSignalPtrs pads, int slot0, int rank, int world, unsigned int seq, int do_signal,
                                int do_wait, int* status) {
+  grid_dep_launch();
+  grid_dep_wait();
   const int r = threadIdx.x;
   if (r >= world) return;
   if (do_signal) {
@@ -169,6 +174,25 @@ __global__ void barrier_kernel(FlSignalPtrs pads, int slot0, int rank, int world
 }
 
 }  // namespace fl
+
+// Waits and barriers are a warp each, often several in a row.  They are launched so that they may be placed while the kernel before
+// them drains; they touch nothing, and poll no flag, before that kernel has ended (grid_dep_wait), so what one polls for is never behind
+// it.  Eight exchanges of 21 MB and their waits, one after the other: 138 -> 126 us; a put of 64 KiB and its wait: 10.2 -> 9.6 us.  The
+// puts themselves, launched like that as well, take longer (176 us): their early CTAs hold shared memory that the running ones' peers want.
+template <typename... P, typename... A>
+static int launch_after(void (*kernel)(P...), unsigned grid, unsigned threads, size_t smem, cudaStream_t stream, const A&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid, 1, 1);
+  cfg.blockDim = dim3(threads, 1, 1);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return (int)cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
 
 extern "C" int fl_put_chunks(const FlPutArgs* args, int num_ctas, int threads, cudaStream_t stream) {
   if (args->nseg < 1 || args->nseg > FL_MAX_SEGS) return -1;
@@ -222,13 +246,11 @@ extern "C" int fl_all_to_all(const void* send, void* const* recv_peers, unsigned
 extern "C" int fl_wait_flags(const FlWaitArgs* args, cudaStream_t stream) {
   if (args->n < 0 || args->n > 16) return -1;
   if (args->n == 0) return 0;
-  fl::wait_flags_kernel<<<1, 32, 0, stream>>>(*args);
-  return (int)cudaGetLastError();
+  return launch_after(fl::wait_flags_kernel, 1, 32, 0, stream, *args);
 }
 
 extern "C" int fl_barrier(FlSignalPtrs pads, int slot0, int rank, int world, unsigned int seq, int do_signal,
                           int do_wait, int* status, cudaStream_t stream) {
   if (world < 1 || world > 8) return -1;
-  fl::barrier_kernel<<<1, 32, 0, stream>>>(pads, slot0, rank, world, seq, do_signal, do_wait, status);
-  return (int)cudaGetLastError();
+  return launch_after(fl::barrier_kernel, 1, 32, 0, stream, pads, slot0, rank, world, seq, do_signal, do_wait, status);
 }
