@@ -10,6 +10,7 @@
 #include "../kernels/comm_kernels.cuh"
 #include "../kernels/embbag.cuh"
 #include "../kernels/interact.cuh"
+#include "../kernels/mlp_bwd.cuh"
 #include "../kernels/kv_pack.cuh"
 #include "../kernels/decoder.cuh"
 #include "../kernels/moe_dispatch.cuh"
@@ -438,6 +439,19 @@ static torch::Tensor moe_route_bwd(torch::Tensor probs, torch::Tensor w, torch::
   check_rc(fl_moe_route_bwd(&a, cur_stream()), "fl_moe_route_bwd");
   return out;
 }
+// gradient of relu(z + bias): (dz, the bias gradient) from dy and the layer's output y, see mlp_bwd.cuh
+static std::pair<torch::Tensor, torch::Tensor> relu_bias_bwd(torch::Tensor dy, torch::Tensor y) {
+  TORCH_CHECK(dy.is_cuda() && dy.device() == y.device() && dy.scalar_type() == torch::kFloat32 && y.scalar_type() == torch::kFloat32 &&
+              dy.dim() == 2 && dy.sizes() == y.sizes() && dy.is_contiguous() && y.is_contiguous() && dy.size(1) <= INT32_MAX, "dy, y: [rows, cols] fp32");
+  c10::cuda::CUDAGuard guard(dy.device());
+  const int64_t rows = dy.size(0);
+  const int cols = (int)dy.size(1);
+  auto dz = torch::empty_like(dy), db = torch::empty({cols}, dy.options()), part = torch::empty({fl_relu_bias_parts(rows, cols), cols}, dy.options());
+  if (rows == 0 || cols == 0) return {dz, db.zero_()};
+  check_rc(fl_relu_bias_bwd(dy.data_ptr<float>(), y.data_ptr<float>(), dz.data_ptr<float>(), part.data_ptr<float>(), db.data_ptr<float>(), rows, cols,
+                            cur_stream()), "fl_relu_bias_bwd");
+  return {dz, db};
+}
 static void moe_zero_tail(int64_t buf, int64_t counts, int64_t experts_local, int64_t cap, int64_t width) {
   check_rc(fl_moe_zero_tail(reinterpret_cast<void*>(buf), reinterpret_cast<const int*>(counts), (int)experts_local,
                             (int)cap, (int)width, cur_stream()), "fl_moe_zero_tail");
@@ -562,6 +576,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("moe_route_bwd", &moe_route_bwd);
   m.def("interact_fwd", &interact_fwd);
   m.def("interact_bwd", &interact_bwd);
+  m.def("relu_bias_bwd", &relu_bias_bwd);
   m.def("dec_act", &dec_act);
   m.def("dec_attention", &dec_attention, py::arg("qkv"), py::arg("pos"), py::arg("k_pool"), py::arg("v_pool"), py::arg("table"),
         py::arg("layer"), py::arg("layers"), py::arg("num_blocks"), py::arg("block_size"), py::arg("heads"), py::arg("kv_heads"),

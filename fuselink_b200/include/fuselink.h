@@ -16,6 +16,7 @@
 #include "../csrc/kernels/interact.cuh"
 #include "../csrc/kernels/kv_pack.cuh"
 #include "../csrc/kernels/decoder.cuh"
+#include "../csrc/kernels/mlp_bwd.cuh"
 #include "../csrc/kernels/moe_dispatch.cuh"
 #include "../csrc/kernels/moe_dispatch_noalloc.cuh"
 #include "../csrc/kernels/moe_route.cuh"

@@ -126,6 +126,48 @@ def _gram(dy: torch.Tensor, r: torch.Tensor) -> torch.Tensor:
     return out if m == B else out.addmm_(dy[m:].t(), r[m:])
 
 
+class _Mlp(torch.autograd.Function):
+    """Linear layers with a ReLU behind each (``relu_last``: behind the last one as well) as one node, params = weight, bias, weight,
+    bias, ...: the ReLU rides along with the product, its gradient and the bias gradient are one pass (csrc/kernels/mlp_bwd.cu).  The
+    rows x may be padded with zeros to an aligned width for the gradients' products: at 479 columns (26 tables) they miss the library's
+    aligned kernels.  The forward product stays at the width of the weight, whose bits decide which ReLUs pass a gradient."""
+
+    @staticmethod
+    def forward(ctx, x, relu_last, *params):
+        acts, n = [x], len(params) // 2
+        for i in range(n):
+            w, b = params[2 * i], params[2 * i + 1]
+            rows = acts[-1] if i else x[:, : w.shape[1]]
+            acts.append(torch._addmm_activation(b, rows, w.t()) if i < n - 1 or relu_last else torch.addmm(b, rows, w.t()))
+        ctx.save_for_backward(*(acts if relu_last else acts[:-1]), *params)
+        ctx.relu_last = relu_last
+        return acts[-1]
+
+    @staticmethod
+    @torch.autograd.function.once_differentiable
+    def backward(ctx, dy):
+        C, saved = require_native(), ctx.saved_tensors
+        n = (len(saved) - ctx.relu_last) // 3
+        acts, params = saved[:n + ctx.relu_last], saved[n + ctx.relu_last:]
+        grads = [None] * (2 * n)
+        for i in range(n - 1, -1, -1):
+            w, x = params[2 * i], acts[i]
+            want_x, want_w, want_b = i > 0 or ctx.needs_input_grad[0], ctx.needs_input_grad[2 + 2 * i], ctx.needs_input_grad[3 + 2 * i]
+            if i < n - 1 or ctx.relu_last:
+                dy, db = C.relu_bias_bwd(dy.contiguous(), acts[i + 1])
+            else:
+                db = dy.sum(0) if want_b else None
+            grads[2 * i + 1] = db if want_b else None
+            if want_w:
+                if x.shape[1] != w.shape[1]:
+                    grads[2 * i] = _gram(dy.contiguous(), x)[:, :w.shape[1]].contiguous()
+                else:
+                    grads[2 * i] = dy.t() @ x
+            if want_x:
+                dy = dy @ (w if x.shape[1] == w.shape[1] else F.pad(w, (0, x.shape[1] - w.shape[1])))
+        return dy if ctx.needs_input_grad[0] else None, None, *grads
+
+
 class _PaddedLinear(torch.autograd.Function):
     """F.linear(r[:, :in], weight, bias) for rows r that are padded with zeros to an aligned width: the gradients' products
     run over the padded width.  At an odd number of columns (479 for 26 tables) they miss the library's aligned kernels."""
@@ -240,15 +282,31 @@ class DLRM(nn.Module):
                             for m in skipped)
                 and all(type(p) is nn.Parameter and p.dtype == torch.float32 for p in self.dense_parameters()))
 
+    def _plain_mlps(self) -> bool:
+        """Whether the MLPs may be called through their parameters: layers as __init__ made them, no hooks on any."""
+        for mlp, relu_last in ((self.bottom, True), (self.top, False)):
+            layers = list(mlp)
+            linear, relu = layers[::2], layers[1::2]
+            if len(linear) != len(relu) + (not relu_last) or not (all(type(m) is nn.Linear and m.bias is not None for m in linear) and
+                                                                  all(type(m) is nn.ReLU for m in relu)):
+                return False
+            if any("forward" in m.__dict__ or m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks
+                   for m in (mlp, *layers)):
+                return False
+        return True
+
     def _dense_forward_fused(self, dense: torch.Tensor, pooled: torch.Tensor) -> torch.Tensor:
         """dense_forward with the gradient of ``pooled`` (over the ranks' mean) written to the buffer the tables' owners read."""
-        x = self.bottom(dense).contiguous()
+        plain = self._plain_mlps()
+        x = (_Mlp.apply(dense, True, *self.bottom.parameters()) if plain else self.bottom(dense)).contiguous()
         if x.data_ptr() % 16:                              # a hook may have put a view of something larger in its place
             x = x.clone()
         n = self.n_inter + self.cfg.dim
         width = (n + 7) // 8 * 8
         anchor = torch.empty(0, device=x.device, requires_grad=True)
         r = _Interaction.apply(x, pooled, self.gpooled.local, 1.0 / self.world, width, (self.iu0, self.iu1), anchor)
+        if plain:
+            return _Mlp.apply(r, False, *self.top.parameters()).squeeze(-1)
         first = self.top[0]
         y = _PaddedLinear.apply(r, first.weight, first.bias)
         return self.top[1:](y).squeeze(-1)
