@@ -16,6 +16,7 @@
 #include <math.h>
 #include <initializer_list>
 #include "../common/fl_ptx.cuh"
+#include "tile_map.cuh"
 
 namespace fl {
 
@@ -81,6 +82,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) dec_embed_kernel(const long long* tokens, const long long* pos, const T* embed, const T* pos_embed,
                                                         T* x, long long rows, int vecs, int seq, int offset, long long vocab,
                                                         long long pos_rows, int* status) {
+  grid_dep_launch();
   const long long total = rows * vecs;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
     const long long n = i / vecs;
@@ -127,6 +129,8 @@ template <typename T, int VPT>
 __global__ void __launch_bounds__(1024) dec_add_norm_kernel(T* x, const T* y, const T* y_bias, const T* w, const T* b, T* h, int hidden,
                                                             float eps) {
   __shared__ float red[32];
+  grid_dep_launch();
+  grid_dep_wait();
   const long long row = blockIdx.x;
   const int vecs = hidden >> 3;
   T* xr = x + row * hidden;
@@ -197,6 +201,8 @@ __global__ void __launch_bounds__(1024) dec_add_norm_kernel(T* x, const T* y, co
 template <typename T>
 __global__ void __launch_bounds__(256) dec_qkv_kernel(T* qkv, const T* bias, const float* rope, long long rope_rows, const long long* pos,
                                                       long long rows, int seq, int heads, int dim, const FlPagedKv kv) {
+  grid_dep_launch();
+  grid_dep_wait();
   const int total_heads = heads + 2 * kv.heads, chunks = dim / 16, half = dim / 2;
   const int per_row = total_heads * chunks;
   const long long total = rows * per_row;
@@ -259,6 +265,8 @@ __global__ void __launch_bounds__(256) dec_qkv_kernel(T* qkv, const T* bias, con
 // ---- activation -----------------------------------------------------------------------------------------------------------
 template <typename T, int KIND>
 __global__ void __launch_bounds__(256) dec_act_kernel(const T* h, const T* bias, T* out, long long rows, int ffn) {
+  grid_dep_launch();
+  grid_dep_wait();
   const int vecs = ffn / 8;
   const long long total = rows * vecs;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
@@ -310,12 +318,128 @@ __device__ __forceinline__ float ld_cluster_f32(uint32_t addr) {
   return v;
 }
 
+// scores of 16 tokens: s[p][e] is token 2 t + e + 8 p of the step, -inf where bit 2 p + e of `there` is off
+template <typename T, int KJ>
+__device__ __forceinline__ void att_scores(const uint32_t (&qa)[KJ][4], const uint4 (&kr)[2][KJ], unsigned there, float scale_log2, float (&s)[2][2]) {
+#pragma unroll
+  for (int p = 0; p < 2; ++p) {
+    s[p][0] = s[p][1] = 0.f;
+#pragma unroll
+    for (int j = 0; j < KJ; ++j) {
+      Num<T>::mma(s[p], qa[j][0], qa[j][1], kr[p][j].x, kr[p][j].y);
+      Num<T>::mma(s[p], qa[j][2], qa[j][3], kr[p][j].z, kr[p][j].w);
+    }
+#pragma unroll
+    for (int e = 0; e < 2; ++e) s[p][e] = there >> (2 * p + e) & 1 ? s[p][e] * scale_log2 : -INFINITY;
+  }
+}
+
+// the step's part of the softmax and of the output; m, l: running maximum and this lane's sum
+template <typename T, int VC>
+__device__ __forceinline__ void att_values(float (&s)[2][2], const uint4 (&vr)[4][VC], float& m, float& l, float (&o)[VC][8][2]) {
+  const float m_old = m;
+  float mx = fmaxf(fmaxf(s[0][0], s[0][1]), fmaxf(s[1][0], s[1][1]));
+  mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+  mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+  // A score may be -inf (an infinite key): 0 stands in for a maximum of -inf, so that a step of nothing else adds nothing.
+  // One that is NaN or +inf makes the sums NaN, and NaN they stay.
+  m = fmaxf(m, mx);
+  const float mn = m == -INFINITY ? 0.f : m;
+  const float f = exp2f(m_old - mn);
+  float add = 0.f;
+#pragma unroll
+  for (int p = 0; p < 2; ++p)
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      s[p][e] = exp2f(s[p][e] - mn);
+      add += s[p][e];
+    }
+  l = l * f + add;                               // this lane's tokens only; summed over the quad at the end
+  const uint32_t p0 = Num<T>::pack(s[0][0], s[0][1]), p1 = Num<T>::pack(s[1][0], s[1][1]);
+#pragma unroll
+  for (int c = 0; c < VC; ++c) {
+    const uint32_t v0[4] = {vr[0][c].x, vr[0][c].y, vr[0][c].z, vr[0][c].w};
+    const uint32_t v1[4] = {vr[1][c].x, vr[1][c].y, vr[1][c].z, vr[1][c].w};
+    const uint32_t v2[4] = {vr[2][c].x, vr[2][c].y, vr[2][c].z, vr[2][c].w};
+    const uint32_t v3[4] = {vr[3][c].x, vr[3][c].y, vr[3][c].z, vr[3][c].w};
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      o[c][j][0] *= f;
+      o[c][j][1] *= f;
+      const uint32_t sel = (j & 1) ? 0x7632u : 0x5410u;
+      Num<T>::mma(o[c][j], p0, p1, __byte_perm(v0[j >> 1], v1[j >> 1], sel), __byte_perm(v2[j >> 1], v3[j >> 1], sel));
+    }
+  }
+}
+
+template <int W> struct AttParts { float m[W][ATT_G], l[W][ATT_G], cm[ATT_G], cl[ATT_G]; };
+
+// Merges the parts of the warps, and those of the CTAs of the cluster, into res [nh][dim].  so: W parts of [ATT_G][DP + 4] in shared
+// memory, so_stride floats apart.
+template <typename T, int DP, int W>
+__device__ __forceinline__ void att_finish(AttParts<W>& parts, float* so, int so_stride, float m, float l, const float (&o)[DP / 64][8][2], int nh,
+                                           int dim, int len, int split, int splits, T* res) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+  auto part = [&](int w, int hg, int d) -> float* { return so + w * so_stride + hg * (DP + 4) + d; };
+  l += __shfl_xor_sync(0xffffffffu, l, 1);
+  l += __shfl_xor_sync(0xffffffffu, l, 2);
+  if (t == 0) { parts.m[warp][g] = m; parts.l[warp][g] = l; }
+#pragma unroll
+  for (int c = 0; c < DP / 64; ++c)
+#pragma unroll
+    for (int j = 0; j < 8; j += 4) {
+      *reinterpret_cast<float4*>(part(warp, g, 64 * c + 16 * t + j)) = make_float4(o[c][j][0], o[c][j + 1][0], o[c][j + 2][0], o[c][j + 3][0]);
+      *reinterpret_cast<float4*>(part(warp, g, 64 * c + 16 * t + 8 + j)) = make_float4(o[c][j][1], o[c][j + 1][1], o[c][j + 2][1], o[c][j + 3][1]);
+    }
+  __syncthreads();
+  // merge the warps: with one split this is the result, otherwise it replaces the first warp's part
+  const int cells = nh * dim;
+  for (int i = threadIdx.x; i < cells; i += W * 32) {
+    const int hg = i / dim, d = i - hg * dim;
+    float mm = -INFINITY;
+#pragma unroll
+    for (int x = 0; x < W; ++x) mm = fmaxf(mm, parts.m[x][hg]);
+    float acc = 0.f, ll = 0.f;
+#pragma unroll
+    for (int x = 0; x < W; ++x) {
+      const float e = parts.l[x][hg] == 0.f ? 0.f : exp2f(parts.m[x][hg] - mm);       // a part without weight; not one whose sum is NaN
+      acc += e * *part(x, hg, d);
+      ll += e * parts.l[x][hg];
+    }
+    if (splits == 1) {
+      res[i] = T(len > 0 ? acc / ll : 0.f);
+    } else {
+      *part(0, hg, d) = acc;
+      if (d == 0) { parts.cm[hg] = mm; parts.cl[hg] = ll; }
+    }
+  }
+  if (splits == 1) return;
+  cluster_sync_all();
+  for (int i = split * W * 32 + threadIdx.x; i < cells; i += splits * W * 32) {
+    const int hg = i / dim, d = i - hg * dim;
+    const uint32_t am = smem_u32(&parts.cm[hg]), al = smem_u32(&parts.cl[hg]), ao = smem_u32(part(0, hg, d));
+    float mm = -INFINITY;
+    for (int x = 0; x < splits; ++x) mm = fmaxf(mm, ld_cluster_f32(map_to_cta(am, x)));
+    float acc = 0.f, ll = 0.f;
+    for (int x = 0; x < splits; ++x) {
+      const float pm = ld_cluster_f32(map_to_cta(am, x)), pl = ld_cluster_f32(map_to_cta(al, x)), po = ld_cluster_f32(map_to_cta(ao, x));
+      const float e = pl == 0.f ? 0.f : exp2f(pm - mm);      // all three on the way before the first is needed
+      acc += e * po;
+      ll += e * pl;
+    }
+    res[i] = T(len > 0 ? acc / ll : 0.f);
+  }
+  cluster_sync_all();                            // nobody leaves while its part is being read
+}
+
 template <typename T, int DP, int W, bool PAGE16>   // DP: head dimension rounded up to a multiple of 64; PAGE16: pages of whole 16s
 __global__ void __launch_bounds__(W * 32, 16 / W) dec_attention_kernel(const T* q, long long q_stride, const long long* pos, const FlPagedKv kv,
                                                                         T* out, int heads, int dim, int group, int gparts, float scale_log2) {
   constexpr int KJ = DP / 32, VC = DP / 64;
-  __shared__ float s_m[W][ATT_G], s_l[W][ATT_G], c_m[ATT_G], c_l[ATT_G];
+  __shared__ AttParts<W> parts;
   __shared__ float s_o[W][ATT_G][DP + 4];
+  grid_dep_launch();
+  grid_dep_wait();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
   const int kh = blockIdx.x / gparts, gp = blockIdx.x - kh * gparts, b = blockIdx.y, split = blockIdx.z, splits = gridDim.z;
   const int h0 = kh * group + gp * ATT_G, nh = min(ATT_G, group - gp * ATT_G);
@@ -393,104 +517,175 @@ __global__ void __launch_bounds__(W * 32, 16 / W) dec_attention_kernel(const T* 
       }
     }
     float s[2][2];
-#pragma unroll
-    for (int p = 0; p < 2; ++p) {
-      s[p][0] = s[p][1] = 0.f;
-#pragma unroll
-      for (int j = 0; j < KJ; ++j) {
-        Num<T>::mma(s[p], qa[j][0], qa[j][1], kr[p][j].x, kr[p][j].y);
-        Num<T>::mma(s[p], qa[j][2], qa[j][3], kr[p][j].z, kr[p][j].w);
-      }
-#pragma unroll
-      for (int e = 0; e < 2; ++e) s[p][e] = there >> (2 * p + e) & 1 ? s[p][e] * scale_log2 : -INFINITY;
-    }
+    att_scores<T, KJ>(qa, kr, there, scale_log2, s);
     blk = blk_next;
     blk_next = page_of(base + 32);
     load_keys(base + 16, blk);
-    const float m_old = m;
-    float mx = fmaxf(fmaxf(s[0][0], s[0][1]), fmaxf(s[1][0], s[1][1]));
-    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
-    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
-    // A score may be -inf (an infinite key): 0 stands in for a maximum of -inf, so that a step of nothing else adds nothing.
-    // One that is NaN or +inf makes the sums NaN, and NaN they stay.
-    m = fmaxf(m, mx);
-    const float mn = m == -INFINITY ? 0.f : m;
-    const float f = exp2f(m_old - mn);
-    float add = 0.f;
+    att_values<T, VC>(s, vr, m, l, o);
+  }
+  att_finish<T, DP, W>(parts, &s_o[0][0][0], ATT_G * (DP + 4), m, l, o, nh, dim, len, split, splits,
+                       out + (long long)b * heads * dim + (long long)h0 * dim);
+}
+
+// The same for heads of whole 64 columns in pages of whole 16 tokens, with the pages on the way through shared memory: a warp has a
+// ring of its own, filled by TMA loads of 16 tokens x 64 columns (2 KB, 128-byte swizzle) that its first lane issues.  Through
+// registers a warp has 4 to 8 KB on the way and waits for the values of every step; here it is three steps ahead (24 KB, of 8 warps
+// per SM).  Nor does it ask for the L1 cache, which has no room beside the products' shared memory (thin_gemm.cu): next to those the
+// loads through registers took 57 us a layer for 16 x 2048 tokens, 8 KV heads of 128; these take 25 (20 us of bytes).  The lanes of a
+// quad take chunks 2 t and 2 t + 1 of a row's eight, so that the reads of two rows meet different banks.  Before the wait for the
+// kernel that writes q and the new token's page, the first steps' pages are asked into L2.
+template <int DP> struct AttRing {
+  static constexpr int kHalf = 16 * 128;                       // one box: 16 tokens x 64 columns
+  static constexpr int kStage = 2 * (DP / 64) * kHalf;         // keys, then values
+  static constexpr int kStages = 3 * (128 / DP);
+  static constexpr int kBytes = kStages * kStage;              // per warp
+};
+
+__device__ __forceinline__ void tma_prefetch_2d(const void* tmap, int x, int y) {
+  asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(tmap), "r"(x), "r"(y) : "memory");
+}
+__device__ __forceinline__ uint4 lds_v4(uint32_t addr) {
+  uint4 v;
+  asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
+  return v;
+}
+
+template <typename T, int DP, int W>
+__global__ void __launch_bounds__(W * 32, 8 / W) dec_attention_ring_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
+                                                                            const T* q, long long q_stride, const long long* pos, const FlPagedKv kv,
+                                                                            T* out, int heads, int group, int gparts, float scale_log2) {
+  using Ring = AttRing<DP>;
+  constexpr int KJ = DP / 32, VC = DP / 64, ST = Ring::kStages;
+  extern __shared__ uint8_t att_smem[];
+  __shared__ AttParts<W> parts;
+  __shared__ uint64_t full[W][ST];
+  __shared__ int abort_flag;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+  const int kh = blockIdx.x / gparts, gp = blockIdx.x - kh * gparts, b = blockIdx.y, split = blockIdx.z, splits = gridDim.z;
+  const int h0 = kh * group + gp * ATT_G, nh = min(ATT_G, group - gp * ATT_G);
+  const int bs = kv.block_size;
+  const long long cap = (long long)kv.table_stride * bs;
+  uint8_t* rings = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(att_smem) + 1023) & ~uintptr_t(1023));
+  uint8_t* ring = rings + warp * Ring::kBytes;
+  const int* table = kv.block_table + (long long)b * kv.table_stride;
+  const int rows = kv.layers * kv.num_blocks * bs;               // rows of the tensor maps: a box from here on reads zeros
+
+  if (lane == 0) {
+    for (int s = 0; s < ST; ++s) mbar_init(&full[warp][s], 1);
+    mbar_fence_init();
+  }
+  if (threadIdx.x == 0) abort_flag = 0;
+  __syncthreads();
+  grid_dep_launch();
+
+  // this warp's tokens: whole groups of 16, dealt out evenly over the warps of all splits
+  int len, first, last, ids;
+  auto plan = [&]() {
+    len = (int)min(max(__ldcg(pos + b) + 1, 0ll), cap);
+    const int units = (len + 15) / 16, nw = splits * W, w = split * W + warp;
+    const int per = units / nw, extra = units % nw;
+    first = w * per + min(w, extra);
+    last = first + per + (w < extra ? 1 : 0);
+  };
+  // the row of a group of 16 tokens in the pools, `rows` if its page is not there; ids: what the lanes hold of the block table
+  auto page_ids = [&](int u0) { ids = u0 + lane < last ? __ldcg(table + (long long)(u0 + lane) * 16 / bs) : -1; };
+  auto row_of = [&](int u, int id) -> int {
+    if (id < 0) id += kv.num_blocks;
+    if (id < 0 || id >= kv.num_blocks) return rows;
+    return (kv.layer * kv.num_blocks + id) * bs + u * 16 % bs;
+  };
+  if (lane == 0) {
+    tma_prefetch_desc(&tm_k);
+    tma_prefetch_desc(&tm_v);
+  }
+  // a look ahead, before the wait: whatever it finds only says what is worth having in L2
+  plan();
+  page_ids(first);
+  if (lane < min(last - first, 2 * ST)) {
+    const int row = row_of(first + lane, ids);
+    if (row < rows) {
 #pragma unroll
-    for (int p = 0; p < 2; ++p)
-#pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        s[p][e] = exp2f(s[p][e] - mn);
-        add += s[p][e];
-      }
-    l = l * f + add;                             // this lane's tokens only; summed over the quad at the end
-    const uint32_t p0 = Num<T>::pack(s[0][0], s[0][1]), p1 = Num<T>::pack(s[1][0], s[1][1]);
-#pragma unroll
-    for (int c = 0; c < VC; ++c) {
-      const uint32_t v0[4] = {vr[0][c].x, vr[0][c].y, vr[0][c].z, vr[0][c].w};
-      const uint32_t v1[4] = {vr[1][c].x, vr[1][c].y, vr[1][c].z, vr[1][c].w};
-      const uint32_t v2[4] = {vr[2][c].x, vr[2][c].y, vr[2][c].z, vr[2][c].w};
-      const uint32_t v3[4] = {vr[3][c].x, vr[3][c].y, vr[3][c].z, vr[3][c].w};
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        o[c][j][0] *= f;
-        o[c][j][1] *= f;
-        const uint32_t sel = (j & 1) ? 0x7632u : 0x5410u;
-        Num<T>::mma(o[c][j], p0, p1, __byte_perm(v0[j >> 1], v1[j >> 1], sel), __byte_perm(v2[j >> 1], v3[j >> 1], sel));
+      for (int c = 0; c < VC; ++c) {
+        tma_prefetch_2d(&tm_k, kh * DP + 64 * c, row);
+        tma_prefetch_2d(&tm_v, kh * DP + 64 * c, row);
       }
     }
   }
-  l += __shfl_xor_sync(0xffffffffu, l, 1);
-  l += __shfl_xor_sync(0xffffffffu, l, 2);
-  if (t == 0) { s_m[warp][g] = m; s_l[warp][g] = l; }
+  grid_dep_wait();
+  plan();
+  page_ids(first);
+
+  int ids_at = first;                                            // lane i holds the page of unit ids_at + i
+  auto fetch = [&](int u) {                                      // every lane calls it
+    if (u >= ids_at + 32) { ids_at += 32; page_ids(ids_at); }
+    const int id = __shfl_sync(0xffffffffu, ids, u - ids_at);
+    const int row = row_of(u, id);
+    if (lane == 0) {
+      const int s = (u - first) % ST;
+      uint8_t* dst = ring + s * Ring::kStage;
+      mbar_arrive_expect_tx(&full[warp][s], Ring::kStage);
+#pragma unroll
+      for (int c = 0; c < VC; ++c) {
+        tma_load_2d(dst + c * Ring::kHalf, &tm_k, &full[warp][s], kh * DP + 64 * c, row);
+        tma_load_2d(dst + (VC + c) * Ring::kHalf, &tm_v, &full[warp][s], kh * DP + 64 * c, row);
+      }
+    }
+    return row < rows;
+  };
+  unsigned present = 0;                                          // bit s: the page in stage s is one of the pool
+  for (int u = first; u < min(last, first + ST); ++u) present |= (fetch(u) ? 1u : 0u) << (u - first);
+
+  uint32_t qa[KJ][4];
+#pragma unroll
+  for (int j = 0; j < KJ; ++j) {
+    const int d = 64 * (j >> 1) + 16 * t + 8 * (j & 1);
+    uint4 u = make_uint4(0, 0, 0, 0);
+    if (g < nh) u = ld_v4(q + (long long)b * q_stride + (long long)(h0 + g) * DP + d);
+    qa[j][0] = u.x; qa[j][1] = u.y; qa[j][2] = u.z; qa[j][3] = u.w;
+  }
+  float o[VC][8][2];
 #pragma unroll
   for (int c = 0; c < VC; ++c)
 #pragma unroll
-    for (int j = 0; j < 8; j += 4) {
-      *reinterpret_cast<float4*>(&s_o[warp][g][64 * c + 16 * t + j]) = make_float4(o[c][j][0], o[c][j + 1][0], o[c][j + 2][0], o[c][j + 3][0]);
-      *reinterpret_cast<float4*>(&s_o[warp][g][64 * c + 16 * t + 8 + j]) = make_float4(o[c][j][1], o[c][j + 1][1], o[c][j + 2][1], o[c][j + 3][1]);
+    for (int j = 0; j < 8; ++j) o[c][j][0] = o[c][j][1] = 0.f;
+  float m = -INFINITY, l = 0.f;
+
+  for (int u = first; u < last; ++u) {
+    const int s = (u - first) % ST;
+    if (!mbar_wait(&full[warp][s], ((u - first) / ST) & 1, &abort_flag, nullptr, kTimeoutMbarFull, 0)) {
+      note(kv.status, FL_DEC_STALLED);
+      for (int j = 0; j < 2000; ++j) __nanosleep(1000);          // copies on the way land before shared memory goes away
+      break;
     }
-  __syncthreads();
-  // merge the warps: with one split this is the result, otherwise it replaces the first warp's part
-  const int cells = nh * dim;
-  T* res = out + (long long)b * heads * dim + (long long)h0 * dim;
-  for (int i = threadIdx.x; i < cells; i += W * 32) {
-    const int hg = i / dim, d = i - hg * dim;
-    float mm = -INFINITY;
+    const uint32_t at = smem_u32(ring + s * Ring::kStage);
+    uint4 kr[2][KJ], vr[4][VC];
 #pragma unroll
-    for (int x = 0; x < W; ++x) mm = fmaxf(mm, s_m[x][hg]);
-    float acc = 0.f, ll = 0.f;
+    for (int p = 0; p < 2; ++p)
 #pragma unroll
-    for (int x = 0; x < W; ++x) {
-      const float e = s_l[x][hg] == 0.f ? 0.f : exp2f(s_m[x][hg] - mm);       // a part without weight; not one whose sum is NaN
-      acc += e * s_o[x][hg][d];
-      ll += e * s_l[x][hg];
+      for (int j = 0; j < KJ; ++j)
+        kr[p][j] = lds_v4(at + (j >> 1) * Ring::kHalf + (8 * p + g) * 128 + (((2 * t + (j & 1)) ^ g) << 4));
+    unsigned there = 0;
+    const bool page = present >> s & 1;
+    if (!page) note(kv.status, FL_DEC_BAD_PAGE);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int tok = 2 * t + (i & 1) + 8 * (i >> 1);
+      const bool in = page && u * 16 + tok < len;
+      there |= (in ? 1u : 0u) << i;
+#pragma unroll
+      for (int c = 0; c < VC; ++c) {
+        vr[i][c] = lds_v4(at + (VC + c) * Ring::kHalf + tok * 128 + ((g ^ (tok & 7)) << 4));
+        if (!in) vr[i][c] = make_uint4(0, 0, 0, 0);              // what a page holds behind the context may be anything
+      }
     }
-    if (splits == 1) {
-      res[i] = T(len > 0 ? acc / ll : 0.f);
-    } else {
-      s_o[0][hg][d] = acc;
-      if (d == 0) { c_m[hg] = mm; c_l[hg] = ll; }
-    }
+    float sc[2][2];
+    att_scores<T, KJ>(qa, kr, there, scale_log2, sc);
+    __syncwarp();                                                // the stage has been read
+    if (u + ST < last) present = (present & ~(1u << s)) | ((fetch(u + ST) ? 1u : 0u) << s);
+    att_values<T, VC>(sc, vr, m, l, o);
   }
-  if (splits == 1) return;
-  cluster_sync_all();
-  for (int i = split * W * 32 + threadIdx.x; i < cells; i += splits * W * 32) {
-    const int hg = i / dim, d = i - hg * dim;
-    const uint32_t am = smem_u32(&c_m[hg]), al = smem_u32(&c_l[hg]), ao = smem_u32(&s_o[0][hg][d]);
-    float mm = -INFINITY;
-    for (int x = 0; x < splits; ++x) mm = fmaxf(mm, ld_cluster_f32(map_to_cta(am, x)));
-    float acc = 0.f, ll = 0.f;
-    for (int x = 0; x < splits; ++x) {
-      const float pm = ld_cluster_f32(map_to_cta(am, x)), pl = ld_cluster_f32(map_to_cta(al, x)), po = ld_cluster_f32(map_to_cta(ao, x));
-      const float e = pl == 0.f ? 0.f : exp2f(pm - mm);      // all three on the way before the first is needed
-      acc += e * po;
-      ll += e * pl;
-    }
-    res[i] = T(len > 0 ? acc / ll : 0.f);
-  }
-  cluster_sync_all();                            // nobody leaves while its part is being read
+  att_finish<T, DP, W>(parts, reinterpret_cast<float*>(rings), Ring::kBytes / 4, m, l, o, nh, DP, len, split, splits,
+                       out + (long long)b * heads * DP + (long long)h0 * DP);
 }
 
 // ---- greedy choice ----------------------------------------------------------------------------------------------------------
@@ -499,6 +694,8 @@ template <typename T>
 __global__ void __launch_bounds__(1024) dec_argmax_kernel(const T* logits, long long* out, long long vocab) {
   __shared__ float sv[32];
   __shared__ long long si[32];
+  grid_dep_launch();
+  grid_dep_wait();
   const T* row = logits + blockIdx.x * vocab;
   float best = -INFINITY;
   long long at = vocab;                                   // vocab: nothing seen yet
@@ -538,6 +735,7 @@ __global__ void __launch_bounds__(1024) dec_argmax_kernel(const T* logits, long 
 
 __global__ void __launch_bounds__(256) dec_advance_kernel(const long long* next, long long* tokens, long long* pos, long long* history,
                                                           long long* step, int batch, int rows) {
+  grid_dep_wait();
   const long long k = *step;
   for (int b = threadIdx.x; b < batch; b += blockDim.x) {
     if (k >= 0 && k < rows) history[k * batch + b] = next[b];
@@ -563,6 +761,23 @@ static bool aligned(std::initializer_list<const void*> pointers) {
   uintptr_t all = 0;
   for (const void* p : pointers) all |= reinterpret_cast<uintptr_t>(p);
   return (all & 15) == 0;
+}
+
+// Launches a kernel that may start while the one before it in the stream ends (it calls grid_dep_wait before it touches memory): the
+// launch itself, 2 to 3 us in a chain of kernels that take no longer, is then out of the way.  dec_embed_kernel is launched
+// without: it begins a chain, in which weights written by whatever came before are complete.
+template <typename... P, typename... A>
+static int launch_chained(void (*kernel)(P...), unsigned grid, unsigned threads, cudaStream_t stream, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid, 1, 1);
+  cfg.blockDim = dim3(threads, 1, 1);
+  cfg.stream = stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return (int)cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
 
 #define FL_DEC_TYPES(dtype, ...)                                             \
@@ -593,10 +808,9 @@ extern "C" int fl_dec_add_norm(int dtype, void* x, const void* y, const void* y_
   // few rows: one vector per thread, as many threads as that takes; many rows: two per thread keeps more CTAs resident
   const int vpt = vecs > 2048 ? 4 : (vecs > 1024 || (rows > 148 && vecs > 128)) ? 2 : 1;
   const int threads = ((vecs + vpt - 1) / vpt + 31) / 32 * 32;
-#define FL_NORM(V) fl::dec_add_norm_kernel<T, V><<<(unsigned)rows, threads, 0, stream>>>((T*)x, (const T*)y, (const T*)y_bias, (const T*)w, (const T*)b, (T*)h, hidden, eps)
+#define FL_NORM(V) return launch_chained(fl::dec_add_norm_kernel<T, V>, (unsigned)rows, threads, stream, (T*)x, (const T*)y, (const T*)y_bias, (const T*)w, (const T*)b, (T*)h, hidden, eps)
   FL_DEC_TYPES(dtype, { if (vpt == 4) FL_NORM(4); else if (vpt == 2) FL_NORM(2); else FL_NORM(1); });
 #undef FL_NORM
-  return (int)cudaGetLastError();
 }
 
 extern "C" int fl_dec_qkv(int dtype, void* qkv, const void* bias, const float* rope, long long rope_rows, const long long* pos,
@@ -604,9 +818,8 @@ extern "C" int fl_dec_qkv(int dtype, void* qkv, const void* bias, const float* r
   if (dim % 16 || dim < 16 || heads < 1 || kv->heads < 1 || kv->block_size < 1 || rows < 0 || (pos == nullptr && seq < 1)) return -2;
   if (!aligned({qkv, bias, kv->k, kv->v})) return -4;
   if (rows == 0) return 0;
-  FL_DEC_TYPES(dtype, (fl::dec_qkv_kernel<T><<<grid_for(rows * (heads + 2 * kv->heads) * (dim / 16)), 256, 0, stream>>>(
-                          (T*)qkv, (const T*)bias, rope, rope_rows, pos, rows, seq, heads, dim, *kv)));
-  return (int)cudaGetLastError();
+  FL_DEC_TYPES(dtype, return launch_chained(fl::dec_qkv_kernel<T>, grid_for(rows * (heads + 2 * kv->heads) * (dim / 16)), 256, stream, (T*)qkv,
+                                            (const T*)bias, rope, rope_rows, pos, rows, seq, heads, dim, *kv));
 }
 
 extern "C" int fl_dec_act(int dtype, int kind, const void* h, const void* bias, void* out, long long rows, int ffn, cudaStream_t stream) {
@@ -614,7 +827,7 @@ extern "C" int fl_dec_act(int dtype, int kind, const void* h, const void* bias, 
   if (!aligned({h, bias, out})) return -4;
   if (rows == 0) return 0;
   const unsigned grid = grid_for(rows * (ffn / 8));
-#define FL_ACT(K) fl::dec_act_kernel<T, K><<<grid, 256, 0, stream>>>((const T*)h, (const T*)bias, (T*)out, rows, ffn)
+#define FL_ACT(K) return launch_chained(fl::dec_act_kernel<T, K>, grid, 256, stream, (const T*)h, (const T*)bias, (T*)out, rows, ffn)
   FL_DEC_TYPES(dtype, {
     if (kind == FL_ACT_SILU_GATED) FL_ACT(FL_ACT_SILU_GATED);
     else if (kind == FL_ACT_RELU) FL_ACT(FL_ACT_RELU);
@@ -622,7 +835,6 @@ extern "C" int fl_dec_act(int dtype, int kind, const void* h, const void* bias, 
     else return -3;
   });
 #undef FL_ACT
-  return (int)cudaGetLastError();
 }
 
 template <typename T, int DP, int W>
@@ -632,14 +844,47 @@ static int launch_attention(const void* q, long long q_stride, const long long* 
   cfg.gridDim = dim3(kv->heads * gparts, batch, splits);
   cfg.blockDim = dim3(W * 32, 1, 1);
   cfg.stream = stream;
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeClusterDimension;
   at[0].val.clusterDim.x = 1; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = splits;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = 2;
   const float scale = 1.4426950408889634f / sqrtf((float)dim);
   auto kernel = kv->block_size % 16 == 0 ? fl::dec_attention_kernel<T, DP, W, true> : fl::dec_attention_kernel<T, DP, W, false>;
   return (int)cudaLaunchKernelEx(&cfg, kernel, (const T*)q, q_stride, pos, *kv, (T*)out, heads, dim, group, gparts, scale);
+}
+
+template <typename T, int DP, int W>
+static int launch_attention_ring(const CUtensorMap& tm_k, const CUtensorMap& tm_v, const void* q, long long q_stride, const long long* pos,
+                                 const FlPagedKv* kv, void* out, int batch, int heads, int group, int gparts, int splits, cudaStream_t stream) {
+  constexpr int smem = W * fl::AttRing<DP>::kBytes + 1024;
+  static bool set_on[64];                          // per device: a process may drive several GPUs
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return (int)e;
+  if (dev < 0 || dev >= 64) return -3;
+  if (!set_on[dev]) {
+    e = cudaFuncSetAttribute(fl::dec_attention_ring_kernel<T, DP, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return (int)e;
+    set_on[dev] = true;
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(kv->heads * gparts, batch, splits);
+  cfg.blockDim = dim3(W * 32, 1, 1);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = 1; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = splits;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 2;
+  const float scale = 1.4426950408889634f / sqrtf((float)DP);
+  return (int)cudaLaunchKernelEx(&cfg, fl::dec_attention_ring_kernel<T, DP, W>, tm_k, tm_v, (const T*)q, q_stride, pos, *kv, (T*)out, heads, group,
+                                 gparts, scale);
 }
 
 // How the context is cut: enough CTAs for sixteen warps per SM (a warp keeps 4 to 8 KB on the way, and that many saturate
@@ -653,11 +898,30 @@ extern "C" int fl_dec_attention(int dtype, const void* q, long long q_stride, co
   if (!aligned({q, kv->k, kv->v})) return -4;
   const int group = heads / kv->heads, gparts = (group + fl::ATT_G - 1) / fl::ATT_G;
   const long long units = (long long)batch * kv->heads * gparts, cap = (long long)kv->table_stride * kv->block_size;
-  long long splits = 4 * 148 / units;
+  // Heads of 64 or 128 in pages of whole 16 tokens, of a pool whose rows 32 bits count: through the ring, two CTAs of four warps per
+  // SM, if that is three steps for each of them.  Below, its start (descriptors, barriers) costs more than it hides: 3 x 400 tokens,
+  // 32 heads of 64, take 13 us through it and 9 without.
+  const long long rows = (long long)kv->layers * kv->num_blocks * kv->block_size;
+  const bool ring = (dim == 64 || dim == 128) && kv->block_size % 16 == 0 && rows > 0 && rows < 0x7fffffffll && units * (cap / 16) >= 3 * 8 * 148;
+  long long splits = (ring ? 2 : 4) * 148 / units;
   if (splits > (cap + 127) / 128) splits = (cap + 127) / 128;
   if (splits > 8) splits = 8;
   if (splits < 1) splits = 1;
-  const bool wide = units * splits <= 2 * 148 && cap >= splits * 8 * 32;
+  const bool wide = units * splits <= (ring ? 1 : 2) * 148 && cap >= splits * 8 * 32;
+  if (ring) {
+    if (dtype != FL_DEC_BF16 && dtype != FL_DEC_FP16) return -1;
+    const int type = dtype == FL_DEC_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
+    CUtensorMap tm_k, tm_v;
+    int rc = fl::tile_map(&tm_k, type, kv->k, (long long)kv->heads * dim, rows, 16);
+    if (rc == 0) rc = fl::tile_map(&tm_v, type, kv->v, (long long)kv->heads * dim, rows, 16);
+    if (rc != 0) return rc;
+#define FL_ATT(D, W) return launch_attention_ring<T, D, W>(tm_k, tm_v, q, q_stride, pos, kv, out, batch, heads, group, gparts, (int)splits, stream)
+    FL_DEC_TYPES(dtype, {
+      if (dim == 64) { if (wide) FL_ATT(64, 8); else FL_ATT(64, 4); }
+      else { if (wide) FL_ATT(128, 8); else FL_ATT(128, 4); }
+    });
+#undef FL_ATT
+  }
 #define FL_ATT(D, W) return launch_attention<T, D, W>(q, q_stride, pos, kv, out, batch, heads, dim, group, gparts, (int)splits, stream)
   FL_DEC_TYPES(dtype, {
     if (dim <= 64) { if (wide) FL_ATT(64, 8); else FL_ATT(64, 4); }
@@ -670,13 +934,11 @@ extern "C" int fl_dec_attention(int dtype, const void* q, long long q_stride, co
 extern "C" int fl_dec_argmax(int dtype, const void* logits, long long* out, int rows, long long vocab, cudaStream_t stream) {
   if (rows < 0 || vocab < 1) return -2;
   if (rows == 0) return 0;
-  FL_DEC_TYPES(dtype, (fl::dec_argmax_kernel<T><<<rows, 1024, 0, stream>>>((const T*)logits, out, vocab)));
-  return (int)cudaGetLastError();
+  FL_DEC_TYPES(dtype, return launch_chained(fl::dec_argmax_kernel<T>, rows, 1024, stream, (const T*)logits, out, vocab));
 }
 
 extern "C" int fl_dec_advance(const long long* next, long long* tokens, long long* pos, long long* history, long long* step, int batch,
                               int rows, cudaStream_t stream) {
   if (batch < 1) return -2;
-  fl::dec_advance_kernel<<<1, 256, 0, stream>>>(next, tokens, pos, history, step, batch, rows);
-  return (int)cudaGetLastError();
+  return launch_chained(fl::dec_advance_kernel, 1, 256, stream, next, tokens, pos, history, step, batch, rows);
 }

@@ -10,7 +10,8 @@ enum FlDecAct : int { FL_ACT_SILU_GATED = 0, FL_ACT_RELU = 1, FL_ACT_GELU_TANH =
 // What a kernel writes to the status word (device memory or mapped host memory, or null) when an index is outside its table; the
 // access is skipped: a row of zeros for the token, no position added, no page written, the page left out of the attention.
 // Negative indices count from the end.
-enum FlDecStatus : int { FL_DEC_BAD_TOKEN = 1, FL_DEC_BAD_POSITION = 2, FL_DEC_BAD_PAGE = 3 };
+enum FlDecStatus : int { FL_DEC_BAD_TOKEN = 1, FL_DEC_BAD_POSITION = 2, FL_DEC_BAD_PAGE = 3,
+                        FL_DEC_STALLED = 4 /* a kernel that waited for its operands in vain */ };
 
 // Where the keys and values of a token go.  Layouts are those of kv_pack.cuh.
 struct FlPagedKv {

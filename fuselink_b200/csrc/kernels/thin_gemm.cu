@@ -1,0 +1,271 @@
+// y = f(x w^T + bias) for a handful of rows x: the matrix products of a decoding step.
+//
+// Bound by reading w once.  A CTA streams 128 rows of w through shared memory, 64 columns (16 KB) per TMA load, and multiplies them
+// with the same columns of x on the tensor cores (tcgen05, M = 128 rows of w, N = 16 rows of x); the sums stay in TMEM until the last
+// block.  Two CTAs of about 100 KB share an SM, so 160 KB of w per SM are on the way.  Matrices with fewer than 148 x 2 such tiles are
+// cut along k over a cluster of up to eight CTAs.  Each stores its sums straight from TMEM into the shared memory of the CTA that owns
+// the row of x, which adds them up, always in the same order: no workspace, no atomics, and the same bits on every run.  (Blocks dealt
+// out evenly over all CTAs, with shared tiles summed through global memory, were tried: the last CTA's trip for the others' sums costs
+// 8 us, more than the uneven grids, 6144 x 4096 and 16 rows: 21 us against 13.)
+//
+// A step is a chain of about ten short kernels per layer.  Launched one after the other, each fills its pipeline from an idle
+// memory and drains it into one.  With `early` a kernel starts as soon as the one before it has started and the SMs have room, and
+// requests its first blocks of w, which do not depend on that kernel; it waits (griddepcontrol.wait) before it reads x.
+//
+// 16 rows, one product after another with w from memory: 6144 x 4096 13.1 us (library 11.7), 4096 x 4096 9.4 (9.3), 2 x 14336 x 4096
+// with the activation 39.8 (40.9 without it), 4096 x 14336 22.3 (23.0); 3 rows: 2048 x 8192 9.4 (17.9), 2048 x 2048 4.3 (6.4).  What
+// counts is the chain: with library products a layer of an 8B model at 16 rows and 2048 tokens took 143 us, with these and the
+// attention's ring (decoder.cu) 121.  At 32 rows they are slower than the library's (15.0, 11.1, 42.6 and 24.5 us against 12.1, 9.4,
+// 41.0 and 27.1), and so is the step, by 6 %: the line is at 16.
+#include "thin_gemm.cuh"
+#include "decoder.cuh"
+#include <cuda_bf16.h>
+#include <cuda_fp16.h>
+#include "../common/fl_ptx.cuh"
+#include "tile_map.cuh"
+
+namespace fl {
+
+constexpr int TG_M = 128;                          // rows of w per tile
+constexpr int TG_N = FL_THIN_MAX_ROWS;             // rows of x, padded
+constexpr int TG_K = 64;                           // columns per block: one 128-byte swizzle row
+constexpr int TG_W_BYTES = TG_M * TG_K * 2;
+constexpr int TG_STAGE_BYTES = TG_W_BYTES + TG_N * TG_K * 2;
+constexpr int TG_STAGES = 5;
+constexpr int TG_PART_BYTES = TG_N * TG_M * 4;     // what the cluster's CTAs send this one: [CTA][row of x][row of w] fp32
+constexpr int TG_SMEM = TG_STAGES * TG_STAGE_BYTES + TG_PART_BYTES + 1024 /*alignment*/;
+constexpr int TG_TMEM_COLS = 32;
+constexpr int TG_THREADS = 128;
+
+template <typename T> struct ThinNum;
+template <> struct ThinNum<__nv_bfloat16> {
+  static constexpr uint32_t kFmt = 1;
+  static __device__ __forceinline__ float round(float a) { return __bfloat162float(__float2bfloat16_rn(a)); }
+};
+template <> struct ThinNum<__half> {
+  static constexpr uint32_t kFmt = 0;
+  static __device__ __forceinline__ float round(float a) { return __half2float(__float2half_rn(a)); }
+};
+
+__device__ __forceinline__ void st_cluster_float(uint32_t addr, float v) {
+  asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
+}
+__device__ __forceinline__ void cluster_arrive_all() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait_all() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+
+template <typename T>
+__global__ void __launch_bounds__(TG_THREADS, 2)
+thin_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_x, const T* bias, T* y, const int rows,
+                 const long long n, const int k, const int splits, const int epilogue, const int early, int* status) {
+  extern __shared__ uint8_t smem_raw[];
+  __shared__ uint64_t full[TG_STAGES], empty[TG_STAGES], done;
+  __shared__ uint32_t tmem_base_s;
+  __shared__ int abort_flag;
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int split = blockIdx.x % splits;                        // = rank in the cluster
+  const long long tile = blockIdx.x / splits;
+  const bool gated = epilogue == FL_THIN_SILU_GATED;
+  const long long n0 = tile * (gated ? TG_M / 2 : TG_M);        // first output column
+  const int blocks = (k + TG_K - 1) / TG_K;
+  const int first = (int)((long long)split * blocks / splits), last = (int)((long long)(split + 1) * blocks / splits);
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < TG_STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
+    mbar_init(&done, 1);
+    abort_flag = 0;
+    mbar_fence_init();
+    tma_prefetch_desc(&tm_w);
+    tma_prefetch_desc(&tm_x);
+  }
+  if (warp == 1) {
+    tmem_alloc(&tmem_base_s, TG_TMEM_COLS);
+    tmem_relinquish();
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  tc_fence_after_sync();
+  if (splits > 1) cluster_arrive_all();                         // waited for before the first store into another CTA
+  grid_dep_launch();
+  const uint32_t tmem_base = tmem_base_s;
+
+  if (warp == 0 && lane == 0) {
+    // ---- loads: w of the first stages before the wait for the kernel that makes x, where w may be read that early
+    auto load_w = [&](int b) {
+      const int s = (b - first) % TG_STAGES;
+      uint8_t* dst = smem + s * TG_STAGE_BYTES;
+      mbar_arrive_expect_tx(&full[s], TG_STAGE_BYTES);
+      if (gated) {                                              // 64 gate rows and the 64 up rows that belong to them
+        tma_load_2d(dst, &tm_w, &full[s], b * TG_K, (int)n0);
+        tma_load_2d(dst + TG_W_BYTES / 2, &tm_w, &full[s], b * TG_K, (int)(n + n0));
+      } else {
+        tma_load_2d(dst, &tm_w, &full[s], b * TG_K, (int)n0);
+      }
+    };
+    auto load_x = [&](int b) {
+      const int s = (b - first) % TG_STAGES;
+      tma_load_2d(smem + s * TG_STAGE_BYTES + TG_W_BYTES, &tm_x, &full[s], b * TG_K, 0);
+    };
+    const int ahead = min(last, first + TG_STAGES);
+    if (!early) grid_dep_wait();
+    for (int b = first; b < ahead; ++b) load_w(b);
+    if (early) grid_dep_wait();
+    for (int b = first; b < ahead; ++b) load_x(b);
+    for (int b = ahead; b < last; ++b) {
+      const int i = b - first;
+      if (!mbar_wait(&empty[i % TG_STAGES], ((i / TG_STAGES) & 1) ^ 1, &abort_flag, nullptr, kTimeoutMbarEmpty, 0)) {
+        for (int j = 0; j < 2000; ++j) __nanosleep(1000);       // copies on the way land before shared memory goes away
+        break;
+      }
+      load_w(b);
+      load_x(b);
+    }
+  } else if (warp == 1 && lane == 0) {
+    // ---- products
+    constexpr uint32_t idesc = make_idesc(ThinNum<T>::kFmt, ThinNum<T>::kFmt, 0, 0, TG_M, TG_N);
+    bool ok = true;
+    for (int b = first; b < last && ok; ++b) {
+      const int i = b - first, s = i % TG_STAGES;
+      ok = mbar_wait(&full[s], (i / TG_STAGES) & 1, &abort_flag, nullptr, kTimeoutMbarFull, 0);
+      if (!ok) break;
+      tc_fence_after_sync();
+      const uint32_t w_base = smem_u32(smem + s * TG_STAGE_BYTES), x_base = w_base + TG_W_BYTES;
+#pragma unroll
+      for (int kk = 0; kk < TG_K / 16; ++kk)
+        umma_f16(tmem_base, make_smem_desc(w_base + kk * 32, 16, 1024), make_smem_desc(x_base + kk * 32, 16, 1024), idesc, (i | kk) != 0);
+      umma_commit(&empty[s]);
+    }
+    if (ok) umma_commit(&done);
+  }
+  __syncwarp();
+  grid_dep_wait();                                              // y may still be read by kernels before this one
+  const bool have = mbar_wait(&done, 0, &abort_flag, nullptr, kTimeoutTmemFull, 0);
+  tc_fence_after_sync();
+  if (!have && status != nullptr) *reinterpret_cast<volatile int*>(status) = FL_DEC_STALLED;
+
+  // ---- sums to the CTAs that own the rows of x: row r belongs to CTA r % splits, as its row r / splits
+  float* part = reinterpret_cast<float*>(smem + TG_STAGES * TG_STAGE_BYTES);
+  const int own = (rows + splits - 1) / splits;                 // rows per CTA; rows <= TG_N and splits divides TG_N: own * splits <= TG_N
+  if (splits > 1) cluster_wait_all();
+  if (have) {
+    uint32_t v[32];                                             // the second half: columns that the products do not write
+    tmem_ld_32x32(tmem_base + ((uint32_t)(warp * 32) << 16), v);
+    tmem_ld_wait();
+    const uint32_t at = smem_u32(part + split * own * TG_M + threadIdx.x);
+#pragma unroll
+    for (int r = 0; r < TG_N; ++r) {
+      if (r < rows) {
+        if (splits == 1) part[r * TG_M + threadIdx.x] = __uint_as_float(v[r]);
+        else st_cluster_float(map_to_cta(at + (uint32_t)(r / splits) * TG_M * 4, r % splits), __uint_as_float(v[r]));
+      }
+    }
+  }
+  tc_fence_before_sync();
+  if (splits > 1) cluster_sync_all();
+  else __syncthreads();
+  if (warp == 1) {
+    tc_fence_after_sync();
+    tmem_dealloc(tmem_base, TG_TMEM_COLS);
+  }
+
+  // ---- this CTA's rows: two neighbouring columns per lane, the CTAs' sums in their order
+  auto sums = [&](int r, int c) -> float2 {
+    const float* p = part + r / splits * TG_M + c;
+    float2 t = *reinterpret_cast<const float2*>(p);
+    for (int s = 1; s < splits; ++s) {
+      const float2 v = *reinterpret_cast<const float2*>(p + s * own * TG_M);
+      t.x += v.x; t.y += v.y;
+    }
+    return t;
+  };
+  auto store = [&](int r, long long col, float a, float b) {
+    T* p = y + (long long)r * n + col;
+    if (col + 1 < n && (n & 1) == 0) {
+      T two[2] = {T(a), T(b)};
+      *reinterpret_cast<uint32_t*>(p) = *reinterpret_cast<const uint32_t*>(two);
+    } else {
+      if (col < n) p[0] = T(a);
+      if (col + 1 < n) p[1] = T(b);
+    }
+  };
+  using R = ThinNum<T>;
+  if (gated) {
+    const int c = 2 * lane;
+    for (int r = split + splits * warp; r < rows; r += 4 * splits) {
+      const float2 g = sums(r, c), u = sums(r, 64 + c);
+      const float g0 = R::round(g.x), g1 = R::round(g.y);
+      store(r, n0 + c, R::round(g0 / (1.f + expf(-g0))) * R::round(u.x), R::round(g1 / (1.f + expf(-g1))) * R::round(u.y));
+    }
+  } else {
+    const int c = 2 * (threadIdx.x & 63);
+    const long long col = n0 + c;
+    const float b0 = bias != nullptr && col < n ? (float)bias[col] : 0.f, b1 = bias != nullptr && col + 1 < n ? (float)bias[col + 1] : 0.f;
+    for (int r = split + splits * (threadIdx.x >> 6); r < rows; r += 2 * splits) {
+      const float2 t = sums(r, c);
+      float a[2] = {R::round(t.x), R::round(t.y)};
+      if (bias != nullptr) { a[0] = R::round(a[0] + b0); a[1] = R::round(a[1] + b1); }
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        if (epilogue == FL_THIN_RELU) a[j] = a[j] < 0.f ? 0.f : a[j];      // keeps NaN
+        else if (epilogue == FL_THIN_GELU_TANH) a[j] = 0.5f * a[j] * (1.f + tanhf(0.7978845608028654f * (a[j] + 0.044715f * a[j] * a[j] * a[j])));
+      }
+      store(r, col, a[0], a[1]);
+    }
+  }
+}
+
+// --------------------------------------------------------------------------------------------------------------------------
+// host side
+// --------------------------------------------------------------------------------------------------------------------------
+template <typename T>
+static int launch_thin(const CUtensorMap& tm_w, const CUtensorMap& tm_x, const void* bias, void* y, int rows, long long n, int k, long long tiles,
+                       int splits, int epilogue, int early, int* status, cudaStream_t stream) {
+  static bool set_on[64];                          // per device: a process may drive several GPUs
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return (int)e;
+  if (dev < 0 || dev >= 64) return -3;
+  if (!set_on[dev]) {
+    e = cudaFuncSetAttribute(thin_gemm_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, TG_SMEM);
+    if (e != cudaSuccess) return (int)e;
+    set_on[dev] = true;
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(tiles * splits), 1, 1);
+  cfg.blockDim = dim3(TG_THREADS, 1, 1);
+  cfg.dynamicSmemBytes = TG_SMEM;
+  cfg.stream = stream;
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = splits; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = early ? 2 : 1;
+  return (int)cudaLaunchKernelEx(&cfg, thin_gemm_kernel<T>, tm_w, tm_x, (const T*)bias, (T*)y, rows, n, k, splits, epilogue, early, status);
+}
+
+}  // namespace fl
+
+extern "C" int fl_thin_gemm(int dtype, const void* x, int rows, const void* w, long long n, int k, const void* bias, int epilogue, void* y, int early,
+                            int* status, cudaStream_t stream) {
+  using namespace fl;
+  if (dtype != FL_DEC_BF16 && dtype != FL_DEC_FP16) return -1;
+  if (rows < 1 || rows > FL_THIN_MAX_ROWS || n < 1 || n > 0x3fffff00ll || k < 8 || k % 8) return -2;
+  if (epilogue < FL_THIN_SILU_GATED || epilogue > FL_THIN_STORE || (epilogue == FL_THIN_SILU_GATED && bias != nullptr)) return -3;
+  if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 15 || reinterpret_cast<uintptr_t>(y) & 3) return -4;
+  const bool gated = epilogue == FL_THIN_SILU_GATED;
+  const int per_tile = gated ? TG_M / 2 : TG_M, blocks = (k + TG_K - 1) / TG_K;
+  const long long tiles = (n + per_tile - 1) / per_tile;
+  // As many CTAs as fit at two per SM, so that all of them run from start to end at an equal share of the memory's rate; clusters of
+  // 1, 2, 4 or 8, since others leave SMs over (6144 x 4096, 16 rows: 17.2 us in clusters of 6, 13.1 in clusters of 4).
+  int splits = 1;
+  while (splits < 8 && 2 * splits * tiles <= 2 * 148 && 2 * splits <= blocks) splits *= 2;
+  const int type = dtype == FL_DEC_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
+  CUtensorMap tm_w, tm_x;
+  int rc = tile_map(&tm_w, type, w, k, gated ? 2 * n : n, per_tile);
+  if (rc == 0) rc = tile_map(&tm_x, type, x, k, rows, TG_N);
+  if (rc != 0) return rc;
+  if (dtype == FL_DEC_BF16) return launch_thin<__nv_bfloat16>(tm_w, tm_x, bias, y, rows, n, k, tiles, splits, epilogue, early, status, stream);
+  return launch_thin<__half>(tm_w, tm_x, bias, y, rows, n, k, tiles, splits, epilogue, early, status, stream);
+}

@@ -13,6 +13,7 @@
 #include "../kernels/mlp_bwd.cuh"
 #include "../kernels/kv_pack.cuh"
 #include "../kernels/decoder.cuh"
+#include "../kernels/thin_gemm.cuh"
 #include "../kernels/moe_dispatch.cuh"
 #include "../kernels/moe_route.cuh"
 #include "../kernels/fp8_gemm.cuh"
@@ -269,8 +270,8 @@ static const long long* dec_i64(const c10::optional<torch::Tensor>& t, int64_t n
   return reinterpret_cast<const long long*>(t->data_ptr<int64_t>());
 }
 // Whether the kernels may read these tensors (None: not given): plain tensors with memory, of `like`'s type and device, contiguous,
-// from a multiple of 16 bytes on.  Native because a shard asks it about some 200 tensors on every call.
-static bool dec_takes(py::list tensors, torch::Tensor like) {
+// from a multiple of 16 bytes on, and matrices of `shape` where that is given.  Native because a shard asks it about some 200 tensors on every call.
+static bool dec_takes(py::list tensors, torch::Tensor like, c10::optional<std::pair<int64_t, int64_t>> shape) {
   const auto dtype = like.scalar_type();
   const auto device = like.device();
   for (py::handle h : tensors) {
@@ -280,6 +281,7 @@ static bool dec_takes(py::list tensors, torch::Tensor like) {
     if (!t.has_storage() || t.scalar_type() != dtype || t.device() != device || !t.is_contiguous() ||
         (reinterpret_cast<uintptr_t>(t.const_data_ptr()) & 15))
       return false;
+    if (shape.has_value() && (t.dim() != 2 || t.size(0) != shape->first || t.size(1) != shape->second)) return false;
   }
   return true;
 }
@@ -357,6 +359,21 @@ static void dec_attention(torch::Tensor qkv, torch::Tensor pos, torch::Tensor k_
   const FlPagedKv kv = dec_kv(k_pool, v_pool, table, FL_KV_LBSHD, layer, layers, num_blocks, block_size, kv_heads, dim, status_addr);
   check_rc(fl_dec_attention(dt, qkv.data_ptr(), width, dec_i64(pos, batch, "positions: int64"), &kv, out.data_ptr(), (int)batch, (int)heads, (int)dim,
                             cur_stream()), "fl_dec_attention");
+}
+// x [rows, k] times w [n, k], see thin_gemm.cuh
+static torch::Tensor dec_product(torch::Tensor x, torch::Tensor w, c10::optional<torch::Tensor> bias, int64_t epilogue, bool early, int64_t status_addr) {
+  const int dt = dec_dtype(x);
+  TORCH_CHECK(x.dim() == 2 && w.dim() == 2 && x.is_contiguous() && w.is_contiguous() && w.is_cuda() && w.scalar_type() == x.scalar_type() &&
+              w.size(1) == x.size(1) && w.device() == x.device(), "product: x [rows, k] and w [n, k], contiguous, of one type and device");
+  TORCH_CHECK(epilogue != FL_THIN_SILU_GATED || w.size(0) % 2 == 0, "product: gate and up rows in equal number");
+  const int64_t n = epilogue == FL_THIN_SILU_GATED ? w.size(0) / 2 : w.size(0);
+  dec_like(bias, x, n, "bias: [n]");
+  TORCH_CHECK(x.size(1) <= INT32_MAX && x.size(0) <= FL_THIN_MAX_ROWS, "product: too large");
+  c10::cuda::CUDAGuard guard(x.device());
+  auto y = torch::empty({x.size(0), n}, x.options());
+  check_rc(fl_thin_gemm(dt, x.data_ptr(), (int)x.size(0), w.data_ptr(), n, (int)x.size(1), opt_ptr(bias), (int)epilogue, y.data_ptr(), early,
+                        reinterpret_cast<int*>(status_addr), cur_stream()), "fl_thin_gemm");
+  return y;
 }
 static torch::Tensor dec_argmax(torch::Tensor logits) {
   const int dt = dec_dtype(logits);
@@ -565,7 +582,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("barrier", &barrier);
   m.def("embbag", &embbag);
   m.def("kv_pack_send", &kv_pack_send);
-  m.def("dec_takes", &dec_takes);
+  m.def("dec_takes", &dec_takes, py::arg("tensors"), py::arg("like"), py::arg("shape") = py::none());
   m.def("dec_embed", &dec_embed, py::arg("tokens"), py::arg("pos"), py::arg("embed"), py::arg("pos_embed"), py::arg("x"), py::arg("seq"),
         py::arg("offset"), py::arg("status_addr") = 0);
   m.def("dec_add_norm", &dec_add_norm);
@@ -581,6 +598,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("dec_attention", &dec_attention, py::arg("qkv"), py::arg("pos"), py::arg("k_pool"), py::arg("v_pool"), py::arg("table"),
         py::arg("layer"), py::arg("layers"), py::arg("num_blocks"), py::arg("block_size"), py::arg("heads"), py::arg("kv_heads"),
         py::arg("dim"), py::arg("out"), py::arg("status_addr") = 0);
+  m.def("dec_product", &dec_product, py::arg("x"), py::arg("w"), py::arg("bias"), py::arg("epilogue"), py::arg("early") = false,
+        py::arg("status_addr") = 0);
   m.def("dec_argmax", &dec_argmax);
   m.def("dec_advance", &dec_advance);
   m.def("moe_dispatch", &moe_dispatch);

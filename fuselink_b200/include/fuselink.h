@@ -21,5 +21,6 @@
 #include "../csrc/kernels/moe_dispatch_noalloc.cuh"
 #include "../csrc/kernels/moe_route.cuh"
 #include "../csrc/kernels/shadow_reduce.cuh"
+#include "../csrc/kernels/thin_gemm.cuh"
 #include "../csrc/mem/vmm.h"
 #include "../csrc/monitor/monitor.h"

@@ -6,8 +6,8 @@ CMakeLists.txt:116-149: model_llama2, model_opt, model_gpt2).
 
 The reference's serving experiment builds `st::model::Gpt<T>` from an external library with dummy weights
 (experiments/serving/model.hh:165-177) and a table of model shapes (common_gpt_hyper_params.h:10-131).
-Here the matrix products and the attention over a prompt are library calls, tensor-parallel over a process group, with
-random-init bf16 weights; hand-written are the KV hand-off between the stages (csrc/kernels/kv_pack.cu), which this model
+Here the attention over a prompt and the matrix products of more than a handful of rows are library calls, tensor-parallel over a
+process group, with random-init bf16 weights; hand-written are the products of a few rows (csrc/kernels/thin_gemm.cu), the KV hand-off between the stages (csrc/kernels/kv_pack.cu), which this model
 feeds layer by layer through ``on_layer_done``, and, for bf16 and fp16 on the GPU, every pass between the products and the
 attention of a decoding step (csrc/kernels/decoder.cu).  The operation-by-operation formulation below is the same
 computation, rounded at the same places; it serves the CPU, fp32 and head sizes the kernels do not take.
@@ -29,6 +29,8 @@ from .._ext import require_native
 KV_BLHSD, KV_LBSHD = 0, 1
 _OPERATIONS = ("_embed", "_norm", "_qkv", "_attn_out", "_mlp", "_logits")      # what the fused route does by itself
 _ACT = {"llama": 0, "opt": 1, "gpt2": 2}          # FlDecAct
+_STORE = 3                                         # FlThinEpi
+_THIN_ROWS = 16                                    # rows up to which csrc/kernels/thin_gemm.cu makes the products
 
 
 @dataclass
@@ -95,6 +97,7 @@ class _Status:
     without waiting for them.  A copied or unpickled shard has a word of its own."""
     WHAT = {1: "a token outside the vocabulary", 2: "a position outside the position embedding or the block table",
             3: "a page id outside the pool"}
+    STALLED = 4                  # FL_DEC_STALLED
 
     def __init__(self):
         self.word = torch.zeros(1, dtype=torch.int32, pin_memory=torch.cuda.is_available())
@@ -278,7 +281,17 @@ class LlamaShard(torch.nn.Module):
         what = 0 if st is None else int(st.word)
         if what:
             st.word.zero_()
+            if what == _Status.STALLED:
+                raise RuntimeError("decoder: a kernel waited for its operands in vain")
             raise IndexError(f"decoder: {_Status.WHAT.get(what, what)}")
+
+    def _thin(self, rows: int, like: torch.Tensor, *matrices) -> bool:
+        """Whether csrc/kernels/thin_gemm.cu makes the products of so many rows with these (list of matrices, rows, columns): plain
+        tensors of the shard's type and device, contiguous, from a multiple of 16 bytes on.  Others stay the library's."""
+        if not (like.is_cuda and 0 < rows <= _THIN_ROWS):
+            return False
+        C = require_native()
+        return all(C.dec_takes(list(ws), like, shape) for ws, *shape in matrices)
 
     def _layers_fused(self, x, pos, seq, k_pool, v_pool, table, layout, num_blocks, attend, on_layer_done=None):
         """Every layer on x [rows, hidden]; ``attend(l, qkv)`` returns the attention output [rows, h_local * D].  Returns
@@ -287,19 +300,30 @@ class LlamaShard(torch.nn.Module):
         rows, kind, status = x.shape[0], _ACT[cfg.arch], self._status_addr()
         rope = self._rope_table(table.shape[1] * cfg.block_size)
         h = torch.empty_like(x)
-        act = torch.empty(rows, self.f_local, dtype=x.dtype, device=x.device)
+        H, q, F2 = cfg.hidden, self.h_local * cfg.head_dim, self.f_local
+        thin = self._thin(rows, x, (self.wqkv, q + 2 * self.kvh_local * cfg.head_dim, H), (self.wo, H, q),
+                          (self.w13, 2 * F2 if self.gated else F2, H), (self.w2, H, F2))
+        act = None if thin else torch.empty(rows, self.f_local, dtype=x.dtype, device=x.device)
+
+        def product(a, w, b=None, epilogue=_STORE):
+            # `early`: the layers' weights were there before the step's first kernel started
+            return C.dec_product(a, w, b, epilogue, True, status) if thin else a @ w.t()
+
         y = bias = None
         for l in range(cfg.layers):
             C.dec_add_norm(x, y, bias, self.n1[l], self.n1b[l], h, cfg.eps)
-            qkv = h @ self.wqkv[l].t()
+            qkv = product(h, self.wqkv[l])
             C.dec_qkv(qkv, self.bqkv[l], rope, pos, seq, k_pool, v_pool, table, layout, l, cfg.layers, num_blocks, cfg.block_size,
                       self.h_local, self.kvh_local, cfg.head_dim, status)
             if on_layer_done is not None:
                 on_layer_done(l)                                                # KV of this layer may leave now
-            y = self._allreduce(attend(l, qkv) @ self.wo[l].t())
+            y = self._allreduce(product(attend(l, qkv), self.wo[l]))
             C.dec_add_norm(x, y, self.bo[l], self.n2[l], self.n2b[l], h, cfg.eps)
-            C.dec_act(h @ self.w13[l].t(), self.b13[l], act, kind)
-            y, bias = self._allreduce(act @ self.w2[l].t()), self.b2[l]
+            if thin:
+                act = product(h, self.w13[l], self.b13[l], kind)
+            else:
+                C.dec_act(h @ self.w13[l].t(), self.b13[l], act, kind)
+            y, bias = self._allreduce(product(act, self.w2[l])), self.b2[l]
         return x, y, bias
 
     def _choose_fused(self, x, y, bias):
@@ -307,8 +331,12 @@ class LlamaShard(torch.nn.Module):
         C = require_native()
         h = torch.empty_like(x)
         C.dec_add_norm(x, y, bias, self.final_norm, self.final_norm_b, h, self.cfg.eps)
-        logits = h @ self.lm_head.t()
-        return C.dec_argmax(logits.flatten(0, -2)).view(logits.shape[:-1])
+        rows = h.flatten(0, -2)
+        if self.lm_head.dim() == 2 and self._thin(rows.shape[0], rows, ([self.lm_head], self.lm_head.shape[0], h.shape[-1])):
+            logits = C.dec_product(rows, self.lm_head, None, _STORE, True, self._status_addr())
+        else:
+            logits = rows @ self.lm_head.t()
+        return C.dec_argmax(logits).view(h.shape[:-1])
 
     def _prefill_fused(self, tokens, k_pool, v_pool, block_table, on_layer_done, last_pos):
         self.check_status()

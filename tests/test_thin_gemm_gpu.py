@@ -1,0 +1,73 @@
+"""Products of a few rows with a large matrix (csrc/kernels/thin_gemm.cu) against PyTorch."""
+import pytest
+import torch
+import torch.nn.functional as F
+
+pytestmark = pytest.mark.gpu
+DT = [torch.bfloat16, torch.float16]
+
+
+def _eighths(*shape, dt, seed):
+    """Multiples of 1/8 in [-1/2, 1/2]: every sum of their products below 2^18 is exact in fp32, in any order."""
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    return (torch.randint(-4, 5, shape, generator=g, device="cuda") / 8).to(dt)
+
+
+# edges of the tiles (128 rows of w, 64 columns, 16 rows of x) and of the cuts along k (8, 4, 2, 1 CTAs per tile)
+@pytest.mark.parametrize("dt", DT)
+@pytest.mark.parametrize("rows,n,k", [(1, 1, 8), (3, 127, 72), (15, 128, 64), (16, 129, 1024), (9, 2048, 2048), (16, 6144, 520),
+                                      (7, 1000, 8200), (5, 12288, 768), (13, 640, 264), (16, 38000, 128), (2, 50257, 768), (4, 128, 65536)])
+@pytest.mark.parametrize("early", [False, True])
+def test_sums_are_exact(dt, rows, n, k, early):
+    from fuselink_b200 import C
+    x, w, b = _eighths(rows, k, dt=dt, seed=1), _eighths(n, k, dt=dt, seed=2), _eighths(n, dt=dt, seed=3)
+    sums = (x.double() @ w.double().t()).to(dt)
+    for _ in range(2):
+        assert torch.equal(C.dec_product(x, w, None, 3, early), sums)
+    assert torch.equal(C.dec_product(x, w, b, 3, early), sums + b)
+    assert torch.equal(C.dec_product(x, w, b, 1, early), F.relu(sums + b))
+    eps = 2.0 ** -8 if dt == torch.bfloat16 else 2.0 ** -11
+    want = F.gelu(sums + b, approximate="tanh")                     # as for the separate activation kernel
+    assert ((C.dec_product(x, w, b, 2, early) - want).float().abs() <= 2.02 * eps * want.float().abs() + 1e-6).all()
+
+
+@pytest.mark.parametrize("dt", DT)
+@pytest.mark.parametrize("rows,n,k", [(1, 8, 64), (16, 64, 2048), (5, 72, 136), (11, 14336, 512), (16, 1000, 264), (2, 20000, 128)])
+def test_gated(dt, rows, n, k):
+    from fuselink_b200 import C
+    x, w = _eighths(rows, k, dt=dt, seed=1), _eighths(2 * n, k, dt=dt, seed=2)
+    h = (x.double() @ w.double().t()).to(dt)
+    want = F.silu(h[:, :n]) * h[:, n:]
+    eps = 2.0 ** -8 if dt == torch.bfloat16 else 2.0 ** -11
+    # the gate may be rounded to its neighbour (2 eps), the product is rounded once more; 6e-8: fp16's smallest step
+    assert ((C.dec_product(x, w, None, 0) - want).float().abs() <= 4.05 * eps * want.float().abs() + 6e-8).all()
+
+
+@pytest.mark.parametrize("rows,n,k", [(16, 6144, 4096), (3, 2048, 8192)])
+def test_error_of_ordinary_values(rows, n, k):
+    from fuselink_b200 import C
+    g = torch.Generator(device="cuda").manual_seed(5)
+    x, w = (torch.randn(a, k, generator=g, device="cuda").to(torch.bfloat16) for a in (rows, n))
+    want = x.double() @ w.double().t()
+    # rounding to bf16, and one rounding of the running sum (at most the sum of the magnitudes) per 16 products
+    bound = 2.0 ** -8 * want.abs() + (k // 16 + 8) * 2.0 ** -23 * (x.double().abs() @ w.double().abs().t())
+    assert ((C.dec_product(x, w, None, 3).double() - want).abs() <= bound).all()
+
+
+def test_not_finite_values_stay_in_their_row_and_column():
+    from fuselink_b200 import C
+    x, w = _eighths(4, 256, dt=torch.bfloat16, seed=1), _eighths(300, 256, dt=torch.bfloat16, seed=2)
+    x[1, 3], w[7, 9] = float("nan"), float("inf")
+    got = C.dec_product(x, w, None, 1)
+    want = F.relu((x.double() @ w.double().t()).to(torch.bfloat16))
+    assert torch.equal(got.isnan(), want.isnan())
+    assert torch.equal(got.nan_to_num(nan=-1), want.nan_to_num(nan=-1))
+
+
+def test_arguments():
+    from fuselink_b200 import C
+    x, w = torch.zeros(2, 64, dtype=torch.half, device="cuda"), torch.zeros(8, 64, dtype=torch.half, device="cuda")
+    for bad in ((x, w[:, :32].contiguous(), None, 3), (x.repeat(9, 1), w, None, 3), (x, w.bfloat16(), None, 3), (x, w, x[0, :7], 3),
+                (x[:, :63].contiguous(), w[:, :63].contiguous(), None, 3), (x, w[:7], None, 0), (x.view(-1)[1:65].view(1, 64), w, None, 3)):
+        with pytest.raises(RuntimeError):
+            C.dec_product(*bad)
