@@ -11,6 +11,7 @@
 // (experiments/serving/model.hh:165-177).
 #include "decoder.cuh"
 #include "kv_pack.cuh"
+#include "thin_gemm.cuh"
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <math.h>
@@ -689,14 +690,17 @@ __global__ void __launch_bounds__(W * 32, 8 / W) dec_attention_ring_kernel(const
 }
 
 // ---- greedy choice ----------------------------------------------------------------------------------------------------------
-// One CTA per row; a vocabulary row (256 KB at 128256 entries) is 16 loads of 16 bytes per thread, read once.
+// A cluster per row, whose CTAs take stretches of it and whose first one compares what they found.  With one CTA per row, 16 loads of
+// 16 bytes per thread and their comparisons one after the other, a row of 128256 entries took 22 us.
 template <typename T>
 __global__ void __launch_bounds__(1024) dec_argmax_kernel(const T* logits, long long* out, long long vocab) {
-  __shared__ float sv[32];
-  __shared__ long long si[32];
+  __shared__ float sv[32], cv[8];
+  __shared__ long long si[32], ci[8];
+  const int parts = gridDim.x, part = blockIdx.x;           // of the row; a cluster is the CTAs of one row
+  if (parts > 1) cluster_sync_all();                        // all of them are there before one writes into the first
   grid_dep_launch();
   grid_dep_wait();
-  const T* row = logits + blockIdx.x * vocab;
+  const T* row = logits + blockIdx.y * vocab;
   float best = -INFINITY;
   long long at = vocab;                                   // vocab: nothing seen yet
   auto better = [](float v, long long i, float w, long long j) {      // (v, i) before (w, j)
@@ -706,15 +710,15 @@ __global__ void __launch_bounds__(1024) dec_argmax_kernel(const T* logits, long 
     return i < j;
   };
   const bool wide = (reinterpret_cast<uintptr_t>(row) & 15) == 0;
-  const long long vecs = wide ? vocab / 8 : 0;
-  for (long long i = threadIdx.x; i < vecs; i += blockDim.x) {
+  const long long vecs = wide ? vocab / 8 : 0, first = part * (long long)blockDim.x + threadIdx.x, step = parts * (long long)blockDim.x;
+  for (long long i = first; i < vecs; i += step) {
     float v[8];
     unpack8<T>(ld_nc_v4(row + i * 8), v);
 #pragma unroll
     for (int j = 0; j < 8; ++j)
       if (better(v[j], i * 8 + j, best, at)) { best = v[j]; at = i * 8 + j; }
   }
-  for (long long i = vecs * 8 + threadIdx.x; i < vocab; i += blockDim.x) {
+  for (long long i = vecs * 8 + first; i < vocab; i += step) {
     const float v = Num<T>::f(row[i]);
     if (better(v, i, best, at)) { best = v; at = i; }
   }
@@ -729,7 +733,20 @@ __global__ void __launch_bounds__(1024) dec_argmax_kernel(const T* logits, long 
   if (threadIdx.x == 0) {
     for (int k = 1; k < (int)blockDim.x / 32; ++k)
       if (better(sv[k], si[k], best, at)) { best = sv[k]; at = si[k]; }
-    out[blockIdx.x] = at < vocab ? at : 0;
+    if (parts == 1) {
+      out[blockIdx.y] = at < vocab ? at : 0;
+    } else {
+      asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(map_to_cta(smem_u32(&cv[part]), 0)), "f"(best) : "memory");
+      asm volatile("st.shared::cluster.b64 [%0], %1;" ::"r"(map_to_cta(smem_u32(&ci[part]), 0)), "l"(at) : "memory");
+    }
+  }
+  if (parts == 1) return;
+  __syncwarp();
+  cluster_sync_all();
+  if (part == 0 && threadIdx.x == 0) {
+    for (int k = 1; k < parts; ++k)
+      if (better(cv[k], ci[k], best, at)) { best = cv[k]; at = ci[k]; }
+    out[blockIdx.y] = at < vocab ? at : 0;
   }
 }
 
@@ -763,11 +780,14 @@ static bool aligned(std::initializer_list<const void*> pointers) {
   return (all & 15) == 0;
 }
 
-// Launches a kernel that may start while the one before it in the stream ends (it calls grid_dep_wait before it touches memory): the
-// launch itself, 2 to 3 us in a chain of kernels that take no longer, is then out of the way.  dec_embed_kernel is launched
-// without: it begins a chain, in which weights written by whatever came before are complete.
+// Whether a kernel over so many rows may start while the one before it in the stream ends (it calls grid_dep_wait before it touches
+// memory): the launch itself, 2 to 3 us in a chain of kernels that take no longer, is then out of the way.  Only as far as the
+// products are thin_gemm.cu's, which take part in it; between library products it costs (23 requests, 8B model: 15.1 ms without, 15.3
+// with).  dec_embed_kernel is launched without: it begins a chain, in which weights written by whatever came before are complete.
+static bool chained(long long rows) { return rows <= FL_THIN_MAX_ROWS; }
+
 template <typename... P, typename... A>
-static int launch_chained(void (*kernel)(P...), unsigned grid, unsigned threads, cudaStream_t stream, A... args) {
+static int launch_chained(void (*kernel)(P...), long long rows, unsigned grid, unsigned threads, cudaStream_t stream, A... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid, 1, 1);
   cfg.blockDim = dim3(threads, 1, 1);
@@ -776,7 +796,7 @@ static int launch_chained(void (*kernel)(P...), unsigned grid, unsigned threads,
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = chained(rows) ? 1 : 0;
   return (int)cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
 
@@ -808,7 +828,7 @@ extern "C" int fl_dec_add_norm(int dtype, void* x, const void* y, const void* y_
   // few rows: one vector per thread, as many threads as that takes; many rows: two per thread keeps more CTAs resident
   const int vpt = vecs > 2048 ? 4 : (vecs > 1024 || (rows > 148 && vecs > 128)) ? 2 : 1;
   const int threads = ((vecs + vpt - 1) / vpt + 31) / 32 * 32;
-#define FL_NORM(V) return launch_chained(fl::dec_add_norm_kernel<T, V>, (unsigned)rows, threads, stream, (T*)x, (const T*)y, (const T*)y_bias, (const T*)w, (const T*)b, (T*)h, hidden, eps)
+#define FL_NORM(V) return launch_chained(fl::dec_add_norm_kernel<T, V>, rows, (unsigned)rows, threads, stream, (T*)x, (const T*)y, (const T*)y_bias, (const T*)w, (const T*)b, (T*)h, hidden, eps)
   FL_DEC_TYPES(dtype, { if (vpt == 4) FL_NORM(4); else if (vpt == 2) FL_NORM(2); else FL_NORM(1); });
 #undef FL_NORM
 }
@@ -818,7 +838,7 @@ extern "C" int fl_dec_qkv(int dtype, void* qkv, const void* bias, const float* r
   if (dim % 16 || dim < 16 || heads < 1 || kv->heads < 1 || kv->block_size < 1 || rows < 0 || (pos == nullptr && seq < 1)) return -2;
   if (!aligned({qkv, bias, kv->k, kv->v})) return -4;
   if (rows == 0) return 0;
-  FL_DEC_TYPES(dtype, return launch_chained(fl::dec_qkv_kernel<T>, grid_for(rows * (heads + 2 * kv->heads) * (dim / 16)), 256, stream, (T*)qkv,
+  FL_DEC_TYPES(dtype, return launch_chained(fl::dec_qkv_kernel<T>, rows, grid_for(rows * (heads + 2 * kv->heads) * (dim / 16)), 256, stream, (T*)qkv,
                                             (const T*)bias, rope, rope_rows, pos, rows, seq, heads, dim, *kv));
 }
 
@@ -827,7 +847,7 @@ extern "C" int fl_dec_act(int dtype, int kind, const void* h, const void* bias, 
   if (!aligned({h, bias, out})) return -4;
   if (rows == 0) return 0;
   const unsigned grid = grid_for(rows * (ffn / 8));
-#define FL_ACT(K) return launch_chained(fl::dec_act_kernel<T, K>, grid, 256, stream, (const T*)h, (const T*)bias, (T*)out, rows, ffn)
+#define FL_ACT(K) return launch_chained(fl::dec_act_kernel<T, K>, rows, grid, 256, stream, (const T*)h, (const T*)bias, (T*)out, rows, ffn)
   FL_DEC_TYPES(dtype, {
     if (kind == FL_ACT_SILU_GATED) FL_ACT(FL_ACT_SILU_GATED);
     else if (kind == FL_ACT_RELU) FL_ACT(FL_ACT_RELU);
@@ -850,7 +870,7 @@ static int launch_attention(const void* q, long long q_stride, const long long* 
   at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
-  cfg.numAttrs = 2;
+  cfg.numAttrs = chained(batch) ? 2 : 1;
   const float scale = 1.4426950408889634f / sqrtf((float)dim);
   auto kernel = kv->block_size % 16 == 0 ? fl::dec_attention_kernel<T, DP, W, true> : fl::dec_attention_kernel<T, DP, W, false>;
   return (int)cudaLaunchKernelEx(&cfg, kernel, (const T*)q, q_stride, pos, *kv, (T*)out, heads, dim, group, gparts, scale);
@@ -881,7 +901,7 @@ static int launch_attention_ring(const CUtensorMap& tm_k, const CUtensorMap& tm_
   at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
-  cfg.numAttrs = 2;
+  cfg.numAttrs = chained(batch) ? 2 : 1;
   const float scale = 1.4426950408889634f / sqrtf((float)DP);
   return (int)cudaLaunchKernelEx(&cfg, fl::dec_attention_ring_kernel<T, DP, W>, tm_k, tm_v, (const T*)q, q_stride, pos, *kv, (T*)out, heads, group,
                                  gparts, scale);
@@ -934,11 +954,30 @@ extern "C" int fl_dec_attention(int dtype, const void* q, long long q_stride, co
 extern "C" int fl_dec_argmax(int dtype, const void* logits, long long* out, int rows, long long vocab, cudaStream_t stream) {
   if (rows < 0 || vocab < 1) return -2;
   if (rows == 0) return 0;
-  FL_DEC_TYPES(dtype, return launch_chained(fl::dec_argmax_kernel<T>, rows, 1024, stream, (const T*)logits, out, vocab));
+  // eight CTAs for rows that have a vector for each of their threads, where all of them find room at once; more rows than a grid's
+  // second dimension takes go in several launches
+  const int parts = vocab >= 8ll * 8 * 512 && rows <= 148 / 4 ? 8 : 1;
+  for (int r = 0; r < rows; r += 65535) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(parts, rows - r < 65535 ? rows - r : 65535, 1);
+    cfg.blockDim = dim3(parts > 1 ? 512 : 1024, 1, 1);
+    cfg.stream = stream;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = parts; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = chained(rows) ? 2 : 1;
+    int rc = 0;
+    FL_DEC_TYPES(dtype, rc = (int)cudaLaunchKernelEx(&cfg, fl::dec_argmax_kernel<T>, (const T*)logits + (long long)r * vocab, out + r, vocab));
+    if (rc != 0) return rc;
+  }
+  return 0;
 }
 
 extern "C" int fl_dec_advance(const long long* next, long long* tokens, long long* pos, long long* history, long long* step, int batch,
                               int rows, cudaStream_t stream) {
   if (batch < 1) return -2;
-  return launch_chained(fl::dec_advance_kernel, 1, 256, stream, next, tokens, pos, history, step, batch, rows);
+  return launch_chained(fl::dec_advance_kernel, batch, 1, 256, stream, next, tokens, pos, history, step, batch, rows);
 }
