@@ -248,6 +248,8 @@ __device__ __forceinline__ void bulk_store(void* gdst, const void* smem_src, uin
                : "memory");
 }
 
+// ask the line at p into L2: a hint, which reads nothing, so it may come before a wait for whoever writes there
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 // bring [p, p + bytes) into L2 without occupying registers or shared memory (p 16-B aligned, bytes a multiple of 16)
 __device__ __forceinline__ void bulk_prefetch_l2(const void* p, uint32_t bytes) {
   asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");

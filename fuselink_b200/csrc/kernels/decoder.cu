@@ -131,9 +131,14 @@ __global__ void __launch_bounds__(1024) dec_add_norm_kernel(T* x, const T* y, co
                                                             float eps) {
   __shared__ float red[32];
   grid_dep_launch();
+  const int vecs = hidden >> 3;
+  if (gridDim.x <= FL_THIN_MAX_ROWS && threadIdx.x < vecs) {     // a step's parameters come from memory: on their way before the wait
+    prefetch_l2(w + threadIdx.x * 8);
+    if (b) prefetch_l2(b + threadIdx.x * 8);
+    if (y_bias) prefetch_l2(y_bias + threadIdx.x * 8);
+  }
   grid_dep_wait();
   const long long row = blockIdx.x;
-  const int vecs = hidden >> 3;
   T* xr = x + row * hidden;
   const T* yr = y ? y + row * hidden : nullptr;
   float v[VPT][8];
@@ -203,6 +208,10 @@ template <typename T>
 __global__ void __launch_bounds__(256) dec_qkv_kernel(T* qkv, const T* bias, const float* rope, long long rope_rows, const long long* pos,
                                                       long long rows, int seq, int heads, int dim, const FlPagedKv kv) {
   grid_dep_launch();
+  if (bias != nullptr && rows <= FL_THIN_MAX_ROWS) {
+    const int c = (blockIdx.x * blockDim.x + threadIdx.x) * 8;
+    if (c < (heads + 2 * kv.heads) * dim) prefetch_l2(bias + c);
+  }
   grid_dep_wait();
   const int total_heads = heads + 2 * kv.heads, chunks = dim / 16, half = dim / 2;
   const int per_row = total_heads * chunks;
@@ -440,17 +449,35 @@ __global__ void __launch_bounds__(W * 32, 16 / W) dec_attention_kernel(const T* 
   __shared__ AttParts<W> parts;
   __shared__ float s_o[W][ATT_G][DP + 4];
   grid_dep_launch();
-  grid_dep_wait();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
   const int kh = blockIdx.x / gparts, gp = blockIdx.x - kh * gparts, b = blockIdx.y, split = blockIdx.z, splits = gridDim.z;
   const int h0 = kh * group + gp * ATT_G, nh = min(ATT_G, group - gp * ATT_G);
   const int bs = kv.block_size;
   const long long cap = (long long)kv.table_stride * bs;
-  const int len = (int)min(max(pos[b] + 1, 0ll), cap);
   const int* table = kv.block_table + (long long)b * kv.table_stride;
   const long long tok_stride = (long long)kv.heads * dim;
+  if (gridDim.y <= FL_THIN_MAX_ROWS) {
+    // a look ahead, before the wait for the kernel that writes q and the new token's page: the keys and values of this warp's first
+    // steps (lanes 0 to 15 and 16 to 31) asked into L2; whatever it finds only says what is worth having there
+    const int units = (int)((min(max(__ldcg(pos + b) + 1, 0ll), cap) + 15) / 16), nw = splits * W, w = split * W + warp;
+    const int from = w * (units / nw) + min(w, units % nw), to = from + units / nw + (w < units % nw ? 1 : 0);
+    for (int u = from; u < min(to, from + 4); ++u) {
+      const int tok = u * 16 + (lane & 15), page = tok / bs;
+      if (page < kv.table_stride) {
+        int id = __ldcg(table + page);
+        if (id < 0) id += kv.num_blocks;
+        if (id >= 0 && id < kv.num_blocks) {
+          const T* r = reinterpret_cast<const T*>(lane < 16 ? kv.k : kv.v) + (((long long)kv.layer * kv.num_blocks + id) * bs + tok % bs) * tok_stride + kh * dim;
+          prefetch_l2(r);
+          if (dim > 64) prefetch_l2(r + dim - 8);
+        }
+      }
+    }
+  }
+  grid_dep_wait();
 
   // this warp's tokens: whole groups of 16, dealt out evenly over the warps of all splits
+  const int len = (int)min(max(pos[b] + 1, 0ll), cap);
   const int units = (len + 15) / 16, nw = splits * W, w = split * W + warp;
   const int per = units / nw, extra = units % nw;
   const int first = (w * per + min(w, extra)) * 16;

@@ -87,6 +87,7 @@ thin_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
   tc_fence_after_sync();
   if (splits > 1) cluster_arrive_all();                         // waited for before the first store into another CTA
   grid_dep_launch();
+  if (bias != nullptr && n0 + threadIdx.x < n) prefetch_l2(bias + n0 + threadIdx.x);
   const uint32_t tmem_base = tmem_base_s;
 
   if (warp == 0 && lane == 0) {
