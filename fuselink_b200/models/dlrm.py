@@ -128,16 +128,16 @@ def _gram(dy: torch.Tensor, r: torch.Tensor) -> torch.Tensor:
 
 class _Mlp(torch.autograd.Function):
     """Linear layers with a ReLU behind each (``relu_last``: behind the last one as well) as one node, params = weight, bias, weight,
-    bias, ...: the ReLU rides along with the product, its gradient and the bias gradient are one pass (csrc/kernels/mlp_bwd.cu).  The
-    rows x may be padded with zeros to an aligned width for the gradients' products: at 479 columns (26 tables) they miss the library's
+    bias, ..., of every layer: the ReLU rides along with the product, its gradient and the bias gradient are one pass (csrc/kernels/mlp_bwd.cu).  The
+    rows x may be ``padded`` with zeros to an aligned width for the gradients' products: at 479 columns (26 tables) they miss the library's
     aligned kernels.  The forward product stays at the width of the weight, whose bits decide which ReLUs pass a gradient."""
 
     @staticmethod
-    def forward(ctx, x, relu_last, *params):
+    def forward(ctx, x, relu_last, padded, *params):
         acts, n = [x], len(params) // 2
         for i in range(n):
             w, b = params[2 * i], params[2 * i + 1]
-            rows = acts[-1] if i else x[:, : w.shape[1]]
+            rows = x[:, : w.shape[1]] if padded and i == 0 else acts[-1]
             acts.append(torch._addmm_activation(b, rows, w.t()) if i < n - 1 or relu_last else torch.addmm(b, rows, w.t()))
         ctx.save_for_backward(*(acts if relu_last else acts[:-1]), *params)
         ctx.relu_last = relu_last
@@ -152,7 +152,7 @@ class _Mlp(torch.autograd.Function):
         grads = [None] * (2 * n)
         for i in range(n - 1, -1, -1):
             w, x = params[2 * i], acts[i]
-            want_x, want_w, want_b = i > 0 or ctx.needs_input_grad[0], ctx.needs_input_grad[2 + 2 * i], ctx.needs_input_grad[3 + 2 * i]
+            want_x, want_w, want_b = i > 0 or ctx.needs_input_grad[0], ctx.needs_input_grad[3 + 2 * i], ctx.needs_input_grad[4 + 2 * i]
             if i < n - 1 or ctx.relu_last:
                 dy, db = C.relu_bias_bwd(dy.contiguous(), acts[i + 1])
             else:
@@ -165,7 +165,11 @@ class _Mlp(torch.autograd.Function):
                     grads[2 * i] = dy.t() @ x
             if want_x:
                 dy = dy @ (w if x.shape[1] == w.shape[1] else F.pad(w, (0, x.shape[1] - w.shape[1])))
-        return dy if ctx.needs_input_grad[0] else None, None, *grads
+        return dy if ctx.needs_input_grad[0] else None, None, None, *grads
+
+    @staticmethod
+    def of(mlp, x, relu_last, padded):
+        return _Mlp.apply(x, relu_last, padded, *(p for m in list(mlp)[::2] for p in (m.weight, m.bias)))
 
 
 class _PaddedLinear(torch.autograd.Function):
@@ -298,7 +302,7 @@ class DLRM(nn.Module):
     def _dense_forward_fused(self, dense: torch.Tensor, pooled: torch.Tensor) -> torch.Tensor:
         """dense_forward with the gradient of ``pooled`` (over the ranks' mean) written to the buffer the tables' owners read."""
         plain = self._plain_mlps()
-        x = (_Mlp.apply(dense, True, *self.bottom.parameters()) if plain else self.bottom(dense)).contiguous()
+        x = (_Mlp.of(self.bottom, dense, True, False) if plain else self.bottom(dense)).contiguous()
         if x.data_ptr() % 16:                              # a hook may have put a view of something larger in its place
             x = x.clone()
         n = self.n_inter + self.cfg.dim
@@ -306,7 +310,7 @@ class DLRM(nn.Module):
         anchor = torch.empty(0, device=x.device, requires_grad=True)
         r = _Interaction.apply(x, pooled, self.gpooled.local, 1.0 / self.world, width, (self.iu0, self.iu1), anchor)
         if plain:
-            return _Mlp.apply(r, False, *self.top.parameters()).squeeze(-1)
+            return _Mlp.of(self.top, r, False, True).squeeze(-1)
         first = self.top[0]
         y = _PaddedLinear.apply(r, first.weight, first.bias)
         return self.top[1:](y).squeeze(-1)

@@ -63,3 +63,26 @@ def test_mlp_nodes_match_the_layers(tables, batch, tf32, monkeypatch):
             # each of the two is within batch roundings of the terms' magnitudes; 1 / batch bounds a sample's gradient of its logit, and
             # the layers' weights, below 1 / sqrt(width) each, do not let it grow
             assert (pa[i] - pb[i]).abs().max() <= 2 * batch * 2.0 ** -24
+
+
+def test_rows_of_another_width_are_refused():
+    """The width of the dense features is the first layer's: neither cut nor filled up."""
+    from fuselink_b200.models.dlrm import DLRM, DLRMConfig, synthetic_batch
+    from fuselink_b200.parallel.symm import SymmetricHeap
+    cfg = DLRMConfig(num_tables=2, rows=50, pooling=3, global_batch=8)
+    heap = SymmetricHeap.create(16 << 20, device=0)
+    try:
+        m = DLRM(cfg, heap, 0, 1, device="cuda", seed=3)
+        dense, idx, labels = synthetic_batch(cfg, 0, 1, "cuda", seed=4)
+        opt = torch.optim.SGD(m.dense_parameters(), lr=0.1)
+        for wrong in (torch.cat([dense, dense], 1), dense[:, :5].contiguous()):
+            with pytest.raises(RuntimeError):
+                m.train_step(wrong, idx, labels, opt)
+        m.bottom[4] = m.bottom[2] = torch.nn.Linear(256, 256, device="cuda")       # one layer in two places
+        m.bottom[0] = torch.nn.Linear(13, 256, device="cuda")
+        m.bottom.extend([torch.nn.Linear(256, 128, device="cuda"), torch.nn.ReLU()])
+        m.train_step(dense, idx, labels, torch.optim.SGD(m.dense_parameters(), lr=0.1))
+        torch.cuda.synchronize()
+        heap.check_status()
+    finally:
+        heap.close()
