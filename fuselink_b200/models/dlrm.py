@@ -128,9 +128,10 @@ def _gram(dy: torch.Tensor, r: torch.Tensor) -> torch.Tensor:
 
 class _Mlp(torch.autograd.Function):
     """Linear layers with a ReLU behind each (``relu_last``: behind the last one as well) as one node, params = weight, bias, weight,
-    bias, ..., of every layer: the ReLU rides along with the product, its gradient and the bias gradient are one pass (csrc/kernels/mlp_bwd.cu).  The
-    rows x may be ``padded`` with zeros to an aligned width for the gradients' products: at 479 columns (26 tables) they miss the library's
-    aligned kernels.  The forward product stays at the width of the weight, whose bits decide which ReLUs pass a gradient."""
+    bias, ..., of every layer: the ReLU's gradient and the bias gradient are one pass (csrc/kernels/mlp_bwd.cu).  The ReLU itself is a pass
+    of its own: as the library products' epilogue it turns NaN into 0 at some sizes.  The rows x may be ``padded`` with zeros to an aligned
+    width for the gradients' products: at 479 columns (26 tables) they miss the library's aligned kernels.  The forward product stays at
+    the width of the weight, whose bits decide which ReLUs pass a gradient."""
 
     @staticmethod
     def forward(ctx, x, relu_last, padded, *params):
@@ -138,7 +139,8 @@ class _Mlp(torch.autograd.Function):
         for i in range(n):
             w, b = params[2 * i], params[2 * i + 1]
             rows = x[:, : w.shape[1]] if padded and i == 0 else acts[-1]
-            acts.append(torch._addmm_activation(b, rows, w.t()) if i < n - 1 or relu_last else torch.addmm(b, rows, w.t()))
+            z = torch.addmm(b, rows, w.t())
+            acts.append(z.relu_() if i < n - 1 or relu_last else z)
         ctx.save_for_backward(*(acts if relu_last else acts[:-1]), *params)
         ctx.relu_last = relu_last
         return acts[-1]

@@ -86,3 +86,42 @@ def test_rows_of_another_width_are_refused():
         heap.check_status()
     finally:
         heap.close()
+
+
+@pytest.mark.parametrize("batch", [7, 2053, 65536])
+@pytest.mark.parametrize("where", ["feature", "weight", "top weight"])
+@pytest.mark.parametrize("tf32", [False, True])
+def test_nan_goes_through_as_through_the_layers(batch, where, tf32, monkeypatch):
+    """A NaN feature or weight makes the loss NaN and the gradients that the layers' own calls make NaN; the rest is the same bits."""
+    from fuselink_b200.models.dlrm import DLRM, DLRMConfig, synthetic_batch
+    from fuselink_b200.parallel.symm import SymmetricHeap
+    monkeypatch.setattr(torch.backends.cuda.matmul, "allow_tf32", tf32)
+    cfg = DLRMConfig(num_tables=3, rows=50, pooling=3, global_batch=batch)
+    res = []
+    for hooked in (False, True):
+        heap = SymmetricHeap.create(2 * batch * 3 * cfg.dim * 4 + (16 << 20), device=0)
+        try:
+            m = DLRM(cfg, heap, 0, 1, device="cuda", seed=3)
+            dense, idx, labels = synthetic_batch(cfg, 0, 1, "cuda", seed=4)
+            if hooked:
+                m.bottom[1].register_forward_hook(lambda *a: None)
+            assert m._plain_mlps() == (not hooked)
+            if where == "feature":
+                dense[batch // 2, 3] = float("nan")
+            else:
+                (m.bottom if where == "weight" else m.top)[0].weight.data[5, 2] = float("nan")
+            grads = {}
+            for i, p in enumerate(m.dense_parameters()):
+                p.register_post_accumulate_grad_hook(lambda p, i=i: grads.__setitem__(i, p.grad.clone()))
+            loss = m.train_step(dense, idx, labels, torch.optim.SGD(m.dense_parameters(), lr=0.0))
+            torch.cuda.synchronize()
+            res.append((loss, m.gpooled.local.clone(), grads))
+        finally:
+            heap.close()
+    (la, ga, pa), (lb, gb, pb) = res
+    assert la.isnan() and lb.isnan()
+    assert gb.isnan().any() and torch.equal(ga.isnan(), gb.isnan()) and torch.equal(ga.nan_to_num(), gb.nan_to_num())
+    for i in pa:
+        assert torch.equal(pa[i].isnan(), pb[i].isnan())
+        if pa[i].dim() == 2:
+            assert torch.equal(pa[i].nan_to_num(), pb[i].nan_to_num())
