@@ -113,9 +113,19 @@ __device__ __forceinline__ bool wait_flag_ge(const uint32_t* p, uint32_t want, i
 }
 
 // 16-byte vector access helpers (used for peer stores/loads: one transaction per 16 B)
+// nc: only for what nobody writes while the kernel runs.  A kernel that is launched to start early (grid_dep_wait) runs while the one
+// before it still writes, so it reads that one's output with ld_v4 or ld_stream_v4.
 __device__ __forceinline__ uint4 ld_nc_v4(const void* p) {
   uint4 v;
   asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
+               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+               : "l"(p));
+  return v;
+}
+// read once: takes no line of the L1 cache
+__device__ __forceinline__ uint4 ld_stream_v4(const void* p) {
+  uint4 v;
+  asm volatile("ld.global.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
                : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
                : "l"(p));
   return v;

@@ -286,12 +286,12 @@ __global__ void __launch_bounds__(256) dec_act_kernel(const T* h, const T* bias,
     if (KIND == FL_ACT_SILU_GATED) {
       float u[8];
       const T* p = h + n * 2 * ffn + c;
-      unpack8<T>(ld_nc_v4(p), a);
-      unpack8<T>(ld_nc_v4(p + ffn), u);
+      unpack8<T>(ld_stream_v4(p), a);
+      unpack8<T>(ld_stream_v4(p + ffn), u);
 #pragma unroll
       for (int j = 0; j < 8; ++j) a[j] = Num<T>::round(a[j] / (1.f + expf(-a[j]))) * u[j];
     } else {
-      unpack8<T>(ld_nc_v4(h + n * ffn + c), a);
+      unpack8<T>(ld_stream_v4(h + n * ffn + c), a);
       if (bias) {
         float e[8];
         load8<T>(bias + c, e);
@@ -506,7 +506,7 @@ __global__ void __launch_bounds__(W * 32, 16 / W) dec_attention_kernel(const T* 
       for (int j = 0; j < KJ; ++j) {
         const int d = 32 * j + 8 * t;
         kr[p][j] = make_uint4(0, 0, 0, 0);
-        if (r != nullptr && d < dim) kr[p][j] = ld_nc_v4(r + d);
+        if (r != nullptr && d < dim) kr[p][j] = ld_stream_v4(r + d);
       }
     }
   };
@@ -541,7 +541,7 @@ __global__ void __launch_bounds__(W * 32, 16 / W) dec_attention_kernel(const T* 
       for (int c = 0; c < VC; ++c) {
         const int d = 64 * c + 8 * g;
         vr[i][c] = make_uint4(0, 0, 0, 0);
-        if (r != nullptr && d < dim) vr[i][c] = ld_nc_v4(r + d);
+        if (r != nullptr && d < dim) vr[i][c] = ld_stream_v4(r + d);
       }
     }
     float s[2][2];
@@ -740,7 +740,7 @@ __global__ void __launch_bounds__(1024) dec_argmax_kernel(const T* logits, long 
   const long long vecs = wide ? vocab / 8 : 0, first = part * (long long)blockDim.x + threadIdx.x, step = parts * (long long)blockDim.x;
   for (long long i = first; i < vecs; i += step) {
     float v[8];
-    unpack8<T>(ld_nc_v4(row + i * 8), v);
+    unpack8<T>(ld_stream_v4(row + i * 8), v);
 #pragma unroll
     for (int j = 0; j < 8; ++j)
       if (better(v[j], i * 8 + j, best, at)) { best = v[j]; at = i * 8 + j; }
@@ -807,8 +807,8 @@ static bool aligned(std::initializer_list<const void*> pointers) {
   return (all & 15) == 0;
 }
 
-// Whether a kernel over so many rows may start while the one before it in the stream ends (it calls grid_dep_wait before it touches
-// memory): the launch itself, 2 to 3 us in a chain of kernels that take no longer, is then out of the way.  Only as far as the
+// Whether a kernel over so many rows may start while the one before it in the stream ends (before grid_dep_wait it touches nothing that
+// decides a result: the attention looks at positions and page ids, for what to ask into L2, and reads them again): the launch itself, 2 to 3 us in a chain of kernels that take no longer, is then out of the way.  Only as far as the
 // products are thin_gemm.cu's, which take part in it; between library products it costs (23 requests, 8B model: 15.1 ms without, 15.3
 // with).  dec_embed_kernel is launched without: it begins a chain, in which weights written by whatever came before are complete.
 static bool chained(long long rows) { return rows <= FL_THIN_MAX_ROWS; }

@@ -1,0 +1,47 @@
+"""Rules of the kernels that are launched to start while the one before them in the stream still runs, read off their source."""
+import os
+import re
+
+import pytest
+
+KERNELS = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "fuselink_b200", "csrc", "kernels")
+EARLY = ["decoder.cu", "thin_gemm.cu", "comm_kernels.cu"]
+
+
+def _functions(name):
+    """{function: body} of the __global__ and __device__ functions of a file, comments removed."""
+    text = re.sub(r"//[^\n]*", "", open(os.path.join(KERNELS, name)).read())
+    found = {}
+    for m in re.finditer(r"\b__(global|device)__\b", text):
+        start, semicolon = text.find("{", m.end()), text.find(";", m.end())
+        if start < 0 or 0 <= semicolon < start:
+            continue
+        head = re.sub(r"__launch_bounds__\s*\([^)]*\)", "", text[m.end():start])
+        depth, at = 1, start + 1
+        while depth:
+            depth += {"{": 1, "}": -1}.get(text[at], 0)
+            at += 1
+        found[re.search(r"(\w+)\s*\(", head).group(1)] = found.get(re.search(r"(\w+)\s*\(", head).group(1), "") + text[start:at]
+    return found
+
+
+def _reached(functions, kernel):
+    """The kernel's body and those of the functions of its file that it calls, through any number of calls."""
+    names, todo = set(), [kernel]
+    while todo:
+        n = todo.pop()
+        if n not in names:
+            names.add(n)
+            todo += [f for f in functions if re.search(rf"\b{f}\b", functions[n])]
+    return {n: functions[n] for n in names}
+
+
+@pytest.mark.parametrize("name", EARLY)
+def test_what_another_kernel_writes_is_not_read_as_read_only(name):
+    """ld.global.nc is defined only for memory that nobody writes while the kernel runs; the kernel before an early one does."""
+    functions = _functions(name)
+    early = [k for k, body in functions.items() if "grid_dep_wait()" in body]
+    assert early
+    for k in early:
+        for n, body in _reached(functions, k).items():
+            assert not re.search(r"ld_nc|\.nc\b|__ldg|__restrict__", body), f"{name}: {n}, reached from {k}"
