@@ -114,10 +114,7 @@ thin_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
     for (int b = first; b < ahead; ++b) load_x(b);
     for (int b = ahead; b < last; ++b) {
       const int i = b - first;
-      if (!mbar_wait(&empty[i % TG_STAGES], ((i / TG_STAGES) & 1) ^ 1, &abort_flag, nullptr, kTimeoutMbarEmpty, 0)) {
-        for (int j = 0; j < 2000; ++j) __nanosleep(1000);       // copies on the way land before shared memory goes away
-        break;
-      }
+      if (!mbar_wait(&empty[i % TG_STAGES], ((i / TG_STAGES) & 1) ^ 1, &abort_flag, nullptr, kTimeoutMbarEmpty, 0)) break;
       load_w(b);
       load_x(b);
     }
@@ -164,6 +161,10 @@ thin_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
   tc_fence_before_sync();
   if (splits > 1) cluster_sync_all();
   else __syncthreads();
+  // whoever gave up, the loader may have copies on the way: they land before this CTA's shared memory and TMEM go away
+  if (*reinterpret_cast<volatile int*>(&abort_flag)) {
+    for (int j = 0; j < 2000; ++j) __nanosleep(1000);
+  }
   if (warp == 1) {
     tc_fence_after_sync();
     tmem_dealloc(tmem_base, TG_TMEM_COLS);
