@@ -122,6 +122,7 @@ thin_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
     // ---- products
     constexpr uint32_t idesc = make_idesc(ThinNum<T>::kFmt, ThinNum<T>::kFmt, 0, 0, TG_M, TG_N);
     bool ok = true;
+    grid_dep_wait();                                            // x comes behind it: the limit of the waits counts from there
     for (int b = first; b < last && ok; ++b) {
       const int i = b - first, s = i % TG_STAGES;
       ok = mbar_wait(&full[s], (i / TG_STAGES) & 1, &abort_flag, nullptr, kTimeoutMbarFull, 0);

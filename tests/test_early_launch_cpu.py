@@ -54,3 +54,12 @@ def test_a_product_that_gave_up_waits_for_its_copies():
     behind = body[body.rindex("mbar_wait"):]                     # nobody gives up later than that
     barrier, look, free = (re.search(r, behind) for r in (r"else __syncthreads\(\);", r"if \([^{;]*abort_flag\)+ \{[^}]*__nanosleep", r"tmem_dealloc"))
     assert barrier and look and free and barrier.end() < look.start() < look.end() < free.start()
+
+
+def test_the_limit_of_a_wait_counts_from_the_end_of_the_kernel_before():
+    """Every bounded wait of an early kernel stands behind a grid_dep_wait of its role: the kernel before may poll a flag for longer."""
+    for name in ("decoder.cu", "thin_gemm.cu"):
+        for n, body in _functions(name).items():
+            roles = re.split(r"\belse if \(warp == 1", body)
+            for role in roles if "mbar_wait" in body else []:
+                assert re.search(r"grid_dep_wait\(\)", role[:role.index("mbar_wait")]), f"{name}: {n}"

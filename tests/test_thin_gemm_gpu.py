@@ -71,3 +71,19 @@ def test_arguments():
                 (x[:, :63].contiguous(), w[:, :63].contiguous(), None, 3), (x, w[:7], None, 0), (x.view(-1)[1:65].view(1, 64), w, None, 3)):
         with pytest.raises(RuntimeError):
             C.dec_product(*bad)
+
+
+def test_the_kernel_before_may_take_longer_than_a_wait():
+    """An early product waits as long as the kernel before it runs, here one that polls a flag for longer than the 2 s of a wait inside
+    a kernel; only then does its own limit count."""
+    from fuselink_b200 import C
+    x, w = _eighths(5, 512, dt=torch.bfloat16, seed=1), _eighths(300, 512, dt=torch.bfloat16, seed=2)
+    flag, timed_out = torch.zeros(1, dtype=torch.int32, device="cuda"), torch.zeros(8, dtype=torch.int32, device="cuda")
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    want = C.dec_product(x, w, None, 3)
+    torch.cuda.synchronize()
+    C.wait_flags([(flag.data_ptr(), 1)], timed_out.data_ptr(), 2600)          # a flag that nothing sets
+    got = C.dec_product(x, w, None, 3, True, status.data_ptr())
+    torch.cuda.synchronize()
+    assert timed_out[0] != 0 and status[0] == 0
+    assert torch.equal(got, want)
