@@ -197,6 +197,12 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
   return true;
 }
 
+// The same by all lanes of a warp, which go on together and with one answer: what follows a wait (shuffles, .aligned instructions,
+// barriers) wants all of them.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status, int code, int where) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, status, code, where));
+}
+
 // ---- programmatic dependent launch --------------------------------------------------------------------
 // wait: everything that the kernels before this one in the stream have written is there (they have ended).  launch: the next kernel,
 // if it was launched to start early, may be started once every CTA of this grid has come here or left.

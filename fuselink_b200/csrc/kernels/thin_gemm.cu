@@ -138,7 +138,7 @@ thin_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
   }
   __syncwarp();
   grid_dep_wait();                                              // y may still be read by kernels before this one
-  const bool have = mbar_wait(&done, 0, &abort_flag, nullptr, kTimeoutTmemFull, 0);
+  const bool have = mbar_wait_warp(&done, 0, &abort_flag, nullptr, kTimeoutTmemFull, 0);
   tc_fence_after_sync();
   if (!have && status != nullptr) *reinterpret_cast<volatile int*>(status) = FL_DEC_STALLED;
 

@@ -63,3 +63,17 @@ def test_the_limit_of_a_wait_counts_from_the_end_of_the_kernel_before():
             roles = re.split(r"\belse if \(warp == 1", body)
             for role in roles if "mbar_wait" in body else []:
                 assert re.search(r"grid_dep_wait\(\)", role[:role.index("mbar_wait")]), f"{name}: {n}"
+
+
+@pytest.mark.parametrize("kernel", ["thin_gemm_kernel"])
+def test_a_warp_goes_on_together_behind_a_wait(kernel):
+    """mbar_wait answers thread by thread; outside of the roles of a single lane it is mbar_wait_warp, since shuffles, cluster barriers
+    and .aligned instructions follow, also where the wait ran out."""
+    body = next(f[kernel] for f in map(_functions, EARLY) if kernel in f)
+    while m := re.search(r"if \([^{}]*lane == 0[^{}]*\) \{", body):
+        depth, at = 1, m.end()
+        while depth:
+            depth += {"{": 1, "}": -1}.get(body[at], 0)
+            at += 1
+        body = body[:m.start()] + body[at:]
+    assert "mbar_wait_warp(" in body and "mbar_wait(" not in body
