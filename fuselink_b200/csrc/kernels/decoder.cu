@@ -680,7 +680,7 @@ __global__ void __launch_bounds__(W * 32, 8 / W) dec_attention_ring_kernel(const
 
   for (int u = first; u < last; ++u) {
     const int s = (u - first) % ST;
-    if (!mbar_wait(&full[warp][s], ((u - first) / ST) & 1, &abort_flag, nullptr, kTimeoutMbarFull, 0)) {
+    if (!mbar_wait_warp(&full[warp][s], ((u - first) / ST) & 1, &abort_flag, nullptr, kTimeoutMbarFull, 0)) {
       note(kv.status, FL_DEC_STALLED);
       for (int j = 0; j < 2000; ++j) __nanosleep(1000);          // copies on the way land before shared memory goes away
       break;

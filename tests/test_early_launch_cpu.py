@@ -65,7 +65,7 @@ def test_the_limit_of_a_wait_counts_from_the_end_of_the_kernel_before():
                 assert re.search(r"grid_dep_wait\(\)", role[:role.index("mbar_wait")]), f"{name}: {n}"
 
 
-@pytest.mark.parametrize("kernel", ["thin_gemm_kernel"])
+@pytest.mark.parametrize("kernel", ["thin_gemm_kernel", "dec_attention_ring_kernel"])
 def test_a_warp_goes_on_together_behind_a_wait(kernel):
     """mbar_wait answers thread by thread; outside of the roles of a single lane it is mbar_wait_warp, since shuffles, cluster barriers
     and .aligned instructions follow, also where the wait ran out."""
