@@ -122,6 +122,8 @@ class LlamaShard(torch.nn.Module):
         self.cfg, self.tp_rank, self.tp_size, self.tp_group = cfg, tp_rank, tp_size, tp_group
         self.h_local, self.kvh_local, self.f_local = cfg.heads // tp_size, cfg.kv_heads // tp_size, cfg.ffn // tp_size
         self.gated = cfg.arch == "llama"                                        # SwiGLU: gate and up in one matrix
+        if torch.device(device).type == "cuda":
+            self._status = _Status()
         D, H = cfg.head_dim, cfg.hidden
         g = torch.Generator(device=device).manual_seed(seed * 31 + 7)           # replicated tensors: same on every shard
         gs = torch.Generator(device=device).manual_seed(seed * 31 + 100 + tp_rank)  # sharded tensors
@@ -266,7 +268,8 @@ class LlamaShard(torch.nn.Module):
         return table
 
     def _status_addr(self) -> int:
-        """Where the kernels note a bad index; 0 (nowhere) if the first call of all is one that is being captured."""
+        """Where the kernels note a bad index or a stall.  The constructor makes the word, since host memory cannot be had under capture;
+        0 (nowhere) only where a shard made elsewhere and moved here is captured in its first call of all."""
         st = self.__dict__.get("_status")
         if st is None:
             if torch.cuda.is_current_stream_capturing():

@@ -226,3 +226,22 @@ def test_attention_leaves_out_a_page_outside_the_pool(bs):
     want = torch.einsum("hn,nhd->hd", (torch.einsum("hd,nhd->hn", q, k) / math.sqrt(dim)).softmax(-1), v).reshape(-1)
     # the probabilities' rounding to the type and the result's
     assert (out[0].float() - want).abs().max() <= 2 * _eps(torch.bfloat16) * v.abs().max() + 1e-5
+
+
+def test_a_first_call_under_capture_notes_what_it_meets():
+    net, pools = _shard("tiny")
+    k, v = pools(2)
+    tok, at = torch.tensor([3], device="cuda"), torch.tensor([5], device="cuda")
+    bt = torch.tensor([[0, 1]], dtype=torch.int32, device="cuda")
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        net.decode_step(tok, at, k, v, bt, 2)
+    for t, bad in ((3, False), (1000, True), (4, False)):
+        tok.fill_(t)
+        g.replay()
+        torch.cuda.synchronize()
+        if bad:
+            with pytest.raises(IndexError, match="token"):
+                net.check_status()
+        else:
+            net.check_status()
