@@ -62,8 +62,8 @@ struct FlGemmDesc {
   // scheduling
   int group_m;      // rasterisation: m-tiles per super-column (default 16)
   int max_ctas;     // 0 => one CTA per SM
-  int expect_rows;  // rows that a group is expected to have, for the choice of tiles (0 => not known)
   int* status;      // device int32[8], zero on success
+  int expect_rows;  // rows that a group is expected to have, for the choice of tiles (0 => not known)
 };
 
 #ifdef __cplusplus
