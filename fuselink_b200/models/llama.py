@@ -323,7 +323,7 @@ class LlamaShard(torch.nn.Module):
             y = self._allreduce(product(attend(l, qkv), self.wo[l]))
             C.dec_add_norm(x, y, self.bo[l], self.n2[l], self.n2b[l], h, cfg.eps)
             if thin:
-                act = product(h, self.w13[l], self.b13[l], kind)
+                act = product(h, self.w13[l], None if self.gated else self.b13[l], kind)
             else:
                 C.dec_act(h @ self.w13[l].t(), self.b13[l], act, kind)
             y, bias = self._allreduce(product(act, self.w2[l])), self.b2[l]

@@ -245,3 +245,19 @@ def test_a_first_call_under_capture_notes_what_it_meets():
                 net.check_status()
         else:
             net.check_status()
+
+
+@pytest.mark.parametrize("batch", [1, 16, 17])
+def test_a_gated_layer_knows_no_bias(batch):
+    """A llama shard's b13 is looked at by no route: neither refused nor added."""
+    net, pools = _shard("tiny")
+    bt = torch.arange(2 * batch, dtype=torch.int32, device="cuda").view(batch, 2)
+    tok, at = torch.arange(batch, device="cuda"), torch.full((batch,), 5, device="cuda")
+    res = []
+    for bias in (None, torch.ones(net.f_local, dtype=torch.bfloat16, device="cuda")):
+        net.b13 = [bias] * net.cfg.layers
+        k, v = pools(2 * batch)
+        assert net._fused(k)
+        res.append((net.decode_step(tok, at, k, v, bt, 2 * batch), k, v))
+    for a, b in zip(*res):
+        assert torch.equal(a, b)
