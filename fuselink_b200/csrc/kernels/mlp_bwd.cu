@@ -11,6 +11,7 @@
 namespace fl {
 
 constexpr int RB_WARPS = 8, RB_ROWS = 4;
+constexpr int RB_MAX_COLS = 0x7fffffff - 127;      // the columns of the last CTA still count in 32 bits
 
 template <int VEC> struct RbVec;
 template <> struct RbVec<4> { using type = float4; };
@@ -83,7 +84,7 @@ __global__ void __launch_bounds__(256) sum_parts_kernel(const float* part, float
 
 // about four CTAs per SM over all column blocks, but no CTA without a few rows for each of its warps
 extern "C" int fl_relu_bias_parts(long long rows, int cols) {
-  if (rows < 1 || cols < 1) return 0;
+  if (rows < 1 || cols < 1 || cols > fl::RB_MAX_COLS) return 0;
   const long long blocks = (cols + 127) / 128, most = (rows + fl::RB_WARPS * fl::RB_ROWS - 1) / (fl::RB_WARPS * fl::RB_ROWS);
   long long n = (4 * 148 + blocks - 1) / blocks;
   if (n > most) n = most;
@@ -91,7 +92,7 @@ extern "C" int fl_relu_bias_parts(long long rows, int cols) {
 }
 
 extern "C" int fl_relu_bias_bwd(const float* dy, const float* y, float* dz, float* part, float* db, long long rows, int cols, cudaStream_t stream) {
-  if (rows < 1 || cols < 1) return -1;
+  if (rows < 1 || cols < 1 || cols > fl::RB_MAX_COLS) return -1;
   const int parts = fl_relu_bias_parts(rows, cols);
   const uintptr_t at = (uintptr_t)dy | (uintptr_t)y | (uintptr_t)dz;
   if (cols % 4 == 0 && (at & 15) == 0)

@@ -1,4 +1,5 @@
 """The C interface (include/fuselink.h) for programs built against an earlier header."""
+import ctypes
 import os
 import shutil
 import subprocess
@@ -27,3 +28,13 @@ int main() {
     assert b.returncode == 0, b.stderr[-3000:]
     end_of_max_ctas, status, expect_rows = map(int, subprocess.run([exe], capture_output=True, text=True, timeout=60).stdout.split())
     assert status == (end_of_max_ctas + 7) // 8 * 8 and expect_rows == status + 8
+
+
+@pytest.mark.parametrize("rows,cols", [(0, 4), (1, 0), (1, 2 ** 31 - 127), (1, 2 ** 31 - 1)])
+def test_the_relu_gradient_refuses_widths_that_32_bits_do_not_count(rows, cols):
+    lib = os.path.join(ROOT, "fuselink_b200", "lib", "libfuselink.so")
+    if not os.path.exists(lib):
+        pytest.skip("libfuselink.so not built")
+    f = ctypes.CDLL(lib).fl_relu_bias_bwd
+    f.argtypes = [ctypes.c_void_p] * 5 + [ctypes.c_longlong, ctypes.c_int, ctypes.c_void_p]
+    assert f(None, None, None, None, None, rows, cols, None) == -1
