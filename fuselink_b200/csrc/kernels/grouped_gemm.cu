@@ -1056,24 +1056,41 @@ static double expected_tiles(double rows, int TM) {
   return t;
 }
 
-// The variant for groups of `expect_rows` rows, `dflt` being the one for thousands.  Few rows per group change what pays, all
-// measured in us on 8 groups of 28672 x 4096 and 4096 x 14336 or 16 of 11264 x 2048 and 2048 x 5632 (0 | 1 | 2):
+// CTA pairs that a launch runs on, of `fit` that the GPU holds at once.
+static int pairs_in_use(const FlGemmDesc* d, int fit) {
+  if (d->max_ctas > 0 && d->max_ctas / 2 < fit) return d->max_ctas / 2 > 0 ? d->max_ctas / 2 : 1;
+  return fit;
+}
+
+// The variant for groups of `expect_rows` rows on `pairs` CTA pairs, `dflt` being the one for thousands.  Few rows per group change what
+// pays, all measured in us on 8 groups of 28672 x 4096 and 4096 x 14336 or 16 of 11264 x 2048 and 2048 x 5632 (0 | 1 | 2):
 //   weight gradients: the contraction is those rows, and a tile is all epilogue: 0 below 448 (250 rows: 704 | 758, 191: 264 | 307;
-//     448: 554 | 541);
+//     448: 554 | 541).  A skewed router moves the line up, not down: where 440 rows is the mean and the fullest expert has 1235, the two
+//     gradients of a layer take 1603 | 1636, at a mean of 520 1770 | 1803;
 //   SWIGLU and DSWIGLU: the wide tiles' single accumulator does not hide such short tiles (448 rows: 321 | 296 | 331; 1000: 1506 |
 //     1491 | 1515); 0 where tiles of 128 rows pad a tenth less than those of 256 (250: 520 | 538 | 553, 125: 358 | 380 | 395);
 //   the others: wide tiles are a tenth cheaper per column, unless their number leaves more pairs idle in the last round (250 rows of
-//     4096 x 14336, 86 tiles on 74 pairs: 289 (1) | 326 (2); 500: 395 | 354; 191 of 2048 x 5632: 90 | 88).
-static int variant_for_rows(const FlGemmDesc* d, int dflt) {
+//     4096 x 14336, 86 tiles on 74 pairs: 289 (1) | 336 (2), on 48 pairs: 343 | 311; 500 on 74: 398 | 365).  The rounds are counted of 2 %
+//     fewer tiles: an average is a little above the number of tiles that the groups mostly take (700 rows: 3.01).
+static int variant_for_rows(const FlGemmDesc* d, int dflt, int pairs) {
   const double rows = d->expect_rows;
   if (d->group_mode == 1) return rows < 448 ? 0 : dflt;
   if (d->N < 512 || rows >= 1024) return dflt;
   const double t256 = expected_tiles(rows, 256);
   if (d->epilogue == FL_EPI_SWIGLU || d->epilogue == FL_EPI_DSWIGLU)
     return 1.1 * 128 * expected_tiles(rows, 128) < 256 * t256 ? 0 : 1;
-  constexpr double kPairs = 74.;
-  const double wide = d->num_groups * t256 * ((d->N + 511) / 512), pair = d->num_groups * t256 * ((d->N + 255) / 256);
-  return 1.8 * ceil(wide / kPairs) < ceil(pair / kPairs) ? 2 : 1;
+  const double share = 0.98 * d->num_groups * t256 / pairs;
+  return 1.8 * ceil(share * ((d->N + 511) / 512)) < ceil(share * ((d->N + 255) / 256)) ? 2 : 1;
+}
+
+extern "C" int fl_gemm_choose(const FlGemmDesc* d, int pairs) {
+  int variant = fl_gemm_get_variant();
+  if (variant == 3) {
+    const bool short_k_long_epilogue = d->group_mode == 0 && d->epilogue == FL_EPI_DSWIGLU && d->K < 8192;
+    variant = (d->N < 512 || short_k_long_epilogue || d->group_mode == 1) ? 1 : 2;
+    if (d->expect_rows > 0) variant = variant_for_rows(d, variant, pairs_in_use(d, pairs));
+  }
+  return variant;
 }
 
 extern "C" int fl_grouped_gemm(const FlGemmDesc* d, cudaStream_t stream) {
@@ -1123,34 +1140,16 @@ extern "C" int fl_grouped_gemm(const FlGemmDesc* d, cudaStream_t stream) {
     p.stagger_ns = forced >= 0 ? forced : (heavy && d->group_mode == 0 ? (d->K / 64) * 650 : 0);
   }
 
-  int variant = fl_gemm_get_variant();
-  if (variant == 3) {
-    const bool short_k_long_epilogue = d->group_mode == 0 && d->epilogue == FL_EPI_DSWIGLU && d->K < 8192;
-    variant = (d->N < 512 || short_k_long_epilogue || d->group_mode == 1) ? 1 : 2;
-    if (d->expect_rows > 0) variant = variant_for_rows(d, variant);
-  }
-  const bool pair = variant >= 1;
-  CUtensorMap tmA, tmB;
-  int rc;
   if (d->group_mode == 0) {
     if (d->a_mn_major) return bad("M-grouped GEMM takes a K-major A (token rows)");
     if (d->K % 8) return bad("K must be a multiple of 8");
     if (d->epilogue == FL_EPI_WGRAD) return bad("WGRAD epilogue needs group_mode 1");
     if ((d->epilogue == FL_EPI_SWIGLU) && (d->N % 256)) return bad("SWIGLU needs N % 256 == 0");
     if ((d->epilogue == FL_EPI_DSWIGLU) && (d->N % 128)) return bad("DSWIGLU needs N % 128 == 0");
-    rc = make_map(&tmA, d->A, d->K, d->cap, d->num_groups, d->lda, d->gsa, 64, BM);
-    if (rc) return rc;
-    if (!d->b_mn_major) rc = make_map(&tmB, d->B, d->K, d->N, d->num_groups, d->ldb, d->gsb, 64, pair ? 128 : BN);
-    else rc = make_map(&tmB, d->B, d->N, d->K, d->num_groups, d->ldb, d->gsb, 64, 64);
-    if (rc) return rc;
   } else {
     if (!d->a_mn_major || !d->b_mn_major) return bad("K-grouped GEMM takes MN-major A and B (token-major buffers)");
     if (d->epilogue != FL_EPI_WGRAD) return bad("K-grouped GEMM supports the WGRAD epilogue only");
     if (d->M % 8) return bad("M must be a multiple of 8");
-    rc = make_map(&tmA, d->A, d->M, d->cap, d->num_groups, d->lda, d->gsa, 64, 64);
-    if (rc) return rc;
-    rc = make_map(&tmB, d->B, d->N, d->cap, d->num_groups, d->ldb, d->gsb, 64, 64);
-    if (rc) return rc;
   }
 
   // per device: a process may drive several GPUs, and the shared-memory attribute belongs to the device's copy of the kernel
@@ -1190,9 +1189,25 @@ extern "C" int fl_grouped_gemm(const FlGemmDesc* d, cudaStream_t stream) {
     cudaGetLastError();
     attr_set = true;
   }
+  const int variant = fl_gemm_choose(d, max_pairs);
+  const bool pair = variant >= 1;
+  CUtensorMap tmA, tmB;
+  int rc;
+  if (d->group_mode == 0) {
+    rc = make_map(&tmA, d->A, d->K, d->cap, d->num_groups, d->lda, d->gsa, 64, BM);
+    if (rc) return rc;
+    if (!d->b_mn_major) rc = make_map(&tmB, d->B, d->K, d->N, d->num_groups, d->ldb, d->gsb, 64, pair ? 128 : BN);
+    else rc = make_map(&tmB, d->B, d->N, d->K, d->num_groups, d->ldb, d->gsb, 64, 64);
+    if (rc) return rc;
+  } else {
+    rc = make_map(&tmA, d->A, d->M, d->cap, d->num_groups, d->lda, d->gsa, 64, 64);
+    if (rc) return rc;
+    rc = make_map(&tmB, d->B, d->N, d->cap, d->num_groups, d->ldb, d->gsb, 64, 64);
+    if (rc) return rc;
+  }
+
   if (pair) {
-    int pairs = max_pairs;
-    if (d->max_ctas > 0 && d->max_ctas / 2 < pairs) pairs = d->max_ctas / 2 > 0 ? d->max_ctas / 2 : 1;
+    const int pairs = pairs_in_use(d, max_pairs);
     if (variant == 2) grouped_gemm_wide_kernel<<<2 * pairs, NUM_THREADS, SMEM3_BYTES, stream>>>(tmA, tmB, p);
     else grouped_gemm_pair_kernel<<<2 * pairs, NUM_THREADS, SMEM2_BYTES, stream>>>(tmA, tmB, p);
     return (int)cudaGetLastError();

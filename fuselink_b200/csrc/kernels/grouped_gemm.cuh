@@ -77,6 +77,8 @@ const char* fl_gemm_last_error(void);
 // Default: FUSELINK_GEMM_PAIR or 3.
 void fl_gemm_set_variant(int pair);
 int fl_gemm_get_variant(void);
+// the variant (0 to 2) that fl_grouped_gemm takes for a description on a GPU that holds `pairs` CTA pairs at once
+int fl_gemm_choose(const FlGemmDesc* desc, int pairs);
 #ifdef __cplusplus
 }
 #endif

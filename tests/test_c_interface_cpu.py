@@ -9,25 +9,49 @@ import pytest
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 
+def _run(tmp_path, source, link=False):
+    """The output of a C++ program against include/fuselink.h (and lib/libfuselink.so)."""
+    cxx = next((c for c in (os.environ.get("CXX"), "g++", "/usr/bin/g++") if c and shutil.which(c)), None)
+    lib = os.path.join(ROOT, "fuselink_b200", "lib")
+    if cxx is None or (link and not os.path.exists(os.path.join(lib, "libfuselink.so"))):
+        pytest.skip("no C++ compiler or library")
+    src, exe = tmp_path / "program.cc", str(tmp_path / "program")
+    src.write_text('#include "fuselink.h"\n#include <stddef.h>\n#include <stdio.h>\n#include <string.h>\n' + source)
+    cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+    b = subprocess.run([cxx, "-std=c++17", "-I", os.path.join(ROOT, "fuselink_b200", "include"), "-I", os.path.join(cuda, "include"), str(src), "-o", exe,
+                        *(["-L", lib, "-lfuselink", f"-Wl,-rpath,{lib}"] if link else [])], capture_output=True, text=True, timeout=300)
+    assert b.returncode == 0, b.stderr[-3000:]
+    r = subprocess.run([exe], capture_output=True, text=True, timeout=60, env={k: v for k, v in os.environ.items() if k != "FUSELINK_GEMM_PAIR"})
+    assert r.returncode == 0, r.stderr
+    return [int(v) for v in r.stdout.split()]
+
+
 def test_a_product_description_keeps_the_places_of_its_fields(tmp_path):
     """Fields are added at the end: a program built before expect_rows passes its status pointer where the library reads it."""
-    cxx = next((c for c in (os.environ.get("CXX"), "g++", "/usr/bin/g++") if c and shutil.which(c)), None)
-    if cxx is None:
-        pytest.skip("no C++ compiler")
-    src, exe = tmp_path / "fields.cc", str(tmp_path / "fields")
-    src.write_text("""#include "fuselink.h"
-#include <stddef.h>
-#include <stdio.h>
-int main() {
+    end_of_max_ctas, status, expect_rows = _run(tmp_path, """int main() {
   printf("%zu %zu %zu", offsetof(FlGemmDesc, max_ctas) + sizeof(int), offsetof(FlGemmDesc, status), offsetof(FlGemmDesc, expect_rows));
 }
 """)
-    cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
-    b = subprocess.run([cxx, "-std=c++17", "-I", os.path.join(ROOT, "fuselink_b200", "include"), "-I", os.path.join(cuda, "include"), str(src), "-o", exe],
-                       capture_output=True, text=True, timeout=300)
-    assert b.returncode == 0, b.stderr[-3000:]
-    end_of_max_ctas, status, expect_rows = map(int, subprocess.run([exe], capture_output=True, text=True, timeout=60).stdout.split())
     assert status == (end_of_max_ctas + 7) // 8 * 8 and expect_rows == status + 8
+
+
+# 8 groups of N columns on a GPU that holds 74 pairs: what the faster tiles were (us, pairs of 256 x 256 | of 256 x 512)
+@pytest.mark.parametrize("N,K,rows,ctas,variant", [
+    (4096, 14336, 250, 0, 1), (4096, 14336, 500, 0, 2), (2048, 5632, 191, 0, 1), (2048, 5632, 700, 0, 1),       # 289|336 398|365 65|99 146|175
+    (4096, 14336, 250, 128, 1), (4096, 14336, 500, 128, 1), (2048, 5632, 500, 128, 1), (2048, 5632, 700, 128, 1),   # 283|330 493|526 129|157 131|160
+    (4096, 14336, 250, 96, 2), (4096, 14336, 191, 96, 1), (2048, 5632, 700, 96, 2),                            # 343|311 289|337 176|169
+    (2048, 5632, 250, 64, 1), (4096, 14336, 700, 64, 2), (4096, 14336, 250, 32, 2), (2048, 5632, 700, 32, 2),  # 115|139 936|834 774|686 383|357
+    (4096, 14336, 0, 32, 2), (4096, 14336, 1024, 32, 2), (256, 14336, 250, 0, 1), (4096, 14336, 250, 1, 2), (4096, 14336, 250, 1000, 1),
+])
+def test_tiles_by_expected_rows_on_the_pairs_that_a_launch_may_use(N, K, rows, ctas, variant, tmp_path):
+    got, = _run(tmp_path, f"""int main() {{
+  FlGemmDesc d;
+  memset(&d, 0, sizeof d);
+  d.num_groups = 8; d.N = {N}; d.K = {K}; d.epilogue = FL_EPI_SCATTER; d.max_ctas = {ctas}; d.expect_rows = {rows};
+  printf("%d", fl_gemm_choose(&d, 74));
+}}
+""", link=True)
+    assert got == variant
 
 
 @pytest.mark.parametrize("rows,cols", [(0, 4), (1, 0), (1, 2 ** 31 - 127), (1, 2 ** 31 - 1)])
