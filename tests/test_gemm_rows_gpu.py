@@ -1,0 +1,113 @@
+"""Tiles chosen by the rows that a group is expected to have (FlGemmDesc::expect_rows): the choice changes no result, whatever the rows
+that the groups then have."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+G, CAP = 3, 1280
+EXPECT = [0, 1, 125, 250, 447, 448, 1023, 1024, 2 ** 31 - 1]       # both sides of every line of the rule
+
+
+@pytest.fixture(autouse=True)
+def _automatic():
+    from fuselink_b200 import C
+    before = C.gemm_get_variant()
+    yield
+    C.gemm_set_variant(before)
+
+
+def _mk(*shape, scale=1.0, seed=0):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    return (torch.randn(*shape, generator=g, device="cuda") * scale).to(torch.bfloat16)
+
+
+def _outcomes(launch):
+    """launch(expect_rows) under every expectation and under each of the three variants by itself."""
+    from fuselink_b200 import C
+    C.gemm_set_variant(3)
+    res = {("rows", e): launch(e) for e in EXPECT}
+    for v in (0, 1, 2):
+        C.gemm_set_variant(v)
+        res["variant", v] = launch(250)
+    return res
+
+
+def _same(launch):
+    """...are the same bits; returns them."""
+    res = _outcomes(launch)
+    first = res["rows", 0]
+    for how, outs in res.items():
+        for a, b in zip(first, outs):
+            assert torch.equal(a, b), how
+    return first
+
+
+def _close(got, want, tol=2e-2):
+    assert (got.float() - want).abs().max() <= tol * want.abs().max()
+
+
+# the fullest and the emptiest that a group may be, edges of the tiles of 128 and 256 rows
+@pytest.mark.parametrize("counts_l", [[1280, 0, 1], [128, 129, 256], [257, 1000, 447]])
+@pytest.mark.parametrize("max_ctas", [0, 10])
+def test_no_result_depends_on_the_expected_rows(counts_l, max_ctas):
+    from fuselink_b200.ops import gemm
+    H, F = 256, 768                                                 # N: 256 (one tile of any kind), 768, 1536
+    counts = torch.tensor(counts_l, dtype=torch.int32, device="cuda")
+    st = torch.zeros(8, dtype=torch.int32, device="cuda")
+    x, w13, w2 = _mk(G * CAP, H, seed=1), _mk(G, 2 * F, H, scale=0.1, seed=2), _mk(G, H, F, scale=0.1, seed=3)
+    act, dy = _mk(G * CAP, F, seed=4), _mk(G * CAP, H, seed=5)
+    for g, c in enumerate(counts_l):                                # a contraction over rows takes whole tiles of them
+        for t in (x, act, dy):
+            t[g * CAP + c:(g + 1) * CAP] = 0
+    fill = lambda *s: torch.full(s, 7.0, dtype=torch.bfloat16, device="cuda")
+    kw = dict(status=st, max_ctas=max_ctas)
+    rows = [slice(g * CAP, g * CAP + c) for g, c in enumerate(counts_l)]
+
+    def swiglu(e):
+        out, gu = fill(G * CAP, F), fill(G * CAP, 2 * F)
+        gemm.grouped_gemm_rows(x, w13, counts, CAP, epilogue=gemm.EPI_SWIGLU, out=out, gu=gu, zero_tail=True, expect_rows=e, **kw)
+        return out, gu
+    out, gu = _same(swiglu)
+    for g, r in enumerate(rows):
+        gate, up = gemm.deinterleave_gate_up(w13[g:g + 1])
+        if counts_l[g]:
+            z = x[r].float()
+            _close(out[r], torch.nn.functional.silu(z @ gate[0].float().t()) * (z @ up[0].float().t()))
+
+    def dswiglu(e):
+        dgu = fill(G * CAP, 2 * F)
+        gemm.grouped_gemm_rows(dy, w2, counts, CAP, b_mn_major=True, epilogue=gemm.EPI_DSWIGLU, gu=gu, dgu=dgu, zero_tail=True, expect_rows=e, **kw)
+        return dgu,
+    _same(dswiglu)
+
+    perm = torch.randperm(G * CAP, generator=torch.Generator().manual_seed(6)).int().cuda()
+
+    def scatter(a, w, n, mn):
+        def launch(e):
+            buf = fill(G * CAP, n)
+            gemm.grouped_gemm_rows(a, w, counts, CAP, b_mn_major=mn, epilogue=gemm.EPI_SCATTER, row_info=perm, peers=[buf.data_ptr()], ldc=n,
+                                   peer_rows=G * CAP, expect_rows=e, **kw)
+            return buf,
+        return launch
+    buf, = _same(scatter(act, w2, H, False))                        # narrower than a wide tile
+    for g, r in enumerate(rows):
+        if counts_l[g]:
+            _close(buf[perm[r].long()], act[r].float() @ w2[g].float().t())
+    _same(scatter(gu, _mk(G, 2 * F, 1024, scale=0.1, seed=7), 1024, True))
+
+    def store(e):
+        c = fill(G * CAP, 2 * F)
+        gemm.grouped_gemm_rows(x, w13, counts, CAP, out=c, zero_tail=True, expect_rows=e, **kw)
+        return c,
+    _same(store)
+
+    def wgrad(e):
+        w = _mk(G, F, H, seed=8)
+        gemm.grouped_gemm_wgrad(act, x, counts, CAP, G, out=w, sgd_lr=0.5, expect_rows=e, **kw)
+        return gemm.grouped_gemm_wgrad(act, x, counts, CAP, G, expect_rows=e, **kw), w
+    dw, _ = _same(wgrad)
+    for g, r in enumerate(rows):
+        if counts_l[g]:
+            _close(dw[g], act[r].float().t() @ x[r].float())
+    assert st[0] == 0
