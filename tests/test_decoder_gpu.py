@@ -135,6 +135,26 @@ def test_argmax(rows, vocab):
     assert torch.equal(got, first)
 
 
+@pytest.mark.parametrize("rows,vocab", [(3, 32767), (3, 32768), (37, 32775), (38, 32775), (2, 128256)])
+@pytest.mark.parametrize("dt", DT)
+def test_argmax_over_the_ctas_of_a_row(rows, vocab, dt):
+    """The line to a cluster per row (32768 entries, 37 rows) and what its CTAs compare: equal values, NaN, nothing but -inf."""
+    from fuselink_b200 import C
+    x = torch.zeros(rows, vocab, dtype=dt, device="cuda")
+    for at in (vocab - 1, vocab // 2, 4097, 4096):
+        x[0, at] = 1
+        assert C.dec_argmax(x)[0] == at
+    x[1, vocab - 2], x[1, 7], x[1, vocab - 9] = float("inf"), float("inf"), float("nan")
+    assert C.dec_argmax(x)[1] == vocab - 9                  # NaN is the largest, as in torch.argmax
+    x[1, vocab // 3] = float("nan")
+    x[-1] = float("-inf")
+    want = torch.zeros(rows, dtype=torch.int64, device="cuda")
+    want[0], want[1] = 4096, vocab // 3
+    if rows == 2:
+        want[1] = 0
+    assert torch.equal(C.dec_argmax(x), want)
+
+
 @pytest.mark.parametrize("kind,ffn", [(0, 512), (1, 24), (2, 3072)])
 def test_activation(kind, ffn):
     from fuselink_b200 import C
@@ -261,3 +281,164 @@ def test_a_gated_layer_knows_no_bias(batch):
         res.append((net.decode_step(tok, at, k, v, bt, 2 * batch), k, v))
     for a, b in zip(*res):
         assert torch.equal(a, b)
+
+
+def _ring(batch, heads, kv_heads, dim, bs, maxblk):
+    """(CTAs per context, warps per CTA) of the attention through the ring, None where the pages go through registers: the rule of
+    fl_dec_attention, so that the cases below reach what they are for."""
+    units, cap = batch * kv_heads * -(-(heads // kv_heads) // 8), maxblk * bs
+    if dim not in (64, 128) or bs % 16 or units * (cap // 16) < 3 * 8 * 148:
+        return None
+    splits = max(1, min(2 * 148 // units, -(-cap // 128), 8))
+    return splits, 8 if units * splits <= 148 and cap >= splits * 8 * 32 else 4
+
+
+def _check(out, q, k, v, dt):
+    """out against the attention of q [heads, dim] over k, v [n, kv_heads, dim], both in fp32 from here on.  Scores are summed up product
+    by product: in a library's matrix product an infinite key may become NaN by inf - inf."""
+    (n, kv_heads, dim), heads = k.shape, q.shape[0]
+    q, k, v = q.float().view(kv_heads, heads // kv_heads, dim), k.float(), v.float()
+    s = torch.stack([(q[:, i].unsqueeze(0) * k).sum(-1).t() for i in range(q.shape[1])], 1)            # [kv_heads, group, n]
+    p = (s / math.sqrt(dim)).softmax(-1)
+    want, size = (torch.einsum("kgn,nkd->kgd", p, t).reshape(-1) for t in (v, v.abs()))
+    got, fine = out.float(), ~want.isnan()
+    assert torch.equal(got.isnan(), want.isnan())
+    # The probabilities are rounded to the type before the second product, and so is the result; 1e-4: scores up to about 30 summed in
+    # fp32 in another order, and the exponentials; in fp16 a probability below 2^-14 loses up to half a step of 2^-24.
+    bound = (1.01 * _eps(dt) + 1e-4) * size + _eps(dt) * want.abs() + (n * 2.0 ** -25 * v.abs().mean() if dt == torch.float16 else 0) + 1e-6
+    assert ((got - want).abs() <= bound)[fine].all(), ((got - want).abs() / bound)[fine].max()
+    return want
+
+
+def _of(pool, pages, n, bad=()):
+    """The first n tokens of `pages` of a pool [blocks, bs, kv_heads, dim], without those of the pages in `bad`."""
+    keep = torch.arange(n, device="cuda")
+    for p in bad:
+        keep = keep[keep // pool.shape[1] != p]
+    return pool[pages.long() % pool.shape[0]].flatten(0, 1)[keep]
+
+
+def _queries(batch, heads, kv_heads, dim, dt):
+    """(qkv, keys [batch, kv_heads, dim]): queries of three times the usual size, so that a head looks at a few tokens and not at the mean
+    of all; and for each KV head a key that its queries give about the weight of the best of some thousand others."""
+    qkv = _rand(batch, (heads + 2 * kv_heads) * dim, dt=dt, seed=4)
+    q = qkv[:, : heads * dim].view(batch, kv_heads, heads // kv_heads, dim)
+    key = (0.33 * q.float().sum(2)).to(dt)
+    q *= 3
+    return qkv, key
+
+
+RING = [  # batch, heads, kv_heads, dim, bs, lens (the first one fills the table), what the rule says
+    (16, 32, 8, 128, 16, [2064 - 67 * i for i in range(16)], (2, 4)),           # the context cut over two CTAs, an early launch
+    (17, 8, 8, 128, 16, [512, 1, 15, 16, 17, 33] + [300 + i for i in range(11)], (2, 4)),      # no early launch
+    (40, 16, 8, 128, 16, [400 - 3 * i for i in range(40)], (1, 4)),
+    (1, 32, 8, 128, 16, [7312], (8, 8)), (1, 8, 8, 128, 32, [7297], (8, 8)),
+    (16, 24, 2, 128, 48, [960 - 50 * i for i in range(16)], (4, 4)),            # twelve heads per KV head: two parts; three steps per page
+    (4, 32, 32, 64, 16, [1008, 17, 500, 999], (2, 4)), (2, 16, 8, 64, 64, [3648, 3], (8, 8)), (30, 8, 8, 64, 16, [256] * 30, (1, 4)),
+    (1, 4, 1, 64, 16, [57000], (8, 8)), (1, 2, 1, 128, 16, [56900], (8, 8)),    # more than 32 steps per warp: its page ids a second time
+    (16, 32, 8, 128, 16, [448 - 13 * i for i in range(16)], (2, 4)), (16, 32, 8, 128, 16, [432 - 13 * i for i in range(16)], None),      # the line
+]
+
+
+@pytest.mark.parametrize("dt", DT)
+@pytest.mark.parametrize("batch,heads,kv_heads,dim,bs,lens,how", RING)
+def test_attention_through_the_ring(dt, batch, heads, kv_heads, dim, bs, lens, how):
+    """Against the same in fp32.  What the pages hold behind a context may be anything: here NaN."""
+    from fuselink_b200 import C
+    L, layer, maxblk = 2, 1, -(-lens[0] // bs)
+    nb = batch * maxblk
+    assert _ring(batch, heads, kv_heads, dim, bs, maxblk) == how
+    kp, vp = (_rand(L, nb, bs, kv_heads, dim, dt=dt, seed=s) for s in (1, 2))
+    bt = torch.randperm(nb, generator=torch.Generator().manual_seed(3)).view(batch, maxblk).int().cuda()
+    qkv, key = _queries(batch, heads, kv_heads, dim, dt)
+    for b, n in enumerate(lens):
+        for tok in (0, n // 2, n - 1):
+            kp[layer, bt[b, tok // bs].long(), tok % bs] = key[b]
+        behind = torch.arange(n, maxblk * bs, device="cuda")
+        for p in (kp, vp):
+            p[layer, bt[b, behind // bs].long(), behind % bs] = float("nan")
+    bt[:, ::3] -= nb                                                # negative ids count from the end
+    pos = torch.tensor(lens, device="cuda") - 1
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    out = torch.full((batch, heads * dim), float("nan"), dtype=dt, device="cuda")
+    C.dec_attention(qkv, pos, kp, vp, bt, layer, L, nb, bs, heads, kv_heads, dim, out, status.data_ptr())
+    assert status.item() == 0
+    for b, n in enumerate(lens):
+        _check(out[b], qkv[b, : heads * dim].view(heads, dim), _of(kp[layer], bt[b], n), _of(vp[layer], bt[b], n), dt)
+
+
+@pytest.mark.parametrize("batch,kv_heads,dim,n,how", [(16, 8, 128, 2064, (2, 4)), (1, 8, 128, 7312, (8, 8)), (4, 32, 64, 1008, (2, 4)), (30, 8, 64, 256, (1, 4))])
+def test_the_ring_leaves_out_a_page_outside_the_pool(batch, kv_heads, dim, n, how):
+    from fuselink_b200 import C
+    bs, heads, dt, maxblk = 16, 2 * kv_heads, torch.bfloat16, n // 16
+    nb = batch * maxblk
+    assert _ring(batch, heads, kv_heads, dim, bs, maxblk) == how
+    kp, vp = (_rand(1, nb, bs, kv_heads, dim, dt=dt, seed=s) for s in (1, 2))
+    bt = torch.randperm(nb, generator=torch.Generator().manual_seed(3)).view(batch, maxblk).int().cuda()
+    outside = {0: nb, 5: -nb - 1, 6: 2 ** 31 - 1, maxblk - 1: -2 ** 31}
+    for p, value in outside.items():
+        bt[batch - 1, p] = value
+    (qkv, _), pos = _queries(batch, heads, kv_heads, dim, dt), torch.full((batch,), n - 1, device="cuda")
+    out, status = torch.empty(batch, heads * dim, dtype=dt, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+    C.dec_attention(qkv, pos, kp, vp, bt, 0, 1, nb, bs, heads, kv_heads, dim, out, status.data_ptr())
+    assert status.item() == 3
+    for b in {0, batch - 1}:
+        k, v = (_of(p[0], bt[b], n, outside if b == batch - 1 else ()) for p in (kp, vp))
+        _check(out[b], qkv[b, : heads * dim].view(heads, dim), k, v, dt)
+
+
+@pytest.mark.parametrize("dt", DT)
+@pytest.mark.parametrize("batch,kv_heads,dim,n,how", [(16, 8, 128, 2049, (2, 4)), (1, 8, 128, 7300, (8, 8)), (4, 32, 64, 1000, (2, 4))])
+@pytest.mark.parametrize("value,where", [(float("nan"), "first"), (float("nan"), "last"), (float("inf"), "middle"), (float("-inf"), "first"), (float("-inf"), "last"),
+                                         (float("-inf"), "all")])
+def test_the_ring_passes_on_what_is_not_finite(dt, batch, kv_heads, dim, n, how, value, where):
+    """As through registers: NaN and infinite scores make the head NaN, those of -inf weigh nothing; other heads and requests as without."""
+    from fuselink_b200 import C
+    bs, heads, maxblk = 16, 2 * kv_heads, -(-n // 16)
+    nb = batch * maxblk
+    assert _ring(batch, heads, kv_heads, dim, bs, maxblk) == how
+    kp, vp = (_rand(1, nb, bs, kv_heads, dim, dt=dt, seed=s) for s in (1, 2))
+    bt = torch.randperm(nb, generator=torch.Generator().manual_seed(3)).view(batch, maxblk).int().cuda()
+    qkv = _rand(batch, (heads + 2 * kv_heads) * dim, dt=dt, seed=4)
+    qkv[:, 0:heads * dim:dim] = 1                                   # every query's first column: the score gets the key's infinity
+    at = {"first": torch.arange(16), "middle": torch.tensor([n // 2]), "last": torch.arange((n - 1) // 16 * 16, n), "all": torch.arange(n)}[where].cuda()
+    kp[0, bt[0, at // bs].long(), at % bs, 1, 0] = value
+    out = torch.empty(batch, heads * dim, dtype=dt, device="cuda")
+    C.dec_attention(qkv, torch.full((batch,), n - 1, device="cuda"), kp, vp, bt, 0, 1, nb, bs, heads, kv_heads, dim, out)
+    for b in {0, batch - 1}:
+        want = _check(out[b], qkv[b, : heads * dim].view(heads, dim), _of(kp[0], bt[b], n), _of(vp[0], bt[b], n), dt)
+        if b == 0:
+            assert want.view(heads, dim)[2:4].isnan().all() == (value != float("-inf") or where == "all")
+
+
+@pytest.mark.parametrize("batch,heads,kv_heads,dim,n", [(16, 32, 8, 128, 2047), (1, 8, 8, 128, 7311), (4, 32, 32, 64, 1007), (3, 4, 4, 64, 389), (17, 8, 8, 128, 511)])
+def test_the_chain_attends_to_the_token_that_was_just_written(batch, heads, kv_heads, dim, n):
+    """Page write and attention, launched one behind the other as a step does, through several layers and steps without a wait in
+    between: every attention sees its own step's keys and values, which weigh more than all others together."""
+    from fuselink_b200 import C
+    L, bs, steps, dt = 6, 16, 2, torch.bfloat16
+    maxblk = (n + steps) // bs + 1
+    nb = batch * maxblk
+    kp, vp = (_rand(L, nb, bs, kv_heads, dim, dt=dt, seed=s) for s in (1, 2))
+    k0, v0 = kp.clone(), vp.clone()
+    bt = torch.randperm(nb, generator=torch.Generator().manual_seed(3)).view(batch, maxblk).int().cuda()
+    qkv = [[_rand(batch, (heads + 2 * kv_heads) * dim, dt=dt, seed=100 * s + l) for l in range(L)] for s in range(steps)]
+    for x in sum(qkv, []):
+        x = x.view(batch, heads + 2 * kv_heads, dim)
+        x[:, heads:heads + kv_heads] = x[:, :heads].float().view(batch, kv_heads, -1, dim).sum(2).to(dt)
+    outs = [[torch.empty(batch, heads * dim, dtype=dt, device="cuda") for _ in range(L)] for _ in range(steps)]
+    pos = [torch.full((batch,), n + s, device="cuda") for s in range(steps)]
+    torch.cuda.synchronize()
+    for s in range(steps):
+        for l in range(L):
+            C.dec_qkv(qkv[s][l], None, None, pos[s], 1, kp, vp, bt, 1, l, L, nb, bs, heads, kv_heads, dim)
+            C.dec_attention(qkv[s][l], pos[s], kp, vp, bt, l, L, nb, bs, heads, kv_heads, dim, outs[s][l])
+    for s in range(steps):
+        for l in range(L):
+            new = qkv[s][l].view(batch, -1, dim)
+            for b in range(batch):
+                page, slot = bt[b, (n + s) // bs].long(), (n + s) % bs
+                k0[l, page, slot], v0[l, page, slot] = new[b, heads:heads + kv_heads], new[b, heads + kv_heads:]
+            for b in {0, batch - 1}:
+                _check(outs[s][l][b], new[b, :heads], _of(k0[l], bt[b], n + s + 1), _of(v0[l], bt[b], n + s + 1), dt)
+    assert torch.equal(kp, k0) and torch.equal(vp, v0)
