@@ -7,6 +7,7 @@
 // Reference parity: none in the reference (it has no kernels); this is the fp8 arm of the MoE expert GEMMs.
 #include "fp8_gemm.cuh"
 #include "../common/fl_ptx.cuh"
+#include "tile_map.cuh"
 #include <cuda.h>
 #include <cuda_fp8.h>
 #include <stdio.h>
@@ -488,21 +489,11 @@ fp8_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
 // ------------------------------------------------------------------------------------------------
 // host
 // ------------------------------------------------------------------------------------------------
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 static thread_local char g_err[256] = "";
 
 static int make_map(CUtensorMap* m, const void* base, long long inner, long long outer, long long groups, int box_inner,
                     int box_outer) {
-  static EncodeTiledFn enc = nullptr;
-  if (!enc) {
-    void* sym = nullptr;
-    cudaDriverEntryPointQueryResult qres;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &sym, cudaEnableDefault, &qres) == cudaSuccess &&
-        qres == cudaDriverEntryPointSuccess)
-      enc = reinterpret_cast<EncodeTiledFn>(sym);
-  }
+  const fl::TileEncodeFn enc = fl::tile_encode();
   if (!enc) { snprintf(g_err, sizeof g_err, "cuTensorMapEncodeTiled entry point not available"); return -10; }
   cuuint64_t dims[3] = {(cuuint64_t)inner, (cuuint64_t)outer, (cuuint64_t)groups};
   cuuint64_t strides[2] = {(cuuint64_t)inner, (cuuint64_t)inner * (cuuint64_t)outer};   // bytes: 1 per element

@@ -21,6 +21,7 @@
 // all-to-alls.  This file is the replacement for that GEMM + the second all-to-all.
 #include "grouped_gemm.cuh"
 #include "../common/fl_ptx.cuh"
+#include "tile_map.cuh"
 #include <cuda.h>
 #include <math.h>
 #include <stdio.h>
@@ -979,28 +980,12 @@ grouped_gemm_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
 // --------------------------------------------------------------------------------------------------
 // host side
 // --------------------------------------------------------------------------------------------------
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
 static thread_local char g_err[256] = "";
-
-static EncodeTiledFn get_encode() {
-  static EncodeTiledFn fn = nullptr;
-  if (!fn) {
-    void* sym = nullptr;
-    cudaDriverEntryPointQueryResult qres;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &sym, cudaEnableDefault, &qres) == cudaSuccess &&
-        qres == cudaDriverEntryPointSuccess)
-      fn = reinterpret_cast<EncodeTiledFn>(sym);
-  }
-  return fn;
-}
 
 // 3-D bf16 view {inner, outer, groups}; box {box_inner, box_outer, 1}; 128-byte swizzle; zero fill.
 static int make_map(CUtensorMap* m, const void* base, long long inner, long long outer, long long groups,
                     long long ld_elems, long long gs_elems, int box_inner, int box_outer) {
-  EncodeTiledFn enc = get_encode();
+  const TileEncodeFn enc = tile_encode();
   if (!enc) {
     snprintf(g_err, sizeof g_err, "cuTensorMapEncodeTiled entry point not available");
     return -10;

@@ -600,6 +600,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         py::arg("dim"), py::arg("out"), py::arg("status_addr") = 0);
   m.def("dec_product", &dec_product, py::arg("x"), py::arg("w"), py::arg("bias"), py::arg("epilogue"), py::arg("early") = false,
         py::arg("status_addr") = 0);
+  m.attr("THIN_MAX_ROWS") = FL_THIN_MAX_ROWS;
   m.def("dec_argmax", &dec_argmax);
   m.def("dec_advance", &dec_advance);
   m.def("moe_dispatch", &moe_dispatch);

@@ -30,7 +30,6 @@ KV_BLHSD, KV_LBSHD = 0, 1
 _OPERATIONS = ("_embed", "_norm", "_qkv", "_attn_out", "_mlp", "_logits")      # what the fused route does by itself
 _ACT = {"llama": 0, "opt": 1, "gpt2": 2}          # FlDecAct
 _STORE = 3                                         # FlThinEpi
-_THIN_ROWS = 16                                    # rows up to which csrc/kernels/thin_gemm.cu makes the products
 
 
 @dataclass
@@ -291,10 +290,10 @@ class LlamaShard(torch.nn.Module):
     def _thin(self, rows: int, like: torch.Tensor, *matrices) -> bool:
         """Whether csrc/kernels/thin_gemm.cu makes the products of so many rows with these (list of matrices, rows, columns): plain
         tensors of the shard's type and device, contiguous, from a multiple of 16 bytes on.  Others stay the library's."""
-        if not (like.is_cuda and 0 < rows <= _THIN_ROWS):
+        if not like.is_cuda:
             return False
         C = require_native()
-        return all(C.dec_takes(list(ws), like, shape) for ws, *shape in matrices)
+        return 0 < rows <= C.THIN_MAX_ROWS and all(C.dec_takes(list(ws), like, shape) for ws, *shape in matrices)
 
     def _layers_fused(self, x, pos, seq, k_pool, v_pool, table, layout, num_blocks, attend, on_layer_done=None):
         """Every layer on x [rows, hidden]; ``attend(l, qkv)`` returns the attention output [rows, h_local * D].  Returns
