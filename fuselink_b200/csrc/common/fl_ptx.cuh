@@ -197,10 +197,30 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
   return true;
 }
 
-// The same by all lanes of a warp, which go on together and with one answer: what follows a wait (shuffles, .aligned instructions,
-// barriers) wants all of them.
+// The same by all lanes of a warp, which look together and go on together with one answer: what follows a wait (shuffles, .aligned
+// instructions, barriers) wants all of them.
 __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status, int code, int where) {
-  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, status, code, where));
+  if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+  const uint64_t t0 = global_timer_ns();
+  uint32_t spins = 0;
+  while (!__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) {
+    if ((++spins & 63u) == 0) {
+      const bool late = global_timer_ns() - t0 > (uint64_t)FL_WAIT_NS;
+      if (__any_sync(0xffffffffu, late || *abort_flag)) {
+        if (late) report(status, code, where);
+        *abort_flag = 1;
+        return false;
+      }
+    }
+  }
+  return true;
+}
+
+// After a wait that ran out: 2 ms, in which copies that are on the way into this CTA's shared memory land.  Not unrolled: the 2000
+// instructions, between those of a kernel of a few microseconds, cost it 0.3 us.
+__device__ __forceinline__ void let_copies_land() {
+#pragma unroll 1
+  for (int j = 0; j < 2000; ++j) __nanosleep(1000);
 }
 
 // ---- programmatic dependent launch --------------------------------------------------------------------

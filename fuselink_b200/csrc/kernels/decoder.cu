@@ -682,7 +682,7 @@ __global__ void __launch_bounds__(W * 32, 8 / W) dec_attention_ring_kernel(const
     const int s = (u - first) % ST;
     if (!mbar_wait_warp(&full[warp][s], ((u - first) / ST) & 1, &abort_flag, nullptr, kTimeoutMbarFull, 0)) {
       note(kv.status, FL_DEC_STALLED);
-      for (int j = 0; j < 2000; ++j) __nanosleep(1000);          // copies on the way land before shared memory goes away
+      let_copies_land();                                         // before shared memory goes away
       break;
     }
     const uint32_t at = smem_u32(ring + s * Ring::kStage);
@@ -808,9 +808,10 @@ static bool aligned(std::initializer_list<const void*> pointers) {
 }
 
 // Whether a kernel over so many rows may start while the one before it in the stream ends (before grid_dep_wait it touches nothing that
-// decides a result: the attention looks at positions and page ids, for what to ask into L2, and reads them again): the launch itself, 2 to 3 us in a chain of kernels that take no longer, is then out of the way.  Only as far as the
-// products are thin_gemm.cu's, which take part in it; between library products it costs (23 requests, 8B model: 15.1 ms without, 15.3
-// with).  dec_embed_kernel is launched without: it begins a chain, in which weights written by whatever came before are complete.
+// decides a result: the attention looks at positions and page ids, for what to ask into L2, and reads them again behind it): the launch
+// itself, 2 to 3 us in a chain of kernels that take no longer, is then out of the way.  Only as far as the products are thin_gemm.cu's,
+// which take part in it; between library products it costs (23 requests, 8B model: 15.1 ms without, 15.3 with).  dec_embed_kernel is
+// launched without: it begins a chain, in which weights written by whatever came before are complete.
 static bool chained(long long rows) { return rows <= FL_THIN_MAX_ROWS; }
 
 template <typename... P, typename... A>
@@ -981,8 +982,9 @@ extern "C" int fl_dec_attention(int dtype, const void* q, long long q_stride, co
 extern "C" int fl_dec_argmax(int dtype, const void* logits, long long* out, int rows, long long vocab, cudaStream_t stream) {
   if (rows < 0 || vocab < 1) return -2;
   if (rows == 0) return 0;
-  // eight CTAs for rows that have a vector for each of their threads, where all of them find room at once; more rows than a grid's
-  // second dimension takes go in several launches
+  // Eight CTAs for rows that have a vector for each of their threads, where all of them find room at once (one CTA | eight, us: 32768
+  // entries, 4 rows 10.4 | 5.5, 37 rows 10.3 | 8.3; 128256, 37 rows 22.7 | 12.5, 64 rows 24.1 | 16.5; 50272, 100 rows 12.8 | 14.4).  More
+  // rows than a grid's second dimension takes go in several launches.
   const int parts = vocab >= 8ll * 8 * 512 && rows <= 148 / 4 ? 8 : 1;
   for (int r = 0; r < rows; r += 65535) {
     cudaLaunchConfig_t cfg = {};

@@ -15,8 +15,14 @@
 // 16 rows, one product after another with w from memory: 6144 x 4096 13.1 us (library 11.7), 4096 x 4096 9.4 (9.3), 2 x 14336 x 4096
 // with the activation 39.8 (40.9 without it), 4096 x 14336 22.3 (23.0); 3 rows: 2048 x 8192 9.4 (17.9), 2048 x 2048 4.3 (6.4).  What
 // counts is the chain: with library products a layer of an 8B model at 16 rows and 2048 tokens took 143 us, with these and the
-// attention's ring (decoder.cu) 121.  At 32 rows they are slower than the library's (15.0, 11.1, 42.6 and 24.5 us against 12.1, 9.4,
-// 41.0 and 27.1), and so is the step, by 6 %: the line is at 16.
+// attention's ring (decoder.cu) 121.  The output head is the last of them and gains least: 128256 x 4096 takes 167 us alone (library
+// 157), a step with it here or there the same within 0.5 % (16 x 2048 tokens 4049 | 4030 us, 1.3B model 16 x 1000 1937 | 1927, 8B
+// 1 x 500 3301 | 3304), GPT-2's less (16 x 500: 486 | 529).
+//
+// The line is at 16 rows, one tile's N.  From 17 on the tile would be of 32 rows, with four stages.  As measured with it, own | library:
+// 17 rows 6144 x 4096 14.0 | 10.9 us, 4096 x 14336 23.3 | 23.7; 24 rows 14.4 | 10.9, 24.1 | 23.7; a step of an 8B model 3794 | 3804 us
+// at 17 requests, 3928 | 3884 at 24, 4040 | 3994 at 31, of a 1.3B model 1608 | 1602 and 1790 | 1745 at 17 and 24; only GPT-2 gains (503 |
+// 526 at 17, 603 | 647 at 28).
 #include "thin_gemm.cuh"
 #include "decoder.cuh"
 #include <cuda_bf16.h>
@@ -162,11 +168,9 @@ thin_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
   tc_fence_before_sync();
   if (splits > 1) cluster_sync_all();
   else __syncthreads();
-  // whoever gave up, the loader may have copies on the way: they land before this CTA's shared memory and TMEM go away
-  if (*reinterpret_cast<volatile int*>(&abort_flag)) {
-    for (int j = 0; j < 2000; ++j) __nanosleep(1000);
-  }
   if (warp == 1) {
+    // whoever gave up, the loader may have copies on the way: they land before TMEM and, with this warp, the CTA's shared memory go away
+    if (*reinterpret_cast<volatile int*>(&abort_flag)) let_copies_land();
     tc_fence_after_sync();
     tmem_dealloc(tmem_base, TG_TMEM_COLS);
   }

@@ -48,11 +48,11 @@ def test_what_another_kernel_writes_is_not_read_as_read_only(name):
 
 
 def test_a_product_that_gave_up_waits_for_its_copies():
-    """Whichever role gives up (the products while the loader has no more blocks to wait for, say), every thread waits behind the
-    CTA's barrier before TMEM is freed and the CTA may end: copies into its shared memory may be on the way."""
+    """Whichever role gives up (the products while the loader has no more blocks to wait for, say), a warp waits behind the CTA's
+    barrier before it frees TMEM and the CTA may end: copies into its shared memory may be on the way."""
     body = _functions("thin_gemm.cu")["thin_gemm_kernel"]
     behind = body[body.rindex("mbar_wait"):]                     # nobody gives up later than that
-    barrier, look, free = (re.search(r, behind) for r in (r"else __syncthreads\(\);", r"if \([^{;]*abort_flag\)+ \{[^}]*__nanosleep", r"tmem_dealloc"))
+    barrier, look, free = (re.search(r, behind) for r in (r"else __syncthreads\(\);", r"if \([^{;]*abort_flag\)+ let_copies_land\(\);", r"tmem_dealloc"))
     assert barrier and look and free and barrier.end() < look.start() < look.end() < free.start()
 
 
