@@ -2,11 +2,26 @@
 //
 //   warp 0      : TMA producer (e4m3 tiles, 128-byte swizzle, never multicast)
 //   warp 1      : MMA issuer   (tcgen05.mma kind::f8f6f4; one 128-deep block per TMEM partial buffer)
-//   warps 2..9  : promotion + epilogue (tcgen05.ld partial -> scale -> fp32 registers -> fused epilogue)
+//   warps 2, 3  : the operands' scales, from memory to shared memory, several blocks ahead
+//   warps 4..11 : promotion + epilogue (tcgen05.ld partial -> scale -> fp32 registers -> fused epilogue); two warps
+//                 share each TMEM lane quadrant and split the tile's columns
+//
+// Bound by the promotion: every partial sum makes a trip from TMEM and takes an fp32 FMA, in a chain that the next multiplication
+// into the same buffer waits for.  So nothing else is in that chain: the scales come through shared memory (read from global
+// memory by the promotion threads, one 4-byte load per row 4 K / 128 bytes apart, they cost a fifth of the kernel's time), a chunk of
+// a partial is on its way while the one before it is added, also from one block to the next, and two FMAs are one instruction.
+// 8 experts, 1024 rows each, hidden 4096, ffn 14336, before and now: second product forward (K = 14336, N = 4096) 582 (scales from
+// global memory, the rest as now) -> 524 us, gradient of the first (K = 28672) 1204 -> 1043; without the FMAs it is 902, without the
+// trips to TMEM 760 (multiplications and loads).  In a training step of 4096 tokens the four products took 4950 us with the loads of
+// the scales, the trips and the FMAs one after the other, now 3905.  Sixteen promotion warps with half the columns each: 1060.
+// The epilogues run between two tiles of a CTA and are not hidden: they store whole sectors through shared memory, ask for the saved
+// gate and up rows a tile ahead, and divide with __fdividef (DSWIGLU product 970 -> 834 us with it; the error against 64 bits is the same
+// to seven digits, 1.6602e-3 of the results' 2-norm, which is the rounding to bf16).
 //
 // Reference parity: none in the reference (it has no kernels); this is the fp8 arm of the MoE expert GEMMs.
 #include "fp8_gemm.cuh"
 #include "../common/fl_ptx.cuh"
+#include "staged_store.cuh"
 #include "tile_map.cuh"
 #include <cuda.h>
 #include <cuda_fp8.h>
@@ -23,9 +38,20 @@ constexpr int STAGES = 4;
 constexpr int A_STAGE = BM * BKB;             // 16 KiB
 constexpr int B_STAGE = BN * BKB;             // 32 KiB
 constexpr int STAGE = A_STAGE + B_STAGE;
-constexpr int NUM_THREADS = 320;
+constexpr int EPI_WARPS = 8;
+constexpr int NUM_THREADS = 128 + 32 * EPI_WARPS;
+// Registers: 384 threads start with 168 each (64512).  The first four warps give 112 each back, the others take 56 more: 128 x 56 +
+// 256 x 224 = 64512.  A promotion thread holds 128 sums, 32 values being added and 32 on their way from TMEM.
+constexpr int PRODUCER_REGS = 56, EPI_REGS = 224;
 constexpr int TMEM_COLS = 512;                // two partial buffers of 256 columns
-constexpr int SMEM_BYTES = STAGES * STAGE + 1024 + 1024;
+constexpr int SC_BLOCKS = 8;                  // blocks of contraction whose scales travel together (a 32-byte sector per row)
+constexpr int SC_STAGES = 2;
+struct ScaleStage {
+  float a[SC_BLOCKS][BM];
+  float b[SC_BLOCKS][2];
+};
+constexpr int SHARED_BYTES = 1024;            // barriers, counts
+constexpr int SMEM_BYTES = STAGES * STAGE + 1024 /*align*/ + SHARED_BYTES + EPI_WARPS * EPI_STAGE_BYTES + SC_STAGES * (int)sizeof(ScaleStage);
 
 struct KParams {
   int num_groups, cap, N, K;
@@ -50,10 +76,14 @@ struct Shared {
   uint64_t empty[STAGES];
   uint64_t pfull[2];
   uint64_t pempty[2];
+  uint64_t sfull[SC_STAGES];
+  uint64_t sempty[SC_STAGES];
   uint32_t tmem_base;
   int abort_flag;
   int counts[FL_GEMM_MAX_GROUPS];
 };
+
+static_assert(sizeof(Shared) <= SHARED_BYTES, "barriers and counts");
 
 struct Tile {
   int g, m0, n0, rows, cnt;
@@ -81,61 +111,6 @@ __device__ __forceinline__ bool map_tile(const KParams& p, const int* counts, in
     acc += tiles;
   }
   return false;
-}
-
-__device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
-  __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
-  return *reinterpret_cast<uint32_t*>(&v);
-}
-__device__ __forceinline__ void store32_bf16(__nv_bfloat16* dst, const float* v) {
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    uint4 o;
-    o.x = pack_bf16(v[8 * i + 0], v[8 * i + 1]);
-    o.y = pack_bf16(v[8 * i + 2], v[8 * i + 3]);
-    o.z = pack_bf16(v[8 * i + 4], v[8 * i + 5]);
-    o.w = pack_bf16(v[8 * i + 6], v[8 * i + 7]);
-    st_v4(dst + 8 * i, o);
-  }
-}
-// 16-column variants: the epilogues that need the saved gate/up beside the 128 accumulators of a thread work on 16
-// columns at a time, which keeps their temporaries (and with them the register spills) small
-__device__ __forceinline__ void store16_bf16(__nv_bfloat16* dst, const float* v) {
-#pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    uint4 o;
-    o.x = pack_bf16(v[8 * i + 0], v[8 * i + 1]);
-    o.y = pack_bf16(v[8 * i + 2], v[8 * i + 3]);
-    o.z = pack_bf16(v[8 * i + 4], v[8 * i + 5]);
-    o.w = pack_bf16(v[8 * i + 6], v[8 * i + 7]);
-    st_v4(dst + 8 * i, o);
-  }
-}
-__device__ __forceinline__ void load16_bf16(const __nv_bfloat16* src, float* v) {
-#pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    uint4 o = ld_v4(src + 8 * i);
-    const uint32_t w[4] = {o.x, o.y, o.z, o.w};
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      __nv_bfloat162 h = *reinterpret_cast<const __nv_bfloat162*>(&w[j]);
-      v[8 * i + 2 * j] = __bfloat162float(h.x);
-      v[8 * i + 2 * j + 1] = __bfloat162float(h.y);
-    }
-  }
-}
-__device__ __forceinline__ void load32_bf16(const __nv_bfloat16* src, float* v) {
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    uint4 o = ld_v4(src + 8 * i);
-    const uint32_t w[4] = {o.x, o.y, o.z, o.w};
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      __nv_bfloat162 h = *reinterpret_cast<const __nv_bfloat162*>(&w[j]);
-      v[8 * i + 2 * j] = __bfloat162float(h.x);
-      v[8 * i + 2 * j + 1] = __bfloat162float(h.y);
-    }
-  }
 }
 
 // 8 neighbouring values; WIDE: the address is a multiple of 16 bytes (otherwise of 8)
@@ -255,11 +230,20 @@ __global__ void __launch_bounds__(256) quantize_blocks_kernel(const __nv_bfloat1
 // and the up value of the same 64 activation columns, and every chunk pair exactly one weight scale block.
 __device__ __forceinline__ int chunk_col(int half, int c) { return (c < 2 ? 0 : 128) + 64 * half + 32 * (c & 1); }
 
+// two fp32 accumulators: acc += v * s, each rounded as fmaf does
+__device__ __forceinline__ void fma2(float2& acc, uint32_t v0, uint32_t v1, float s) {
+  asm volatile("{\n\t.reg .b64 a, v, s;\n\tmov.b64 a, {%0, %1};\n\tmov.b64 v, {%2, %3};\n\tmov.b64 s, {%4, %4};\n\t"
+      "fma.rn.f32x2 a, v, s, a;\n\tmov.b64 {%0, %1}, a;\n\t}"
+      : "+f"(acc.x), "+f"(acc.y) : "r"(v0), "r"(v1), "f"(s));
+}
+
+template <int EPI>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 fp8_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const KParams p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   Shared* sh = reinterpret_cast<Shared*>(smem + STAGES * STAGE);
+  ScaleStage* sc_ring = reinterpret_cast<ScaleStage*>(smem + STAGES * STAGE + SHARED_BYTES + EPI_WARPS * EPI_STAGE_BYTES);
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const int KB = p.K / 128;
@@ -271,7 +255,11 @@ fp8_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(&sh->pfull[b], 1);
-      mbar_init(&sh->pempty[b], 8);
+      mbar_init(&sh->pempty[b], EPI_WARPS);
+    }
+    for (int i = 0; i < SC_STAGES; ++i) {
+      mbar_init(&sh->sfull[i], 2);
+      mbar_init(&sh->sempty[i], EPI_WARPS);
     }
     sh->abort_flag = 0;
     mbar_fence_init();
@@ -293,122 +281,169 @@ fp8_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
   volatile int* abort_flag = &sh->abort_flag;
   const int* counts = sh->counts;
 
-  if (warp == 0) {
-    if (lane == 0) {
-      uint32_t it = 0;
-      bool ok = true;
-      Tile t;
-      for (int id = blockIdx.x; ok && map_tile(p, counts, id, t); id += gridDim.x) {
-        for (int kb = 0; kb < KB && ok; ++kb, ++it) {
-          const int s = it % STAGES;
-          const uint32_t ph = (it / STAGES) & 1;
-          ok = mbar_wait(&sh->empty[s], ph ^ 1, abort_flag, p.status, kTimeoutMbarEmpty, 2100 + s);
-          if (!ok) break;
-          uint8_t* a_dst = smem + s * STAGE;
-          uint8_t* b_dst = a_dst + A_STAGE;
-          mbar_arrive_expect_tx(&sh->full[s], STAGE);
-          const int k0 = kb * 128;
-          tma_load_3d(a_dst, &tmA, &sh->full[s], k0, t.m0, t.g);
-          if (!p.b_mn) {
-            tma_load_3d(b_dst, &tmB, &sh->full[s], k0, t.n0, t.g);
-          } else {
+  if (warp < 4) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(PRODUCER_REGS));
+    if (warp == 0) {
+      if (lane == 0) {
+        uint32_t it = 0;
+        bool ok = true;
+        Tile t;
+        for (int id = blockIdx.x; ok && map_tile(p, counts, id, t); id += gridDim.x) {
+          for (int kb = 0; kb < KB && ok; ++kb, ++it) {
+            const int s = it % STAGES;
+            const uint32_t ph = (it / STAGES) & 1;
+            ok = mbar_wait(&sh->empty[s], ph ^ 1, abort_flag, p.status, kTimeoutMbarEmpty, 2100 + s);
+            if (!ok) break;
+            uint8_t* a_dst = smem + s * STAGE;
+            uint8_t* b_dst = a_dst + A_STAGE;
+            mbar_arrive_expect_tx(&sh->full[s], STAGE);
+            const int k0 = kb * 128;
+            tma_load_3d(a_dst, &tmA, &sh->full[s], k0, t.m0, t.g);
+            if (!p.b_mn) {
+              tma_load_3d(b_dst, &tmB, &sh->full[s], k0, t.n0, t.g);
+            } else {
 #pragma unroll
-            for (int j = 0; j < BN / 128; ++j)
-              tma_load_3d(b_dst + j * (128 * BKB), &tmB, &sh->full[s], t.n0 + 128 * j, k0, t.g);
+              for (int j = 0; j < BN / 128; ++j)
+                tma_load_3d(b_dst + j * (128 * BKB), &tmB, &sh->full[s], t.n0 + 128 * j, k0, t.g);
+            }
+          }
+        }
+        if (!ok) let_copies_land();
+      }
+    } else if (warp == 1) {
+      if (lane == 0) {
+        const uint32_t idesc = make_idesc(0, 0, 0u, p.b_mn ? 1u : 0u, BM, BN);   // e4m3 x e4m3 -> fp32
+        uint32_t it = 0;
+        bool ok = true;
+        Tile t;
+        for (int id = blockIdx.x; ok && map_tile(p, counts, id, t); id += gridDim.x) {
+          for (int kb = 0; kb < KB && ok; ++kb, ++it) {
+            const int s = it % STAGES;
+            const uint32_t ph = (it / STAGES) & 1;
+            const int b = it & 1;
+            const uint32_t bph = (it >> 1) & 1;
+            ok = mbar_wait(&sh->pempty[b], bph ^ 1, abort_flag, p.status, kTimeoutTmemEmpty, 2200 + b);
+            if (!ok) break;
+            ok = mbar_wait(&sh->full[s], ph, abort_flag, p.status, kTimeoutMbarFull, 2300 + s);
+            if (!ok) break;
+            tc_fence_after_sync();
+            const uint32_t a_base = smem_u32(smem + s * STAGE);
+            const uint32_t b_base = a_base + A_STAGE;
+            const uint32_t d_tmem = tmem_base + b * BN;
+#pragma unroll
+            for (int kk = 0; kk < 4; ++kk) {   // 4 x (K = 32) per 128-deep block
+              const uint64_t da = make_smem_desc(a_base + kk * 32, 16, 1024);
+              const uint64_t db = p.b_mn ? make_smem_desc(b_base + kk * 4096, 128 * BKB, 1024)
+                                         : make_smem_desc(b_base + kk * 32, 16, 1024);
+              umma_f8(d_tmem, da, db, idesc, kk != 0 ? 1u : 0u);
+            }
+            umma_commit(&sh->empty[s]);
+            umma_commit(&sh->pfull[b]);
           }
         }
       }
-      if (!ok) {
-        for (int i = 0; i < 2000; ++i) __nanosleep(1000);
-      }
-    }
-  } else if (warp == 1) {
-    if (lane == 0) {
-      const uint32_t idesc = make_idesc(0, 0, 0u, p.b_mn ? 1u : 0u, BM, BN);   // e4m3 x e4m3 -> fp32
+    } else {
+      const int i = (warp - 2) * 32 + lane;
+      const int NB = p.N / 128;
       uint32_t it = 0;
       bool ok = true;
       Tile t;
       for (int id = blockIdx.x; ok && map_tile(p, counts, id, t); id += gridDim.x) {
-        for (int kb = 0; kb < KB && ok; ++kb, ++it) {
-          const int s = it % STAGES;
-          const uint32_t ph = (it / STAGES) & 1;
-          const int b = it & 1;
-          const uint32_t bph = (it >> 1) & 1;
-          ok = mbar_wait(&sh->pempty[b], bph ^ 1, abort_flag, p.status, kTimeoutTmemEmpty, 2200 + b);
-          if (!ok) break;
-          ok = mbar_wait(&sh->full[s], ph, abort_flag, p.status, kTimeoutMbarFull, 2300 + s);
-          if (!ok) break;
-          tc_fence_after_sync();
-          const uint32_t a_base = smem_u32(smem + s * STAGE);
-          const uint32_t b_base = a_base + A_STAGE;
-          const uint32_t d_tmem = tmem_base + b * BN;
+        const float* a0 = p.a_scale + ((long long)t.g * p.cap + t.m0 + i) * KB;
+        // of block kb: b0[kb * next_k] and b0[kb * next_k + next_n]
+        const long long nb = t.n0 / 128, next_n = p.b_mn ? 1 : KB, next_k = p.b_mn ? NB : 1;
+        const float* b0 = p.b_scale + (p.b_mn ? (long long)t.g * KB * NB + nb : ((long long)t.g * NB + nb) * KB);
+        for (int kb = 0; kb < KB; kb += SC_BLOCKS, ++it) {
+          const int n = min(SC_BLOCKS, KB - kb);
+          float v[2][SC_BLOCKS], w = 0.f;
 #pragma unroll
-          for (int kk = 0; kk < 4; ++kk) {   // 4 x (K = 32) per 128-deep block
-            const uint64_t da = make_smem_desc(a_base + kk * 32, 16, 1024);
-            const uint64_t db = p.b_mn ? make_smem_desc(b_base + kk * 4096, 128 * BKB, 1024)
-                                       : make_smem_desc(b_base + kk * 32, 16, 1024);
-            umma_f8(d_tmem, da, db, idesc, kk != 0 ? 1u : 0u);
-          }
-          umma_commit(&sh->empty[s]);
-          umma_commit(&sh->pfull[b]);
+          for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int k = 0; k < SC_BLOCKS; ++k) v[h][k] = k < n && i + 64 * h < t.rows ? a0[64ll * h * KB + kb + k] : 0.f;
+          if (i < 2 * n) w = b0[(kb + (i >> 1)) * next_k + (i & 1) * next_n];
+          const int s = it % SC_STAGES;
+          ok = mbar_wait_warp(&sh->sempty[s], ((it / SC_STAGES) & 1) ^ 1, abort_flag, p.status, kTimeoutMbarEmpty, 2600 + s);
+          if (!ok) break;
+          ScaleStage& st = sc_ring[s];
+#pragma unroll
+          for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int k = 0; k < SC_BLOCKS; ++k) st.a[k][i + 64 * h] = v[h][k];
+          if (i < 2 * n) st.b[i >> 1][i & 1] = w;
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&sh->sfull[s]);
         }
       }
     }
   } else {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(EPI_REGS));
     const int q = warp & 3;
-    const int half = (warp - 2) >> 2;
-    uint32_t it = 0;
+    const int half = (warp - 4) >> 2;
+    uint8_t* stg = smem + STAGES * STAGE + SHARED_BYTES + (warp - 4) * EPI_STAGE_BYTES;
+    const int r_in_tile = q * 32 + lane;
+    uint32_t it = 0, sit = 0;                     // blocks and stages of scales so far
     bool ok = true;
     Tile t;
     for (int id = blockIdx.x; ok && map_tile(p, counts, id, t); id += gridDim.x) {
-      const int r_in_tile = q * 32 + lane;
       const int row = t.m0 + r_in_tile;
       const long long grow = (long long)t.g * p.cap + row;
       const bool valid = r_in_tile < t.rows;
-      const int NB = p.N / 128;
-      const int nb0 = t.n0 / 128;
-      float acc[128];
+      if (EPI == FL_EPI_DSWIGLU && half == 0 && valid)      // the saved gate/up of this row: in L2 by the time they are wanted
+        bulk_prefetch_l2(p.gu + grow * p.ldgu + 2ll * t.n0, BN * 2 * 2);
+      float2 acc[64];                                                 // chunk c: acc[16 c .. 16 c + 15]
 #pragma unroll
-      for (int i = 0; i < 128; ++i) acc[i] = 0.f;
-      const float* sa_row = p.a_scale + grow * KB;
-      for (int kb = 0; kb < KB && ok; ++kb, ++it) {
-        const int b = it & 1;
-        const uint32_t bph = (it >> 1) & 1;
-        // scales of this block (loaded before the wait so their latency overlaps it)
-        const float sa = valid ? sa_row[kb] : 0.f;
-        float sb0, sb1;
-        if (!p.b_mn) {
-          sb0 = p.b_scale[((long long)t.g * NB + nb0) * KB + kb];
-          sb1 = p.b_scale[((long long)t.g * NB + nb0 + 1) * KB + kb];
-        } else {
-          sb0 = p.b_scale[((long long)t.g * KB + kb) * NB + nb0];
-          sb1 = p.b_scale[((long long)t.g * KB + kb) * NB + nb0 + 1];
-        }
-        const float s0 = sa * sb0, s1 = sa * sb1;
-        ok = mbar_wait(&sh->pfull[b], bph, abort_flag, p.status, kTimeoutTmemFull, 2400 + b);
-        if (!ok) break;
+      for (int i = 0; i < 64; ++i) acc[i] = make_float2(0.f, 0.f);
+      // A chunk is on its way from TMEM while the one before it is added, over the ends of blocks as well: what bounds this loop is
+      // the chain of trips to TMEM, not their number of bytes or the additions.
+      auto t_addr = [&](int c) { return tmem_base + (it & 1) * BN + ((uint32_t)(q * 32) << 16) + chunk_col(half, c); };
+      auto partial = [&]() {                      // block `it` has been multiplied
+        ok = mbar_wait_warp(&sh->pfull[it & 1], (it >> 1) & 1, abort_flag, p.status, kTimeoutTmemFull, 2400 + (it & 1));
         tc_fence_after_sync();
-        const uint32_t t_addr = tmem_base + b * BN + ((uint32_t)(q * 32) << 16);
+      };
+      uint32_t r[2][32];
+      partial();
+      if (!ok) break;
+      tmem_ld_32x32(t_addr(0), r[0]);
+      for (int kb = 0; kb < KB; ++kb) {
+        const int k = kb % SC_BLOCKS, s = sit % SC_STAGES;
+        if (k == 0) ok = mbar_wait_warp(&sh->sfull[s], (sit / SC_STAGES) & 1, abort_flag, p.status, kTimeoutMbarFull, 2700 + s);
+        if (!ok) break;
+        const float sa = sc_ring[s].a[k][r_in_tile];
+        const float sc[2] = {sa * sc_ring[s].b[k][0], sa * sc_ring[s].b[k][1]};
+        tmem_ld_wait();
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
-          uint32_t r[32];
-          tmem_ld_32x32(t_addr + chunk_col(half, c), r);
-          tmem_ld_wait();
-          const float sc = c < 2 ? s0 : s1;
+          if (c < 3) {
+            tmem_ld_32x32(t_addr(c + 1), r[(c + 1) & 1]);
+          } else {                                // everything of this block is in registers
+            tc_fence_before_sync();
+            __syncwarp();
+            const bool scales_done = k == SC_BLOCKS - 1 || kb == KB - 1;
+            if (lane == 0) {
+              mbar_arrive(&sh->pempty[it & 1]);
+              if (scales_done) mbar_arrive(&sh->sempty[s]);
+            }
+            sit += scales_done;
+            ++it;
+            if (kb + 1 < KB) {
+              partial();
+              if (ok) tmem_ld_32x32(t_addr(0), r[0]);
+            }
+          }
 #pragma unroll
-          for (int i = 0; i < 32; ++i) acc[c * 32 + i] = fmaf(__uint_as_float(r[i]), sc, acc[c * 32 + i]);
+          for (int i = 0; i < 16; ++i) fma2(acc[c * 16 + i], r[c & 1][2 * i], r[c & 1][2 * i + 1], sc[c >> 1]);
+          if (c < 3) tmem_ld_wait();
         }
-        tc_fence_before_sync();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&sh->pempty[b]);
+        if (!ok) break;
       }
       if (!ok) break;
       // ---- fused epilogue from registers ----------------------------------------------------------
       const bool zero_row = !valid && p.zero_tail && row < min(p.cap, (t.cnt + 127) / 128 * 128);
-      if (p.epilogue == FL_EPI_STORE || p.epilogue == FL_EPI_SCATTER) {
+      auto at = [](__nv_bfloat16* d) { return reinterpret_cast<unsigned long long>(d); };
+      if (EPI == FL_EPI_STORE || EPI == FL_EPI_SCATTER) {
         __nv_bfloat16* dst = nullptr;
-        if (p.epilogue == FL_EPI_STORE) {
-          dst = p.C + grow * p.ldc;
+        if (EPI == FL_EPI_STORE) {
+          if (valid || zero_row) dst = p.C + grow * p.ldc;
         } else if (valid) {
           const int info = p.row_info[grow];
           const int rk = (info >> 28) & 0xF;
@@ -418,64 +453,74 @@ fp8_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
           else
             report(p.status, kBadIndex, 2500);   // names no rank / no slot of the receive buffer: not stored
         }
-        if ((valid && dst != nullptr) || (zero_row && p.epilogue == FL_EPI_STORE)) {
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          uint32_t pk[16];
+#pragma unroll
+          for (int i = 0; i < 16; ++i) pk[i] = valid ? pack_bf16(acc[c * 16 + i].x, acc[c * 16 + i].y) : 0u;
+          staged_store_packed(stg, lane, pk, dst != nullptr ? at(dst + t.n0 + chunk_col(half, c)) : 0ull);
+        }
+      } else if (EPI == FL_EPI_SWIGLU) {
+        const bool st = valid || zero_row;
+        __nv_bfloat16* act = p.C + grow * p.ldc + t.n0 / 2 + 64 * half;
+        __nv_bfloat16* gu = p.gu ? p.gu + grow * p.ldgu + t.n0 : nullptr;
+        uint32_t pk[16];
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {                                 // gate in chunk c, up in chunk c + 2
+#pragma unroll
+          for (int i = 0; i < 16; ++i) {
+            const float2 g = valid ? acc[c * 16 + i] : make_float2(0.f, 0.f), u = valid ? acc[32 + c * 16 + i] : make_float2(0.f, 0.f);
+            pk[i] = pack_bf16(__fdividef(g.x, 1.f + __expf(-g.x)) * u.x, __fdividef(g.y, 1.f + __expf(-g.y)) * u.y);
+          }
+          staged_store_packed(stg, lane, pk, st ? at(act + 32 * c) : 0ull);
+        }
+        if (gu) {
 #pragma unroll
           for (int c = 0; c < 4; ++c) {
-            float v[32];
 #pragma unroll
-            for (int i = 0; i < 32; ++i) v[i] = valid ? acc[c * 32 + i] : 0.f;
-            store32_bf16(dst + t.n0 + chunk_col(half, c), v);
-          }
-        }
-      } else if (p.epilogue == FL_EPI_SWIGLU) {
-        if (valid || zero_row) {
-          __nv_bfloat16* act = p.C + grow * p.ldc + t.n0 / 2 + 64 * half;
-          __nv_bfloat16* gu = p.gu ? p.gu + grow * p.ldgu + t.n0 + 64 * half : nullptr;
-#pragma unroll
-          for (int c = 0; c < 4; ++c) {                        // 16 columns at a time: gate in acc[0, 64), up in acc[64, 128)
-            float g[16], u[16], a[16];
-#pragma unroll
-            for (int i = 0; i < 16; ++i) {
-              g[i] = valid ? acc[c * 16 + i] : 0.f;
-              u[i] = valid ? acc[64 + c * 16 + i] : 0.f;
-              a[i] = g[i] / (1.f + __expf(-g[i])) * u[i];
-            }
-            store16_bf16(act + 16 * c, a);
-            if (gu) {
-              store16_bf16(gu + 16 * c, g);
-              store16_bf16(gu + 128 + 16 * c, u);
-            }
+            for (int i = 0; i < 16; ++i) pk[i] = valid ? pack_bf16(acc[c * 16 + i].x, acc[c * 16 + i].y) : 0u;
+            staged_store_packed(stg, lane, pk, st ? at(gu + chunk_col(half, c)) : 0ull);
           }
         }
       } else {  // FL_EPI_DSWIGLU: acc = dAct over 256 activation columns
-        if (valid || zero_row) {
+        const bool st = valid || zero_row;
 #pragma unroll
-          for (int c = 0; c < 8; ++c) {                        // 16 columns at a time: acc[16 c, 16 c + 16)
-            const int a_col = t.n0 + chunk_col(half, c >> 1) + 16 * (c & 1);
-            const long long gcol = (long long)(a_col >> 7) * 256 + (a_col & 127);
-            float dg[16], du[16];
+        for (int c = 0; c < 4; ++c) {
+          const int a_col = t.n0 + chunk_col(half, c);
+          const long long gcol = (long long)(a_col >> 7) * 256 + (a_col & 127);
+          uint32_t pdg[16], pdu[16];
+#pragma unroll
+          for (int h = 0; h < 4; ++h) {                               // 8 columns at a time
+            uint4 g8 = make_uint4(0, 0, 0, 0), u8 = make_uint4(0, 0, 0, 0);
             if (valid) {
-              float g[16], u[16];
-              load16_bf16(p.gu + grow * p.ldgu + gcol, g);
-              load16_bf16(p.gu + grow * p.ldgu + gcol + 128, u);
-#pragma unroll
-              for (int i = 0; i < 16; ++i) {
-                const float da = acc[c * 16 + i];
-                const float sg = 1.f / (1.f + __expf(-g[i]));
-                dg[i] = da * u[i] * (sg * (1.f + g[i] * (1.f - sg)));
-                du[i] = da * g[i] * sg;
-              }
-            } else {
-#pragma unroll
-              for (int i = 0; i < 16; ++i) dg[i] = du[i] = 0.f;
+              g8 = ld_v4(p.gu + grow * p.ldgu + gcol + 8 * h);
+              u8 = ld_v4(p.gu + grow * p.ldgu + gcol + 128 + 8 * h);
             }
-            store16_bf16(p.dgu + grow * p.ldgu + gcol, dg);
-            store16_bf16(p.dgu + grow * p.ldgu + gcol + 128, du);
+            const uint32_t gw[4] = {g8.x, g8.y, g8.z, g8.w}, uw[4] = {u8.x, u8.y, u8.z, u8.w};
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              float g[2], u[2], dg[2], du[2];
+              unpack_bf16(gw[i], g[0], g[1]);
+              unpack_bf16(uw[i], u[0], u[1]);
+              const float2 d2 = acc[c * 16 + 4 * h + i];
+#pragma unroll
+              for (int e = 0; e < 2; ++e) {
+                const float da = e ? d2.y : d2.x;
+                const float sg = __fdividef(1.f, 1.f + __expf(-g[e]));
+                dg[e] = da * u[e] * (sg * (1.f + g[e] * (1.f - sg)));
+                du[e] = da * g[e] * sg;
+              }
+              pdg[4 * h + i] = valid ? pack_bf16(dg[0], dg[1]) : 0u;
+              pdu[4 * h + i] = valid ? pack_bf16(du[0], du[1]) : 0u;
+            }
           }
+          __nv_bfloat16* dst = p.dgu + grow * p.ldgu + gcol;
+          staged_store_packed(stg, lane, pdg, st ? at(dst) : 0ull);
+          staged_store_packed(stg, lane, pdu, st ? at(dst + 128) : 0ull);
         }
       }
     }
-    if (p.epilogue == FL_EPI_SCATTER) fence_sys();
+    if (EPI == FL_EPI_SCATTER) fence_sys();
   }
 
   tc_fence_before_sync();
@@ -508,6 +553,24 @@ static int make_map(CUtensorMap* m, const void* base, long long inner, long long
                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) { snprintf(g_err, sizeof g_err, "cuTensorMapEncodeTiled failed with CUresult %d", (int)r); return -12; }
   return 0;
+}
+
+template <int EPI>
+static int launch(const CUtensorMap& tmA, const CUtensorMap& tmB, const KParams& p, int max_ctas, cudaStream_t stream) {
+  static int sms_of[64];                       // per device: the shared-memory attribute belongs to the device's copy of the kernel
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= 64) { snprintf(g_err, sizeof g_err, "device ordinal out of range"); return -1; }
+  int& num_sms = sms_of[dev];
+  if (!num_sms) {
+    cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev);
+    cudaError_t e = cudaFuncSetAttribute(fp8_grouped_gemm_kernel<EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
+    if (e != cudaSuccess) { num_sms = 0; return (int)e; }
+  }
+  int grid = num_sms;
+  if (max_ctas > 0 && max_ctas < grid) grid = max_ctas;
+  fp8_grouped_gemm_kernel<EPI><<<grid, NUM_THREADS, SMEM_BYTES, stream>>>(tmA, tmB, p);
+  return (int)cudaGetLastError();
 }
 
 }  // namespace fl8
@@ -544,20 +607,12 @@ extern "C" int fl_fp8_grouped_gemm(const FlFp8GemmDesc* d, cudaStream_t stream) 
   rc = d->b_mn_major ? make_map(&tmB, d->B, d->N, d->K, d->num_groups, 128, 128)
                      : make_map(&tmB, d->B, d->K, d->N, d->num_groups, 128, BN);
   if (rc) return rc;
-  static int sms_of[64];                       // per device: the shared-memory attribute belongs to the device's copy of the kernel
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev < 0 || dev >= 64) return bad("device ordinal out of range");
-  int& num_sms = sms_of[dev];
-  if (!num_sms) {
-    cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaError_t e = cudaFuncSetAttribute(fp8_grouped_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
-    if (e != cudaSuccess) { num_sms = 0; return (int)e; }
+  switch (d->epilogue) {
+    case FL_EPI_STORE: return launch<FL_EPI_STORE>(tmA, tmB, p, d->max_ctas, stream);
+    case FL_EPI_SWIGLU: return launch<FL_EPI_SWIGLU>(tmA, tmB, p, d->max_ctas, stream);
+    case FL_EPI_SCATTER: return launch<FL_EPI_SCATTER>(tmA, tmB, p, d->max_ctas, stream);
+    default: return launch<FL_EPI_DSWIGLU>(tmA, tmB, p, d->max_ctas, stream);
   }
-  int grid = num_sms;
-  if (d->max_ctas > 0 && d->max_ctas < grid) grid = d->max_ctas;
-  fp8_grouped_gemm_kernel<<<grid, NUM_THREADS, SMEM_BYTES, stream>>>(tmA, tmB, p);
-  return (int)cudaGetLastError();
 }
 
 extern "C" int fl_fp8_quantize_rows(const void* x, void* q, float* scale, long long rows, int K, const int* counts, int cap,

@@ -67,6 +67,32 @@ def test_fp8_rows_store(K, b_mn):
         assert (out[g * cap + end:(g + 1) * cap] == 7.0).all()
 
 
+@pytest.mark.parametrize("b_mn", [False, True])
+@pytest.mark.parametrize("blocks", [7, 8, 9, 16, 17])
+def test_fp8_scales_through_their_ring(blocks, b_mn):
+    """The scales travel eight blocks of contraction at a time, in two stages: one block less, as many, one more, over several tiles
+    per CTA (two CTAs), rows that end inside a tile and an expert without rows.  Scales differ by powers of two from block to block, so that
+    one taken from the wrong block or row shows."""
+    from fuselink_b200.ops import fp8
+    G, cap, N, K = 3, 384, 768, 128 * blocks
+    counts_l = [383, 0, 130]
+    counts = torch.tensor(counts_l, dtype=torch.int32, device="cuda")
+    g = torch.Generator(device="cuda").manual_seed(blocks)
+    aq = torch.randint(-8, 9, (G * cap, K), generator=g, device="cuda").float().to(fp8.FP8)
+    wq = torch.randint(-8, 9, (G, K, N) if b_mn else (G, N, K), generator=g, device="cuda").float().to(fp8.FP8)
+    asc = 2.0 ** torch.randint(-3, 4, (G * cap, blocks), generator=g, device="cuda").float()
+    wsc = 2.0 ** torch.randint(-3, 4, (G, wq.shape[1] // 128, wq.shape[2] // 128), generator=g, device="cuda").float()
+    st = torch.zeros(8, dtype=torch.int32, device="cuda")
+    out = fp8.grouped_gemm_rows_fp8(aq, asc, wq, wsc, counts, cap, b_mn_major=b_mn, max_ctas=2, status=st)
+    torch.cuda.synchronize()
+    assert st[0].item() == 0, st.tolist()
+    ad, wd = fp8.dequantize_rows(aq, asc).double(), fp8.dequantize_blocks(wq, wsc).double()
+    for i, c in enumerate(counts_l):
+        ref = ad[i * cap:i * cap + c] @ (wd[i] if b_mn else wd[i].t())
+        # products of small integers and powers of two: sums exact in fp32, the results rounded to bf16 once (2^-9)
+        assert ((out[i * cap:i * cap + c].double() - ref).abs() <= ref.abs() * 2.0 ** -8).all()
+
+
 def test_fp8_swiglu_scatter_and_dswiglu():
     import torch.nn.functional as F
     from fuselink_b200.ops import fp8, gemm
