@@ -11,130 +11,213 @@
 
 namespace fl {
 
-constexpr int BULK_SLOTS = 4;
+// Bound by memory (or the link): every byte is read once and written once, and small launches by their start and end.  One thread per
+// CTA streams through a ring of 16 KiB slots in shared memory with the bulk-copy engine.  A launch is split evenly, in slots, over two
+// CTAs per SM, which drain their ring once per segment; dealt out in chunks, each drained before the next was asked for, 320 chunks
+// left some SMs with three and some with two.  The next kernel may be placed when every CTA is done copying.  8 exchanges of 8 x 2.6 MB
+// in a row 125 -> 102 us, 4 of 4 x 8.4 MB 78 -> 64, 2 of 2 x 67 MB 107 -> 100; a put of 16 MiB 10.4 -> 8.6, 64 MiB 24.6 -> 23.3, 256 MiB 100 -> 94.
+// One CTA per SM with 12 slots: 129, 64, 101, 7.9, 23.2, 94; three with 4: 113, 69, 101, 9.3, 23.0, 94.
 constexpr int BULK_SLOT_BYTES = 16 * 1024;
+constexpr int BULK_MAX_SLOTS = 6;
 
-__device__ __forceinline__ void copy_vec(const uint8_t* __restrict__ src, uint8_t* __restrict__ dst,
-                                         unsigned long long bytes) {
-  const int tid = threadIdx.x, nt = blockDim.x;
-  if (((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 15) == 0) {
-    const unsigned long long n16 = bytes >> 4;
-    const uint4* s = reinterpret_cast<const uint4*>(src);
-    uint4* d = reinterpret_cast<uint4*>(dst);
-    unsigned long long i = tid;
-    // 4 independent 16-byte loads in flight per thread before the first store
-    for (; i + 3ull * nt < n16; i += 4ull * nt) {
-      uint4 a = ld_nc_v4(s + i), b = ld_nc_v4(s + i + nt), c = ld_nc_v4(s + i + 2 * nt), e = ld_nc_v4(s + i + 3 * nt);
-      st_v4(d + i, a); st_v4(d + i + nt, b); st_v4(d + i + 2 * nt, c); st_v4(d + i + 3 * nt, e);
-    }
-    for (; i < n16; i += nt) st_v4(d + i, ld_nc_v4(s + i));
-    for (unsigned long long b = (n16 << 4) + tid; b < bytes; b += nt) dst[b] = src[b];
-  } else {
-    for (unsigned long long b = tid; b < bytes; b += nt) dst[b] = src[b];
-  }
+__device__ __forceinline__ void copy_bytes(const uint8_t* src, uint8_t* dst, unsigned long long bytes) {
+  for (unsigned long long b = threadIdx.x; b < bytes; b += blockDim.x) dst[b] = src[b];
 }
 
-// One thread streams the chunk through a ring of shared-memory slots with the bulk-copy engine:
+// src and dst at the same distance from a multiple of 16, by all threads of the CTA
+__device__ __forceinline__ void copy_vec(const uint8_t* __restrict__ src, uint8_t* __restrict__ dst, unsigned long long bytes) {
+  const unsigned long long to16 = (16 - (reinterpret_cast<uintptr_t>(dst) & 15)) & 15, head = to16 < bytes ? to16 : bytes;
+  copy_bytes(src, dst, head);
+  const int tid = threadIdx.x, nt = blockDim.x;
+  const unsigned long long n16 = (bytes - head) >> 4;
+  const uint4* s = reinterpret_cast<const uint4*>(src + head);
+  uint4* d = reinterpret_cast<uint4*>(dst + head);
+  unsigned long long i = tid;
+  // 4 independent 16-byte loads in flight per thread before the first store
+  for (; i + 3ull * nt < n16; i += 4ull * nt) {
+    uint4 a = ld_nc_v4(s + i), b = ld_nc_v4(s + i + nt), c = ld_nc_v4(s + i + 2 * nt), e = ld_nc_v4(s + i + 3 * nt);
+    st_v4(d + i, a); st_v4(d + i + nt, b); st_v4(d + i + 2 * nt, c); st_v4(d + i + 3 * nt, e);
+  }
+  for (; i < n16; i += nt) st_v4(d + i, ld_nc_v4(s + i));
+  copy_bytes(src + head + (n16 << 4), dst + head + (n16 << 4), bytes - head - (n16 << 4));
+}
+
+// 16 bytes from `sh` bytes (1 to 15) into the 32 that a and b hold
+__device__ __forceinline__ uint4 shifted(const uint4& a, const uint4& b, unsigned sh) {
+  const bool two = sh & 8, one = sh & 4;
+  const unsigned bits = (sh & 3) * 8;
+  uint32_t w[6] = {two ? a.z : a.x, two ? a.w : a.y, two ? b.x : a.z, two ? b.y : a.w, two ? b.z : b.x, two ? b.w : b.y};
+#pragma unroll
+  for (int i = 0; i < 5; ++i) w[i] = one ? w[i + 1] : w[i];
+  return make_uint4(__funnelshift_r(w[0], w[1], bits), __funnelshift_r(w[1], w[2], bits), __funnelshift_r(w[2], w[3], bits),
+                    __funnelshift_r(w[3], w[4], bits));
+}
+
+// src and dst at different distances from a multiple of 16, by all threads of the CTA: whole vectors of dst from two neighbouring
+// vectors of src each (the second of them is in L1).  Only vectors that lie inside [src, src + bytes) are read; the ends go byte by
+// byte.  Byte by byte throughout, an exchange of blocks of an odd number of elements took 33 times as long as one of a multiple of eight
+// (8 ranks, 8 x 2.6 MB each: 4358 us against 125; now 138).
+__device__ __forceinline__ void copy_shifted(const uint8_t* src, uint8_t* dst, unsigned long long bytes) {
+  constexpr int U = 4;
+  const unsigned long long to16 = (16 - (reinterpret_cast<uintptr_t>(dst) & 15)) & 15;
+  const unsigned long long head = to16 + 16;                                    // then src + head - sh is not before src
+  const unsigned sh = (unsigned)(reinterpret_cast<uintptr_t>(src + head) & 15);
+  const long long body = (long long)bytes - (long long)head - 16 + (long long)sh;   // bytes of src up to the last vector that may be a second one
+  if (body < 16) { copy_bytes(src, dst, bytes); return; }
+  const unsigned long long n = (unsigned long long)body >> 4;
+  const uint8_t* s = src + head - sh;
+  uint8_t* d = dst + head;
+  const unsigned tid = threadIdx.x, nt = blockDim.x;
+  unsigned long long i = tid;
+  for (; i + (U - 1ull) * nt < n; i += (unsigned long long)U * nt) {
+    uint4 a[U], b[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      a[u] = ld_v4(s + 16 * (i + (unsigned long long)u * nt));
+      b[u] = ld_v4(s + 16 * (i + (unsigned long long)u * nt) + 16);
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) st_v4(d + 16 * (i + (unsigned long long)u * nt), shifted(a[u], b[u], sh));
+  }
+  for (; i < n; i += nt) st_v4(d + 16 * i, shifted(ld_v4(s + 16 * i), ld_v4(s + 16 * i + 16), sh));
+  copy_bytes(src, dst, head);
+  copy_bytes(src + head + 16 * n, dst + head + 16 * n, bytes - head - 16 * n);
+}
+
+// One thread streams `bytes` (a multiple of 16, as src and dst are) through the ring of shared-memory slots with the bulk-copy engine:
 // global -> smem (mbarrier completion) then smem -> global (bulk group).  No multicast anywhere.
-__device__ __forceinline__ bool copy_bulk(const uint8_t* src, uint8_t* dst, unsigned long long bytes,
-                                          uint8_t* ring, uint64_t* bars, uint32_t& phase_bits, int* abort_flag,
-                                          int* status) {
+__device__ __forceinline__ bool copy_bulk(const uint8_t* src, uint8_t* dst, unsigned long long bytes, uint8_t* ring, int slots, uint64_t* bars,
+                                          uint32_t& phase_bits, int* abort_flag, int* status) {
   const int n = (int)((bytes + BULK_SLOT_BYTES - 1) / BULK_SLOT_BYTES);
   auto slot_bytes = [&](int j) {
     unsigned long long off = (unsigned long long)j * BULK_SLOT_BYTES;
     unsigned long long left = bytes - off;
     return (uint32_t)(left < BULK_SLOT_BYTES ? left : BULK_SLOT_BYTES);
   };
-  auto issue_load = [&](int j) {
-    const int s = j % BULK_SLOTS;
+  auto issue_load = [&](int j, int s) {
     mbar_arrive_expect_tx(&bars[s], slot_bytes(j));
     bulk_load(ring + s * BULK_SLOT_BYTES, src + (unsigned long long)j * BULK_SLOT_BYTES, slot_bytes(j), &bars[s]);
   };
-  for (int j = 0; j < n && j < BULK_SLOTS - 1; ++j) issue_load(j);
+  for (int j = 0; j < n && j < slots - 1; ++j) issue_load(j, j);
   bool ok = true;
+  int s = 0;
   for (int j = 0; j < n; ++j) {
-    const int s = j % BULK_SLOTS;
     ok = mbar_wait(&bars[s], (phase_bits >> s) & 1, abort_flag, status, kTimeoutMbarFull, 500 + s);
     if (!ok) break;
     phase_bits ^= 1u << s;
     fence_proxy_async_smem();
     bulk_store(dst + (unsigned long long)j * BULK_SLOT_BYTES, ring + s * BULK_SLOT_BYTES, slot_bytes(j));
     tma_store_commit();
-    const int nj = j + BULK_SLOTS - 1;  // reuses the slot read by store j-1
+    const int nj = j + slots - 1, ns = s == 0 ? slots - 1 : s - 1;  // reuses the slot read by store j-1
     if (nj < n) {
       tma_store_wait_read<1>();
-      issue_load(nj);
+      issue_load(nj, ns);
     }
+    s = s + 1 == slots ? 0 : s + 1;
   }
-  tma_store_wait<0>();  // all writes of this chunk performed before the flag is published
-  if (!ok) {
-    for (int i = 0; i < 1000; ++i) __nanosleep(1000);  // let a stray in-flight load land
-  }
+  tma_store_wait<0>();  // all writes of this piece performed before the flag is published
+  if (!ok) let_copies_land();
   return ok;
 }
 
-__global__ void __launch_bounds__(1024) put_chunks_kernel(const FlPutArgs a) {
+// The CTA to which unit u of U falls when CTA b of G has the units [U b / G, U (b + 1) / G)
+__host__ __device__ __forceinline__ unsigned put_owner(unsigned long long u, unsigned long long U, unsigned G) {
+  return (unsigned)(((u + 1) * G - 1) / U);
+}
+
+__global__ void __launch_bounds__(1024) put_chunks_kernel(const __grid_constant__ FlPutArgs a, const int slots, const unsigned long long even_units) {
   extern __shared__ __align__(128) uint8_t dyn_smem[];
-  __shared__ uint64_t bars[BULK_SLOTS];
+  __shared__ uint64_t bars[BULK_MAX_SLOTS];
   __shared__ int abort_flag;
   __shared__ int wait_ok;
   uint32_t phase_bits = 0;
   if (threadIdx.x == 0) {
     abort_flag = 0;
     if (a.use_bulk) {
-      for (int s = 0; s < BULK_SLOTS; ++s) mbar_init(&bars[s], 1);
+      for (int s = 0; s < slots; ++s) mbar_init(&bars[s], 1);
       mbar_fence_init();
     }
   }
   __syncthreads();
-  grid_dep_launch();
+  grid_dep_wait();
 
-  unsigned long long chunks_before = 0;
+  // by all threads; false if the copy was given up
+  auto copy = [&](const uint8_t* s, uint8_t* d, unsigned long long len) -> bool {
+    if ((reinterpret_cast<uintptr_t>(s) ^ reinterpret_cast<uintptr_t>(d)) & 15) {
+      copy_shifted(s, d, len);
+    } else if (!a.use_bulk) {
+      copy_vec(s, d, len);
+    } else {
+      const unsigned long long to16 = (16 - (reinterpret_cast<uintptr_t>(d) & 15)) & 15, head = to16 < len ? to16 : len, body = (len - head) & ~15ull;
+      if (threadIdx.x == 0 && body != 0) {
+        if (!copy_bulk(s + head, d + head, body, dyn_smem, slots, bars, phase_bits, &abort_flag, a.status)) abort_flag = 1;
+        fence_proxy_async_all();
+      }
+      copy_bytes(s, d, head);
+      copy_bytes(s + head + body, d + head + body, len - head - body);
+    }
+    __syncthreads();
+    return abort_flag == 0;
+  };
+  // The flag update is itself a release at system scope: it orders this thread's bulk stores (complete, see
+  // copy_bulk) and, through the barrier above, the other threads' stores before the flag becomes visible.
+  unsigned long long chunks_before = 0, units_before = 0;
   bool live = true;
   for (int si = 0; si < a.nseg && live; ++si) {
     const FlSeg& sg = a.seg[si];
     const unsigned long long nch = (sg.bytes + a.chunk_bytes - 1) / a.chunk_bytes;
     unsigned long long done_here = 0;      // thread 0: bytes of this segment this CTA has finished
-    // CTAs take chunks round-robin over the concatenation of all segments
-    unsigned long long first = (blockIdx.x + gridDim.x - (chunks_before % gridDim.x)) % gridDim.x;
-    for (unsigned long long c = first; c < nch && live; c += gridDim.x) {
-      const unsigned long long off = c * a.chunk_bytes;
-      const unsigned long long len = (sg.bytes - off) < a.chunk_bytes ? (sg.bytes - off) : a.chunk_bytes;
-      if (sg.wait_flags) {
-        if (threadIdx.x == 0) wait_ok = wait_flag_ge(sg.wait_flags + c, a.seq, a.status, 600 + si) ? 1 : 0;
-        __syncthreads();
-        const int okv = wait_ok;
-        __syncthreads();
-        if (!okv) { live = false; break; }
-      }
-      const uint8_t* s = reinterpret_cast<const uint8_t*>(sg.src) + off;
-      uint8_t* d = reinterpret_cast<uint8_t*>(sg.dst) + off;
-      const bool bulk_ok = a.use_bulk && ((reinterpret_cast<uintptr_t>(s) | reinterpret_cast<uintptr_t>(d) | len) & 15) == 0;
-      if (bulk_ok) {
-        if (threadIdx.x == 0) {
-          if (!copy_bulk(s, d, len, dyn_smem, bars, phase_bits, &abort_flag, a.status)) abort_flag = 1;
-          fence_proxy_async_all();
+    if (even_units != 0) {
+      // Evenly: a contiguous piece per CTA, whatever the chunks.  The CTAs that have a part of a segment, at most as many as it has
+      // chunks, add one each to its arrival counter when they are done, the first of them the rest.
+      const unsigned long long U = even_units, n = (sg.bytes + BULK_SLOT_BYTES - 1) / BULK_SLOT_BYTES, u0 = units_before, u1 = u0 + n;
+      const unsigned long long mine0 = U * blockIdx.x / gridDim.x, mine1 = U * (blockIdx.x + 1) / gridDim.x;
+      const unsigned long long from = mine0 > u0 ? mine0 : u0, to = mine1 < u1 ? mine1 : u1;
+      units_before = u1;
+      if (from < to) {
+        const unsigned long long off = (from - u0) * BULK_SLOT_BYTES, end = (to - u0) * BULK_SLOT_BYTES, len = (end < sg.bytes ? end : sg.bytes) - off;
+        live = copy(reinterpret_cast<const uint8_t*>(sg.src) + off, reinterpret_cast<uint8_t*>(sg.dst) + off, len);
+        if (live && threadIdx.x == 0) {
+          if (sg.flag_mode == FL_FLAG_COUNT) {
+            const unsigned first = put_owner(u0, U, gridDim.x), last = put_owner(u1 - 1, U, gridDim.x);
+            red_release_sys_add(sg.flags, blockIdx.x == first ? (unsigned)(nch - (last - first)) : 1u);
+          }
+          if (sg.bytes_done != nullptr) {
+            if (a.done_scratch != nullptr) done_here += len;
+            else atomicAdd_system(sg.bytes_done, len);
+          }
         }
-      } else {
-        copy_vec(s, d, len);
       }
-      __syncthreads();
-      if (abort_flag) { live = false; break; }
-      // The flag update is itself a release at system scope: it orders this thread's bulk stores (complete, see
-      // copy_bulk) and, through the barrier above, the other threads' stores before the flag becomes visible.
-      if (threadIdx.x == 0 && sg.flag_mode != FL_FLAG_NONE) {
-        if (sg.flag_mode == FL_FLAG_SEQ_PER_CHUNK) st_release_sys(sg.flags + c, a.seq);
-        else red_release_sys_add(sg.flags, 1u);
-      }
-      // device-side completion counter: the host monitor folds it into the path's completed bytes
-      if (threadIdx.x == 0 && sg.bytes_done != nullptr) {
-        if (a.done_scratch != nullptr) done_here += len;
-        else atomicAdd_system(sg.bytes_done, (unsigned long long)len);
+    } else {
+      // CTAs take chunks round-robin over the concatenation of all segments
+      unsigned long long first = (blockIdx.x + gridDim.x - (chunks_before % gridDim.x)) % gridDim.x;
+      for (unsigned long long c = first; c < nch && live; c += gridDim.x) {
+        const unsigned long long off = c * a.chunk_bytes;
+        const unsigned long long len = (sg.bytes - off) < a.chunk_bytes ? (sg.bytes - off) : a.chunk_bytes;
+        if (sg.wait_flags) {
+          if (threadIdx.x == 0) wait_ok = wait_flag_ge(sg.wait_flags + c, a.seq, a.status, 600 + si) ? 1 : 0;
+          __syncthreads();
+          const int okv = wait_ok;
+          __syncthreads();
+          if (!okv) { live = false; break; }
+        }
+        live = copy(reinterpret_cast<const uint8_t*>(sg.src) + off, reinterpret_cast<uint8_t*>(sg.dst) + off, len);
+        if (!live) break;
+        if (threadIdx.x == 0 && sg.flag_mode != FL_FLAG_NONE) {
+          if (sg.flag_mode == FL_FLAG_SEQ_PER_CHUNK) st_release_sys(sg.flags + c, a.seq);
+          else red_release_sys_add(sg.flags, 1u);
+        }
+        // device-side completion counter: the host monitor folds it into the path's completed bytes
+        if (threadIdx.x == 0 && sg.bytes_done != nullptr) {
+          if (a.done_scratch != nullptr) done_here += len;
+          else atomicAdd_system(sg.bytes_done, (unsigned long long)len);
+        }
       }
     }
     if (threadIdx.x == 0 && done_here != 0) atomicAdd(a.done_scratch + si, done_here);
     chunks_before += nch;
   }
+  grid_dep_launch();
   if (a.done_scratch != nullptr && threadIdx.x == 0) {
     // every CTA takes a ticket, also one that gave up a wait; the last one forwards the totals and rearms the words
     __threadfence();
@@ -175,10 +258,9 @@ __global__ void barrier_kernel(FlSignalPtrs pads, int slot0, int rank, int world
 
 }  // namespace fl
 
-// Waits and barriers are a warp each, often several in a row.  They are launched so that they may be placed while the kernel before
+// Puts, waits and barriers, often several in a row, are launched so that they may be placed while the kernel before
 // them drains; they touch nothing, and poll no flag, before that kernel has ended (grid_dep_wait), so what one polls for is never behind
-// it.  Eight exchanges of 21 MB and their waits, one after the other: 138 -> 126 us; a put of 64 KiB and its wait: 10.2 -> 9.6 us.  The
-// puts themselves, launched like that as well, take longer (176 us): their early CTAs hold shared memory that the running ones' peers want.
+// it.  The waits and barriers alone: eight exchanges of 21 MB 138 -> 126 us; a put of 64 KiB and its wait: 10.2 -> 9.6 us.
 template <typename... P, typename... A>
 static int launch_after(void (*kernel)(P...), unsigned grid, unsigned threads, size_t smem, cudaStream_t stream, const A&... args) {
   cudaLaunchConfig_t cfg = {};
@@ -194,25 +276,66 @@ static int launch_after(void (*kernel)(P...), unsigned grid, unsigned threads, s
   return (int)cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
 
+constexpr unsigned PUT_CTAS = 2 * 148;
+
+// Whether the launch may be split evenly in slots over its G CTAs (see the kernel): nothing is waited for or flagged chunk by chunk, and no
+// segment is shared by more CTAs than it has chunks to count.
+static unsigned long long even_split(const FlPutArgs* a, unsigned G) {
+  unsigned long long U = 0;
+  for (int i = 0; i < a->nseg; ++i) {
+    if (a->seg[i].wait_flags != nullptr || a->seg[i].flag_mode == FL_FLAG_SEQ_PER_CHUNK) return 0;
+    U += (a->seg[i].bytes + fl::BULK_SLOT_BYTES - 1) / fl::BULK_SLOT_BYTES;
+  }
+  if (U < G) return 0;
+  unsigned long long u0 = 0;
+  for (int i = 0; i < a->nseg; ++i) {
+    const unsigned long long n = (a->seg[i].bytes + fl::BULK_SLOT_BYTES - 1) / fl::BULK_SLOT_BYTES;
+    const unsigned long long chunks = (a->seg[i].bytes + a->chunk_bytes - 1) / a->chunk_bytes;
+    if (n != 0 && a->seg[i].flag_mode == FL_FLAG_COUNT && fl::put_owner(u0 + n - 1, U, G) - fl::put_owner(u0, U, G) + 1ull > chunks) return 0;
+    u0 += n;
+  }
+  return U;
+}
+
 extern "C" int fl_put_chunks(const FlPutArgs* args, int num_ctas, int threads, cudaStream_t stream) {
   if (args->nseg < 1 || args->nseg > FL_MAX_SEGS) return -1;
   if (args->chunk_bytes == 0 || (args->chunk_bytes & 15)) return -2;
   if (threads <= 0 || threads > 1024) threads = 512;
   if (num_ctas <= 0) num_ctas = 1;
-  size_t smem = args->use_bulk ? fl::BULK_SLOTS * fl::BULK_SLOT_BYTES : 0;
+  int slots = 0;
+  unsigned long long even = 0;
+  if (args->use_bulk) {
+    // as many slots as a CTA will fill; threads beyond the one that feeds the engine only where bytes have to be shifted
+    for (int i = 0; i < args->nseg; ++i)
+      if (((uintptr_t)args->seg[i].src ^ (uintptr_t)args->seg[i].dst) & 15) threads = 512;
+    const unsigned G = (unsigned)num_ctas < PUT_CTAS ? (unsigned)num_ctas : PUT_CTAS;
+    even = even_split(args, G);
+    unsigned long long per_cta = (args->chunk_bytes + fl::BULK_SLOT_BYTES - 1) / fl::BULK_SLOT_BYTES;
+    slots = 4;
+    if (even != 0) {
+      num_ctas = (int)G;
+      per_cta = (even + G - 1) / G;
+      slots = fl::BULK_MAX_SLOTS;
+    }
+    if (per_cta + 1 < (unsigned long long)slots) slots = (int)per_cta + 1;
+  } else {
+    even = even_split(args, (unsigned)num_ctas);
+  }
+  const size_t smem = (size_t)slots * fl::BULK_SLOT_BYTES;
   if (smem > 48 * 1024) {
     static bool set_on[64];                 // per device: a process may drive several GPUs
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64) return -3;
     if (!set_on[dev]) {
-      cudaError_t e = cudaFuncSetAttribute(fl::put_chunks_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      cudaError_t e = cudaFuncSetAttribute(fl::put_chunks_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, fl::BULK_MAX_SLOTS * fl::BULK_SLOT_BYTES);
+      // without it an SM is set up for one of these CTAs at a time (eight exchanges 148 us, with it 108)
+      if (e == cudaSuccess) e = cudaFuncSetAttribute(fl::put_chunks_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
       if (e != cudaSuccess) return (int)e;
       set_on[dev] = true;
     }
   }
-  fl::put_chunks_kernel<<<num_ctas, threads, smem, stream>>>(*args);
-  return (int)cudaGetLastError();
+  return launch_after(fl::put_chunks_kernel, (unsigned)num_ctas, (unsigned)threads, smem, stream, *args, slots, even);
 }
 
 extern "C" int fl_all_to_all(const void* send, void* const* recv_peers, unsigned long long bytes_per_peer, int rank,

@@ -45,6 +45,51 @@ def test_unaligned_put(heaps):
 
 
 @pytest.mark.parametrize("engine", ["ldst", "bulk"])
+@pytest.mark.parametrize("nbytes", [1, 47, 48, 49, 65535, 65537, 196608 + 31, (5 << 20) + 7])
+def test_put_at_any_alignment(heaps, engine, nbytes):
+    """The same distance from a multiple of 16 on both sides (ends byte by byte, the rest in vectors or through the engine) and
+    different ones (vectors put together from two), around the sizes at which either begins, slots and chunks end."""
+    from fuselink_b200.ops.comm import Channel
+    chans = [Channel(h, "al", engine=engine) for h in heaps]
+    off = heaps[0].alloc_tensor([nbytes + 64], torch.uint8).offset
+    for h in heaps[1:]:
+        h.alloc_tensor([nbytes + 64], torch.uint8)
+    g = torch.Generator(device="cuda").manual_seed(nbytes)
+    src = torch.randint(0, 255, (nbytes + 32,), dtype=torch.uint8, device="cuda", generator=g)
+    got = heaps[2].tensor(off, [nbytes + 64], torch.uint8)
+    for s, d in ((0, 0), (5, 5), (13, 13), (0, 8), (8, 0), (1, 0), (0, 1), (2, 12), (15, 3), (3, 15), (4, 6)):
+        got.fill_(255)
+        chans[0].put(src[s:s + nbytes], 2, off + 16 + d)
+        chans[2].expect(0, nbytes)
+        chans[2].wait()
+        torch.cuda.synchronize()
+        heaps[2].check_status()
+        assert torch.equal(got[16 + d:16 + d + nbytes], src[s:s + nbytes]), (s, d)
+        assert (got[:16 + d] == 255).all() and (got[16 + d + nbytes:] == 255).all(), (s, d)
+
+
+@pytest.mark.parametrize("engine", ["ldst", "bulk"])
+@pytest.mark.parametrize("n", [513, 100_003, 600_001])
+def test_all_to_all_of_odd_blocks(heaps, engine, n):
+    """Blocks that begin anywhere: of some pairs of ranks at the same distance from a multiple of 16, of others not."""
+    from fuselink_b200.ops.comm import Channel, all_to_all
+    W = 4
+    chans = [Channel(h, "odd", engine=engine) for h in heaps]
+    recv = [h.alloc_tensor([W, n], torch.bfloat16) for h in heaps]
+    for it in range(2):
+        send = [torch.randn(W, n, device="cuda").bfloat16() for _ in range(W)]
+        for r in range(W):
+            all_to_all(chans[r], send[r], recv[r], wait=False)
+        for r in range(W):
+            chans[r].wait()
+        torch.cuda.synchronize()
+        for r in range(W):
+            heaps[r].check_status()
+            for s in range(W):
+                assert torch.equal(recv[r].local[s], send[s][r]), (it, r, s)
+
+
+@pytest.mark.parametrize("engine", ["ldst", "bulk"])
 def test_all_to_all(heaps, engine):
     from fuselink_b200.ops.comm import Channel, all_to_all
     W, n = 4, 300_000
