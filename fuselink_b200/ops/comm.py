@@ -10,6 +10,7 @@ the receiver waits for its running total.  No word is ever reset.
 """
 from __future__ import annotations
 
+import functools
 from typing import Optional, Sequence, Tuple
 
 import torch
@@ -28,13 +29,17 @@ def chunking(nbytes: int, chunk_bytes: Optional[int] = None) -> Tuple[int, int]:
     Large messages use the configured chunk (512 KiB, the reference's NCCL_P2P_NET_CHUNKSIZE setting); smaller
     ones are cut so that every SM gets about one chunk, never below 64 KiB.
     """
-    cfg = chunk_bytes or _chunk_default()
+    return _cut(nbytes, chunk_bytes or _chunk_default(), _chunk_min())
+
+
+@functools.lru_cache(maxsize=1024)
+def _cut(nbytes: int, cfg: int, least: int) -> Tuple[int, int]:
     if nbytes <= 0:
         return cfg, 0
     c = cfg
     # about one chunk per SM for mid sizes; a chunk is never cut below 64 KiB (a CTA streams it through a ring of
     # 16 KiB slots, and every chunk costs one remote flag update)
-    while c > _chunk_min() and nbytes // c < _NUM_SMS:
+    while c > least and nbytes // c < _NUM_SMS:
         c //= 2
     c = max(16, (c + 15) // 16 * 16)
     return c, (nbytes + c - 1) // c
@@ -79,6 +84,10 @@ class Channel:
         self.C = require_native()
         self.slot0 = heap.signal_slots(f"chan:{name}", heap.world)
         self.expected = [0] * heap.world
+        # addresses do not change while the heap is open: this rank's words, and the word of this rank on every other
+        self._words = heap.sig_addr(self.slot0)
+        self._word_on = [heap.sig_addr(self.slot0 + heap.rank, r) for r in range(heap.world)]
+        self._status_addr = heap.status_addr
         self.engine = engine or knobs().copy_engine
         self.counters = None      # optional pinned int64[world]: bytes this rank has finished sending to each peer
 
@@ -101,12 +110,14 @@ class Channel:
         cb, n = chunking(nbytes, chunk_bytes)
         if n == 0:
             return 0
-        seg = (src.data_ptr(), self.heap.addr(dst_offset, dst_rank), nbytes,
-               self.heap.sig_addr(self.slot0 + self.heap.rank, dst_rank), FLAG_COUNT, 0)
+        seg = (src.data_ptr(), self.heap.base[dst_rank] + dst_offset, nbytes, self._word_on[dst_rank], FLAG_COUNT, 0)
         ctas, threads = _launch_shape(n, self.engine)
-        ctr = [self.counters.data_ptr() + 8 * dst_rank] if self.counters is not None else []
-        scratch = self.counter_scratch.data_ptr() if ctr and getattr(self, "counter_scratch", None) is not None else 0
-        self.C.put_chunks([seg], cb, 0, self.engine == "bulk", ctas, threads, self.heap.status_addr, ctr, scratch)
+        if self.counters is None:
+            self.C.put_chunks([seg], cb, 0, self.engine == "bulk", ctas, threads, self._status_addr)
+            return n
+        ctr = [self.counters.data_ptr() + 8 * dst_rank]
+        scratch = self.counter_scratch.data_ptr() if getattr(self, "counter_scratch", None) is not None else 0
+        self.C.put_chunks([seg], cb, 0, self.engine == "bulk", ctas, threads, self._status_addr, ctr, scratch)
         return n
 
     def put_many(self, items: Sequence[Tuple[int, int, int, int]], chunk_bytes: int) -> None:
@@ -135,9 +146,10 @@ class Channel:
     def wait(self, src_ranks: Optional[Sequence[int]] = None) -> None:
         """Enqueue a wait (on the current stream) until everything announced with expect() has arrived."""
         ranks = range(self.heap.world) if src_ranks is None else src_ranks
-        flags = [(self.heap.sig_addr(self.slot0 + r), self.expected[r] & 0xFFFFFFFF) for r in ranks if self.expected[r] > 0]
+        words, expected = self._words, self.expected
+        flags = [(words + 4 * r, expected[r] & 0xFFFFFFFF) for r in ranks if expected[r] > 0]
         for i in range(0, len(flags), 16):
-            self.C.wait_flags(flags[i:i + 16], self.heap.status_addr)
+            self.C.wait_flags(flags[i:i + 16], self._status_addr)
 
 
 def barrier(heap: SymmetricHeap, name: str = "barrier", signal: bool = True, wait: bool = True) -> None:
@@ -161,14 +173,14 @@ def all_to_all(chan: Channel, send: torch.Tensor, recv: SymTensor, wait: bool = 
     heap = chan.heap
     W = heap.world
     assert send.shape[0] == W and send.is_contiguous()
-    per = send[0].numel() * send.element_size()
+    per = send.numel() // W * send.element_size()
     cb, n = chunking(per)
     for r in range(W):
         chan.expected[r] += n
     ctas, threads = _launch_shape(n * W, chan.engine)
     want = [e & 0xFFFFFFFF for e in chan.expected] if wait else []
     chan.C.all_to_all(send.data_ptr(), recv.peers(), per, heap.rank, heap.pads(), chan.slot0, cb, want,
-                      chan.engine == "bulk", ctas, threads, heap.status_addr)
+                      chan.engine == "bulk", ctas, threads, chan._status_addr)
 
 
 def all_to_all_v(chan: Channel, send: torch.Tensor, send_offsets: Sequence[int], send_bytes: Sequence[int],
