@@ -25,7 +25,7 @@ __device__ __forceinline__ void copy_bytes(const uint8_t* src, uint8_t* dst, uns
 }
 
 // src and dst at the same distance from a multiple of 16, by all threads of the CTA
-__device__ __forceinline__ void copy_vec(const uint8_t* __restrict__ src, uint8_t* __restrict__ dst, unsigned long long bytes) {
+__device__ __forceinline__ void copy_vec(const uint8_t* src, uint8_t* dst, unsigned long long bytes) {
   const unsigned long long to16 = (16 - (reinterpret_cast<uintptr_t>(dst) & 15)) & 15, head = to16 < bytes ? to16 : bytes;
   copy_bytes(src, dst, head);
   const int tid = threadIdx.x, nt = blockDim.x;
@@ -35,10 +35,10 @@ __device__ __forceinline__ void copy_vec(const uint8_t* __restrict__ src, uint8_
   unsigned long long i = tid;
   // 4 independent 16-byte loads in flight per thread before the first store
   for (; i + 3ull * nt < n16; i += 4ull * nt) {
-    uint4 a = ld_nc_v4(s + i), b = ld_nc_v4(s + i + nt), c = ld_nc_v4(s + i + 2 * nt), e = ld_nc_v4(s + i + 3 * nt);
+    uint4 a = ld_stream_v4(s + i), b = ld_stream_v4(s + i + nt), c = ld_stream_v4(s + i + 2 * nt), e = ld_stream_v4(s + i + 3 * nt);
     st_v4(d + i, a); st_v4(d + i + nt, b); st_v4(d + i + 2 * nt, c); st_v4(d + i + 3 * nt, e);
   }
-  for (; i < n16; i += nt) st_v4(d + i, ld_nc_v4(s + i));
+  for (; i < n16; i += nt) st_v4(d + i, ld_stream_v4(s + i));
   copy_bytes(src + head + (n16 << 4), dst + head + (n16 << 4), bytes - head - (n16 << 4));
 }
 
