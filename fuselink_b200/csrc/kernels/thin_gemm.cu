@@ -8,7 +8,7 @@
 // out evenly over all CTAs, with shared tiles summed through global memory, were tried: the last CTA's trip for the others' sums costs
 // 8 us, more than the uneven grids, 6144 x 4096 and 16 rows: 21 us against 13.)
 //
-// A step is a chain of about ten short kernels per layer.  Launched one after the other, each fills its pipeline from an idle
+// A step is a chain of seven or eight short kernels per layer.  Launched one after the other, each fills its pipeline from an idle
 // memory and drains it into one.  With `early` a kernel starts as soon as the one before it has started and the SMs have room, and
 // requests its first blocks of w, which do not depend on that kernel; it waits (griddepcontrol.wait) before it reads x.
 //
@@ -25,6 +25,7 @@
 // 526 at 17, 603 | 647 at 28).
 #include "thin_gemm.cuh"
 #include "decoder.cuh"
+#include "kv_pack.cuh"
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include "../common/fl_ptx.cuh"
@@ -46,10 +47,22 @@ constexpr int TG_THREADS = 128;
 template <typename T> struct ThinNum;
 template <> struct ThinNum<__nv_bfloat16> {
   static constexpr uint32_t kFmt = 1;
+  using two = __nv_bfloat162;
+  static __device__ __forceinline__ float2 f2(uint32_t w) { return __bfloat1622float2(*reinterpret_cast<two*>(&w)); }
+  static __device__ __forceinline__ uint32_t pack(float a, float b) {
+    two h = __floats2bfloat162_rn(a, b);
+    return *reinterpret_cast<uint32_t*>(&h);
+  }
   static __device__ __forceinline__ float round(float a) { return __bfloat162float(__float2bfloat16_rn(a)); }
 };
 template <> struct ThinNum<__half> {
   static constexpr uint32_t kFmt = 0;
+  using two = __half2;
+  static __device__ __forceinline__ float2 f2(uint32_t w) { return __half22float2(*reinterpret_cast<two*>(&w)); }
+  static __device__ __forceinline__ uint32_t pack(float a, float b) {
+    two h = __floats2half2_rn(a, b);
+    return *reinterpret_cast<uint32_t*>(&h);
+  }
   static __device__ __forceinline__ float round(float a) { return __half2float(__float2half_rn(a)); }
 };
 
@@ -59,10 +72,16 @@ __device__ __forceinline__ void st_cluster_float(uint32_t addr, float v) {
 __device__ __forceinline__ void cluster_arrive_all() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait_all() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 
-template <typename T>
-__global__ void __launch_bounds__(TG_THREADS, 2)
+// OUT: what becomes of the sums, FL_THIN_QKV by itself, the others (FL_THIN_STORE here) by `epilogue`.  For FL_THIN_QKV a fifth warp looks
+// up where the keys and values go while the products run.  As a kernel of its own between product and attention the pass was one more link
+// of the chain: 1.2 us per layer of a 1.3B model at 3 requests (16 steps 17.35 ms, now 16.89), nothing that shows beside the bytes of an 8B
+// model at 16.  (The norms in the products on both sides of them were tried as well: normalised on its way in, x comes 2.8 us later, and
+// the norm's own kernel costs 1 to 2.)
+template <typename T, int OUT>
+__global__ void __launch_bounds__(OUT == FL_THIN_QKV ? TG_THREADS + 32 : TG_THREADS, 2)
 thin_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_x, const T* bias, T* y, const int rows,
-                 const long long n, const int k, const int splits, const int epilogue, const int early, int* status) {
+                 const long long n, const int k, const int splits, const int epilogue, const int early, int* status,
+                 const __grid_constant__ FlThinQkv qk) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ uint64_t full[TG_STAGES], empty[TG_STAGES], done;
   __shared__ uint32_t tmem_base_s;
@@ -71,10 +90,11 @@ thin_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int split = blockIdx.x % splits;                        // = rank in the cluster
   const long long tile = blockIdx.x / splits;
-  const bool gated = epilogue == FL_THIN_SILU_GATED;
+  const bool gated = OUT == FL_THIN_STORE && epilogue == FL_THIN_SILU_GATED;
   const long long n0 = tile * (gated ? TG_M / 2 : TG_M);        // first output column
   const int blocks = (k + TG_K - 1) / TG_K;
   const int first = (int)((long long)split * blocks / splits), last = (int)((long long)(split + 1) * blocks / splits);
+  using R = ThinNum<T>;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < TG_STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
@@ -93,8 +113,12 @@ thin_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
   tc_fence_after_sync();
   if (splits > 1) cluster_arrive_all();                         // waited for before the first store into another CTA
   grid_dep_launch();
-  if (bias != nullptr && n0 + threadIdx.x < n) prefetch_l2(bias + n0 + threadIdx.x);
+  if (bias != nullptr && threadIdx.x < TG_THREADS && n0 + threadIdx.x < n) prefetch_l2(bias + n0 + threadIdx.x);
   const uint32_t tmem_base = tmem_base_s;
+
+  // FL_THIN_QKV: of this CTA's rows, the row of the page (before layer and head; -1: none) and the angles (0: not turned)
+  __shared__ int qk_page[OUT == FL_THIN_QKV ? TG_N : 1], qk_slot[OUT == FL_THIN_QKV ? TG_N : 1], qk_turn[OUT == FL_THIN_QKV ? TG_N : 1];
+  __shared__ float qk_angle[OUT == FL_THIN_QKV ? TG_N * TG_M : 1];
 
   if (warp == 0 && lane == 0) {
     // ---- loads: w of the first stages before the wait for the kernel that makes x, where w may be read that early
@@ -141,6 +165,42 @@ thin_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
       umma_commit(&empty[s]);
     }
     if (ok) umma_commit(&done);
+  } else if (OUT == FL_THIN_QKV && warp == 4) {
+    // ---- this CTA's rows: page and slot of the position, and its angles
+    grid_dep_wait();
+    const int own_rows = (rows - split + splits - 1) / splits;
+    int turn = -1;
+    if (lane < own_rows) {
+      const int r = split + lane * splits;
+      const long long at = __ldcg(qk.pos + r);
+      const int at32 = (int)at;                                 // a position beyond 32 bits is in no table
+      int page = at32 / qk.kv.block_size, slot = at32 - page * qk.kv.block_size, blk = -1;
+      if (slot < 0) { slot += qk.kv.block_size; page -= 1; }
+      if (page < 0) page += qk.kv.table_stride;                 // negative positions and page ids count from the end, as indexing does
+      int what = 0;
+      if (at32 != at || page < 0 || page >= qk.kv.table_stride) {
+        what = FL_DEC_BAD_POSITION;
+      } else {
+        blk = __ldcg(qk.kv.block_table + (long long)r * qk.kv.table_stride + page);
+        if (blk < 0) blk += qk.kv.num_blocks;
+        if (blk < 0 || blk >= qk.kv.num_blocks) { what = FL_DEC_BAD_PAGE; blk = -1; }
+      }
+      if (what != 0 && qk.kv.status != nullptr) *reinterpret_cast<volatile int*>(qk.kv.status) = what;
+      const long long t = at < 0 ? -at : at;
+      turn = qk.rope != nullptr && t < qk.rope_rows ? (int)t : -1;
+      qk_page[lane] = blk;
+      qk_slot[lane] = slot;
+      qk_turn[lane] = turn < 0 ? 0 : at < 0 ? -1 : 1;
+    }
+    if (qk.rope != nullptr) {
+#pragma unroll 4
+      for (int j = 0; j < own_rows; ++j) {
+        const int t = __shfl_sync(0xffffffffu, turn, j);
+        if (t >= 0)
+          for (int c = lane * 4; c < qk.dim; c += 128)
+            *reinterpret_cast<float4*>(qk_angle + j * TG_M + c) = __ldcg(reinterpret_cast<const float4*>(qk.rope + (long long)t * qk.dim + c));
+      }
+    }
   }
   __syncwarp();
   grid_dep_wait();                                              // y may still be read by kernels before this one
@@ -152,7 +212,7 @@ thin_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
   float* part = reinterpret_cast<float*>(smem + TG_STAGES * TG_STAGE_BYTES);
   const int own = (rows + splits - 1) / splits;                 // rows per CTA; rows <= TG_N and splits divides TG_N: own * splits <= TG_N
   if (splits > 1) cluster_wait_all();
-  if (have) {
+  if (have && (OUT != FL_THIN_QKV || warp < 4)) {
     uint32_t v[32];                                             // the second half: columns that the products do not write
     tmem_ld_32x32(tmem_base + ((uint32_t)(warp * 32) << 16), v);
     tmem_ld_wait();
@@ -195,8 +255,48 @@ thin_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
       if (col + 1 < n) p[1] = T(b);
     }
   };
-  using R = ThinNum<T>;
-  if (gated) {
+  const int c2 = 2 * (threadIdx.x & 63);
+  const long long col = n0 + c2;
+  if (OUT == FL_THIN_QKV) {
+    // Whole heads: dim divides the tile.  Bias, rotation of q and k by the position's angles, q to y, k and v to their pages.
+    const int dim = qk.dim, half = dim / 2, in = c2 % dim;      // even, as half is: a thread's two columns turn alike
+    const long long head = col / dim;
+    const bool is_q = head < qk.heads, is_v = head >= qk.heads + qk.kv.heads, low = in < half;
+    const int other = low ? c2 + half : c2 - half;
+    if (threadIdx.x < TG_THREADS && col < n) {
+      const long long oc = n0 + other;
+      float ba[2] = {0.f, 0.f}, bo[2] = {0.f, 0.f};
+      if (bias != nullptr) { ba[0] = (float)bias[col]; ba[1] = (float)bias[col + 1]; bo[0] = (float)bias[oc]; bo[1] = (float)bias[oc + 1]; }
+      for (int r = split + splits * (threadIdx.x >> 6); r < rows; r += 2 * splits) {
+        const int j = r / splits, turn = is_v ? 0 : qk_turn[j];
+        const float2 t = sums(r, c2);
+        float a[2] = {R::round(t.x), R::round(t.y)};
+        if (bias != nullptr) { a[0] = R::round(a[0] + ba[0]); a[1] = R::round(a[1] + ba[1]); }
+        if (turn != 0) {
+          const float2 u = sums(r, other);
+          float o[2] = {R::round(u.x), R::round(u.y)};
+          if (bias != nullptr) { o[0] = R::round(o[0] + bo[0]); o[1] = R::round(o[1] + bo[1]); }
+          const float* cs = qk_angle + j * TG_M + (low ? in : in - half);      // half cosines, half sines
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            // the products of the second half's value are rounded by themselves, as dec_qkv_kernel's are
+            const float co = cs[e], si = turn < 0 ? -cs[half + e] : cs[half + e];
+            a[e] = low ? fmaf(a[e], co, -__fmul_rn(o[e], si)) : fmaf(o[e], si, __fmul_rn(a[e], co));
+          }
+        }
+        const uint32_t two = R::pack(a[0], a[1]);
+        if (is_q) {
+          *reinterpret_cast<uint32_t*>(y + (long long)r * n + col) = two;
+        } else if (qk_page[j] >= 0) {
+          const long long blk = qk_page[j], slot = qk_slot[j];
+          const int kh = (int)(head - qk.heads - (is_v ? qk.kv.heads : 0));
+          const long long at = qk.kv.layout == FL_KV_BLHSD ? ((blk * qk.kv.layers + qk.kv.layer) * qk.kv.heads + kh) * qk.kv.block_size + slot
+                                                           : (((long long)qk.kv.layer * qk.kv.num_blocks + blk) * qk.kv.block_size + slot) * qk.kv.heads + kh;
+          *reinterpret_cast<uint32_t*>(reinterpret_cast<T*>(is_v ? qk.kv.v : qk.kv.k) + at * dim + in) = two;
+        }
+      }
+    }
+  } else if (gated) {
     const int c = 2 * lane;
     for (int r = split + splits * warp; r < rows; r += 4 * splits) {
       const float2 g = sums(r, c), u = sums(r, 64 + c);
@@ -204,11 +304,9 @@ thin_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
       store(r, n0 + c, R::round(g0 / (1.f + expf(-g0))) * R::round(u.x), R::round(g1 / (1.f + expf(-g1))) * R::round(u.y));
     }
   } else {
-    const int c = 2 * (threadIdx.x & 63);
-    const long long col = n0 + c;
     const float b0 = bias != nullptr && col < n ? (float)bias[col] : 0.f, b1 = bias != nullptr && col + 1 < n ? (float)bias[col + 1] : 0.f;
     for (int r = split + splits * (threadIdx.x >> 6); r < rows; r += 2 * splits) {
-      const float2 t = sums(r, c);
+      const float2 t = sums(r, c2);
       float a[2] = {R::round(t.x), R::round(t.y)};
       if (bias != nullptr) { a[0] = R::round(a[0] + b0); a[1] = R::round(a[1] + b1); }
 #pragma unroll
@@ -224,22 +322,27 @@ thin_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
 // --------------------------------------------------------------------------------------------------------------------------
 // host side
 // --------------------------------------------------------------------------------------------------------------------------
-template <typename T>
-static int launch_thin(const CUtensorMap& tm_w, const CUtensorMap& tm_x, const void* bias, void* y, int rows, long long n, int k, long long tiles,
-                       int splits, int epilogue, int early, int* status, cudaStream_t stream) {
+struct FlThinStep {
+  int dtype; const void* x; int rows; const void* w; long long n; int k; const void* bias; int epilogue; void* y; int early; int* status;
+  FlThinQkv qkv;
+};
+
+template <typename T, int OUT>
+static int launch_thin(const CUtensorMap& tm_w, const CUtensorMap& tm_x, const FlThinStep& a, long long tiles, int splits, cudaStream_t stream) {
   static bool set_on[64];                          // per device: a process may drive several GPUs
+  const auto kernel = thin_gemm_kernel<T, OUT>;
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return (int)e;
   if (dev < 0 || dev >= 64) return -3;
   if (!set_on[dev]) {
-    e = cudaFuncSetAttribute(thin_gemm_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, TG_SMEM);
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TG_SMEM);
     if (e != cudaSuccess) return (int)e;
     set_on[dev] = true;
   }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(tiles * splits), 1, 1);
-  cfg.blockDim = dim3(TG_THREADS, 1, 1);
+  cfg.blockDim = dim3(OUT == FL_THIN_QKV ? TG_THREADS + 32 : TG_THREADS, 1, 1);
   cfg.dynamicSmemBytes = TG_SMEM;
   cfg.stream = stream;
   cudaLaunchAttribute at[2];
@@ -248,31 +351,50 @@ static int launch_thin(const CUtensorMap& tm_w, const CUtensorMap& tm_x, const v
   at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
-  cfg.numAttrs = early ? 2 : 1;
-  return (int)cudaLaunchKernelEx(&cfg, thin_gemm_kernel<T>, tm_w, tm_x, (const T*)bias, (T*)y, rows, n, k, splits, epilogue, early, status);
+  cfg.numAttrs = a.early ? 2 : 1;
+  return (int)cudaLaunchKernelEx(&cfg, kernel, tm_w, tm_x, (const T*)a.bias, (T*)a.y, a.rows, a.n, a.k, splits, a.epilogue, a.early, a.status, a.qkv);
 }
 
 }  // namespace fl
 
-extern "C" int fl_thin_gemm(int dtype, const void* x, int rows, const void* w, long long n, int k, const void* bias, int epilogue, void* y, int early,
-                            int* status, cudaStream_t stream) {
+static int thin_step(const fl::FlThinStep* a, cudaStream_t stream) {
   using namespace fl;
-  if (dtype != FL_DEC_BF16 && dtype != FL_DEC_FP16) return -1;
-  if (rows < 1 || rows > FL_THIN_MAX_ROWS || n < 1 || n > 0x3fffff00ll || k < 8 || k % 8) return -2;
-  if (epilogue < FL_THIN_SILU_GATED || epilogue > FL_THIN_STORE || (epilogue == FL_THIN_SILU_GATED && bias != nullptr)) return -3;
-  if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 15 || reinterpret_cast<uintptr_t>(y) & 3) return -4;
-  const bool gated = epilogue == FL_THIN_SILU_GATED;
-  const int per_tile = gated ? TG_M / 2 : TG_M, blocks = (k + TG_K - 1) / TG_K;
-  const long long tiles = (n + per_tile - 1) / per_tile;
+  const bool gated = a->epilogue == FL_THIN_SILU_GATED, qkv = a->epilogue == FL_THIN_QKV;
+  if (a->dtype != FL_DEC_BF16 && a->dtype != FL_DEC_FP16) return -1;
+  if (a->rows < 1 || a->rows > FL_THIN_MAX_ROWS || a->n < 1 || a->n > 0x3fffff00ll || a->k < 8 || a->k % 8) return -2;
+  if (a->epilogue < FL_THIN_SILU_GATED || a->epilogue > FL_THIN_QKV || (gated && a->bias != nullptr)) return -3;
+  if (((uintptr_t)a->x | (uintptr_t)a->w) & 15 || (uintptr_t)a->y & 3) return -4;
+  if (qkv) {
+    const FlThinQkv& q = a->qkv;
+    if (q.pos == nullptr || q.dim < 16 || q.dim % 16 || TG_M % q.dim || q.heads < 1 || q.kv.heads < 1 || q.kv.block_size < 1 || q.kv.table_stride < 1 ||
+        (long long)(q.heads + 2ll * q.kv.heads) * q.dim != a->n || ((uintptr_t)q.kv.k | (uintptr_t)q.kv.v) & 3 || (uintptr_t)q.rope & 15)
+      return -5;
+  }
+  const int per_tile = gated ? TG_M / 2 : TG_M, blocks = (a->k + TG_K - 1) / TG_K;
+  const long long tiles = (a->n + per_tile - 1) / per_tile;
   // As many CTAs as fit at two per SM, so that all of them run from start to end at an equal share of the memory's rate; clusters of
   // 1, 2, 4 or 8, since others leave SMs over (6144 x 4096, 16 rows: 17.2 us in clusters of 6, 13.1 in clusters of 4).
   int splits = 1;
   while (splits < 8 && 2 * splits * tiles <= 2 * 148 && 2 * splits <= blocks) splits *= 2;
-  const int type = dtype == FL_DEC_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
+  const int type = a->dtype == FL_DEC_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
   CUtensorMap tm_w, tm_x;
-  int rc = tile_map(&tm_w, type, w, k, gated ? 2 * n : n, per_tile);
-  if (rc == 0) rc = tile_map(&tm_x, type, x, k, rows, TG_N);
+  int rc = tile_map(&tm_w, type, a->w, a->k, gated ? 2 * a->n : a->n, per_tile);
+  if (rc == 0) rc = tile_map(&tm_x, type, a->x, a->k, a->rows, TG_N);
   if (rc != 0) return rc;
-  if (dtype == FL_DEC_BF16) return launch_thin<__nv_bfloat16>(tm_w, tm_x, bias, y, rows, n, k, tiles, splits, epilogue, early, status, stream);
-  return launch_thin<__half>(tm_w, tm_x, bias, y, rows, n, k, tiles, splits, epilogue, early, status, stream);
+  if (a->dtype == FL_DEC_BF16) return qkv ? launch_thin<__nv_bfloat16, FL_THIN_QKV>(tm_w, tm_x, *a, tiles, splits, stream)
+                                          : launch_thin<__nv_bfloat16, FL_THIN_STORE>(tm_w, tm_x, *a, tiles, splits, stream);
+  return qkv ? launch_thin<__half, FL_THIN_QKV>(tm_w, tm_x, *a, tiles, splits, stream) : launch_thin<__half, FL_THIN_STORE>(tm_w, tm_x, *a, tiles, splits, stream);
+}
+
+extern "C" int fl_thin_gemm(int dtype, const void* x, int rows, const void* w, long long n, int k, const void* bias, int epilogue, void* y, int early,
+                            int* status, cudaStream_t stream) {
+  if (epilogue == FL_THIN_QKV) return -3;
+  const fl::FlThinStep a = {dtype, x, rows, w, n, k, bias, epilogue, y, early, status, {}};
+  return thin_step(&a, stream);
+}
+
+extern "C" int fl_thin_qkv(int dtype, const void* x, int rows, const void* w, long long n, int k, const void* bias, const FlThinQkv* qkv, void* y,
+                           int early, int* status, cudaStream_t stream) {
+  const fl::FlThinStep a = {dtype, x, rows, w, n, k, bias, FL_THIN_QKV, y, early, status, *qkv};
+  return thin_step(&a, stream);
 }

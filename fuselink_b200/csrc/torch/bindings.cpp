@@ -375,6 +375,34 @@ static torch::Tensor dec_product(torch::Tensor x, torch::Tensor w, c10::optional
                         reinterpret_cast<int*>(status_addr), cur_stream()), "fl_thin_gemm");
   return y;
 }
+// queries of [rows, (heads + 2 kv_heads) * dim] (the rest is unwritten); keys and values to their pages, as dec_qkv
+static torch::Tensor dec_qkv_product(torch::Tensor x, torch::Tensor w, c10::optional<torch::Tensor> bias, c10::optional<torch::Tensor> rope,
+                                     torch::Tensor pos, torch::Tensor k_pool, torch::Tensor v_pool, torch::Tensor table, int64_t layout, int64_t layer,
+                                     int64_t layers, int64_t num_blocks, int64_t block_size, int64_t heads, int64_t kv_heads, int64_t dim, bool early,
+                                     int64_t status_addr) {
+  const int dt = dec_dtype(x);
+  TORCH_CHECK(x.dim() == 2 && w.dim() == 2 && x.is_contiguous() && w.is_contiguous() && w.is_cuda() && w.scalar_type() == x.scalar_type() &&
+              w.size(1) == x.size(1) && w.device() == x.device(), "product: x [rows, k] and w [n, k], contiguous, of one type and device");
+  const int64_t rows = x.size(0), n = w.size(0);
+  TORCH_CHECK(n == (heads + 2 * kv_heads) * dim, "w: [(heads + 2 kv_heads) * dim, hidden]");
+  TORCH_CHECK(x.size(1) <= INT32_MAX && rows <= FL_THIN_MAX_ROWS, "product: too large");
+  TORCH_CHECK(k_pool.scalar_type() == x.scalar_type() && v_pool.scalar_type() == x.scalar_type(), "pools of the model's type expected");
+  TORCH_CHECK(table.size(0) >= rows, "block_table: one row per request");
+  TORCH_CHECK(!rope.has_value() || (rope->is_cuda() && rope->scalar_type() == torch::kFloat32 && rope->is_contiguous() && rope->size(-1) == dim),
+              "rope: [positions, dim] fp32");
+  dec_like(bias, x, n, "bias: [(heads + 2 kv_heads) * dim]");
+  c10::cuda::CUDAGuard guard(x.device());
+  FlThinQkv q = {};
+  q.rope = rope.has_value() ? rope->data_ptr<float>() : nullptr;
+  q.rope_rows = rope.has_value() ? rope->size(0) : 0;
+  q.pos = dec_i64(pos, rows, "positions: int64");
+  q.heads = (int)heads; q.dim = (int)dim;
+  q.kv = dec_kv(k_pool, v_pool, table, layout, layer, layers, num_blocks, block_size, kv_heads, dim, status_addr);
+  auto y = torch::empty({rows, n}, x.options());
+  check_rc(fl_thin_qkv(dt, x.data_ptr(), (int)rows, w.data_ptr(), n, (int)x.size(1), opt_ptr(bias), &q, y.data_ptr(), early,
+                       reinterpret_cast<int*>(status_addr), cur_stream()), "fl_thin_qkv");
+  return y;
+}
 static torch::Tensor dec_argmax(torch::Tensor logits) {
   const int dt = dec_dtype(logits);
   TORCH_CHECK(logits.dim() == 2 && logits.is_contiguous(), "logits: [rows, vocab]");
@@ -600,6 +628,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         py::arg("dim"), py::arg("out"), py::arg("status_addr") = 0);
   m.def("dec_product", &dec_product, py::arg("x"), py::arg("w"), py::arg("bias"), py::arg("epilogue"), py::arg("early") = false,
         py::arg("status_addr") = 0);
+  m.def("dec_qkv_product", &dec_qkv_product);
   m.attr("THIN_MAX_ROWS") = FL_THIN_MAX_ROWS;
   m.def("dec_argmax", &dec_argmax);
   m.def("dec_advance", &dec_advance);

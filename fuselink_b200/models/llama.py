@@ -311,12 +311,18 @@ class LlamaShard(torch.nn.Module):
             # `early`: the layers' weights were there before the step's first kernel started
             return C.dec_product(a, w, b, epilogue, True, status) if thin else a @ w.t()
 
+        # A step's keys and values go to their pages where their sums are, if heads divide a tile's 128 columns.  A prefill's attention
+        # reads them beside the queries.
+        pages_in_product = thin and pos is not None and 128 % cfg.head_dim == 0
         y = bias = None
         for l in range(cfg.layers):
             C.dec_add_norm(x, y, bias, self.n1[l], self.n1b[l], h, cfg.eps)
-            qkv = product(h, self.wqkv[l])
-            C.dec_qkv(qkv, self.bqkv[l], rope, pos, seq, k_pool, v_pool, table, layout, l, cfg.layers, num_blocks, cfg.block_size,
-                      self.h_local, self.kvh_local, cfg.head_dim, status)
+            where = (k_pool, v_pool, table, layout, l, cfg.layers, num_blocks, cfg.block_size, self.h_local, self.kvh_local, cfg.head_dim)
+            if pages_in_product:
+                qkv = C.dec_qkv_product(h, self.wqkv[l], self.bqkv[l], rope, pos, *where, True, status)
+            else:
+                qkv = product(h, self.wqkv[l])
+                C.dec_qkv(qkv, self.bqkv[l], rope, pos, seq, *where, status)
             if on_layer_done is not None:
                 on_layer_done(l)                                                # KV of this layer may leave now
             y = self._allreduce(product(attend(l, qkv), self.wo[l]))

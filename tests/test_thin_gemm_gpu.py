@@ -87,3 +87,51 @@ def test_the_kernel_before_may_take_longer_than_a_wait():
     torch.cuda.synchronize()
     assert timed_out[0] != 0 and status[0] == 0
     assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("dt", DT)
+@pytest.mark.parametrize("rows,k,heads,kv_heads,dim", [(1, 64, 1, 1, 16), (3, 2048, 32, 32, 64), (16, 512, 5, 1, 128), (9, 264, 3, 2, 32), (13, 4096, 32, 8, 128)])
+@pytest.mark.parametrize("rope,bias", [(True, False), (False, True), (True, True)])
+@pytest.mark.parametrize("layout", [0, 1])
+def test_qkv_with_rotation_and_pages(dt, rows, k, heads, kv_heads, dim, rope, bias, layout):
+    """Against the product and the pass behind it, bit by bit: negative positions and pages, positions beyond the table of angles, a
+    page outside the pool and one outside the block table among them."""
+    from fuselink_b200 import C
+    n, L, nblk, bs, layer = (heads + 2 * kv_heads) * dim, 2, 40, 16, 1
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    x, w = _eighths(rows, k, dt=dt, seed=1), _eighths(n, k, dt=dt, seed=2)
+    b = _eighths(n, dt=dt, seed=3) if bias else None
+    ang = torch.rand(30, dim // 2, generator=g, device="cuda") * 6
+    table = torch.cat([ang.cos(), ang.sin()], 1).contiguous() if rope else None
+    bt = torch.randperm(nblk, generator=g, device="cuda")[:16 * 2].int().view(16, 2).contiguous()
+    pos = torch.randint(0, 32, (rows,), generator=g, device="cuda")
+    if rows > 4:
+        pos[1], pos[2], bt[3], pos[4] = -3, 1000, nblk, 2 ** 33
+        bt[0] -= nblk
+    pools = [[torch.zeros(nblk * L * bs * kv_heads * dim, dtype=dt, device="cuda") for _ in range(2)] for _ in range(2)]
+    st = torch.zeros(2, dtype=torch.int32, device="cuda")
+    qkv = C.dec_product(x, w, None, 3)
+    C.dec_qkv(qkv, b, table, pos, 1, *pools[0], bt, layout, layer, L, nblk, bs, heads, kv_heads, dim, st.data_ptr())
+    got = C.dec_qkv_product(x, w, b, table, pos, *pools[1], bt, layout, layer, L, nblk, bs, heads, kv_heads, dim, True, st.data_ptr() + 4)
+    assert torch.equal(got[:, :heads * dim], qkv[:, :heads * dim])
+    for p, q in zip(*pools):
+        assert torch.equal(p, q) and p.any()
+    assert (st[0] != 0) == (st[1] != 0) == (rows > 4)
+
+
+def test_arguments_of_qkv():
+    from fuselink_b200 import C
+    cuda = dict(dtype=torch.half, device="cuda")
+    x, w = torch.zeros(2, 64, **cuda), torch.zeros(96, 64, **cuda)
+    pos, bt, pool = torch.zeros(2, dtype=torch.long, device="cuda"), torch.zeros(2, 1, dtype=torch.int32, device="cuda"), torch.zeros(4 * 16 * 48, **cuda)
+
+    def call(x=x, w=w, bias=None, rope=None, pos=pos, k=pool, v=pool, bt=bt, layer=0, blocks=4, heads=1, kv_heads=1, dim=32):
+        return C.dec_qkv_product(x, w, bias, rope, pos, k, v, bt, 1, layer, 1, blocks, 16, heads, kv_heads, dim, True, 0)
+
+    call()
+    rope = torch.zeros(4, 32, device="cuda")
+    for bad in (dict(dim=16), dict(w=torch.zeros(144, 64, **cuda), dim=48), dict(pos=pos[:1]), dict(bt=bt[:1]), dict(layer=1), dict(blocks=64), dict(bias=x[0]),
+                dict(rope=rope[:, :16]), dict(rope=rope.half()), dict(k=pool.bfloat16()), dict(x=x.repeat(9, 1)), dict(w=w.bfloat16()),
+                dict(rope=torch.zeros(130, device="cuda")[1:129].view(4, 32)), dict(x=torch.zeros(200, **cuda)[1:129].view(2, 64))):
+        with pytest.raises(RuntimeError):
+            call(**bad)
