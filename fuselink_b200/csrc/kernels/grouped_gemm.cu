@@ -530,17 +530,107 @@ struct SharedPair {
   uint64_t empty[STAGES2];
   uint64_t tmem_full[2];
   uint64_t tmem_empty[2];
+  uint64_t w_full[8][2];                         // DW: the weights that an epilogue warp updates have come into its buffer
   uint32_t tmem_base;
   int abort_flag;
   int counts[FL_GEMM_MAX_GROUPS];
 };
 
+// The weight-gradient epilogue of the pair kernel: a warp's 32 rows x 128 columns of the tile in two blocks of 64 columns, each stored
+// by one TMA store from a buffer of the warp's own (two of 4 KiB, 128-byte swizzle), and with the fused update brought there by a TMA
+// load first, asked for before the accumulator is ready.  Bound by memory's writes where experts have few rows (a tile is then three or
+// four k-blocks and 64 KiB of output per CTA; a fill reaches 3.2 to 3.6 TB/s), by the products and the power cap beyond about 500.  From
+// registers, 64 bytes of a row at a time, a warp waited for its weights and its own stores in every 32 columns.  us, gradients stored |
+// update in place, before (the better of one CTA per tile and pairs) -> now:
+//   16 experts of 11264 x 2048, 191 rows each: 274 | 527 -> 243 | 370;  512: 344 | 592 -> 344 | 418;  1024: 637 | 747 -> 637 | 638
+//   8 experts of 28672 x 4096, 250 rows: 701 | 1381 -> 590 | 927;  1024: 1540 | 1805 -> 1475 | 1601
+// One stage less of operands than the other pair kernel pays for the buffers.  Asking for the next tile's weights into L2 as well costs
+// 5 to 15 % (1023 against 927 at 250 rows).
+constexpr int DW_STAGES = 5;
+constexpr int DW_BUF_BYTES = 32 * ROW_BYTES;
+constexpr int SMEM_DW_BYTES = DW_STAGES * STAGE2_BYTES + 1024 /*align*/ + 1024 /*barriers, counts*/ + 8 * 2 * DW_BUF_BYTES;
+
+struct DwWarp {
+  uint8_t* buf;        // [2][DW_BUF_BYTES]
+  uint64_t* full;      // [2]
+  uint32_t blocks;     // 64-column blocks done so far
+};
+
+// Asks for the weights of the tile's blocks (lane 0).  The buffers' last stores have been read by then.
+__device__ __forceinline__ void dw_request(const KParams& p, const CUtensorMap* tmC, const DwWarp& w, int g, int row, int col) {
+  tma_store_wait_read<0>();
+  for (int j = 0; j < 2; ++j) {
+    if (row >= p.M || col + 64 * j >= p.N) break;
+    const uint32_t b = (w.blocks + j) & 1;
+    mbar_arrive_expect_tx(&w.full[b], DW_BUF_BYTES);
+    tma_load_3d(w.buf + b * DW_BUF_BYTES, tmC, &w.full[b], col + 64 * j, row, g);
+  }
+}
+
+__device__ __forceinline__ bool dw_blocks(const KParams& p, const CUtensorMap* tmC, DwWarp& w, int g, int row, int col, uint32_t t_addr, bool have_acc,
+                                          int lane, volatile int* abort_flag) {
+  const bool update = p.sgd_lr != 0.f;
+#pragma unroll 1
+  for (int j = 0; j < 2; ++j) {
+    if (row >= p.M || col + 64 * j >= p.N) break;
+    const uint32_t b = w.blocks & 1;
+    uint8_t* buf = w.buf + b * DW_BUF_BYTES;
+    if (update) {
+      if (!mbar_wait_warp(&w.full[b], (w.blocks >> 1) & 1, abort_flag, p.status, kTimeoutMbarFull, 1500 + b)) return false;
+    } else {
+      if (lane == 0) tma_store_wait_read<1>();     // the store before the last one has left this buffer
+      __syncwarp();
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      uint32_t r[32];
+      if (have_acc) {
+        tmem_ld_32x32(t_addr + 64 * j + 32 * h, r);
+        tmem_ld_wait();
+      } else {
+#pragma unroll
+        for (int i = 0; i < 32; ++i) r[i] = 0u;
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        uint4* at = reinterpret_cast<uint4*>(buf + lane * ROW_BYTES + (((4 * h + i) ^ (lane & 7)) << 4));
+        float v[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) v[e] = __uint_as_float(r[8 * i + e]);
+        if (update) {
+          const uint4 old = *at;
+          const uint32_t ow[4] = {old.x, old.y, old.z, old.w};
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            float w0, w1;
+            unpack_bf16(ow[e], w0, w1);
+            v[2 * e] = w0 - p.sgd_lr * v[2 * e];
+            v[2 * e + 1] = w1 - p.sgd_lr * v[2 * e + 1];
+          }
+        }
+        *at = make_uint4(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]), pack_bf16(v[6], v[7]));
+      }
+    }
+    fence_proxy_async_smem();
+    __syncwarp();
+    if (lane == 0) {
+      tma_store_3d(tmC, buf, col + 64 * j, row, g);
+      tma_store_commit();
+    }
+    ++w.blocks;
+  }
+  return true;
+}
+
+// DW: the weight-gradient GEMM into a matrix of this GPU, through the epilogue above.
+template <bool DW>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
-grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
+grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const __grid_constant__ CUtensorMap tmC,
                          const KParams p) {
+  constexpr int ST = DW ? DW_STAGES : STAGES2;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  SharedPair* sh = reinterpret_cast<SharedPair*>(smem + STAGES2 * STAGE2_BYTES);
+  SharedPair* sh = reinterpret_cast<SharedPair*>(smem + ST * STAGE2_BYTES);
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const uint32_t rank = cluster_cta_rank();       // 0 = leader (issues the MMAs), 1 = peer
@@ -549,7 +639,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
   constexpr int TM = 2 * BM;                      // rows of a pair's tile
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < STAGES2; ++s) {
+    for (int s = 0; s < ST; ++s) {
       mbar_init(&sh->full[s], 1);                 // used in the leader: one arrive.expect_tx covering both CTAs' bytes
       mbar_init(&sh->empty[s], 1);                // one multicast commit from the leader's MMA thread
     }
@@ -557,6 +647,8 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
       mbar_init(&sh->tmem_full[a], 1);
       mbar_init(&sh->tmem_empty[a], 16);          // used in the leader: 8 epilogue warps of each CTA
     }
+    if (DW)
+      for (int w = 0; w < 8; ++w) { mbar_init(&sh->w_full[w][0], 1); mbar_init(&sh->w_full[w][1], 1); }
     sh->abort_flag = 0;
     mbar_fence_init();
   }
@@ -569,6 +661,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
   if (warp == 0 && lane == 0) {
     tma_prefetch_desc(&tmA);
     tma_prefetch_desc(&tmB);
+    if (DW) tma_prefetch_desc(&tmC);
   }
   tc_fence_before_sync();
   __syncthreads();
@@ -586,8 +679,8 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
       Tile t;
       for (int id = pair_id; ok && map_tile(p, counts, id, t, TM); id += num_pairs) {
         for (int kb = 0; kb < t.kblocks && ok; ++kb, ++it) {
-          const int s = it % STAGES2;
-          const uint32_t ph = (it / STAGES2) & 1;
+          const int s = it % ST;
+          const uint32_t ph = (it / ST) & 1;
           ok = mbar_wait(&sh->empty[s], ph ^ 1, abort_flag, p.status, kTimeoutMbarEmpty, 1100 + s);
           if (!ok) break;
           uint8_t* a_dst = smem + s * STAGE2_BYTES;
@@ -635,8 +728,8 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
         tc_fence_after_sync();
         const uint32_t d_tmem = tmem_base + acc * BN;
         for (int kb = 0; kb < t.kblocks && ok; ++kb, ++it) {
-          const int s = it % STAGES2;
-          const uint32_t ph = (it / STAGES2) & 1;
+          const int s = it % ST;
+          const uint32_t ph = (it / ST) & 1;
           ok = mbar_wait(&sh->full[s], ph, abort_flag, p.status, kTimeoutMbarFull, 1300 + s);
           if (!ok) break;
           tc_fence_after_sync();
@@ -668,14 +761,26 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
     uint32_t tile_i = 0;
     bool ok = true;
     Tile t;
+    DwWarp dw = {smem + ST * STAGE2_BYTES + 1024 + (warp - 2) * 2 * DW_BUF_BYTES, sh->w_full[warp - 2], 0};
     for (int id = pair_id; ok && map_tile(p, counts, id, t, TM); id += num_pairs, ++tile_i) {
       const int acc = tile_i & 1;
       const uint32_t acc_ph = (tile_i >> 1) & 1;
+      if (DW) {
+        const int row = t.m0 + 128 * (int)rank + 32 * q, col = t.n0 + 128 * half;
+        if (p.sgd_lr != 0.f && lane == 0) dw_request(p, &tmC, dw, t.g, row, col);
+        ok = mbar_wait_warp(&sh->tmem_full[acc], acc_ph, abort_flag, p.status, kTimeoutTmemFull, 1400 + acc);
+        if (!ok) break;
+        tc_fence_after_sync();
+        ok = dw_blocks(p, &tmC, dw, t.g, row, col, tmem_base + acc * BN + ((uint32_t)(q * 32) << 16) + 128 * half, t.kblocks > 0, lane, abort_flag);
+        if (!ok) break;
+        tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(&sh->tmem_empty[acc]), 0));
+        continue;
+      }
       if (p.epilogue == FL_EPI_DSWIGLU && half == 0)
         prefetch_saved_gate_up(p, t.g, t.m0 + 128 * (int)rank, min(128, t.cnt - (t.m0 + 128 * (int)rank)), t.n0, min(BN, p.N - t.n0),
                                q * 32 + lane);
-      if (p.epilogue == FL_EPI_WGRAD && p.sgd_lr != 0.f && half == 0)
-        prefetch_weights(p, t.g, t.m0 + 128 * (int)rank, t.n0, min(BN, p.N - t.n0), q * 32 + lane);
       ok = mbar_wait(&sh->tmem_full[acc], acc_ph, abort_flag, p.status, kTimeoutTmemFull, 1400 + acc);
       if (!ok) break;
       tc_fence_after_sync();
@@ -683,10 +788,14 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
       e.g = t.g; e.row0 = t.m0 + 128 * (int)rank; e.n0 = t.n0; e.have_acc = t.kblocks > 0;
       e.valid_rows = p.group_mode == 0 ? min(128, t.cnt - e.row0) : 128;
       e.zero_limit = p.group_mode == 0 ? min(p.cap, (t.cnt + 127) / 128 * 128) : 0;
-      epilogue_slab(p, e, tmem_base + acc * BN, q, half, lane, smem + STAGES2 * STAGE2_BYTES + 1024 + (warp - 2) * EPI_STAGE_BYTES);
+      epilogue_slab(p, e, tmem_base + acc * BN, q, half, lane, smem + ST * STAGE2_BYTES + 1024 + (warp - 2) * EPI_STAGE_BYTES);
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(&sh->tmem_empty[acc]), 0));
+    }
+    if (DW && lane == 0) {
+      if (!ok) let_copies_land();
+      tma_store_wait<0>();
     }
     if (p.epilogue == FL_EPI_SCATTER || p.push_world > 0) fence_sys();
   }
@@ -1009,9 +1118,7 @@ static int pairs_in_use(const FlGemmDesc* d, int fit) {
 
 // The variant for groups of `expect_rows` rows on `pairs` CTA pairs, `dflt` being the one for thousands.  Few rows per group change what
 // pays, all measured in us on 8 groups of 28672 x 4096 and 4096 x 14336 or 16 of 11264 x 2048 and 2048 x 5632 (0 | 1 | 2):
-//   weight gradients: the contraction is those rows, and a tile is all epilogue: 0 below 448 (250 rows: 704 | 758, 191: 264 | 307;
-//     448: 554 | 541).  A skewed router moves the line up, not down: where 440 rows is the mean and the fullest expert has 1235, the two
-//     gradients of a layer take 1603 | 1636, at a mean of 520 1770 | 1803;
+//   weight gradients: pairs at any number of rows (with the update in place: 191 rows 527 | 370 | 541, 1024: 1991 | 1609 | 2607);
 //   SWIGLU and DSWIGLU: the wide tiles' single accumulator does not hide such short tiles (448 rows: 321 | 296 | 331; 1000: 1506 |
 //     1491 | 1515); 0 where tiles of 128 rows pad a tenth less than those of 256 (250: 520 | 538 | 553, 125: 358 | 380 | 395);
 //   the others: wide tiles are a tenth cheaper per column, unless their number leaves more pairs idle in the last round (250 rows of
@@ -1019,8 +1126,7 @@ static int pairs_in_use(const FlGemmDesc* d, int fit) {
 //     fewer tiles: an average is a little above the number of tiles that the groups mostly take (700 rows: 3.01).
 static int variant_for_rows(const FlGemmDesc* d, int dflt, int pairs) {
   const double rows = d->expect_rows;
-  if (d->group_mode == 1) return rows < 448 ? 0 : dflt;
-  if (d->N < 512 || rows >= 1024) return dflt;
+  if (d->group_mode == 1 || d->N < 512 || rows >= 1024) return dflt;
   const double t256 = expected_tiles(rows, 256);
   if (d->epilogue == FL_EPI_SWIGLU || d->epilogue == FL_EPI_DSWIGLU)
     return 1.1 * 128 * expected_tiles(rows, 128) < 256 * t256 ? 0 : 1;
@@ -1111,7 +1217,9 @@ extern "C" int fl_grouped_gemm(const FlGemmDesc* d, cudaStream_t stream) {
     cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev);
     cudaError_t e = cudaFuncSetAttribute(grouped_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
     if (e != cudaSuccess) return (int)e;
-    e = cudaFuncSetAttribute(grouped_gemm_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM2_BYTES);
+    e = cudaFuncSetAttribute(grouped_gemm_pair_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM2_BYTES);
+    if (e != cudaSuccess) return (int)e;
+    e = cudaFuncSetAttribute(grouped_gemm_pair_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_DW_BYTES);
     if (e != cudaSuccess) return (int)e;
     e = cudaFuncSetAttribute(grouped_gemm_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM3_BYTES);
     if (e != cudaSuccess) return (int)e;
@@ -1127,7 +1235,7 @@ extern "C" int fl_grouped_gemm(const FlGemmDesc* d, cudaStream_t stream) {
     cfg.attrs = &at;
     cfg.numAttrs = 1;
     int nclusters = 0;
-    if (cudaOccupancyMaxActiveClusters(&nclusters, grouped_gemm_pair_kernel, &cfg) == cudaSuccess && nclusters > 0)
+    if (cudaOccupancyMaxActiveClusters(&nclusters, grouped_gemm_pair_kernel<false>, &cfg) == cudaSuccess && nclusters > 0)
       max_pairs = nclusters;
     else
       max_pairs = num_sms / 2;
@@ -1154,7 +1262,12 @@ extern "C" int fl_grouped_gemm(const FlGemmDesc* d, cudaStream_t stream) {
   if (pair) {
     const int pairs = pairs_in_use(d, max_pairs);
     if (variant == 2) grouped_gemm_wide_kernel<<<2 * pairs, NUM_THREADS, SMEM3_BYTES, stream>>>(tmA, tmB, p);
-    else grouped_gemm_pair_kernel<<<2 * pairs, NUM_THREADS, SMEM2_BYTES, stream>>>(tmA, tmB, p);
+    else if (d->group_mode == 1 && d->push_world == 0) {
+      CUtensorMap tmC;
+      rc = make_map(&tmC, d->C, d->N, d->M, d->num_groups, d->ldc, d->gsc, 64, 32);
+      if (rc) return rc;
+      grouped_gemm_pair_kernel<true><<<2 * pairs, NUM_THREADS, SMEM_DW_BYTES, stream>>>(tmA, tmB, tmC, p);
+    } else grouped_gemm_pair_kernel<false><<<2 * pairs, NUM_THREADS, SMEM2_BYTES, stream>>>(tmA, tmB, tmB, p);
     return (int)cudaGetLastError();
   }
   int grid = num_sms;

@@ -111,3 +111,37 @@ def test_no_result_depends_on_the_expected_rows(counts_l, max_ctas):
         if counts_l[g]:
             _close(dw[g], act[r].float().t() @ x[r].float())
     assert st[0] == 0
+
+
+@pytest.mark.parametrize("M,N", [(8, 32), (40, 96), (264, 288), (512, 544), (1000, 64), (256, 1056)])
+@pytest.mark.parametrize("rows", [[3, 0, 190], [64, 65, 384]])
+@pytest.mark.parametrize("lr", [0.0, 0.25])
+def test_weight_gradients_through_the_pair_kernel(M, N, rows, lr):
+    """Bit by bit what one CTA per tile stores from registers: matrices that end inside a block of 32 rows x 64 columns or inside a tile, an
+    expert without rows, a contraction that ends inside a k-block, several tiles per pair, and nothing written behind the matrices."""
+    from fuselink_b200 import C
+    from fuselink_b200.ops.gemm import grouped_gemm_wgrad
+    G, cap = len(rows), 384
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    a, b = (torch.randn(G * cap, n, generator=g, device="cuda").to(torch.bfloat16) for n in (M, N))
+    for i, n in enumerate(rows):                       # the rows behind an expert's last are zeros, as the kernels before leave them
+        a[i * cap + n:(i + 1) * cap], b[i * cap + n:(i + 1) * cap] = 0, 0
+    counts = torch.tensor(rows, dtype=torch.int32, device="cuda")
+    w = torch.randn(G * M * N + 4096, generator=g, device="cuda").to(torch.bfloat16)
+    st = torch.zeros(8, dtype=torch.int32, device="cuda")
+    got, before = {}, C.gemm_get_variant()
+    try:
+        for v in (0, 1):
+            C.gemm_set_variant(v)
+            got[v] = w.clone()
+            for _ in range(2):
+                grouped_gemm_wgrad(a, b, counts, cap, G, out=got[v][: G * M * N].view(G, M, N), sgd_lr=lr, max_ctas=4, status=st)
+            torch.cuda.synchronize()
+            assert st[0].item() == 0, st.tolist()
+    finally:
+        C.gemm_set_variant(before)
+    assert torch.equal(got[0], got[1]) and torch.equal(got[1][G * M * N:], w[G * M * N:])
+    if lr == 0.0:
+        want = torch.stack([a[i * cap:i * cap + n].double().t() @ b[i * cap:i * cap + n].double() for i, n in enumerate(rows)])
+        # rounded to bf16 once; sums of up to 384 products in fp32
+        assert ((got[1][: G * M * N].view(G, M, N).double() - want).abs() <= 2.0 ** -8 * want.abs() + 384 * 2.0 ** -23 * 16).all()
