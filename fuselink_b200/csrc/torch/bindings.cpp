@@ -497,6 +497,51 @@ static std::pair<torch::Tensor, torch::Tensor> relu_bias_bwd(torch::Tensor dy, t
                             cur_stream()), "fl_relu_bias_bwd");
   return {dz, db};
 }
+// An MLP's layers behind one another, and their gradients (models/dlrm.py, _Mlp).  Native because a small batch takes the GPU less time than
+// the host needs for some forty calls.  params: weight, bias of every layer.
+static std::vector<torch::Tensor> mlp_forward(torch::Tensor x, bool relu_last, bool padded, const std::vector<torch::Tensor>& params) {
+  const size_t n = params.size() / 2;
+  TORCH_CHECK(params.size() == 2 * n && n > 0, "params: weight and bias of every layer");
+  std::vector<torch::Tensor> acts;
+  for (size_t i = 0; i < n; ++i) {
+    const torch::Tensor &w = params[2 * i], &b = params[2 * i + 1];
+    const torch::Tensor& rows = i == 0 ? x : acts.back();
+    auto z = at::addmm(b, padded && i == 0 ? rows.narrow(1, 0, w.size(1)) : rows, w.t());
+    if (i + 1 < n || relu_last) z.relu_();
+    acts.push_back(z);
+  }
+  return acts;
+}
+// dy^T r over slices of `slice` rows, the slices' results added up in fp32
+static torch::Tensor sliced_gram(const torch::Tensor& dy, const torch::Tensor& r, int64_t slice) {
+  const int64_t B = dy.size(0), n = B / slice, m = n * slice;
+  if (n < 2) return at::mm(dy.t(), r);
+  auto out = at::bmm(dy.narrow(0, 0, m).view({n, slice, dy.size(1)}).transpose(1, 2), r.narrow(0, 0, m).view({n, slice, r.size(1)})).sum(0);
+  return m == B ? out : out.addmm_(dy.narrow(0, m, B - m).t(), r.narrow(0, m, B - m));
+}
+// inputs: x, then the outputs of the layers that have a ReLU.  want: of x, then of every parameter.  Returns the gradients in that order.
+static std::vector<c10::optional<torch::Tensor>> mlp_backward(torch::Tensor dy, const std::vector<torch::Tensor>& inputs, bool relu_last,
+                                                              const std::vector<torch::Tensor>& params, const std::vector<bool>& want, int64_t slice) {
+  const size_t n = params.size() / 2;
+  TORCH_CHECK(inputs.size() == n + relu_last && want.size() == 2 * n + 1, "one input per layer");
+  std::vector<c10::optional<torch::Tensor>> grads(2 * n + 1);
+  for (size_t i = n; i-- > 0;) {
+    const torch::Tensor &w = params[2 * i], &x = inputs[i];
+    const int64_t width = x.size(1), cols = w.size(1);
+    torch::Tensor db;
+    if (i + 1 < n || relu_last) {
+      std::tie(dy, db) = relu_bias_bwd(dy.contiguous(), inputs[i + 1]);
+    } else if (want[2 * i + 2]) {
+      db = dy.sum(0);
+    }
+    if (want[2 * i + 2]) grads[2 * i + 2] = db;
+    if (want[2 * i + 1])
+      grads[2 * i + 1] = width != cols ? sliced_gram(dy.contiguous(), x, slice).narrow(1, 0, cols).contiguous() : at::mm(dy.t(), x);
+    if (i > 0 || want[0]) dy = at::mm(dy, width == cols ? w : at::constant_pad_nd(w, {0, width - cols}));
+  }
+  if (want[0]) grads[0] = dy;
+  return grads;
+}
 static void moe_zero_tail(int64_t buf, int64_t counts, int64_t experts_local, int64_t cap, int64_t width) {
   check_rc(fl_moe_zero_tail(reinterpret_cast<void*>(buf), reinterpret_cast<const int*>(counts), (int)experts_local,
                             (int)cap, (int)width, cur_stream()), "fl_moe_zero_tail");
@@ -622,6 +667,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("interact_fwd", &interact_fwd);
   m.def("interact_bwd", &interact_bwd);
   m.def("relu_bias_bwd", &relu_bias_bwd);
+  m.def("mlp_forward", &mlp_forward);
+  m.def("mlp_backward", &mlp_backward);
   m.def("dec_act", &dec_act);
   m.def("dec_attention", &dec_attention, py::arg("qkv"), py::arg("pos"), py::arg("k_pool"), py::arg("v_pool"), py::arg("table"),
         py::arg("layer"), py::arg("layers"), py::arg("num_blocks"), py::arg("block_size"), py::arg("heads"), py::arg("kv_heads"),

@@ -69,6 +69,14 @@ def _mlp(sizes, last_act: bool) -> nn.Sequential:
     return nn.Sequential(*layers)
 
 
+def _parameters(mlp) -> list:
+    """list(mlp.parameters()), without the general walk for what _mlp makes: a step asks for them several times."""
+    if type(mlp) is not nn.Sequential or mlp._parameters or any(type(m) not in (nn.Linear, nn.ReLU) or m._modules for m in mlp._modules.values()):
+        return list(mlp.parameters())
+    found = {id(p): p for m in mlp._modules.values() for p in m._parameters.values() if p is not None}
+    return list(found.values())
+
+
 def _tf32_allowed() -> bool:
     """Whether the program lets fp32 products run in tf32.  `fp32_precision` answers for both of the framework's settings; the
     older flag raises once the newer setting has been used."""
@@ -135,43 +143,22 @@ class _Mlp(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, x, relu_last, padded, *params):
-        acts, n = [x], len(params) // 2
-        for i in range(n):
-            w, b = params[2 * i], params[2 * i + 1]
-            rows = x[:, : w.shape[1]] if padded and i == 0 else acts[-1]
-            z = torch.addmm(b, rows, w.t())
-            acts.append(z.relu_() if i < n - 1 or relu_last else z)
-        ctx.save_for_backward(*(acts if relu_last else acts[:-1]), *params)
+        acts = require_native().mlp_forward(x, relu_last, padded, params)
+        ctx.save_for_backward(x, *(acts if relu_last else acts[:-1]), *params)
         ctx.relu_last = relu_last
         return acts[-1]
 
     @staticmethod
     @torch.autograd.function.once_differentiable
     def backward(ctx, dy):
-        C, saved = require_native(), ctx.saved_tensors
-        n = (len(saved) - ctx.relu_last) // 3
-        acts, params = saved[:n + ctx.relu_last], saved[n + ctx.relu_last:]
-        grads = [None] * (2 * n)
-        for i in range(n - 1, -1, -1):
-            w, x = params[2 * i], acts[i]
-            want_x, want_w, want_b = i > 0 or ctx.needs_input_grad[0], ctx.needs_input_grad[3 + 2 * i], ctx.needs_input_grad[4 + 2 * i]
-            if i < n - 1 or ctx.relu_last:
-                dy, db = C.relu_bias_bwd(dy.contiguous(), acts[i + 1])
-            else:
-                db = dy.sum(0) if want_b else None
-            grads[2 * i + 1] = db if want_b else None
-            if want_w:
-                if x.shape[1] != w.shape[1]:
-                    grads[2 * i] = _gram(dy.contiguous(), x)[:, :w.shape[1]].contiguous()
-                else:
-                    grads[2 * i] = dy.t() @ x
-            if want_x:
-                dy = dy @ (w if x.shape[1] == w.shape[1] else F.pad(w, (0, x.shape[1] - w.shape[1])))
-        return dy if ctx.needs_input_grad[0] else None, None, None, *grads
+        saved, want = ctx.saved_tensors, ctx.needs_input_grad
+        n = (len(saved) - ctx.relu_last) // 3 + ctx.relu_last
+        dx, *grads = require_native().mlp_backward(dy, saved[:n], ctx.relu_last, saved[n:], [want[0], *want[3:]], _GRAM_ROWS)
+        return dx, None, None, *grads
 
     @staticmethod
     def of(mlp, x, relu_last, padded):
-        return _Mlp.apply(x, relu_last, padded, *(p for m in list(mlp)[::2] for p in (m.weight, m.bias)))
+        return _Mlp.apply(x, relu_last, padded, *(m._parameters[name] for m in list(mlp._modules.values())[::2] for name in ("weight", "bias")))
 
 
 class _PaddedLinear(torch.autograd.Function):
@@ -318,7 +305,7 @@ class DLRM(nn.Module):
         return self.top[1:](y).squeeze(-1)
 
     def dense_parameters(self):
-        return list(self.bottom.parameters()) + list(self.top.parameters())
+        return _parameters(self.bottom) + _parameters(self.top)
 
     # ---- one training step (public API) --------------------------------------------------------------------
     def train_step(self, dense: torch.Tensor, indices: torch.Tensor, labels: torch.Tensor, opt: torch.optim.Optimizer):
