@@ -273,6 +273,13 @@ __global__ void __launch_bounds__(256) dec_qkv_kernel(T* qkv, const T* bias, con
 }
 
 // ---- activation -----------------------------------------------------------------------------------------------------------
+// Bound by memory, where its arithmetic lets it be: an exponential and an IEEE division per element took 573 us for 32768 x 14336 in
+// bf16 (2.8 GB, 436 us at the rate of a copy), with the hardware's 443.  Their error, some 2^-21, does not show behind the rounding to
+// bf16 (against 64 bits 2.4132767e-3 either way); behind that to fp16 it does in the eighth digit, so fp16 keeps the others.  Both sides of
+// the quotient are a sixteenth: __fdividef gives 0 for divisors beyond 2^126, which 1 + e^-x is below x = -87.3.
+template <typename T> __device__ __forceinline__ float silu_of(float x) { return x / (1.f + expf(-x)); }
+template <> __device__ __forceinline__ float silu_of<__nv_bfloat16>(float x) { return __fdividef(0.0625f * x, fmaf(__expf(-x), 0.0625f, 0.0625f)); }
+
 template <typename T, int KIND>
 __global__ void __launch_bounds__(256) dec_act_kernel(const T* h, const T* bias, T* out, long long rows, int ffn) {
   grid_dep_launch();
@@ -289,7 +296,7 @@ __global__ void __launch_bounds__(256) dec_act_kernel(const T* h, const T* bias,
       unpack8<T>(ld_stream_v4(p), a);
       unpack8<T>(ld_stream_v4(p + ffn), u);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) a[j] = Num<T>::round(a[j] / (1.f + expf(-a[j]))) * u[j];
+      for (int j = 0; j < 8; ++j) a[j] = Num<T>::round(silu_of<T>(a[j])) * u[j];
     } else {
       unpack8<T>(ld_stream_v4(h + n * ffn + c), a);
       if (bias) {

@@ -165,6 +165,22 @@ def test_activation(kind, ffn):
     assert ((out - want).float().abs() <= 2.02 * 2.0 ** -8 * want.float().abs() + 1e-6).all()
 
 
+@pytest.mark.parametrize("dt", DT)
+def test_silu_of_every_value(dt):
+    """Of every 16-bit value, against 64 bits: rounded once, as is the product with 1.  4e-37 and 6e-8: the largest result that e^-x = inf
+    (x < -88.7) loses, and fp16's smallest step."""
+    from fuselink_b200 import C
+    x = torch.arange(-32768, 32768, device="cuda").to(torch.int16).view(dt).view(16, 4096)
+    out = torch.empty_like(x)
+    C.dec_act(torch.cat([x, torch.ones_like(x)], 1), None, out, 0)
+    want = F.silu(x.double())
+    want[x == float("-inf")] = float("nan")                          # -inf / inf, as before
+    eps = 2.0 ** -8 if dt == torch.bfloat16 else 2.0 ** -11
+    fin = want.isfinite()
+    assert torch.equal(out.isnan(), want.isnan()) and torch.equal(out[~fin & ~want.isnan()].double(), want[~fin & ~want.isnan()])
+    assert ((out.double() - want)[fin].abs() <= 1.01 * eps * want[fin].abs() + (4e-37 if dt == torch.bfloat16 else 6e-8)).all()
+
+
 def _shard(model):
     from fuselink_b200.models.llama import MODEL_ZOO, LlamaShard
     net = LlamaShard(MODEL_ZOO[model], device="cuda", seed=2)
