@@ -293,6 +293,7 @@ __device__ __forceinline__ void epilogue_slab(const KParams& p, const EpiSlab& e
     // Saved gate/up of the next 32-column chunk are fetched (packed bf16, 2 x 64 B) while the current chunk's
     // accumulator read and math are in flight, so the global-load latency is paid once per tile, not per chunk.
     const int c0 = half * (BN / 64), c1 = c0 + BN / 64;
+    if (e.n0 + c0 * 32 >= p.N) return;                          // N is a multiple of 128: a warp's columns are all there or none is
     auto gate_col = [&](int c) {
       const int a_col = e.n0 + c * 32;                          // column of dAct
       return (long long)(a_col >> 7) * 256 + (a_col & 127);     // gate position in the interleaved row; up is +128

@@ -145,3 +145,35 @@ def test_weight_gradients_through_the_pair_kernel(M, N, rows, lr):
         want = torch.stack([a[i * cap:i * cap + n].double().t() @ b[i * cap:i * cap + n].double() for i, n in enumerate(rows)])
         # rounded to bf16 once; sums of up to 384 products in fp32
         assert ((got[1][: G * M * N].view(G, M, N).double() - want).abs() <= 2.0 ** -8 * want.abs() + 384 * 2.0 ** -23 * 16).all()
+
+
+@pytest.mark.parametrize("N,K", [(128, 64), (384, 200), (512, 1024)])
+@pytest.mark.parametrize("rows", [[1, 0, 128], [129, 31, 256], [257, 300, 384]])
+@pytest.mark.parametrize("mn", [False, True])
+def test_activation_gradients_through_the_pair_kernel(N, K, rows, mn):
+    """Bit by bit what one CTA per tile stores from registers: columns that end in the middle of a tile, rows that end inside a block of 32,
+    a CTA of the pair without rows, an expert without any; zeros up to a whole 128 rows and nothing behind them."""
+    from fuselink_b200 import C
+    from fuselink_b200.ops.gemm import EPI_DSWIGLU, grouped_gemm_rows
+    G, cap = len(rows), 384
+    g = torch.Generator(device="cuda").manual_seed(N + K)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda").to(torch.bfloat16)
+    a, b, gu = rnd(G * cap, K), rnd(G, K, N) if mn else rnd(G, N, K), rnd(G * cap, 2 * N) * 3
+    counts = torch.tensor(rows, dtype=torch.int32, device="cuda")
+    st = torch.zeros(8, dtype=torch.int32, device="cuda")
+    got, before = {}, C.gemm_get_variant()
+    try:
+        for v in (0, 1):
+            C.gemm_set_variant(v)
+            got[v] = torch.full((G * cap + 40, 2 * N), 7.0, dtype=torch.bfloat16, device="cuda")
+            for _ in range(2):
+                grouped_gemm_rows(a, b, counts, cap, b_mn_major=mn, epilogue=EPI_DSWIGLU, gu=gu, dgu=got[v], zero_tail=True, max_ctas=4, status=st)
+            torch.cuda.synchronize()
+            assert st[0].item() == 0, st.tolist()
+    finally:
+        C.gemm_set_variant(before)
+    assert torch.equal(got[0], got[1])
+    for i, n in enumerate(rows):
+        end = (n + 127) // 128 * 128
+        assert (got[1][i * cap + n:i * cap + end] == 0).all() and (got[1][i * cap + end:(i + 1) * cap] == 7).all()
+        assert n == 0 or got[1][i * cap:i * cap + n].float().abs().amax(1).min() > 0
