@@ -623,12 +623,70 @@ __device__ __forceinline__ bool dw_blocks(const KParams& p, const CUtensorMap* t
   return true;
 }
 
-// DW: the weight-gradient GEMM into a matrix of this GPU, through the epilogue above.
-template <bool DW>
+// The activation gradient's epilogue of the pair kernel, through the same buffers: 64 columns of dAct and the gate and up that belong to
+// them, which come by TMA and leave as dGate and dUp.  Loaded and stored row by row from registers, every 16 bytes were half of a
+// sector's request and the epilogue cost the GEMM up to a seventh of its time.  us, before -> now: 16 experts of 5632 x 2048, 191 rows each
+// 131 -> 126, 400: 218 -> 199, 1024: 424 -> 365; 8 of 14336 x 4096, 512 rows 456 -> 440, 1024: 1019 -> 970; 32 of 2048 x 1024, 400 rows 131 ->
+// 117.  (SWIGLU's three outputs that way: 437 against 430 at 250 rows, 622 against 623 at 1024; not used.)
+__device__ __forceinline__ int gate_column(int act_column) { return (act_column >> 7) * 256 + (act_column & 127); }   // up: 128 further
+__device__ __forceinline__ void dswiglu_request(const CUtensorMap* tm_gu, const DwWarp& w, int g, int row, int col) {
+  tma_store_wait_read<0>();
+  mbar_arrive_expect_tx(&w.full[0], 2 * DW_BUF_BYTES);
+  tma_load_3d(w.buf, tm_gu, &w.full[0], gate_column(col), row, g);
+  tma_load_3d(w.buf + DW_BUF_BYTES, tm_gu, &w.full[0], gate_column(col) + 128, row, g);
+}
+__device__ __forceinline__ bool dswiglu_block(const KParams& p, const CUtensorMap* tm_dgu, DwWarp& w, int g, int row, int col, bool valid, uint32_t t_addr,
+                                              int lane, volatile int* abort_flag) {
+  if (!mbar_wait_warp(&w.full[0], w.blocks & 1, abort_flag, p.status, kTimeoutMbarFull, 1510)) return false;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    uint32_t r[32];
+    tmem_ld_32x32(t_addr + 32 * h, r);
+    tmem_ld_wait();
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      uint8_t* at = w.buf + lane * ROW_BYTES + (((4 * h + i) ^ (lane & 7)) << 4);
+      const uint4 gq = *reinterpret_cast<const uint4*>(at), uq = *reinterpret_cast<const uint4*>(at + DW_BUF_BYTES);
+      const uint32_t gw[4] = {gq.x, gq.y, gq.z, gq.w}, uw[4] = {uq.x, uq.y, uq.z, uq.w};
+      uint32_t pdg[4], pdu[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        float g0, g1, u0, u1;
+        unpack_bf16(gw[j], g0, g1);
+        unpack_bf16(uw[j], u0, u1);
+        const float da0 = __uint_as_float(r[8 * i + 2 * j]), da1 = __uint_as_float(r[8 * i + 2 * j + 1]);
+        // as in epilogue_slab
+        const float s0 = sigmoid_f(g0), s1 = sigmoid_f(g1);
+        const float t0 = g0 * s0, t1 = g1 * s1;
+        pdg[j] = valid ? pack_bf16((da0 * u0) * (fmaf(-t0, s0, t0) + s0), (da1 * u1) * (fmaf(-t1, s1, t1) + s1)) : 0u;
+        pdu[j] = valid ? pack_bf16(da0 * t0, da1 * t1) : 0u;
+      }
+      *reinterpret_cast<uint4*>(at) = make_uint4(pdg[0], pdg[1], pdg[2], pdg[3]);
+      *reinterpret_cast<uint4*>(at + DW_BUF_BYTES) = make_uint4(pdu[0], pdu[1], pdu[2], pdu[3]);
+    }
+  }
+  fence_proxy_async_smem();
+  __syncwarp();
+  if (lane == 0) {
+    tma_store_3d(tm_dgu, w.buf, gate_column(col), row, g);
+    tma_store_3d(tm_dgu, w.buf + DW_BUF_BYTES, gate_column(col) + 128, row, g);
+    tma_store_commit();
+  }
+  ++w.blocks;
+  return true;
+}
+
+// What a pair's epilogue is: PAIR_ANY epilogue_slab, PAIR_DW the weight gradient of matrices of this GPU, PAIR_DSWIGLU the activation's
+// gradient with rows up to a whole 128 written (zero_tail), so that every block of 32 rows is written whole or not at all.
+enum PairEpilogue { PAIR_ANY, PAIR_DW, PAIR_DSWIGLU };
+
+// tmC: PAIR_DW the matrices, PAIR_DSWIGLU dGate and dUp; tmG: PAIR_DSWIGLU gate and up.
+template <int KIND>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
 grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const __grid_constant__ CUtensorMap tmC,
-                         const KParams p) {
-  constexpr int ST = DW ? DW_STAGES : STAGES2;
+                         const __grid_constant__ CUtensorMap tmG, const KParams p) {
+  constexpr bool DW = KIND == PAIR_DW, BUFFERED = KIND != PAIR_ANY;
+  constexpr int ST = BUFFERED ? DW_STAGES : STAGES2;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   SharedPair* sh = reinterpret_cast<SharedPair*>(smem + ST * STAGE2_BYTES);
@@ -648,7 +706,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
       mbar_init(&sh->tmem_full[a], 1);
       mbar_init(&sh->tmem_empty[a], 16);          // used in the leader: 8 epilogue warps of each CTA
     }
-    if (DW)
+    if (BUFFERED)
       for (int w = 0; w < 8; ++w) { mbar_init(&sh->w_full[w][0], 1); mbar_init(&sh->w_full[w][1], 1); }
     sh->abort_flag = 0;
     mbar_fence_init();
@@ -662,7 +720,8 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
   if (warp == 0 && lane == 0) {
     tma_prefetch_desc(&tmA);
     tma_prefetch_desc(&tmB);
-    if (DW) tma_prefetch_desc(&tmC);
+    if (BUFFERED) tma_prefetch_desc(&tmC);
+    if (KIND == PAIR_DSWIGLU) tma_prefetch_desc(&tmG);
   }
   tc_fence_before_sync();
   __syncthreads();
@@ -779,6 +838,26 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
         if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(&sh->tmem_empty[acc]), 0));
         continue;
       }
+      if (KIND == PAIR_DSWIGLU) {
+        const int slab = t.m0 + 128 * (int)rank, row = slab + 32 * q, col = t.n0 + 128 * half;
+        const bool valid = row + lane < t.cnt, write = slab < t.cnt && col < p.N;      // all of the slab, zeros behind the last row
+        if (write && lane == 0) dswiglu_request(&tmG, dw, t.g, row, col);
+        ok = mbar_wait_warp(&sh->tmem_full[acc], acc_ph, abort_flag, p.status, kTimeoutTmemFull, 1400 + acc);
+        if (!ok) break;
+        tc_fence_after_sync();
+        const uint32_t t_addr = tmem_base + acc * BN + ((uint32_t)(q * 32) << 16) + 128 * half;
+        if (write) {
+          ok = dswiglu_block(p, &tmC, dw, t.g, row, col, valid, t_addr, lane, abort_flag);
+          if (!ok) break;
+          if (lane == 0) dswiglu_request(&tmG, dw, t.g, row, col + 64);
+          ok = dswiglu_block(p, &tmC, dw, t.g, row, col + 64, valid, t_addr + 64, lane, abort_flag);
+          if (!ok) break;
+        }
+        tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(&sh->tmem_empty[acc]), 0));
+        continue;
+      }
       if (p.epilogue == FL_EPI_DSWIGLU && half == 0)
         prefetch_saved_gate_up(p, t.g, t.m0 + 128 * (int)rank, min(128, t.cnt - (t.m0 + 128 * (int)rank)), t.n0, min(BN, p.N - t.n0),
                                q * 32 + lane);
@@ -794,7 +873,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(&sh->tmem_empty[acc]), 0));
     }
-    if (DW && lane == 0) {
+    if (BUFFERED && lane == 0) {
       if (!ok) let_copies_land();
       tma_store_wait<0>();
     }
@@ -1121,7 +1200,8 @@ static int pairs_in_use(const FlGemmDesc* d, int fit) {
 // pays, all measured in us on 8 groups of 28672 x 4096 and 4096 x 14336 or 16 of 11264 x 2048 and 2048 x 5632 (0 | 1 | 2):
 //   weight gradients: pairs at any number of rows (with the update in place: 191 rows 527 | 370 | 541, 1024: 1991 | 1609 | 2607);
 //   SWIGLU and DSWIGLU: the wide tiles' single accumulator does not hide such short tiles (448 rows: 321 | 296 | 331; 1000: 1506 |
-//     1491 | 1515); 0 where tiles of 128 rows pad a tenth less than those of 256 (250: 520 | 538 | 553, 125: 358 | 380 | 395);
+//     1491 | 1515); 0 where tiles of 128 rows pad a tenth less than those of 256 (SWIGLU 250: 520 | 538 | 553, 125: 358 | 380 | 395), for DSWIGLU
+//     a sixth (264 rows each: 384 | 432, 128: 110 | 114, 250: 292 | 261);
 //   the others: wide tiles are a tenth cheaper per column, unless their number leaves more pairs idle in the last round (250 rows of
 //     4096 x 14336, 86 tiles on 74 pairs: 289 (1) | 336 (2), on 48 pairs: 343 | 311; 500 on 74: 398 | 365).  The rounds are counted of 2 %
 //     fewer tiles: an average is a little above the number of tiles that the groups mostly take (700 rows: 3.01).
@@ -1130,7 +1210,7 @@ static int variant_for_rows(const FlGemmDesc* d, int dflt, int pairs) {
   if (d->group_mode == 1 || d->N < 512 || rows >= 1024) return dflt;
   const double t256 = expected_tiles(rows, 256);
   if (d->epilogue == FL_EPI_SWIGLU || d->epilogue == FL_EPI_DSWIGLU)
-    return 1.1 * 128 * expected_tiles(rows, 128) < 256 * t256 ? 0 : 1;
+    return (d->epilogue == FL_EPI_SWIGLU ? 1.1 : 1.2) * 128 * expected_tiles(rows, 128) < 256 * t256 ? 0 : 1;
   const double share = 0.98 * d->num_groups * t256 / pairs;
   return 1.8 * ceil(share * ((d->N + 511) / 512)) < ceil(share * ((d->N + 255) / 256)) ? 2 : 1;
 }
@@ -1218,9 +1298,11 @@ extern "C" int fl_grouped_gemm(const FlGemmDesc* d, cudaStream_t stream) {
     cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev);
     cudaError_t e = cudaFuncSetAttribute(grouped_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
     if (e != cudaSuccess) return (int)e;
-    e = cudaFuncSetAttribute(grouped_gemm_pair_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM2_BYTES);
+    e = cudaFuncSetAttribute(grouped_gemm_pair_kernel<PAIR_ANY>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM2_BYTES);
     if (e != cudaSuccess) return (int)e;
-    e = cudaFuncSetAttribute(grouped_gemm_pair_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_DW_BYTES);
+    e = cudaFuncSetAttribute(grouped_gemm_pair_kernel<PAIR_DW>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_DW_BYTES);
+    if (e != cudaSuccess) return (int)e;
+    e = cudaFuncSetAttribute(grouped_gemm_pair_kernel<PAIR_DSWIGLU>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_DW_BYTES);
     if (e != cudaSuccess) return (int)e;
     e = cudaFuncSetAttribute(grouped_gemm_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM3_BYTES);
     if (e != cudaSuccess) return (int)e;
@@ -1236,7 +1318,7 @@ extern "C" int fl_grouped_gemm(const FlGemmDesc* d, cudaStream_t stream) {
     cfg.attrs = &at;
     cfg.numAttrs = 1;
     int nclusters = 0;
-    if (cudaOccupancyMaxActiveClusters(&nclusters, grouped_gemm_pair_kernel<false>, &cfg) == cudaSuccess && nclusters > 0)
+    if (cudaOccupancyMaxActiveClusters(&nclusters, grouped_gemm_pair_kernel<PAIR_ANY>, &cfg) == cudaSuccess && nclusters > 0)
       max_pairs = nclusters;
     else
       max_pairs = num_sms / 2;
@@ -1267,8 +1349,15 @@ extern "C" int fl_grouped_gemm(const FlGemmDesc* d, cudaStream_t stream) {
       CUtensorMap tmC;
       rc = make_map(&tmC, d->C, d->N, d->M, d->num_groups, d->ldc, d->gsc, 64, 32);
       if (rc) return rc;
-      grouped_gemm_pair_kernel<true><<<2 * pairs, NUM_THREADS, SMEM_DW_BYTES, stream>>>(tmA, tmB, tmC, p);
-    } else grouped_gemm_pair_kernel<false><<<2 * pairs, NUM_THREADS, SMEM2_BYTES, stream>>>(tmA, tmB, tmB, p);
+      grouped_gemm_pair_kernel<PAIR_DW><<<2 * pairs, NUM_THREADS, SMEM_DW_BYTES, stream>>>(tmA, tmB, tmC, tmC, p);
+    } else if (d->zero_tail && d->epilogue == FL_EPI_DSWIGLU) {
+      const long long gs = (long long)d->cap * d->ldgu;
+      CUtensorMap tmC, tmG;
+      rc = make_map(&tmC, d->dgu, 2ll * d->N, d->cap, d->num_groups, d->ldgu, gs, 64, 32);
+      if (rc == 0) rc = make_map(&tmG, d->gu, 2ll * d->N, d->cap, d->num_groups, d->ldgu, gs, 64, 32);
+      if (rc) return rc;
+      grouped_gemm_pair_kernel<PAIR_DSWIGLU><<<2 * pairs, NUM_THREADS, SMEM_DW_BYTES, stream>>>(tmA, tmB, tmC, tmG, p);
+    } else grouped_gemm_pair_kernel<PAIR_ANY><<<2 * pairs, NUM_THREADS, SMEM2_BYTES, stream>>>(tmA, tmB, tmB, tmB, p);
     return (int)cudaGetLastError();
   }
   int grid = num_sms;
