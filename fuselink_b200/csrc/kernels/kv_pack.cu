@@ -136,7 +136,7 @@ __global__ void __launch_bounds__(256, 6) kv_pack_send_kernel(const FlKvSendArgs
 // 243; 13 x 1280 of one layer, 32 of 64 77 | 60.  Units of 16 KiB in six slots: 1506, 146, 258, 64; of 8 KiB in twelve: 2420 (a store costs
 // the engine over a microsecond whatever its size), so pages of less than 16 KiB stay with the other kernel (4 x 1584 of 32 layers, 2 heads
 // of 128: 100 | 113).
-constexpr int KVB_SLOTS = 3, KVB_SLOT_BYTES = 32 * 1024, KVB_LEAST = 16 * 1024;
+constexpr int KVB_SLOTS = 3, KVB_SLOT_BYTES = 32 * 1024, KVB_LEAST = 16 * 1024, KVB_LEAST_CALL = 16 << 20;
 
 __global__ void __launch_bounds__(32) kv_pack_bulk_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
                                                           const FlKvSendArgs a, const int group /* heads per unit */) {
@@ -275,7 +275,8 @@ static int kv_map(CUtensorMap* m, void* base, const FlKvSendArgs* a, int group) 
 }
 
 // Heads per unit of the bulk kernel, 0 if it does not take the call: heads of at most 256 columns and pages of at most 256 slots (a
-// box's sides), contiguous in the source, units of 16 to 32 KiB, pools from a multiple of 16 bytes on.
+// box's sides), contiguous in the source, units of 16 to 32 KiB, pools from a multiple of 16 bytes on.  Not below 16 MiB of pages: two
+// tensor maps cost the host 4 us a launch, and a prefill of small models sends layer by layer (GPT-2, 4 x 64 tokens: 2106 us, 2163 with them).
 static int kv_group(const FlKvSendArgs* a) {
   const long long head = (long long)a->block_size * a->head_dim * 2;
   if (a->src_layout != FL_KV_BLHSD || a->batch > KV_BATCH || a->head_dim < 8 || a->head_dim > 256 || a->block_size < 1 || a->block_size > 256 ||
@@ -285,7 +286,8 @@ static int kv_group(const FlKvSendArgs* a) {
   long long g = KVB_SLOT_BYTES / head;
   if (g > a->heads) g = a->heads;
   if (g > 256) g = 256;
-  return g * head >= KVB_LEAST ? (int)g : 0;
+  const double bytes = 2. * a->batch * a->max_blocks * (a->layer_end - a->layer_begin) * (double)a->heads * (double)head;
+  return g * head >= KVB_LEAST && bytes >= KVB_LEAST_CALL ? (int)g : 0;
 }
 
 }  // namespace fl

@@ -142,10 +142,7 @@ def test_online_trace_batches_with_pool_credits():
             h.close()
 
 
-# through the copy engine from 16 KiB on: (9, 16, 128) ends in one head of a unit of eight, (32, 32, 256) are two units of one head each and
-# more, (16, 16, 32) is the smallest unit, (15, 16, 32) one of the other kernel's, (1, 64, 128) one head, (300, 1, 32) a box of 256 heads
-@pytest.mark.parametrize("H,S,D,layout", [(9, 16, 128, 1), (32, 32, 256, 1), (16, 16, 32, 1), (15, 16, 32, 1), (1, 64, 128, 1), (300, 1, 32, 1), (9, 16, 128, 0),
-                                          (1, 1, 8, 1), (3, 5, 24, 1), (12, 16, 64, 1), (64, 64, 128, 1), (7, 16, 128, 0)])
+@pytest.mark.parametrize("H,S,D,layout", [(1, 1, 8, 1), (3, 5, 24, 1), (12, 16, 64, 1), (64, 64, 128, 1), (7, 16, 128, 0)])
 @pytest.mark.parametrize("batch", [1, 37, 1500])                       # the last: more requests than the table of totals holds
 def test_kv_pack_send_over_page_shapes(H, S, D, layout, batch):
     """Odd head counts and page sizes, pages of 2^16 vectors and more, empty requests; every page lands, nothing else moves."""
@@ -200,3 +197,12 @@ def test_decode_stage_follows_its_parameters_after_the_capture(input_len, steps)
         assert got.shape == (3, 1 + steps) and torch.equal(got, want)
     finally:
         heap.close()
+
+
+# (9, 16, 128) ends in one head of a unit of eight, (32, 32, 256) are units of two heads, (16, 16, 32) is the smallest unit and (15, 16, 32) one
+# of the other kernel's, (1, 64, 128) is one head, (300, 1, 32) a box of 256 heads; on both sides of 16 MiB of pages
+@pytest.mark.parametrize("H,S,D,layout", [(9, 16, 128, 1), (32, 32, 256, 1), (16, 16, 32, 1), (15, 16, 32, 1), (1, 64, 128, 1), (300, 1, 32, 1), (9, 16, 128, 0)])
+@pytest.mark.parametrize("more", [-1, 1, 20])
+def test_kv_pack_send_through_the_copy_engine(H, S, D, layout, more):
+    least = -(-(16 << 20) // (2 * 3 * H * S * D * 2))               # requests of three pages, keys and values
+    test_kv_pack_send_over_page_shapes(H, S, D, layout, least + more)
