@@ -15,6 +15,7 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <math.h>
+#include <type_traits>
 #include <initializer_list>
 #include "../common/fl_ptx.cuh"
 #include "tile_map.cuh"
@@ -277,8 +278,11 @@ __global__ void __launch_bounds__(256) dec_qkv_kernel(T* qkv, const T* bias, con
 // bf16 (2.8 GB, 436 us at the rate of a copy), with the hardware's 443.  Their error, some 2^-21, does not show behind the rounding to
 // bf16 (against 64 bits 2.4132767e-3 either way); behind that to fp16 it does in the eighth digit, so fp16 keeps the others.  Both sides of
 // the quotient are a sixteenth: __fdividef gives 0 for divisors beyond 2^126, which 1 + e^-x is below x = -87.3.
-template <typename T> __device__ __forceinline__ float silu_of(float x) { return x / (1.f + expf(-x)); }
-template <> __device__ __forceinline__ float silu_of<__nv_bfloat16>(float x) { return __fdividef(0.0625f * x, fmaf(__expf(-x), 0.0625f, 0.0625f)); }
+template <typename T>
+__device__ __forceinline__ float silu_of(float x) {
+  if constexpr (std::is_same_v<T, __nv_bfloat16>) return __fdividef(0.0625f * x, fmaf(__expf(-x), 0.0625f, 0.0625f));
+  else return x / (1.f + expf(-x));
+}
 
 template <typename T, int KIND>
 __global__ void __launch_bounds__(256) dec_act_kernel(const T* h, const T* bias, T* out, long long rows, int ffn) {
