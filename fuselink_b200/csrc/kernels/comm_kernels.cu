@@ -217,7 +217,7 @@ __global__ void __launch_bounds__(1024) put_chunks_kernel(const __grid_constant_
     if (threadIdx.x == 0 && done_here != 0) atomicAdd(a.done_scratch + si, done_here);
     chunks_before += nch;
   }
-  grid_dep_launch();
+  if (a.nwait == 0) grid_dep_launch();  // a launch that polls lets nobody take a place before it has seen its flags
   if (a.done_scratch != nullptr && threadIdx.x == 0) {
     // every CTA takes a ticket, also one that gave up a wait; the last one forwards the totals and rearms the words
     __threadfence();
@@ -236,16 +236,16 @@ __global__ void __launch_bounds__(1024) put_chunks_kernel(const __grid_constant_
     wait_flag_ge(a.wait_flag[threadIdx.x], a.wait_want[threadIdx.x], a.status, 650 + threadIdx.x);
 }
 
+// Neither of these two lets the next kernel start while it may still have to poll: a put behind one would fill the shared memory of every
+// SM meanwhile, and what a peer waits for before it sets the flags may be a kernel of another stream that then finds no place.
 __global__ void wait_flags_kernel(const FlWaitArgs a) {
-  grid_dep_launch();
-  grid_dep_wait();
   const int i = threadIdx.x;
+  grid_dep_wait();
   if (i < a.n) wait_flag_ge(a.flag[i], a.want[i], a.status, 700 + i, a.limit_ns ? a.limit_ns : (uint64_t)FL_FLAG_WAIT_NS);
 }
 
 __global__ void barrier_kernel(FlSignalPtrs pads, int slot0, int rank, int world, unsigned int seq, int do_signal,
                                int do_wait, int* status) {
-  grid_dep_launch();
   grid_dep_wait();
   const int r = threadIdx.x;
   if (r >= world) return;

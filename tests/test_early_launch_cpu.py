@@ -77,3 +77,16 @@ def test_a_warp_goes_on_together_behind_a_wait(kernel):
             at += 1
         body = body[:m.start()] + body[at:]
     assert "mbar_wait_warp(" in body and "mbar_wait(" not in body
+
+
+def test_a_kernel_that_polls_flags_lets_nobody_start_before_it_has_seen_them():
+    """The next kernel's CTAs would hold their SMs while flags are polled, and what a peer waits for before it sets them may need those SMs."""
+    functions = _functions("comm_kernels.cu")
+    polling = [k for k, body in functions.items() if "grid_dep_wait()" in body and any("wait_flag_ge" in b for b in _reached(functions, k).values())]
+    assert sorted(polling) == ["barrier_kernel", "put_chunks_kernel", "wait_flags_kernel"]
+    for k in polling:
+        body = functions[k].replace("if (a.nwait == 0) grid_dep_launch();", "nobody_polls_from_here();")
+        assert "grid_dep_launch()" not in body, k
+        if "nobody_polls_from_here" in body:                     # what is polled behind it is a loop over a.nwait flags
+            behind = body[body.index("nobody_polls_from_here"):]
+            assert all("a.nwait" in line for line in re.findall(r"if \([^;]*wait_flag_ge", behind)) and behind.count("wait_flag_ge") == 1
