@@ -236,8 +236,8 @@ __global__ void __launch_bounds__(1024) put_chunks_kernel(const __grid_constant_
     wait_flag_ge(a.wait_flag[threadIdx.x], a.wait_want[threadIdx.x], a.status, 650 + threadIdx.x);
 }
 
-// Neither of these two lets the next kernel start while it may still have to poll: a put behind one would fill the shared memory of every
-// SM meanwhile, and what a peer waits for before it sets the flags may be a kernel of another stream that then finds no place.
+// Neither of these two lets the next kernel start while it may still have to poll: what stands behind one would hold its SMs meanwhile,
+// and what a peer waits for before it sets the flags may be a kernel of another stream that then finds no place.
 __global__ void wait_flags_kernel(const FlWaitArgs a) {
   const int i = threadIdx.x;
   grid_dep_wait();
@@ -258,9 +258,8 @@ __global__ void barrier_kernel(FlSignalPtrs pads, int slot0, int rank, int world
 
 }  // namespace fl
 
-// Puts, waits and barriers, often several in a row, are launched so that they may be placed while the kernel before
-// them drains; they touch nothing, and poll no flag, before that kernel has ended (grid_dep_wait), so what one polls for is never behind
-// it.  The waits and barriers alone: eight exchanges of 21 MB 138 -> 126 us; a put of 64 KiB and its wait: 10.2 -> 9.6 us.
+// Small puts, waits and barriers, often several in a row, are launched so that they may be placed while the kernel before
+// them drains; they touch nothing, and poll no flag, before that kernel has ended (grid_dep_wait), so what one polls for is never behind it.
 template <typename... P, typename... A>
 static int launch_after(void (*kernel)(P...), unsigned grid, unsigned threads, size_t smem, cudaStream_t stream, const A&... args) {
   cudaLaunchConfig_t cfg = {};
@@ -277,6 +276,10 @@ static int launch_after(void (*kernel)(P...), unsigned grid, unsigned threads, s
 }
 
 constexpr unsigned PUT_CTAS = 2 * 148;
+// Up to so many CTAs a put is launched early.  With its wait, one of 4 KiB takes 7.4 us launched plainly and 5.8 us early, 64 KiB 8.3 and
+// 6.9, 1 MiB 10.2 and 9.6; with more CTAs it is the other way round on most GPUs: 16 MiB 13.9 and 14.4, eight exchanges of 1 MB 95.6 and
+// 98.4, of 21 MB 127 and 141 (on one kind of GPU 108 and 103).  So few CTAs also leave room for other streams while they wait their turn.
+constexpr int PUT_EARLY_CTAS = 32;
 
 // Whether the launch may be split evenly in slots over its G CTAs (see the kernel): nothing is waited for or flagged chunk by chunk, and no
 // segment is shared by more CTAs than it has chunks to count.
@@ -334,6 +337,10 @@ extern "C" int fl_put_chunks(const FlPutArgs* args, int num_ctas, int threads, c
       if (e != cudaSuccess) return (int)e;
       set_on[dev] = true;
     }
+  }
+  if (num_ctas > PUT_EARLY_CTAS) {
+    fl::put_chunks_kernel<<<num_ctas, threads, smem, stream>>>(*args, slots, even);
+    return (int)cudaGetLastError();
   }
   return launch_after(fl::put_chunks_kernel, (unsigned)num_ctas, (unsigned)threads, smem, stream, *args, slots, even);
 }
