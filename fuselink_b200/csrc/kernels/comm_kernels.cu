@@ -278,7 +278,7 @@ static int launch_after(void (*kernel)(P...), unsigned grid, unsigned threads, s
 constexpr unsigned PUT_CTAS = 2 * 148;
 // Up to so many CTAs a put is launched early.  With its wait, one of 4 KiB takes 7.4 us launched plainly and 5.8 us early, 64 KiB 8.3 and
 // 6.9, 1 MiB 10.2 and 9.6; with more CTAs it is the other way round on most GPUs: 16 MiB 13.9 and 14.4, eight exchanges of 1 MB 95.6 and
-// 98.4, of 21 MB 127 and 141 (on one kind of GPU 108 and 103).  So few CTAs also leave room for other streams while they wait their turn.
+// 98.4, of 21 MB 128 and 139 (but 125 and 103 on other GPUs of the same model).  So few CTAs also leave room for other streams while they wait their turn.
 constexpr int PUT_EARLY_CTAS = 32;
 
 // Whether the launch may be split evenly in slots over its G CTAs (see the kernel): nothing is waited for or flagged chunk by chunk, and no
@@ -332,7 +332,7 @@ extern "C" int fl_put_chunks(const FlPutArgs* args, int num_ctas, int threads, c
     if (dev < 0 || dev >= 64) return -3;
     if (!set_on[dev]) {
       cudaError_t e = cudaFuncSetAttribute(fl::put_chunks_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, fl::BULK_MAX_SLOTS * fl::BULK_SLOT_BYTES);
-      // without it an SM is set up for one of these CTAs at a time (eight exchanges 148 us, with it 108)
+      // without it an SM is set up for one of these CTAs at a time (eight exchanges launched early 148 us, with it 108)
       if (e == cudaSuccess) e = cudaFuncSetAttribute(fl::put_chunks_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
       if (e != cudaSuccess) return (int)e;
       set_on[dev] = true;
