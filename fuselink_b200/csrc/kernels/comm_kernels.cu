@@ -325,7 +325,7 @@ extern "C" int fl_put_chunks(const FlPutArgs* args, int num_ctas, int threads, c
     even = even_split(args, (unsigned)num_ctas);
   }
   const size_t smem = (size_t)slots * fl::BULK_SLOT_BYTES;
-  if (smem > 48 * 1024) {
+  if (smem > 0) {                           // three slots are 48 KiB, which with the kernel's own few words is more than a launch gets unasked
     static bool set_on[64];                 // per device: a process may drive several GPUs
     int dev = 0;
     cudaGetDevice(&dev);

@@ -137,3 +137,27 @@ def test_striped_relay(heaps):
         h.check_status()
     assert torch.equal(dst[1].local, src)
     C.monitor_close(mon, False)
+
+
+@pytest.mark.parametrize("nbytes", [16384 + 16, 32768])
+def test_first_put_of_a_process(nbytes):
+    """Two units for one CTA: a ring of 48 KiB, more than a launch may have before the kernel's limit has been raised.  In a process of its own,
+    since any larger put raises it."""
+    import os
+    import subprocess
+    import sys
+    program = f"""
+import torch
+from fuselink_b200.ops.comm import Channel
+from fuselink_b200.parallel.symm import SymmetricHeap
+heaps = SymmetricHeap.emulated(2, 8 << 20)
+chans = [Channel(h, "t") for h in heaps]
+dst = [h.alloc_tensor([{nbytes}], torch.uint8) for h in heaps]
+src = torch.randint(0, 255, ({nbytes},), dtype=torch.uint8, device="cuda")
+chans[0].put(src, 1, dst[1].offset)
+torch.cuda.synchronize()
+assert torch.equal(heaps[1].tensor(dst[1].offset, [{nbytes}], torch.uint8), src)
+"""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", program], cwd=root, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
