@@ -248,16 +248,17 @@ __global__ void __launch_bounds__(32) kv_pack_bulk_kernel(const __grid_constant_
     fence_proxy_async_all();
     fence_sys();
   }
-  int last = 0;
-  if (lane == 0) last = atomicAdd(a.cta_counter, 1u) == gridDim.x - 1;
-  if (!__shfl_sync(0xffffffffu, last, 0)) return;
-  if (a.hdr_bytes > 0 && a.hdr_src && a.hdr_dst)
+  unsigned before = 0;
+  if (lane == 0) before = atomicAdd(a.cta_counter, fl_kv_ticket(ok));
+  const FlKvEnd end = fl_kv_end(__shfl_sync(0xffffffffu, before, 0), ok, gridDim.x);
+  if (!end.last) return;
+  if (end.publish && a.hdr_bytes > 0 && a.hdr_src && a.hdr_dst)
     for (int i = lane; i < a.hdr_bytes; i += 32) reinterpret_cast<uint8_t*>(a.hdr_dst)[i] = reinterpret_cast<const uint8_t*>(a.hdr_src)[i];
   __syncwarp();
   if (lane == 0) {
     *a.cta_counter = 0;
     fence_sys();
-    if (a.done_flag) st_release_sys(a.done_flag, a.seq);
+    if (end.publish && a.done_flag) st_release_sys(a.done_flag, a.seq);
   }
 }
 

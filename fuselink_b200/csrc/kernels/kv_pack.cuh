@@ -29,6 +29,24 @@ struct FlKvSendArgs {
   int* status;
 };
 
+// How the CTAs of a launch end: each adds its ticket to cta_counter, with a mark if it gave up waiting for a copy.  The last one resets the
+// word and publishes header and flag only where nobody gave up, so that the receiver's own wait tells it of pages that never came.
+constexpr unsigned int FL_KV_GAVE_UP = 1u << 16;   // a launch has fewer CTAs
+struct FlKvEnd { bool last, publish; };
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+inline unsigned int fl_kv_ticket(bool ok) { return ok ? 1u : 1u + FL_KV_GAVE_UP; }
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+inline FlKvEnd fl_kv_end(unsigned int before, bool ok, unsigned int ctas) {
+  FlKvEnd e;
+  e.last = before % FL_KV_GAVE_UP == ctas - 1;
+  e.publish = e.last && ok && before < FL_KV_GAVE_UP;
+  return e;
+}
+
 #ifdef __cplusplus
 extern "C" {
 #endif

@@ -62,3 +62,31 @@ def test_the_relu_gradient_refuses_widths_that_32_bits_do_not_count(rows, cols):
     f = ctypes.CDLL(lib).fl_relu_bias_bwd
     f.argtypes = [ctypes.c_void_p] * 5 + [ctypes.c_longlong, ctypes.c_int, ctypes.c_void_p]
     assert f(None, None, None, None, None, rows, cols, None) == -1
+
+
+@pytest.mark.parametrize("ctas", [1, 2, 7, 296])
+def test_a_hand_off_with_a_cta_that_gave_up_is_not_published(ctas, tmp_path):
+    """fl_kv_ticket and fl_kv_end over a launch's CTAs, where nobody gives up, then where the first, the last or all of them do: one CTA is the
+    last, and it publishes only what is whole."""
+    published = _run(tmp_path, f"""int main() {{
+  const unsigned n = {ctas};
+  for (unsigned who = 0; who < 4; ++who) {{
+    unsigned counter = 0, lasts = 0, published = 0;
+    for (unsigned c = 0; c < n; ++c) {{
+      const bool ok = who == 0 || !(who == 3 || (who == 1 && c == 0) || (who == 2 && c == n - 1));
+      const unsigned before = counter;
+      counter += fl_kv_ticket(ok);
+      const FlKvEnd e = fl_kv_end(before, ok, n);
+      lasts += e.last; published += e.publish;
+      if (e.last && c != n - 1) return 1;
+    }}
+    if (lasts != 1) return 1;
+    printf("%u ", published);
+  }}
+}}
+""")
+    assert published == [1, 0, 0, 0]
+    text = open(os.path.join(ROOT, "fuselink_b200", "csrc", "kernels", "kv_pack.cu")).read()
+    body = text[text.index("kv_pack_bulk_kernel("):]
+    behind = body[body.index("if (!ok) let_copies_land"):body.index("st_release_sys(a.done_flag")]
+    assert "fl_kv_ticket(ok)" in behind and "if (end.publish && a.hdr_bytes" in behind and behind.endswith("if (end.publish && a.done_flag) ")
