@@ -118,7 +118,7 @@ thin_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
 
   // FL_THIN_QKV: of this CTA's rows, the row of the page (before layer and head; -1: none) and the angles (0: not turned)
   __shared__ int qk_page[OUT == FL_THIN_QKV ? TG_N : 1], qk_slot[OUT == FL_THIN_QKV ? TG_N : 1], qk_turn[OUT == FL_THIN_QKV ? TG_N : 1];
-  __shared__ float qk_angle[OUT == FL_THIN_QKV ? TG_N * TG_M : 1];
+  __shared__ __align__(16) float qk_angle[OUT == FL_THIN_QKV ? TG_N * TG_M : 1];
 
   if (warp == 0 && lane == 0) {
     // ---- loads: w of the first stages before the wait for the kernel that makes x, where w may be read that early
