@@ -158,7 +158,7 @@ class _Mlp(torch.autograd.Function):
 
     @staticmethod
     def of(mlp, x, relu_last, padded):
-        return _Mlp.apply(x, relu_last, padded, *(m._parameters[name] for m in list(mlp._modules.values())[::2] for name in ("weight", "bias")))
+        return _Mlp.apply(x, relu_last, padded, *(p for m in list(mlp)[::2] for p in (m.weight, m.bias)))
 
 
 class _PaddedLinear(torch.autograd.Function):

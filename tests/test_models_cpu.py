@@ -372,3 +372,15 @@ def test_embedding_rows_summed_per_warp():
     for asked, rows, dim, want in [(24, 10 ** 6, 128, 24), (64, 10 ** 6, 128, 24), (10 ** 6, 10 ** 9, 128, 24), (25, 10 ** 6, 128, 24), (23, 10 ** 6, 128, 23), (24, 5, 128, 5),
                                    (24, 10 ** 6, 256, 12), (24, 10 ** 6, 384, 8), (24, 10 ** 6, 512, 6), (24, 10 ** 6, 3072, 1), (24, 10 ** 6, 4096, 0), (-1, 10 ** 6, 128, -1)]:
         assert f(asked, rows, dim) == want
+
+
+def test_mlp_node_takes_weights_that_are_no_parameters():
+    """A layer whose weight or bias the program computes (an attribute in the parameter's place) is a plain layer to the route."""
+    from fuselink_b200.models.dlrm import DLRM, DLRMConfig, _Mlp
+    m = DLRM(DLRMConfig(num_tables=3, rows=10, global_batch=4), device="cpu")
+    theta = torch.randn(m.bottom[0].weight.shape, requires_grad=True)
+    del m.bottom[0].weight, m.bottom[2].bias
+    m.bottom[0].weight, m.bottom[2].bias = theta * 2, torch.ones(m.bottom[2].weight.shape[0])
+    assert m._plain_dense() and m._plain_mlps()
+    x = torch.randn(4, m.bottom[0].weight.shape[1])
+    assert torch.equal(_Mlp.of(m.bottom, x, True, False), m.bottom(x))
