@@ -13,10 +13,10 @@
 // 8 experts, 1024 rows each, hidden 4096, ffn 14336, before and now: second product forward (K = 14336, N = 4096) 582 (scales from
 // global memory, the rest as now) -> 524 us, gradient of the first (K = 28672) 1204 -> 1043; without the FMAs it is 902, without the
 // trips to TMEM 760 (multiplications and loads).  In a training step of 4096 tokens the four products took 4950 us with the loads of
-// the scales, the trips and the FMAs one after the other, now 3905.  Sixteen promotion warps with half the columns each: 1060.
-// The epilogues run between two tiles of a CTA and are not hidden: they store whole sectors through shared memory, ask for the saved
-// gate and up rows a tile ahead, and divide with __fdividef (DSWIGLU product 970 -> 834 us with it; the error against 64 bits is the same
-// to seven digits, 1.6602e-3 of the results' 2-norm, which is the rounding to bf16).
+// the scales, the trips and the FMAs one after the other, now 4230.  Sixteen promotion warps with half the columns each: 1060.
+// The epilogues run between two tiles of a CTA and are not hidden: they store whole sectors through shared memory and ask for the saved
+// gate and up rows a tile ahead.  Their quotients are IEEE divisions: __fdividef takes 1228 instead of 1423 us (SWIGLU in that step) and
+// 872 instead of 1020 (DSWIGLU), but rounds more results to the wrong bf16 neighbour (74 of 8388608 for 60) and gives 0 for gates below -87.3.
 //
 // Reference parity: none in the reference (it has no kernels); this is the fp8 arm of the MoE expert GEMMs.
 #include "fp8_gemm.cuh"
@@ -470,7 +470,7 @@ fp8_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
 #pragma unroll
           for (int i = 0; i < 16; ++i) {
             const float2 g = valid ? acc[c * 16 + i] : make_float2(0.f, 0.f), u = valid ? acc[32 + c * 16 + i] : make_float2(0.f, 0.f);
-            pk[i] = pack_bf16(__fdividef(g.x, 1.f + __expf(-g.x)) * u.x, __fdividef(g.y, 1.f + __expf(-g.y)) * u.y);
+            pk[i] = pack_bf16(g.x / (1.f + __expf(-g.x)) * u.x, g.y / (1.f + __expf(-g.y)) * u.y);
           }
           staged_store_packed(stg, lane, pk, st ? at(act + 32 * c) : 0ull);
         }
@@ -506,7 +506,7 @@ fp8_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
 #pragma unroll
               for (int e = 0; e < 2; ++e) {
                 const float da = e ? d2.y : d2.x;
-                const float sg = __fdividef(1.f, 1.f + __expf(-g[e]));
+                const float sg = 1.f / (1.f + __expf(-g[e]));
                 dg[e] = da * u[e] * (sg * (1.f + g[e] * (1.f - sg)));
                 du[e] = da * g[e] * sg;
               }

@@ -198,3 +198,38 @@ def test_block_quantizer_at_8_byte_addresses():
     q, s = fp8.quantize_blocks(w)
     q0, s0 = fp8.quantize_blocks(w.clone())
     assert torch.equal(q.view(torch.uint8), q0.view(torch.uint8)) and torch.equal(s, s0)
+
+
+def test_fp8_epilogues_at_gates_whose_sigmoid_is_subnormal():
+    """1 + e^-g is beyond 2^126 below g = -87.3, where the hardware's fast quotient gives 0.  One product per sum, so gate, up and dAct are
+    exact; what is left is the exponential (CUDA's bound for __expf at 88.6: 105 ulp, below 2^-16) and the rounding to bf16 (2^-8: eight bits)."""
+    from fuselink_b200.ops import fp8, gemm
+    cap, H, Fd = 256, 128, 256
+    tol = 1.02 * 2.0 ** -8
+    st = torch.zeros(8, dtype=torch.int32, device="cuda")
+    first, second = (torch.zeros(1, Fd, H, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    first[:, :, 0], second[:, :, 1] = 1, 1                              # gate: the row's first value, up: its second
+    w = gemm.interleave_gate_up(first, second).float().to(fp8.FP8)
+    x = torch.zeros(cap, H, device="cuda")
+    x[:, 0], x[:, 1] = -1, 4
+    scale = torch.linspace(80, 88.6, cap, device="cuda").view(cap, 1)
+    act = fp8.grouped_gemm_rows_fp8(x.to(fp8.FP8), scale, w, torch.ones(1, 2 * Fd // 128, 1, device="cuda"), None, cap, epilogue=fp8.EPI_SWIGLU,
+                                    gu=torch.empty(cap, 2 * Fd, dtype=torch.bfloat16, device="cuda"), status=st)
+    g, u = -scale.double(), 4 * scale.double()
+    want = (g * torch.sigmoid(g) * u).expand(cap, Fd)
+    assert ((act.double() - want).abs() <= tol * want.abs()).all()
+
+    gate, up = scale.neg().to(torch.bfloat16).expand(cap, Fd), torch.full((cap, Fd), 4., dtype=torch.bfloat16, device="cuda")
+    gu = gemm.interleave_gate_up(gate.t().unsqueeze(0), up.t().unsqueeze(0))[0].t().contiguous()
+    dgu = torch.empty_like(gu)
+    w2 = torch.zeros(1, H, Fd, device="cuda")
+    w2[:, 0] = -1
+    fp8.grouped_gemm_rows_fp8(x.to(fp8.FP8), torch.ones(cap, 1, device="cuda"), w2.to(fp8.FP8), torch.ones(1, 1, Fd // 128, device="cuda"), None, cap,
+                              b_mn_major=True, epilogue=fp8.EPI_DSWIGLU, gu=gu, dgu=dgu, status=st)
+    dg, du = (t[0].t().double() for t in gemm.deinterleave_gate_up(dgu.t().contiguous().unsqueeze(0)))
+    g = gate.double()                                                   # dAct = 1
+    sg = torch.sigmoid(g)
+    assert (g >= -88.5).all()                                           # what -88.6 rounds to; e^89 is inf
+    for got, want in ((du, g * sg), (dg, 4 * sg * (1 + g * (1 - sg)))):
+        assert ((got - want).abs() <= tol * want.abs()).all()
+    assert st[0].item() == 0
