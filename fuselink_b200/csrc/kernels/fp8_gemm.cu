@@ -308,7 +308,6 @@ fp8_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
             }
           }
         }
-        if (!ok) let_copies_land();
       }
     } else if (warp == 1) {
       if (lane == 0) {
@@ -520,12 +519,15 @@ fp8_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
         }
       }
     }
+    if (!ok) tmem_ld_wait();                      // a chunk may be on its way
     if (EPI == FL_EPI_SCATTER) fence_sys();
   }
 
   tc_fence_before_sync();
   __syncthreads();
   if (warp == 1) {
+    // whoever gave up, copies may be on the way and products running: they end before TMEM and, with this warp, the CTA's shared memory go away
+    if (*abort_flag) let_copies_land();
     tc_fence_after_sync();
     tmem_dealloc(tmem_base, TMEM_COLS);
   }

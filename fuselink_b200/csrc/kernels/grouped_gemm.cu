@@ -435,10 +435,6 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
           }
         }
       }
-      if (!ok) {
-        // give copies that are still in flight time to land before the CTA (and its shared memory) goes away
-        for (int i = 0; i < 2000; ++i) __nanosleep(1000);
-      }
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
@@ -509,6 +505,8 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
   tc_fence_before_sync();
   __syncthreads();
   if (warp == 1) {
+    // whoever gave up, copies may be on the way and products running: they end before TMEM and, with this warp, the CTA's shared memory go away
+    if (*abort_flag) let_copies_land();
     tc_fence_after_sync();
     tmem_dealloc(tmem_base, TMEM_COLS);
   }
@@ -769,9 +767,6 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
           }
         }
       }
-      if (!ok) {
-        for (int i = 0; i < 2000; ++i) __nanosleep(1000);
-      }
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer (leader CTA only)
@@ -873,15 +868,13 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(&sh->tmem_empty[acc]), 0));
     }
-    if (BUFFERED && lane == 0) {
-      if (!ok) let_copies_land();
-      tma_store_wait<0>();
-    }
+    if (BUFFERED && lane == 0) tma_store_wait<0>();
     if (p.epilogue == FL_EPI_SCATTER || p.push_world > 0) fence_sys();
   }
 
   tc_fence_before_sync();
   __syncthreads();
+  if (warp == 1 && *abort_flag) let_copies_land(); // as in the kernel above; the pair's other CTA waits for this one
   cluster_sync_all();                              // neither CTA frees TMEM while the other may still use the pair's
   if (warp == 1) {
     tc_fence_after_sync();
@@ -1002,9 +995,6 @@ grouped_gemm_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
           }
         }
       }
-      if (!ok) {
-        for (int i = 0; i < 2000; ++i) __nanosleep(1000);
-      }
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer (leader CTA only)
@@ -1119,6 +1109,7 @@ grouped_gemm_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
 
   tc_fence_before_sync();
   __syncthreads();
+  if (warp == 1 && *abort_flag) let_copies_land();
   cluster_sync_all();
   if (warp == 1) {
     tc_fence_after_sync();

@@ -90,3 +90,17 @@ def test_a_kernel_that_polls_flags_lets_nobody_start_before_it_has_seen_them():
         if "nobody_polls_from_here" in body:                     # what is polled behind it is a loop over a.nwait flags
             behind = body[body.index("nobody_polls_from_here"):]
             assert all("a.nwait" in line for line in re.findall(r"if \([^;]*wait_flag_ge", behind)) and behind.count("wait_flag_ge") == 1
+
+
+@pytest.mark.parametrize("name,kernel", [("fp8_gemm.cu", "fp8_grouped_gemm_kernel"), ("grouped_gemm.cu", "grouped_gemm_kernel"),
+                                         ("grouped_gemm.cu", "grouped_gemm_pair_kernel"), ("grouped_gemm.cu", "grouped_gemm_wide_kernel")])
+def test_a_grouped_product_that_gave_up_waits_for_its_copies(name, kernel):
+    """As above: behind the CTA's barrier, before TMEM is freed, whichever role gave up and although the loader may have ended before that."""
+    text = re.sub(r"//[^\n]*", "", open(os.path.join(KERNELS, name)).read())
+    start = re.search(rf"\n{kernel}\(const __grid_constant__", text).start()
+    body = text[start:text.index("\n}\n", start)]
+    behind = body[body.rindex("mbar_wait"):]
+    barrier, look, free = (re.search(r, behind) for r in (r"\n  __syncthreads\(\);", r"if \([^{;]*\*abort_flag\) let_copies_land\(\);", r"tmem_dealloc"))
+    assert barrier and look and free and barrier.end() < look.start() < look.end() < free.start()
+    if kernel.startswith("fp8"):                                 # sums are asked for ahead of their use: none is on its way at the end
+        assert re.search(r"if \(!ok\) tmem_ld_wait\(\);", behind[:barrier.start()])
