@@ -487,7 +487,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         prefetch_saved_gate_up(p, t.g, t.m0, t.rows, t.n0, min(BN, p.N - t.n0), q * 32 + lane);
       if (p.epilogue == FL_EPI_WGRAD && p.sgd_lr != 0.f && half == 0)
         prefetch_weights(p, t.g, t.m0, t.n0, min(BN, p.N - t.n0), q * 32 + lane);
-      ok = mbar_wait(&sh->tmem_full[acc], acc_ph, abort_flag, p.status, kTimeoutTmemFull, 400 + acc);
+      ok = mbar_wait_warp(&sh->tmem_full[acc], acc_ph, abort_flag, p.status, kTimeoutTmemFull, 400 + acc);
       if (!ok) break;
       tc_fence_after_sync();
       EpiSlab e;
@@ -856,7 +856,7 @@ grouped_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
       if (p.epilogue == FL_EPI_DSWIGLU && half == 0)
         prefetch_saved_gate_up(p, t.g, t.m0 + 128 * (int)rank, min(128, t.cnt - (t.m0 + 128 * (int)rank)), t.n0, min(BN, p.N - t.n0),
                                q * 32 + lane);
-      ok = mbar_wait(&sh->tmem_full[acc], acc_ph, abort_flag, p.status, kTimeoutTmemFull, 1400 + acc);
+      ok = mbar_wait_warp(&sh->tmem_full[acc], acc_ph, abort_flag, p.status, kTimeoutTmemFull, 1400 + acc);
       if (!ok) break;
       tc_fence_after_sync();
       EpiSlab e;
@@ -1090,7 +1090,7 @@ grouped_gemm_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
       if (p.epilogue == FL_EPI_WGRAD && p.sgd_lr != 0.f && half == 0)
         prefetch_weights(p, t.g, t.m0 + 128 * (int)rank, t.n0, min(WIDE_N, p.N - t.n0), q * 32 + lane);
       for (int h = 0; h < 2 && ok; ++h) {
-        ok = mbar_wait(&sh->half_full[h], ph, abort_flag, p.status, kTimeoutTmemFull, 2400 + h);
+        ok = mbar_wait_warp(&sh->half_full[h], ph, abort_flag, p.status, kTimeoutTmemFull, 2400 + h);
         if (!ok) break;
         tc_fence_after_sync();
         EpiSlab e;

@@ -104,3 +104,13 @@ def test_a_grouped_product_that_gave_up_waits_for_its_copies(name, kernel):
     assert barrier and look and free and barrier.end() < look.start() < look.end() < free.start()
     if kernel.startswith("fp8"):                                 # sums are asked for ahead of their use: none is on its way at the end
         assert re.search(r"if \(!ok\) tmem_ld_wait\(\);", behind[:barrier.start()])
+
+
+@pytest.mark.parametrize("kernel", ["grouped_gemm_kernel", "grouped_gemm_pair_kernel", "grouped_gemm_wide_kernel"])
+def test_an_epilogue_warp_goes_on_together_behind_a_wait(kernel):
+    """Loads from TMEM and the stores through shared memory want the whole warp, also where a wait ran out; single lanes wait by themselves."""
+    text = re.sub(r"//[^\n]*", "", open(os.path.join(KERNELS, "grouped_gemm.cu")).read())
+    start = re.search(rf"\n{kernel}\(const __grid_constant__", text).start()
+    body = text[start:text.index("\n}\n", start)]
+    epilogue = body[body.index("half = (warp - 2) >> 2"):]
+    assert "mbar_wait_warp(" in epilogue and "mbar_wait(" not in epilogue
