@@ -206,3 +206,43 @@ def test_decode_stage_follows_its_parameters_after_the_capture(input_len, steps)
 def test_kv_pack_send_through_the_copy_engine(H, S, D, layout, more):
     least = -(-(16 << 20) // (2 * 3 * H * S * D * 2))               # requests of three pages, keys and values
     test_kv_pack_send_over_page_shapes(H, S, D, layout, least + more)
+
+
+@pytest.mark.parametrize("layout", [0, 1])
+@pytest.mark.parametrize("ctas", [3, 0])
+@pytest.mark.parametrize("hdr_bytes,shift", [(8192 + 8, 0), (8192, 8), (8, 0)])     # whole vectors and a rest; not at 16 bytes; less than a vector
+def test_kv_hand_off_through_the_copy_engine(layout, ctas, hdr_bytes, shift):
+    """What test_kv_pack_send_matches_page_gather checks and ids outside their pools, above 16 MiB: two launches on one counter with header
+    and flag, by a few CTAs (many units each) and by all; only the valid pages move, the others are reported."""
+    from fuselink_b200 import C
+    L, H, S, D, B, maxb = 4, 8, 16, 128, 40, 5                           # a unit is a page of 32 KiB; two layers hold 25 MiB
+    n = B * maxb
+    g = torch.Generator().manual_seed(ctas)
+    src = [torch.randint(-32768, 32768, (n, L, H, S, D), generator=g, dtype=torch.int16).cuda().view(torch.bfloat16) for _ in range(2)]
+    shape = (n, L, H, S, D) if layout == 0 else (L, n, S, H, D)
+    dst = [torch.full(shape, -7.0, dtype=torch.bfloat16, device="cuda") for _ in range(2)]
+    nb = torch.randint(0, maxb + 1, (B,), generator=g).int()
+    nb[0], nb[7], nb[B - 1] = maxb, 0, maxb
+    sbt, dbt = (torch.randperm(n, generator=g).view(B, maxb).int() for _ in range(2))
+    valid = torch.arange(maxb).unsqueeze(0) < nb.unsqueeze(1)
+    for table, b, j, bad in ((sbt, 0, 1, n), (sbt, B - 1, 4, -1), (dbt, 0, 0, n + 5), (dbt, B - 1, 2, -2 ** 31), (dbt, 0, 4, 2 ** 31 - 1)):
+        table[b, j] = bad
+        valid[b, j] = False
+    status, counter, flag = torch.zeros(8, dtype=torch.int32, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda"), torch.zeros(4, dtype=torch.int32, device="cuda")
+    hdr = torch.randint(0, 256, (hdr_bytes + shift,), generator=g, dtype=torch.uint8).cuda()[shift:]
+    hdr_dst = torch.zeros(hdr_bytes + 32, dtype=torch.uint8, device="cuda")
+    tables = sbt.cuda(), dbt.cuda(), nb.cuda()
+    for l0, l1, seq in [(0, 2, 1), (2, 4, 2)]:
+        C.kv_pack_send(src[0], src[1], dst[0].data_ptr(), dst[1].data_ptr(), 0, layout, n, n, L, H, S, D, l0, l1, *tables,
+                       hdr if seq == 2 else None, hdr_dst.data_ptr() if seq == 2 else 0, flag.data_ptr(), seq, counter, ctas, status.data_ptr())
+        assert flag[0].item() == seq and counter.item() == 0
+    assert status[0].item() == 6                                         # kBadIndex: recorded, access skipped
+    assert torch.equal(hdr_dst[:hdr_bytes], hdr) and (hdr_dst[hdr_bytes:] == 0).all() and (flag[1:] == 0).all()
+    si, di = sbt[valid].long().cuda(), dbt[valid].long().cuda()
+    for s, d in zip(src, dst):
+        want = torch.full_like(d, -7.0)
+        if layout == 0:
+            want[di] = s[si]
+        else:
+            want[:, di] = s[si].permute(1, 0, 3, 2, 4)
+        assert torch.equal(d.view(torch.int16), want.view(torch.int16))
