@@ -53,18 +53,24 @@ __device__ __forceinline__ uint4 shifted(const uint4& a, const uint4& b, unsigne
                     __funnelshift_r(w[3], w[4], bits));
 }
 
+// Only vectors that lie inside [src, src + bytes) are read, the second of the last pair too.
+__host__ __device__ __forceinline__ FlPutShifted put_shifted(unsigned long long src, unsigned long long dst, unsigned long long bytes) {
+  FlPutShifted p = {((16 - (dst & 15)) & 15) + 16, 0, 0};                      // 16 more: then src + head - shift is not before src
+  p.shift = (unsigned)((src + p.head) & 15);
+  const long long body = (long long)bytes - (long long)p.head - 16 + (long long)p.shift;   // bytes of src up to the last vector that may be a second one
+  if (body >= 16) p.vectors = (unsigned long long)body >> 4;
+  return p;
+}
+
 // src and dst at different distances from a multiple of 16, by all threads of the CTA: whole vectors of dst from two neighbouring
-// vectors of src each (the second of them is in L1).  Only vectors that lie inside [src, src + bytes) are read; the ends go byte by
-// byte.  Byte by byte throughout, an exchange of blocks of an odd number of elements took 33 times as long as one of a multiple of eight
-// (8 ranks, 8 x 2.6 MB each: 4358 us against 125; now 138).
+// vectors of src each (the second of them is in L1).  Byte by byte throughout, an exchange of blocks of an odd number of elements took 33
+// times as long as one of a multiple of eight (8 ranks, 8 x 2.6 MB each: 4358 us against 125; now 138).
 __device__ __forceinline__ void copy_shifted(const uint8_t* src, uint8_t* dst, unsigned long long bytes) {
   constexpr int U = 4;
-  const unsigned long long to16 = (16 - (reinterpret_cast<uintptr_t>(dst) & 15)) & 15;
-  const unsigned long long head = to16 + 16;                                    // then src + head - sh is not before src
-  const unsigned sh = (unsigned)(reinterpret_cast<uintptr_t>(src + head) & 15);
-  const long long body = (long long)bytes - (long long)head - 16 + (long long)sh;   // bytes of src up to the last vector that may be a second one
-  if (body < 16) { copy_bytes(src, dst, bytes); return; }
-  const unsigned long long n = (unsigned long long)body >> 4;
+  const FlPutShifted span = put_shifted(reinterpret_cast<uintptr_t>(src), reinterpret_cast<uintptr_t>(dst), bytes);
+  const unsigned long long head = span.head, n = span.vectors;
+  const unsigned sh = span.shift;
+  if (n == 0) { copy_bytes(src, dst, bytes); return; }
   const uint8_t* s = src + head - sh;
   uint8_t* d = dst + head;
   const unsigned tid = threadIdx.x, nt = blockDim.x;
@@ -298,6 +304,19 @@ static unsigned long long even_split(const FlPutArgs* a, unsigned G) {
     u0 += n;
   }
   return U;
+}
+
+extern "C" unsigned long long fl_put_even_slots(const FlPutArgs* args, unsigned int num_ctas) {
+  if (args->nseg < 1 || args->nseg > FL_MAX_SEGS || args->chunk_bytes == 0 || num_ctas == 0) return 0;
+  return even_split(args, num_ctas);
+}
+extern "C" unsigned int fl_put_slot_owner(unsigned long long slot, unsigned long long slots, unsigned int num_ctas) {
+  return fl::put_owner(slot, slots, num_ctas);
+}
+extern "C" int fl_put_shifted(unsigned long long src, unsigned long long dst, unsigned long long bytes, FlPutShifted* out) {
+  if (((src ^ dst) & 15) == 0) return -1;
+  *out = fl::put_shifted(src, dst, bytes);
+  return 0;
 }
 
 extern "C" int fl_put_chunks(const FlPutArgs* args, int num_ctas, int threads, cudaStream_t stream) {

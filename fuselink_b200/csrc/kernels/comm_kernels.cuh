@@ -16,7 +16,8 @@
 enum FlFlagMode : int {
   FL_FLAG_NONE = 0,
   FL_FLAG_SEQ_PER_CHUNK = 1,  // flags[chunk] = seq          (relay staging: one word per chunk)
-  FL_FLAG_COUNT = 2,          // flags[0]   += 1 per chunk   (final destination: arrival counter)
+  FL_FLAG_COUNT = 2,          // flags[0]   += the number of chunks in all (final destination: arrival counter).  The total says that
+                              //              everything is there; a smaller count does not say how much is
 };
 
 struct FlSeg {
@@ -44,9 +45,17 @@ struct FlPutArgs {
   int nwait;
   // optional, with bytes_done: FL_MAX_SEGS + 1 zeroed 64-bit words of DEVICE memory owned by the caller's channel.  The
   // CTAs add up their finished bytes there and the last CTA of the launch forwards one total per segment to bytes_done, so
-  // a launch costs one host-memory atomic per segment instead of one per chunk (each takes about a microsecond over PCIe
-  // and they serialise).  Launches that share the words must be stream-ordered.  Null: one host atomic per chunk.
+  // a launch costs one host-memory atomic per segment instead of one per chunk or per CTA (each takes about a microsecond over
+  // PCIe and they serialise).  Launches that share the words must be stream-ordered.  Null: one host atomic per chunk, or, where the
+  // launch is split evenly, per CTA that has a part of the segment.
   unsigned long long* done_scratch;
+};
+
+// Bytes [head, head + 16 vectors) of the destination are whole vectors; vector i comes from the two of the source that begin at
+// head - shift + 16 i and 16 bytes further.  The rest goes byte by byte.
+struct FlPutShifted {
+  unsigned long long head, vectors;
+  unsigned int shift;
 };
 
 struct FlWaitArgs {
@@ -65,6 +74,11 @@ struct FlSignalPtrs {
 extern "C" {
 #endif
 int fl_put_chunks(const FlPutArgs* args, int num_ctas, int threads, cudaStream_t stream);
+// What fl_put_chunks goes by, for its tests.  The 16 KiB slots over which num_ctas CTAs split the launch evenly, 0 where they take chunks in
+// turn; the CTA to which a slot falls; what a copy between addresses that differ modulo 16 moves as vectors.
+unsigned long long fl_put_even_slots(const FlPutArgs* args, unsigned int num_ctas);
+unsigned int fl_put_slot_owner(unsigned long long slot, unsigned long long slots, unsigned int num_ctas);
+int fl_put_shifted(unsigned long long src, unsigned long long dst, unsigned long long bytes, FlPutShifted* out);
 int fl_wait_flags(const FlWaitArgs* args, cudaStream_t stream);
 // Uniform all-to-all in one launch: block p of `send` ([world, bytes_per_peer]) goes to recv_peers[p] + rank *
 // bytes_per_peer; arrival counters live at pads.p[dst][slot0 + src]; with want != NULL the launch also waits
