@@ -275,9 +275,10 @@ __global__ void __launch_bounds__(256) dec_qkv_kernel(T* qkv, const T* bias, con
 
 // ---- activation -----------------------------------------------------------------------------------------------------------
 // Bound by memory, where its arithmetic lets it be: an exponential and an IEEE division per element took 573 us for 32768 x 14336 in
-// bf16 (2.8 GB, 436 us at the rate of a copy), with the hardware's 443.  Their error, some 2^-21, does not show behind the rounding to
-// bf16 (against 64 bits 2.4132767e-3 either way); behind that to fp16 it does in the eighth digit, so fp16 keeps the others.  Both sides of
-// the quotient are a sixteenth: __fdividef gives 0 for divisors beyond 2^126, which 1 + e^-x is below x = -87.3.
+// bf16 (2.8 GB, 436 us at the rate of a copy), with the hardware's 443.  The result is rounded to bf16 before it is used, and of every
+// bf16 gate that gives the bits of expf and an IEEE division, though __expf's error grows to some 2^-17 at |x| = 87.  fp16 has three bits
+// more, behind which it shows, so fp16 keeps the others.  Both sides of the quotient are a sixteenth: __fdividef gives 0 for divisors
+// beyond 2^126, which 1 + e^-x is below x = -87.3.
 template <typename T>
 __device__ __forceinline__ float silu_of(float x) {
   if constexpr (std::is_same_v<T, __nv_bfloat16>) return __fdividef(0.0625f * x, fmaf(__expf(-x), 0.0625f, 0.0625f));

@@ -181,6 +181,18 @@ def test_silu_of_every_value(dt):
     assert ((out.double() - want)[fin].abs() <= 1.01 * eps * want[fin].abs() + (4e-37 if dt == torch.bfloat16 else 6e-8)).all()
 
 
+def test_silu_of_bf16_gates_is_that_of_full_precision():
+    """The hardware's exponential and quotient stand before a rounding to bf16: of every gate the bits that expf and an IEEE division give,
+    which are also the decoding products' (thin_gemm.cu)."""
+    from fuselink_b200 import C
+    x = torch.arange(-32768, 32768, device="cuda").to(torch.int16).view(torch.bfloat16).view(512, 128)
+    out = torch.empty_like(x)
+    C.dec_act(torch.cat([x, torch.ones_like(x)], 1), None, out, 0)
+    want = (x.float() / (1 + torch.exp(-x.float()))).to(torch.bfloat16)
+    assert torch.equal(out.isnan(), want.isnan())
+    assert torch.equal(out.view(torch.int16)[~out.isnan()], want.view(torch.int16)[~out.isnan()])
+
+
 def _shard(model):
     from fuselink_b200.models.llama import MODEL_ZOO, LlamaShard
     net = LlamaShard(MODEL_ZOO[model], device="cuda", seed=2)
