@@ -115,7 +115,7 @@ def test_no_result_depends_on_the_expected_rows(counts_l, max_ctas):
 
 @pytest.mark.parametrize("M,N", [(8, 32), (40, 96), (264, 288), (512, 544), (1000, 64), (256, 1056)])
 @pytest.mark.parametrize("rows", [[3, 0, 190], [64, 65, 384]])
-@pytest.mark.parametrize("lr", [0.0, 0.25])
+@pytest.mark.parametrize("lr", [0.0, 0.25, 0.01])                       # 0.01: a product that is not exact, so that one rounding more or less shows
 def test_weight_gradients_through_the_pair_kernel(M, N, rows, lr):
     """Bit by bit what one CTA per tile stores from registers: matrices that end inside a block of 32 rows x 64 columns or inside a tile, an
     expert without rows, a contraction that ends inside a k-block, several tiles per pair, and nothing written behind the matrices."""
