@@ -51,6 +51,15 @@ struct FlPutArgs {
   unsigned long long* done_scratch;
 };
 
+// An even split: CTA b of G has the slots (of 16 KiB, those of one segment behind those of the one before) [slots b / G, slots (b + 1) / G).
+// The CTAs that have a part of a segment, at most as many as it has chunks, add to its arrival counter when they are done.
+struct FlPutSplit {
+  unsigned int slots;                     // of all segments; 0: not even, the CTAs take chunks in turn
+  unsigned int slot_end[FL_MAX_SEGS];     // running totals
+  unsigned int first_cta[FL_MAX_SEGS];    // the CTA that has the segment's first slot ...
+  unsigned int first_adds[FL_MAX_SEGS];   // ... and what it adds; the others add 1
+};
+
 // Bytes [head, head + 16 vectors) of the destination are whole vectors; vector i comes from the two of the source that begin at
 // head - shift + 16 i and 16 bytes further.  The rest goes byte by byte.
 struct FlPutShifted {
@@ -74,10 +83,9 @@ struct FlSignalPtrs {
 extern "C" {
 #endif
 int fl_put_chunks(const FlPutArgs* args, int num_ctas, int threads, cudaStream_t stream);
-// What fl_put_chunks goes by, for its tests.  The 16 KiB slots over which num_ctas CTAs split the launch evenly, 0 where they take chunks in
-// turn; the CTA to which a slot falls; what a copy between addresses that differ modulo 16 moves as vectors.
-unsigned long long fl_put_even_slots(const FlPutArgs* args, unsigned int num_ctas);
-unsigned int fl_put_slot_owner(unsigned long long slot, unsigned long long slots, unsigned int num_ctas);
+// What fl_put_chunks goes by, for its tests: the split of a launch over num_ctas CTAs, and what a copy between addresses that differ
+// modulo 16 moves as vectors.
+int fl_put_split(const FlPutArgs* args, unsigned int num_ctas, FlPutSplit* out);
 int fl_put_shifted(unsigned long long src, unsigned long long dst, unsigned long long bytes, FlPutShifted* out);
 int fl_wait_flags(const FlWaitArgs* args, cudaStream_t stream);
 // Uniform all-to-all in one launch: block p of `send` ([world, bytes_per_peer]) goes to recv_peers[p] + rank *

@@ -22,6 +22,10 @@ class Put(ct.Structure):                  # FlPutArgs
                 ("done_scratch", ct.c_void_p)]
 
 
+class Split(ct.Structure):                # FlPutSplit
+    _fields_ = [("slots", ct.c_uint), ("slot_end", ct.c_uint * MAX_SEGS), ("first_cta", ct.c_uint * MAX_SEGS), ("first_adds", ct.c_uint * MAX_SEGS)]
+
+
 class Shifted(ct.Structure):              # FlPutShifted
     _fields_ = [("head", ct.c_ulonglong), ("vectors", ct.c_ulonglong), ("shift", ct.c_uint)]
 
@@ -31,19 +35,17 @@ def lib():
     if not os.path.exists(LIB):
         pytest.skip("libfuselink.so not built")
     lib = ct.CDLL(LIB)
-    lib.fl_put_even_slots.restype = ct.c_ulonglong
-    lib.fl_put_even_slots.argtypes = [ct.POINTER(Put), ct.c_uint]
-    lib.fl_put_slot_owner.restype = ct.c_uint
-    lib.fl_put_slot_owner.argtypes = [ct.c_ulonglong, ct.c_ulonglong, ct.c_uint]
+    lib.fl_put_split.argtypes = [ct.POINTER(Put), ct.c_uint, ct.POINTER(Split)]
     lib.fl_put_shifted.argtypes = [ct.c_ulonglong] * 3 + [ct.POINTER(Shifted)]
     return lib
 
 
-def even_slots(lib, sizes, chunk, G, mode=FLAG_COUNT, wait=None):
-    put = Put(nseg=len(sizes), chunk_bytes=chunk, use_bulk=1)
+def split(lib, sizes, chunk, G, mode=FLAG_COUNT, wait=None):
+    out, put = Split(), Put(nseg=len(sizes), chunk_bytes=chunk, use_bulk=1)
     for s, b in zip(put.seg, sizes):
         s.bytes, s.flag_mode, s.wait_flags = b, mode, wait
-    return lib.fl_put_even_slots(ct.byref(put), G)
+    assert lib.fl_put_split(ct.byref(put), G, ct.byref(out)) == 0
+    return out
 
 
 @pytest.mark.parametrize("seed", range(40))
@@ -56,11 +58,13 @@ def test_arrivals_of_an_even_split(lib, seed):
         sizes = [rng.randint(0, most) if rng.random() < 0.8 else 16 * rng.randint(0, 100) for _ in range(rng.randint(1, 8))]
         chunks = [-(-b // chunk) for b in sizes]
         G = min(max(sum(chunks), 1), 296)
-        U = even_slots(lib, sizes, chunk, G)
+        sp = split(lib, sizes, chunk, G)
+        U = sp.slots
     assert U == sum(-(-b // SLOT) for b in sizes) >= G
     u0 = 0
-    for b, n_chunks in zip(sizes, chunks):
+    for i, (b, n_chunks) in enumerate(zip(sizes, chunks)):
         n = -(-b // SLOT)
+        assert sp.slot_end[i] == u0 + n
         if n == 0:
             continue
         took = []                         # (CTA, first slot, last slot)
@@ -69,9 +73,8 @@ def test_arrivals_of_an_even_split(lib, seed):
             if lo < hi:
                 took.append((c, lo, hi))
         assert [t[1] for t in took[1:]] == [t[2] for t in took[:-1]] and took[0][1] == u0 and took[-1][2] == u0 + n
-        first, last = lib.fl_put_slot_owner(u0, U, G), lib.fl_put_slot_owner(u0 + n - 1, U, G)
-        assert [t[0] for t in took] == list(range(first, last + 1))
-        adds = [n_chunks - (last - first) if c == first else 1 for c, _, _ in took]
+        assert [t[0] for t in took] == list(range(took[0][0], took[-1][0] + 1)) and took[0][0] == sp.first_cta[i]
+        adds = [sp.first_adds[i] if c == sp.first_cta[i] else 1 for c, _, _ in took]
         assert sum(adds) == n_chunks and min(adds) >= 1         # none finishes without adding: n_chunks is reached by the last
         u0 += n
 
@@ -81,8 +84,15 @@ def test_common_launches_are_split_evenly(lib):
     for sizes in ([64 << 10], [16 << 20], [1 << 30], [2621440] * 8, [8 << 20] * 4):
         chunk, n = chunking(sizes[0])
         G = min(n * len(sizes), 296)
-        assert even_slots(lib, sizes, chunk, G) > 0
-        assert even_slots(lib, sizes, chunk, G, FLAG_SEQ_PER_CHUNK) == 0 and even_slots(lib, sizes, chunk, G, wait=16) == 0
+        assert split(lib, sizes, chunk, G).slots > 0
+        assert split(lib, sizes, chunk, G, FLAG_SEQ_PER_CHUNK).slots == 0 and split(lib, sizes, chunk, G, wait=16).slots == 0
+
+
+def test_what_the_kernel_multiplies_fits_32_bits(lib):
+    for G in (1, 37, 296):
+        most = (2 ** 32 - 1) // G
+        assert split(lib, [most * SLOT], 1 << 30, G).slots == (most if most * SLOT >> 30 >= G - 1 else 0)
+        assert split(lib, [most * SLOT + 1], 1 << 30, G).slots == 0
 
 
 @pytest.mark.parametrize("sh", range(1, 16))
