@@ -14,9 +14,9 @@ namespace fl {
 // Bound by memory (or the link): every byte is read once and written once, and small launches by their start and end.  One thread per
 // CTA streams through a ring of 16 KiB slots in shared memory with the bulk-copy engine.  A launch is split evenly, in slots, over two
 // CTAs per SM, which drain their ring once per segment; dealt out in chunks, each drained before the next was asked for, 320 chunks
-// left some SMs with three and some with two.  The next kernel may be placed when every CTA is done copying.  8 exchanges of 8 x 2.6 MB
-// in a row 125 -> 102 us, 4 of 4 x 8.4 MB 78 -> 64, 2 of 2 x 67 MB 107 -> 100; a put of 16 MiB 10.4 -> 8.6, 64 MiB 24.6 -> 23.3, 256 MiB 100 -> 94.
-// One CTA per SM with 12 slots: 129, 64, 101, 7.9, 23.2, 94; three with 4: 113, 69, 101, 9.3, 23.0, 94.
+// left some SMs with three and some with two.  In chunks | evenly, us: 8 exchanges of 8 x 2.6 MB in a row 137 | 117, of 8 x 131 KB 91 | 70, 4 of
+// 4 x 8.4 MB 86 | 75, 2 of 2 x 67 MB 111 | 107; a put and its wait of 64 KiB 8.3 | 6.4, 4 MiB 9.7 | 9.4, 16 MiB 12.9 | 13.3, 64 MiB 27.7 | 27.9, 256 MiB
+// 102 | 98.  One CTA per SM with 12 slots: 131, 70, 72, 105; 6.4, 9.4, 10.9, 26, 96; three with 4: 131, 71, 79, 108; 6.4, 9.4, 13.2, 27.4, 99.
 constexpr int BULK_SLOT_BYTES = 16 * 1024;
 constexpr int BULK_MAX_SLOTS = 6;
 
@@ -64,7 +64,7 @@ __host__ __device__ __forceinline__ FlPutShifted put_shifted(unsigned long long 
 
 // src and dst at different distances from a multiple of 16, by all threads of the CTA: whole vectors of dst from two neighbouring
 // vectors of src each (the second of them is in L1).  Byte by byte throughout, an exchange of blocks of an odd number of elements took 33
-// times as long as one of a multiple of eight (8 ranks, 8 x 2.6 MB each: 4358 us against 125; now 138).
+// times as long as one of a multiple of eight (8 ranks, 8 x 2.6 MB each: 4427 us against 137; now 134 against 117).
 __device__ __forceinline__ void copy_shifted(const uint8_t* src, uint8_t* dst, unsigned long long bytes) {
   constexpr int U = 4;
   const FlPutShifted span = put_shifted(reinterpret_cast<uintptr_t>(src), reinterpret_cast<uintptr_t>(dst), bytes);
@@ -257,7 +257,7 @@ __global__ void barrier_kernel(FlSignalPtrs pads, int slot0, int rank, int world
 
 }  // namespace fl
 
-// Small puts, waits and barriers, often several in a row, are launched so that they may be placed while the kernel before
+// Small puts of one segment, waits and barriers, often several in a row, are launched so that they may be placed while the kernel before
 // them drains; they touch nothing, and poll no flag, before that kernel has ended (grid_dep_wait), so what one polls for is never behind it.
 template <typename... P, typename... A>
 static int launch_after(void (*kernel)(P...), unsigned grid, unsigned threads, size_t smem, cudaStream_t stream, const A&... args) {
@@ -275,42 +275,41 @@ static int launch_after(void (*kernel)(P...), unsigned grid, unsigned threads, s
 }
 
 constexpr unsigned PUT_CTAS = 2 * 148;
-// Up to so many CTAs a put is launched early.  With its wait, one of 4 KiB takes 7.4 us launched plainly and 5.8 us early, 64 KiB 8.3 and
-// 6.9, 1 MiB 10.2 and 9.6; with more CTAs it is the other way round on most GPUs: 16 MiB 13.9 and 14.4, eight exchanges of 1 MB 95.6 and
-// 98.4, of 21 MB 128 and 139 (but 125 and 103 on other GPUs of the same model).  So few CTAs also leave room for other streams while they wait their turn.
+// Up to so many CTAs a put is launched early, an exchange (several segments) never.  Plainly | early, us: a put and its wait of 4 KiB 6.3 | 5.2,
+// 64 KiB 7.6 | 6.4, 512 KiB (8 CTAs) 9.0 | 8.8, 1 MiB (16) 8.8 | 8.8, 2 MiB (32) 9.5 | 8.9, 8 MiB (128) 9.5 | 9.1, 16 MiB (256) 13.5 | 13.9; beyond 32 the
+// half microsecond is not worth the room that CTAs take from other streams while they wait their turn.  Eight exchanges of 0.5 MB (8 CTAs)
+// 69.8 | 74, of 1 MB (16) 69.5 | 75, of 2 MB (32) 71 | 75, of 4 MB (64) 74 | 74.6, of 21 MB (256) 117 | 140 (on other GPUs of the same model 125 | 103).
 constexpr int PUT_EARLY_CTAS = 32;
 
 // The even split of the launch over its G CTAs, where nothing is waited for or flagged chunk by chunk, and no segment is shared by more CTAs
 // than it has chunks to count.  Made here, since the kernel's 64-bit divisions stood before its first load: eight exchanges of 1 MB 94 us with
 // them, 77 without, of 21 MB 127 and 117, a put of 4 MiB 9.3 and 8.2.  What the kernel multiplies fits 32 bits (up to 237 GB on 296 CTAs).
-static FlPutSplit even_split(const FlPutArgs* a, unsigned G) {
-  const FlPutSplit none = {};
-  FlPutSplit sp = {};
+static void even_split(const FlPutArgs* a, unsigned G, FlPutSplit* sp) {
+  sp->slots = 0;
   unsigned long long U = 0;
   for (int i = 0; i < a->nseg; ++i) {
-    if (a->seg[i].wait_flags != nullptr || a->seg[i].flag_mode == FL_FLAG_SEQ_PER_CHUNK) return none;
+    if (a->seg[i].wait_flags != nullptr || a->seg[i].flag_mode == FL_FLAG_SEQ_PER_CHUNK) return;
     U += (a->seg[i].bytes + fl::BULK_SLOT_BYTES - 1) / fl::BULK_SLOT_BYTES;
-    if (U > 0xffffffffull / G) return none;
-    sp.slot_end[i] = (unsigned)U;
+    if (U * G > 0xffffffffull) return;
+    sp->slot_end[i] = (unsigned)U;
   }
-  if (U < G) return none;
+  if (U < G) return;
+  const unsigned slots = (unsigned)U;
   for (int i = 0; i < a->nseg; ++i) {
-    const unsigned s0 = i == 0 ? 0 : sp.slot_end[i - 1], s1 = sp.slot_end[i];
+    const unsigned s0 = i == 0 ? 0 : sp->slot_end[i - 1], s1 = sp->slot_end[i];
     if (s0 == s1) continue;
     const unsigned long long chunks = (a->seg[i].bytes + a->chunk_bytes - 1) / a->chunk_bytes;
-    auto owner = [&](unsigned s) { return (unsigned)(((s + 1ull) * G - 1) / U); };
-    const unsigned first = owner(s0), others = owner(s1 - 1) - first;
-    if (a->seg[i].flag_mode == FL_FLAG_COUNT && others + 1ull > chunks) return none;
-    sp.first_cta[i] = first;
-    sp.first_adds[i] = (unsigned)(chunks - others);
+    const unsigned first = s0 == 0 ? 0 : ((s0 + 1) * G - 1) / slots, others = (s1 == slots ? G - 1 : (s1 * G - 1) / slots) - first;
+    if (a->seg[i].flag_mode == FL_FLAG_COUNT && others >= chunks) return;
+    sp->first_cta[i] = first;
+    sp->first_adds[i] = (unsigned)(chunks - others);
   }
-  sp.slots = (unsigned)U;
-  return sp;
+  sp->slots = slots;
 }
 
 extern "C" int fl_put_split(const FlPutArgs* args, unsigned int num_ctas, FlPutSplit* out) {
   if (args->nseg < 1 || args->nseg > FL_MAX_SEGS || args->chunk_bytes == 0 || num_ctas == 0) return -1;
-  *out = even_split(args, num_ctas);
+  even_split(args, num_ctas, out);
   return 0;
 }
 extern "C" int fl_put_shifted(unsigned long long src, unsigned long long dst, unsigned long long bytes, FlPutShifted* out) {
@@ -325,13 +324,13 @@ extern "C" int fl_put_chunks(const FlPutArgs* args, int num_ctas, int threads, c
   if (threads <= 0 || threads > 1024) threads = 512;
   if (num_ctas <= 0) num_ctas = 1;
   int slots = 0;
-  FlPutSplit even = {};
+  FlPutSplit even;
   if (args->use_bulk) {
     // as many slots as a CTA will fill; threads beyond the one that feeds the engine only where bytes have to be shifted
     for (int i = 0; i < args->nseg; ++i)
       if (((uintptr_t)args->seg[i].src ^ (uintptr_t)args->seg[i].dst) & 15) threads = 512;
     const unsigned G = (unsigned)num_ctas < PUT_CTAS ? (unsigned)num_ctas : PUT_CTAS;
-    even = even_split(args, G);
+    even_split(args, G, &even);
     unsigned long long per_cta = (args->chunk_bytes + fl::BULK_SLOT_BYTES - 1) / fl::BULK_SLOT_BYTES;
     slots = 4;
     if (even.slots != 0) {
@@ -341,7 +340,7 @@ extern "C" int fl_put_chunks(const FlPutArgs* args, int num_ctas, int threads, c
     }
     if (per_cta + 1 < (unsigned long long)slots) slots = (int)per_cta + 1;
   } else {
-    even = even_split(args, (unsigned)num_ctas);
+    even_split(args, (unsigned)num_ctas, &even);
   }
   const size_t smem = (size_t)slots * fl::BULK_SLOT_BYTES;
   if (smem > 0) {                           // three slots are 48 KiB, which with the kernel's own few words is more than a launch gets unasked
@@ -351,13 +350,13 @@ extern "C" int fl_put_chunks(const FlPutArgs* args, int num_ctas, int threads, c
     if (dev < 0 || dev >= 64) return -3;
     if (!set_on[dev]) {
       cudaError_t e = cudaFuncSetAttribute(fl::put_chunks_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, fl::BULK_MAX_SLOTS * fl::BULK_SLOT_BYTES);
-      // without it an SM is set up for one of these CTAs at a time (eight exchanges launched early 148 us, with it 108)
+      // two CTAs per SM are what the split counts on; left to the driver it is the same where launches follow one another (117 us either way)
       if (e == cudaSuccess) e = cudaFuncSetAttribute(fl::put_chunks_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
       if (e != cudaSuccess) return (int)e;
       set_on[dev] = true;
     }
   }
-  if (num_ctas > PUT_EARLY_CTAS) {
+  if (num_ctas > PUT_EARLY_CTAS || args->nseg > 1) {
     fl::put_chunks_kernel<<<num_ctas, threads, smem, stream>>>(*args, even, slots);
     return (int)cudaGetLastError();
   }
