@@ -126,7 +126,35 @@ __device__ __forceinline__ bool copy_bulk(const uint8_t* src, uint8_t* dst, unsi
   return ok;
 }
 
-__global__ void __launch_bounds__(1024) put_chunks_kernel(const __grid_constant__ FlPutArgs a, const __grid_constant__ FlPutSplit even, const int slots) {
+// What the kernel is launched with: FlPutArgs and FlPutSplit in the room of the former.  The host's time per launch moves with the size, us
+// of a put of 64 KiB: 688 bytes (both structures as they are) 4.45, 640 and 624 4.35, 608 and 600 4.0, 592 4.27; hence the last field.
+struct PutSeg {
+  const uint8_t* src;
+  uint8_t* dst;
+  unsigned long long bytes;
+  uint32_t* flags;
+  union {
+    const uint32_t* wait_flags;                            // chunks in turn
+    struct { unsigned first_cta, first_adds; };            // evenly
+  };
+  unsigned long long* bytes_done;
+  int flag_mode;
+  unsigned slot_end;
+};
+struct PutLaunch {
+  PutSeg seg[FL_MAX_SEGS];
+  int nseg, use_bulk, slots;                               // slots: of a CTA's ring
+  unsigned chunk_bytes, seq, even_slots;
+  int* status;
+  const uint32_t* wait_flag[8];
+  unsigned wait_want[8];
+  int nwait;
+  unsigned long long* done_scratch;
+  unsigned long long unused;
+};
+static_assert(sizeof(PutLaunch) == 600, "see above");
+
+__global__ void __launch_bounds__(1024) put_chunks_kernel(const __grid_constant__ PutLaunch a) {
   extern __shared__ __align__(128) uint8_t dyn_smem[];
   __shared__ uint64_t bars[BULK_MAX_SLOTS];
   __shared__ int abort_flag;
@@ -135,7 +163,7 @@ __global__ void __launch_bounds__(1024) put_chunks_kernel(const __grid_constant_
   if (threadIdx.x == 0) {
     abort_flag = 0;
     if (a.use_bulk) {
-      for (int s = 0; s < slots; ++s) mbar_init(&bars[s], 1);
+      for (int s = 0; s < a.slots; ++s) mbar_init(&bars[s], 1);
       mbar_fence_init();
     }
   }
@@ -151,7 +179,7 @@ __global__ void __launch_bounds__(1024) put_chunks_kernel(const __grid_constant_
     } else {
       const unsigned long long to16 = (16 - (reinterpret_cast<uintptr_t>(d) & 15)) & 15, head = to16 < len ? to16 : len, body = (len - head) & ~15ull;
       if (threadIdx.x == 0 && body != 0) {
-        if (!copy_bulk(s + head, d + head, body, dyn_smem, slots, bars, phase_bits, &abort_flag, a.status)) abort_flag = 1;
+        if (!copy_bulk(s + head, d + head, body, dyn_smem, a.slots, bars, phase_bits, &abort_flag, a.status)) abort_flag = 1;
         fence_proxy_async_all();
       }
       copy_bytes(s, d, head);
@@ -163,19 +191,19 @@ __global__ void __launch_bounds__(1024) put_chunks_kernel(const __grid_constant_
   // The flag update is itself a release at system scope: it orders this thread's bulk stores (complete, see
   // copy_bulk) and, through the barrier above, the other threads' stores before the flag becomes visible.
   bool live = true;
-  if (even.slots != 0) {
+  if (a.even_slots != 0) {
     // a contiguous piece per CTA, whatever the chunks
-    const unsigned mine0 = even.slots * blockIdx.x / gridDim.x, mine1 = even.slots * (blockIdx.x + 1) / gridDim.x;
+    const unsigned mine0 = a.even_slots * blockIdx.x / gridDim.x, mine1 = a.even_slots * (blockIdx.x + 1) / gridDim.x;
     for (int si = 0; si < a.nseg && live; ++si) {
-      const FlSeg& sg = a.seg[si];
-      const unsigned s0 = si == 0 ? 0 : even.slot_end[si - 1], s1 = even.slot_end[si];
+      const PutSeg& sg = a.seg[si];
+      const unsigned s0 = si == 0 ? 0 : a.seg[si - 1].slot_end, s1 = sg.slot_end;
       const unsigned from = mine0 > s0 ? mine0 : s0, to = mine1 < s1 ? mine1 : s1;
       if (from >= to) continue;
       const unsigned long long off = (unsigned long long)(from - s0) * BULK_SLOT_BYTES, end = (unsigned long long)(to - s0) * BULK_SLOT_BYTES;
       const unsigned long long len = (end < sg.bytes ? end : sg.bytes) - off;
-      live = copy(reinterpret_cast<const uint8_t*>(sg.src) + off, reinterpret_cast<uint8_t*>(sg.dst) + off, len);
+      live = copy(sg.src + off, sg.dst + off, len);
       if (live && threadIdx.x == 0) {
-        if (sg.flag_mode == FL_FLAG_COUNT) red_release_sys_add(sg.flags, blockIdx.x == even.first_cta[si] ? even.first_adds[si] : 1u);
+        if (sg.flag_mode == FL_FLAG_COUNT) red_release_sys_add(sg.flags, blockIdx.x == sg.first_cta ? sg.first_adds : 1u);
         if (sg.bytes_done != nullptr) {
           if (a.done_scratch != nullptr) atomicAdd(a.done_scratch + si, len);
           else atomicAdd_system(sg.bytes_done, len);
@@ -186,7 +214,7 @@ __global__ void __launch_bounds__(1024) put_chunks_kernel(const __grid_constant_
     // CTAs take chunks round-robin over the concatenation of all segments
     unsigned long long chunks_before = 0;
     for (int si = 0; si < a.nseg && live; ++si) {
-      const FlSeg& sg = a.seg[si];
+      const PutSeg& sg = a.seg[si];
       const unsigned long long nch = (sg.bytes + a.chunk_bytes - 1) / a.chunk_bytes;
       unsigned long long done_here = 0;      // thread 0: bytes of this segment this CTA has finished
       unsigned long long first = (blockIdx.x + gridDim.x - (chunks_before % gridDim.x)) % gridDim.x;
@@ -200,7 +228,7 @@ __global__ void __launch_bounds__(1024) put_chunks_kernel(const __grid_constant_
           __syncthreads();
           if (!okv) { live = false; break; }
         }
-        live = copy(reinterpret_cast<const uint8_t*>(sg.src) + off, reinterpret_cast<uint8_t*>(sg.dst) + off, len);
+        live = copy(sg.src + off, sg.dst + off, len);
         if (!live) break;
         if (threadIdx.x == 0 && sg.flag_mode != FL_FLAG_NONE) {
           if (sg.flag_mode == FL_FLAG_SEQ_PER_CHUNK) st_release_sys(sg.flags + c, a.seq);
@@ -356,11 +384,34 @@ extern "C" int fl_put_chunks(const FlPutArgs* args, int num_ctas, int threads, c
       set_on[dev] = true;
     }
   }
+  fl::PutLaunch k;
+  for (int i = 0; i < args->nseg; ++i) {
+    const FlSeg& from = args->seg[i];
+    k.seg[i].src = reinterpret_cast<const uint8_t*>(from.src);
+    k.seg[i].dst = reinterpret_cast<uint8_t*>(from.dst);
+    k.seg[i].bytes = from.bytes;
+    k.seg[i].flags = from.flags;
+    k.seg[i].bytes_done = from.bytes_done;
+    k.seg[i].flag_mode = from.flag_mode;
+    if (even.slots != 0) {
+      k.seg[i].slot_end = even.slot_end[i];
+      k.seg[i].first_cta = even.first_cta[i];
+      k.seg[i].first_adds = even.first_adds[i];
+    } else {
+      k.seg[i].wait_flags = from.wait_flags;
+    }
+  }
+  k.nseg = args->nseg; k.use_bulk = args->use_bulk; k.slots = slots;
+  k.chunk_bytes = args->chunk_bytes; k.seq = args->seq; k.even_slots = even.slots;
+  k.status = args->status;
+  k.nwait = args->nwait;
+  for (int i = 0; i < args->nwait && i < 8; ++i) { k.wait_flag[i] = args->wait_flag[i]; k.wait_want[i] = args->wait_want[i]; }
+  k.done_scratch = args->done_scratch;
   if (num_ctas > PUT_EARLY_CTAS || args->nseg > 1) {
-    fl::put_chunks_kernel<<<num_ctas, threads, smem, stream>>>(*args, even, slots);
+    fl::put_chunks_kernel<<<num_ctas, threads, smem, stream>>>(k);
     return (int)cudaGetLastError();
   }
-  return launch_after(fl::put_chunks_kernel, (unsigned)num_ctas, (unsigned)threads, smem, stream, *args, even, slots);
+  return launch_after(fl::put_chunks_kernel, (unsigned)num_ctas, (unsigned)threads, smem, stream, k);
 }
 
 extern "C" int fl_all_to_all(const void* send, void* const* recv_peers, unsigned long long bytes_per_peer, int rank,
