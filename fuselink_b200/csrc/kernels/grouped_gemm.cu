@@ -1189,7 +1189,8 @@ static int pairs_in_use(const FlGemmDesc* d, int fit) {
 
 // The variant for groups of `expect_rows` rows on `pairs` CTA pairs, `dflt` being the one for thousands.  Few rows per group change what
 // pays, all measured in us on 8 groups of 28672 x 4096 and 4096 x 14336 or 16 of 11264 x 2048 and 2048 x 5632 (0 | 1 | 2):
-//   weight gradients: pairs at any number of rows (with the update in place: 191 rows 527 | 370 | 541, 1024: 1991 | 1609 | 2607);
+//   weight gradients: pairs at any number of rows (with the update in place: 191 rows 527 | 370 | 541, 1024: 1991 | 1609 | 2607), but 0
+//     below 448 where they are pushed to other ranks, from registers (such an epilogue, stored here: 250 rows 704 | 758, 448: 554 | 541);
 //   SWIGLU and DSWIGLU: the wide tiles' single accumulator does not hide such short tiles (448 rows: 321 | 296 | 331; 1000: 1506 |
 //     1491 | 1515); 0 where tiles of 128 rows pad a tenth less than those of 256 (SWIGLU 250: 520 | 538 | 553, 125: 358 | 380 | 395), for DSWIGLU
 //     a sixth (264 rows each: 384 | 432, 128: 110 | 114, 250: 292 | 261);
@@ -1198,7 +1199,8 @@ static int pairs_in_use(const FlGemmDesc* d, int fit) {
 //     fewer tiles: an average is a little above the number of tiles that the groups mostly take (700 rows: 3.01).
 static int variant_for_rows(const FlGemmDesc* d, int dflt, int pairs) {
   const double rows = d->expect_rows;
-  if (d->group_mode == 1 || d->N < 512 || rows >= 1024) return dflt;
+  if (d->group_mode == 1) return d->push_world > 0 && rows < 448 ? 0 : dflt;
+  if (d->N < 512 || rows >= 1024) return dflt;
   const double t256 = expected_tiles(rows, 256);
   if (d->epilogue == FL_EPI_SWIGLU || d->epilogue == FL_EPI_DSWIGLU)
     return (d->epilogue == FL_EPI_SWIGLU ? 1.1 : 1.2) * 128 * expected_tiles(rows, 128) < 256 * t256 ? 0 : 1;

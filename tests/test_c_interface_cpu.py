@@ -54,6 +54,19 @@ def test_tiles_by_expected_rows_on_the_pairs_that_a_launch_may_use(N, K, rows, c
     assert got == variant
 
 
+@pytest.mark.parametrize("push_world,rows,variant", [(0, 191, 1), (0, 1024, 1), (2, 191, 0), (8, 447, 0), (2, 448, 1), (2, 1024, 1), (2, 0, 1)])
+def test_tiles_of_weight_gradients_that_other_ranks_receive(push_world, rows, variant, tmp_path):
+    """Pairs store a gradient of few rows faster only where it leaves through shared memory, which it does if it stays on this GPU."""
+    got, = _run(tmp_path, f"""int main() {{
+  FlGemmDesc d;
+  memset(&d, 0, sizeof d);
+  d.group_mode = 1; d.num_groups = 8; d.M = 28672; d.N = 4096; d.epilogue = FL_EPI_WGRAD; d.push_world = {push_world}; d.expect_rows = {rows};
+  printf("%d", fl_gemm_choose(&d, 74));
+}}
+""", link=True)
+    assert got == variant
+
+
 @pytest.mark.parametrize("rows,cols", [(0, 4), (1, 0), (1, 2 ** 31 - 127), (1, 2 ** 31 - 1)])
 def test_the_relu_gradient_refuses_widths_that_32_bits_do_not_count(rows, cols):
     lib = os.path.join(ROOT, "fuselink_b200", "lib", "libfuselink.so")
